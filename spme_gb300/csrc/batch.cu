@@ -869,7 +869,7 @@ int apply_body(_spme_batch_t *b, double alpha, const T *f, double beta, T *u) {
         BTRY_CUDA(cudaStreamWaitEvent(rss, b->ev_fork, 0));
     }
     BTRY_CUDA(launch_realspace_batch<T>((const RealArgs<T> *)b->d_real_sys, b->d_pre_real,
-                                        b->nsys, b->tot_real, rss));
+                                        b->nsys, b->tot_real, b->R, rss));
     if (conc) BTRY_CUDA(cudaEventRecord(b->ev_rs_join, rss));
     mark(b, 3);
     launch_gather_cols_rows<T>((const T *)b->d_F, b->d_ridx2, n, C, (T *)b->d_Fs, s);

@@ -191,24 +191,24 @@ cudaError_t launch_zfft_influence(const CUtensorMap &map, T *G, const T *tab2, c
                                   cudaStream_t s);
 
 // ---- real-space pair sum + self term (realspace.cu) -----------------------
-// cpos: float4 for T = float, double4_32a for T = double (cell-relative).
-template <typename T>
-cudaError_t launch_realspace(int nc, const int *cell_off, const int *cell_perm, const void *cpos,
-                             const T *F, int R, double L, double rc, double xi, double a,
-                             int with_self, T *W, cudaStream_t s);
-// Piecewise Chebyshev table of the real-space pair functions F(r), G(r) for FP64
-// engines (xi and a fixed per engine): degree kPairDeg on nseg1 segments of
-// [r_lo, r_mid) and nseg2 of [r_mid, r_hi]; coef (device) holds the F and G
-// coefficients interleaved per segment.  A null coef means no table.
-constexpr int kPairDeg = 10;
+// Table of the real-space pair functions for FP64 engines (xi and a fixed per
+// engine), in s = r^2: A = F and B = G / s as polynomials of degree kPairDeg in
+// the offset from the segment's centre, interleaved.  Segments split each
+// octave of s evenly (2^(20 - shift) of them), so the segment is the top bits
+// of s: segment g = high word >> shift has index g - base below mid = (2a)^2
+// and one more from mid on (the segment holding mid carries both forms).  Used
+// for lo <= s <= hi (compared as bits); a null coef means no table.
+constexpr int kPairDeg = 6;
 struct PairTable {
     const double *coef = nullptr;
-    double r_lo = 0, r_mid = 0, r_hi = 0, inv_h1 = 0, inv_h2 = 0;
-    int nseg1 = 0, nseg2 = 0;
+    long long lo_bits = 0, mid_bits = 0, hi_bits = 0;
+    int base = 0, shift = 14;
 };
 // Fits the table on the host (checked between nodes to 2e-13 relative);
-// false if no fit meets that within 4096 segments.
+// false if no fit meets that within 1024 segments per octave.
 bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef, PairTable *t);
+// cpos: float4 for T = float, double4_32a for T = double (cell-relative); FP32 in
+// realspace.cu (tab unused), FP64 in realspace_fp64.cu.
 template <typename T>
 cudaError_t launch_realspace(int nc, const int *cell_off, const int *cell_perm, const void *cpos,
                              const T *F, int R, double L, double rc, double xi, double a,
@@ -242,10 +242,26 @@ template <typename T>
 RealArgs<T> real_args(int nc, const int *cell_off, const int *cell_perm, const void *cpos,
                       const T *F, int R, double L, double rc, double xi, double a, int with_self,
                       const PairTable &tab, T *W);
-// All systems in one persistent launch over their cells (prefix as for the spread).
+// All systems (R right-hand sides each) in one persistent launch over their cells
+// (prefix as for the spread).
 template <typename T>
 cudaError_t launch_realspace_batch(const RealArgs<T> *sys, const int *prefix, int nsys,
-                                   int total, cudaStream_t s);
+                                   int total, int R, cudaStream_t s);
+
+template <>
+cudaError_t launch_realspace<float>(int, const int *, const int *, const void *, const float *,
+                                    int, double, double, double, double, int, const PairTable &,
+                                    float *, cudaStream_t);
+template <>
+cudaError_t launch_realspace<double>(int, const int *, const int *, const void *, const double *,
+                                     int, double, double, double, double, int, const PairTable &,
+                                     double *, cudaStream_t);
+template <>
+cudaError_t launch_realspace_batch<float>(const RealArgs<float> *, const int *, int, int, int,
+                                          cudaStream_t);
+template <>
+cudaError_t launch_realspace_batch<double>(const RealArgs<double> *, const int *, int, int, int,
+                                           cudaStream_t);
 
 // ---- layout conversions (pack.cu) -----------------------------------------
 // W = self_c * F (the self term alone, when no real-space sum is requested)
