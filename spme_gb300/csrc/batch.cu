@@ -506,14 +506,14 @@ int record_stride(const _spme_batch_t *b) {
 template <typename T>
 int build_tiles(_spme_batch_t *b) {
     int off = 0;
-    size_t smem = 0;
+    bool tile_ok = true;
     for (BatchSys &x : b->sys) {
         set_geo(x, b->tile);
         x.tile_off = off;
         off += x.g.ntx * x.g.nty * x.g.ntz;
-        smem = std::max(smem, interp_smem_bytes(x.g, sizeof(T)));
+        tile_ok = tile_ok && interp_tile_ok(x.g, sizeof(T));
     }
-    if (smem > 220 * 1024) return SPME_ERR_UNSUPPORTED;
+    if (!tile_ok) return SPME_ERR_UNSUPPORTED;
     cudaFree(b->d_cnt1);
     cudaFree(b->d_off1);
     b->d_cnt1 = b->d_off1 = nullptr;

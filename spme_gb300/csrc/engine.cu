@@ -1150,8 +1150,7 @@ int spme_set_tile(spme_t *e, int tx, int ty, int tz) {
     g.tx = tx;
     g.ty = ty;
     g.tz = tz;
-    if (spme::interp_smem_bytes(g, e->elem) > 220 * 1024)
-        return e->last_error = SPME_ERR_UNSUPPORTED;
+    if (!spme::interp_tile_ok(g, e->elem)) return e->last_error = SPME_ERR_UNSUPPORTED;
     e->tile[0] = tx;
     e->tile[1] = ty;
     e->tile[2] = tz;

@@ -1,5 +1,6 @@
-// Interpolation of the 3R mesh components back to the particles (restates
-// old-version/spme_kernel.c:8-70: v_i = sum_j P_ij grid[c][ind_ij]).
+// FP32 interpolation of the 3R mesh components back to the particles (restates
+// old-version/spme_kernel.c:8-70: v_i = sum_j P_ij grid[c][ind_ij]; FP64 in
+// interp_fp64.cu).
 //
 // One CTA per mesh tile.  For CG components at a time it stages the tile
 // plus its (p-1) upper halo in shared memory as a dense box
@@ -26,11 +27,10 @@ namespace spme {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kHX = 24;  // staged row width (elements)
+constexpr int kHX = kInterpMaxRow;  // staged row width (elements)
 
 template <typename T> struct Vec16;
 template <> struct Vec16<float> { using type = float4; static constexpr int n = 4; };
-template <> struct Vec16<double> { using type = double2; static constexpr int n = 2; };
 
 // A half-warp's copy of one particle record for interp_pairs: lane j of the
 // half holds weights j and 16 + j (the record's 3p weights: x, y, z), plus
@@ -345,7 +345,7 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
 
 template <typename T, int P, int CG>
 // blocks per SM that the 4-component box's shared memory allows (16x8x4 tiles)
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 5 : 2)
+__global__ void __launch_bounds__(kThreads, 5)
 k_interp(const __grid_constant__ CUtensorMap tmap, InterpArgs<T> A) {
     // tiles z fastest: blocks launched together are z neighbours, whose boxes
     // share p - 1 of their tz + p - 1 planes (read from L2 by the later ones)
@@ -417,7 +417,8 @@ bool encode_box(CUtensorMap *m, const void *mesh, int K, int C, const MeshGeom &
     const cuuint64_t dims[4] = {(cuuint64_t)K, (cuuint64_t)K, (cuuint64_t)K, (cuuint64_t)C};
     const cuuint64_t strides[3] = {(cuuint64_t)K * elem, (cuuint64_t)K * K * elem,
                                    (cuuint64_t)K * K * K * elem};
-    const cuuint32_t box[4] = {(cuuint32_t)kHX, (cuuint32_t)(g.ty + g.p - 1),
+    const int row = elem == 8 ? interp64_row(g.tx + g.p - 1) : kHX;
+    const cuuint32_t box[4] = {(cuuint32_t)row, (cuuint32_t)(g.ty + g.p - 1),
                                (cuuint32_t)(g.tz + g.p - 1), (cuuint32_t)CG};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     if (box[1] > 256 || box[2] > 256) return false;
@@ -431,15 +432,23 @@ bool encode_box(CUtensorMap *m, const void *mesh, int K, int C, const MeshGeom &
 }  // namespace
 
 size_t interp_smem_bytes(const MeshGeom &g, size_t elem) {
-    return (size_t)4 * (g.tz + g.p - 1) * (g.ty + g.p - 1) * kHX * elem + 128;
+    const size_t rows = (size_t)(g.tz + g.p - 1) * (g.ty + g.p - 1);
+    // FP64: the box and one row sum per thread
+    if (elem == 8)
+        return (rows * interp64_row(g.tx + g.p - 1) + kInterp64Threads) * elem + 128;
+    return 4 * rows * kHX * elem + 128;
+}
+
+bool interp_tile_ok(const MeshGeom &g, size_t elem) {
+    return (size_t)4 * (g.tz + g.p - 1) * (g.ty + g.p - 1) * kHX * elem + 128 <= 220 * 1024;
 }
 
 bool make_interp_box(CUtensorMap *map, const void *mesh, int C, const MeshGeom &g, size_t elem) {
-    return encode_box(map, mesh, g.K, C, g, elem, 4);
+    return encode_box(map, mesh, g.K, C, g, elem, elem == 8 ? 1 : 4);
 }
 
 bool make_interp_maps(InterpMaps *maps, const void *mesh, int C, const MeshGeom &g, size_t elem) {
-    maps->ok4 = encode_box(&maps->cg4, mesh, g.K, C, g, elem, 4);
+    maps->ok4 = encode_box(&maps->cg4, mesh, g.K, C, g, elem, elem == 8 ? 1 : 4);
     return maps->ok4;
 }
 
@@ -478,15 +487,9 @@ cudaError_t launch_interp_batch(const InterpSys<T> *sys, const int *prefix, int 
 
 template cudaError_t launch_interp_batch<float>(const InterpSys<float> *, const int *, int, int,
                                                 size_t, cudaStream_t, size_t);
-template cudaError_t launch_interp_batch<double>(const InterpSys<double> *, const int *, int, int,
-                                                 size_t, cudaStream_t, size_t);
 template cudaError_t launch_interp<float>(const InterpMaps &, const int *, int, const int *,
                                           const uint32_t *, const float *, const float *, int,
                                           int, int, const MeshGeom &, float *, int, int *,
                                           cudaStream_t);
-template cudaError_t launch_interp<double>(const InterpMaps &, const int *, int, const int *,
-                                           const uint32_t *, const double *, const double *, int,
-                                           int, int, const MeshGeom &, double *, int, int *,
-                                           cudaStream_t);
 
 }  // namespace spme

@@ -92,15 +92,41 @@ cudaError_t launch_spread_cols_batch(const SpreadColsSys<T> *sys, const int *pre
 template <typename T>
 cudaError_t launch_spread_cols(const int *start_off, const uint32_t *rec_start, const T *rec_w,
                                const T *Fs, int C, const MeshGeom &g, T *mesh, cudaStream_t s);
+// Spread through per-tile boxes (spread_box.cu), for few components: records in
+// tile order, any K; boxes: scratch of nslot * spread_box_bytes (nslot
+// components per launch).  Usable when spread_box_ok(g, elem).
+// bt: make_box_table's offsets on the device (3 K entries of four) and the most
+// tiles that cover a coordinate of each axis; false if one has over four.
+struct BoxTable {
+    const int4 *tab = nullptr;
+    int most[3] = {0, 0, 0};
+};
+bool spread_box_ok(const MeshGeom &g, size_t elem);
+size_t spread_box_bytes(const MeshGeom &g, size_t elem);
+bool make_box_table(const MeshGeom &g, std::vector<int> *tab, int (*most)[3]);
+template <typename T>
+cudaError_t launch_spread_box(const int *tile_off, const int *rec_idx, const uint32_t *rec_start,
+                              const T *rec_w, const T *F, int C, const MeshGeom &g, T *boxes,
+                              int nslot, const BoxTable &bt, T *mesh, cudaStream_t s);
 // TMA descriptor of the real mesh [C][K][K][K] for the interpolation halo
-// boxes (4 components per box: more blocks per SM than 8, measured faster).
+// boxes: FP32 (interp.cu) 4 components of rows of kInterpMaxRow points (more
+// blocks per SM than 8 components, measured faster), FP64 (interp_fp64.cu) one
+// component of rows of interp64_row(tx + p - 1) points.
+constexpr int kInterpMaxRow = 24;
+constexpr int kInterp64Threads = 128;
+// Row length of an FP64 box: the least r >= n that is 2 (mod 4) (bank spread of
+// neighbouring rows; whole 16-byte vectors).
+__host__ __device__ constexpr int interp64_row(int n) { return n + (6 - n % 4) % 4; }
 struct InterpMaps {
     CUtensorMap cg4;
     bool ok4 = false;
 };
 bool make_interp_maps(InterpMaps *maps, const void *mesh, int C, const MeshGeom &g, size_t elem);
-// Shared memory the interpolation kernel needs (4-component boxes).
+// Dynamic shared memory of the interpolation kernel.
 size_t interp_smem_bytes(const MeshGeom &g, size_t elem);
+// Tile shapes the engines accept: four components of the tile and its halo, rows
+// of kInterpMaxRow points, within 220 KB.
+bool interp_tile_ok(const MeshGeom &g, size_t elem);
 // Arguments of one system's interpolation (records indexed by sorted slot,
 // stride ws; tile_off indexed by this system's tiles; W rows by particle).
 template <typename T>
@@ -116,14 +142,14 @@ struct InterpArgs {
     int C, cb, ce, accumulate, use_tma, ws;
 };
 // One system of a batched interpolation: its arguments and, when args.use_tma
-// is set, its 4-component TMA box over its own mesh (make_interp_box; read by
-// the kernel from this global work list, 64-byte aligned).
+// is set, its TMA box over its own mesh (make_interp_box; read by the kernel
+// from this global work list, 64-byte aligned).
 template <typename T>
 struct InterpSys {
     CUtensorMap tmap;
     InterpArgs<T> args;
 };
-// The 4-component TMA box of one mesh (false where TMA does not apply: K * elem
+// The TMA box of one mesh (false where TMA does not apply: K * elem
 // not a multiple of 16 bytes, an unaligned mesh, or no driver entry point).
 bool make_interp_box(CUtensorMap *map, const void *mesh, int C, const MeshGeom &g, size_t elem);
 // All systems in one persistent launch over their tiles (prefix as for the
@@ -132,13 +158,20 @@ bool make_interp_box(CUtensorMap *map, const void *mesh, int C, const MeshGeom &
 template <typename T>
 cudaError_t launch_interp_batch(const InterpSys<T> *sys, const int *prefix, int nsys, int total,
                                 size_t smem, cudaStream_t s, size_t smem_limit = 0);
-// Components [cb, ce) of the C-component mesh (cb a multiple of 4) into
+// Components [cb, ce) of the C-component mesh (cb a multiple of 12, or 0) into
 // W[n][C]; err: device flag set to 1 if a TMA wait timed out.
 template <typename T>
 cudaError_t launch_interp(const InterpMaps &maps, const int *tile_off, int n, const int *rec_idx,
                           const uint32_t *rec_start, const T *rec_w, const T *mesh, int C,
                           int cb, int ce, const MeshGeom &g, T *W, int accumulate, int *err,
                           cudaStream_t s);
+template <>
+cudaError_t launch_interp<double>(const InterpMaps &, const int *, int, const int *,
+                                  const uint32_t *, const double *, const double *, int, int, int,
+                                  const MeshGeom &, double *, int, int *, cudaStream_t);
+template <>
+cudaError_t launch_interp_batch<double>(const InterpSys<double> *, const int *, int, int, size_t,
+                                        cudaStream_t, size_t);
 
 // ---- host tables (engine.cu) ----------------------------------------------
 // |b(m)|^2 = 1 / |sum_{j<p-1} M_p(j+1) e^{i j 2 pi m'/K}|^2 (old-version/spme.c:109-126).
