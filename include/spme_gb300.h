@@ -123,12 +123,15 @@ long spme_launch_count(const spme_t *spme);
  * and the concurrent sum only slows them down). */
 int spme_set_overlap(spme_t *spme, int on);
 
-/* Spread kernel.  1 (default): column gather where it applies (K >= 32; in
- * FP32 from 9 components on, below that the tile kernel is faster), each mesh
- * column visits only the particles whose stencil covers it, force components
- * across the lanes of a warp.  0: tile kernel always, threads own the columns
- * of a mesh tile and visit every particle staged for the tile.  Mode 1 on an
- * engine without the column-gather buffers returns SPME_ERR_UNSUPPORTED. */
+/* Spread kernel.  1 (default): for few components (most FP64 engines of up to
+ * 3 right-hand sides, FP32 ones of 1 or 2 at K >= 96) per-tile boxes, one
+ * particle's stencil points across the lanes of a warp; else the column gather
+ * where it applies (FP32 from 9 components on), each mesh column visits only
+ * the particles whose stencil covers it; else the tile kernel.  0: tile kernel
+ * always, threads own the columns of a mesh tile and visit every particle
+ * staged for the tile.  Mode 1 on an engine whose mesh is too small for the
+ * column gather (K < p + 15 in FP32, p + 7 in FP64) returns
+ * SPME_ERR_UNSUPPORTED (its default kernel stays). */
 int spme_set_spread_mode(spme_t *spme, int mode);
 
 /* Transform strategy of the mesh pass.  1: cuFFT 2D (y, x) transforms of

@@ -371,7 +371,7 @@ class Engine:
         _check(load().spme_set_overlap(self.h, 1 if on else 0), "spme_set_overlap")
 
     def set_spread_mode(self, mode: int):
-        """1: column-gather spread (default where it applies); 0: tile spread."""
+        """1: box or column-gather spread (default where they apply); 0: tile spread."""
         _check(load().spme_set_spread_mode(self.h, int(mode)), "spme_set_spread_mode")
 
     def set_fft_mode(self, mode: int):

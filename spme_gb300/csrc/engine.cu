@@ -137,7 +137,17 @@ struct _spme_t {
     void *d_rec_w = nullptr;
     // column-gather spread: records sorted by stencil-start cell (K^3 keys)
     bool cols = false;
-    int spread_mode = 1;  // 1: column-gather kernel where it applies, 0: tile kernel
+    bool cols_fit = false;  // the mesh admits it (spread mode 1 is accepted)
+    // box spread (few components): scratch for box_slots components' boxes of the
+    // current tile (0 slots: not used)
+    bool box = false;
+    void *d_box = nullptr;
+    size_t box_cap = 0;
+    int box_slots = 0;
+    int *d_boxtab = nullptr;  // coverage offsets of the current tile (3 K entries of 4)
+    spme::BoxTable boxtab;
+    int boxtab_tile[3] = {0, 0, 0};
+    int spread_mode = 1;  // 1: box or column-gather kernel where they apply, 0: tile kernel
     int *d_scount = nullptr, *d_soff = nullptr, *d_sperm = nullptr, *d_srec_idx = nullptr;
     uint32_t *d_srec_start = nullptr;
     void *d_srec_w = nullptr;
@@ -270,7 +280,65 @@ int record_width(const spme_t *e) {
     return (raw + per16 - 1) / per16 * per16;
 }
 
+// Whether an engine of C components spreads through boxes (spread_box.cu; its
+// default 8x8x8 tile).  The box kernel's cost grows with C, the column gather's is
+// per visit up to 16 components and needs its own sort.  Spread + position build
+// measured on GB300, box vs the other kernel (ms):
+// FP64 (vs column gather), p = 6: N = 1e5, K = 128: C = 3 0.42 vs 1.16, C = 9
+// 0.93 vs 1.17, C = 15 1.55 vs 1.17; N = 2000, K = 64: C = 9 0.142 vs 0.163;
+// p = 4: C = 6 0.43 vs 0.50, C = 9 0.59 vs 0.50; p = 8: C = 9 1.56 vs 2.42, but
+// 0.92 vs 0.86 at K = 90, where tiles that do not divide K make the sum slower.
+// FP32 (vs the tile kernel, spread alone): p = 6: C = 3 0.119 vs 0.145, C = 6
+// 0.214 vs 0.197; p = 4: C = 6 0.145 vs 0.170; p = 8: C = 3 0.176 vs 0.166; K = 64:
+// 0.019 vs 0.016 (one more launch).
+bool box_pays(size_t elem, int p, int C, int K) {
+    if (elem == 8) return C <= (p == 4 || K % 8 != 0 ? 6 : 9);
+    return K >= 96 && ((p == 4 && C <= 6) || (p == 6 && C <= 3));
+}
+// Scratch bounds: boxes of as many components at a time as fit in kBoxScratch,
+// and no box spread where one component's boxes exceed kBoxMax (then the
+// column-gather or the tile kernel runs).
+constexpr size_t kBoxScratch = (size_t)1 << 30, kBoxMax = (size_t)4 << 30;
+
+// Scratch and coverage table for the current tile; without them (too large, or no
+// memory) the box spread is off.
+void alloc_box(spme_t *e) {
+    if (!e->box || (e->boxtab.tab && e->boxtab_tile[0] == e->g.tx &&
+                    e->boxtab_tile[1] == e->g.ty && e->boxtab_tile[2] == e->g.tz))
+        return;
+    const size_t one = spme::spread_box_bytes(e->g, e->elem);
+    e->box_slots = 0;
+    e->boxtab = spme::BoxTable{};
+    if (one > kBoxMax || !spme::spread_box_ok(e->g, e->elem)) return;
+    const int slots = (int)std::max<size_t>(1, std::min<size_t>(e->Cmax, kBoxScratch / one));
+    if (one * slots > e->box_cap) {
+        dfree(e->d_box);
+        e->d_box = nullptr;
+        e->box_cap = 0;
+        if (dalloc(&e->d_box, one * slots) != SPME_OK) return;
+        e->box_cap = one * slots;
+    }
+    std::vector<int> tab;
+    spme::BoxTable bt;
+    if (!spme::make_box_table(e->g, &tab, &bt.most)) return;
+    if (!e->d_boxtab && dalloc(&e->d_boxtab, sizeof(int) * tab.size()) != SPME_OK) return;
+    // (the previous tile's table may still be read by work on the stream)
+    if (cudaStreamSynchronize(e->stream) != cudaSuccess ||
+        cudaMemcpy(e->d_boxtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice) !=
+            cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    bt.tab = reinterpret_cast<const int4 *>(e->d_boxtab);
+    e->boxtab = bt;
+    e->boxtab_tile[0] = e->g.tx;
+    e->boxtab_tile[1] = e->g.ty;
+    e->boxtab_tile[2] = e->g.tz;
+    e->box_slots = slots;
+}
+
 int alloc_tiles(spme_t *e) {
+    alloc_box(e);
     size_t need = (size_t)e->ntiles;
     if (need <= e->cap_tiles && e->d_tcount) return SPME_OK;
     dfree(e->d_tcount);
@@ -483,7 +551,12 @@ int create_impl(const spme_params &prm, spme_t **out) {
         TRY(dalloc(&e->d_pstart, sizeof(uint32_t) * n));
         TRY(dalloc(&e->d_pfrac, e->elem * 3 * n));
     }
-    e->cols = (prm.terms & SPME_TERM_RECIP) && spme::spread_cols_ok((int)K, (int)C, e->elem, prm.porder);
+    e->cols_fit = (prm.terms & SPME_TERM_RECIP) && spme::spread_cols_ok((int)K, (int)C, e->elem, prm.porder);
+    e->box = (prm.terms & SPME_TERM_RECIP) && box_pays(e->elem, prm.porder, (int)C, (int)K);
+    alloc_box(e);
+    e->box = e->box_slots > 0;
+    // (FP32 passes of fewer than 9 components never take the column gather)
+    e->cols = e->cols_fit && !e->box && (e->elem == 8 || C >= 9);
     if (e->cols) {
         const size_t K3 = K * K * K;
         TRY(dalloc(&e->d_scount, sizeof(int) * K3));
@@ -657,7 +730,8 @@ void destroy_impl(spme_t *e) {
                     e->d_W,      e->d_fstage,  e->d_ustage, e->d_err,  e->d_ztw,
                     e->d_zip,    e->d_f2tab,    e->d_scount,  e->d_soff,   e->d_sperm, e->d_srec_idx,
                     e->d_srec_start, e->d_srec_w, e->d_Fs, e->d_W2, e->d_pair, e->d_key2,
-                    e->d_key3,   e->d_pstart, e->d_pfrac};
+                    e->d_key3,   e->d_pstart, e->d_pfrac, e->d_box,
+                    e->d_boxtab};
     for (void *b : bufs) dfree(b);
     for (int i = 0; i <= kStages; i++)
         if (e->ev[i]) cudaEventDestroy(e->ev[i]);
@@ -814,7 +888,12 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
                               spme::spread_cols_ok(K, C, e->elem, e->g.p) &&
                               (e->elem == 8 || C >= 9) &&
                               (long long)n * spme::spread_cols_row_width(C) < (1LL << 31);
-        if (use_cols) {
+        if (e->box_slots > 0 && e->spread_mode == 1) {
+            TRY_CUDA(spme::launch_spread_box<T>(e->d_toff, e->d_rec_idx, e->d_rec_start,
+                                                (const T *)e->d_rec_w, F, C, e->g, (T *)e->d_box,
+                                                e->box_slots, e->boxtab, (T *)e->d_mesh, s));
+            e->launches += 2 * ((C + e->box_slots - 1) / e->box_slots) - 1;
+        } else if (use_cols) {
             spme::launch_gather_cols_rows<T>(F, e->d_srec_idx, n, C, (T *)e->d_Fs, s);
             TRY_CUDA(spme::launch_spread_cols<T>(e->d_soff, e->d_srec_start,
                                                  (const T *)e->d_srec_w, (const T *)e->d_Fs, C,
@@ -1171,7 +1250,7 @@ int spme_set_overlap(spme_t *e, int on) {
 int spme_set_spread_mode(spme_t *e, int mode) {
     if (!e || (mode != 0 && mode != 1)) return SPME_ERR_INVALID;
     DeviceGuard dg(e->device);
-    if (mode == 1 && !e->cols) return e->last_error = SPME_ERR_UNSUPPORTED;
+    if (mode == 1 && !e->cols_fit) return e->last_error = SPME_ERR_UNSUPPORTED;
     if (e->stream) cudaStreamSynchronize(e->stream);
     drop_graphs(e);
     e->spread_mode = mode;
