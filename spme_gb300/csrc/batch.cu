@@ -600,6 +600,12 @@ int create_t(_spme_batch_t *b) {
     for (auto &kv : byK) {
         FftGroup grp;
         grp.K = kv.first;
+        // a group starts on a 256-byte boundary: with an odd number of right-hand sides
+        // the meshes of an odd K before it hold an odd number of values, and cuFFT's real
+        // data and the spread's stores of column pairs need 8-byte (FP64: 16-byte)
+        // alignment (inside a group of even K every mesh keeps it)
+        mesh = (mesh + 63) / 64 * 64;
+        spec = (spec + 63) / 64 * 64;
         grp.mesh_off = mesh;
         grp.spec_off = spec;
         grp.nsys = (int)kv.second.size();
