@@ -126,8 +126,9 @@ int spme_set_overlap(spme_t *spme, int on);
 /* Spread kernel.  1 (default): for few components (most FP64 engines of up to
  * 3 right-hand sides, FP32 ones of 1 or 2 at K >= 96) per-tile boxes, one
  * particle's stencil points across the lanes of a warp; else the column gather
- * where it applies (FP32 from 9 components on), each mesh column visits only
- * the particles whose stencil covers it; else the tile kernel.  0: tile kernel
+ * where it applies (FP32 from 9 components on, mostly in its z-marching form),
+ * each mesh column visits only the particles whose stencil covers it; else the
+ * tile kernel.  0: tile kernel
  * always, threads own the columns of a mesh tile and visit every particle
  * staged for the tile.  Mode 1 on an engine whose mesh is too small for the
  * column gather (K < p + 15 in FP32, p + 7 in FP64) returns

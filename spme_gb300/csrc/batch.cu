@@ -728,16 +728,19 @@ int create_t(_spme_batch_t *b) {
     std::vector<InflSys> fs(ns);
     std::vector<int> ps(ns + 1, 0), pr(ns + 1, 0), pf(ns + 1, 0);
     const int RW = spread_cols_row_width(C);
+    long columns = 0;
+    for (const BatchSys &x : b->sys) columns += spread_cols_grid(x.s.dim, C, sizeof(T), 0).columns;
     for (int k = 0; k < ns; k++) {
         const BatchSys &x = b->sys[k];
         const int K = x.s.dim;
-        const int TZ = sizeof(T) == 4 ? 16 : 8;
+        const SpreadColsGrid sg = spread_cols_grid(K, C, sizeof(T), columns);
         ss[k].args = SpreadColsArgs<T>{b->d_off2 + x.start_off, b->d_rst2, (const T *)b->d_rw2,
                                        (const T *)b->d_Fs, (T *)b->d_mesh + x.mesh_off, C, RW, K,
-                                       (K + TZ - 1) / TZ, b->ws};
+                                       sg.nzt, sg.zseg, b->ws};
         ss[k].p = x.s.porder;
-        ss[k].gx = (K + 15) / 16;
-        ps[k + 1] = ps[k] + spread_cols_blocks(K, C, sizeof(T));
+        ss[k].gx = sg.x;
+        ss[k].gy = sg.y;
+        ps[k + 1] = ps[k] + sg.blocks;
         rs[k] = real_args<T>(x.nc, b->d_off3 + x.cell_off, b->d_perm3, b->d_cpos, (const T *)b->d_F,
                              b->R, x.s.box_size, x.s.rcut, x.s.xi, x.s.radius, 1, ptab[k],
                              (T *)b->d_W);

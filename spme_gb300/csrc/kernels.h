@@ -74,21 +74,40 @@ struct SpreadColsArgs {
     const T *rec_w;
     const T *Fs;
     T *mesh;
-    int C, RW, K, nzt, ws;
+    int C, RW, K, nzt, zseg, ws;  // nzt z tiles or segments of zseg planes
 };
-// A system of a batched launch: its arguments, order and blocks along x.
+// A system of a batched launch: its arguments, order and blocks along x and y.
 template <typename T>
 struct SpreadColsSys {
     SpreadColsArgs<T> args;
-    int p, gx;
+    int p, gx, gy;
 };
-// Blocks of one system's column-gather spread (all component chunks).
-int spread_cols_blocks(int K, int C, size_t elem);
+// Blocks of one system's column-gather spread: along x and y, z tiles or segments
+// (and their planes), in all (with component chunks), and without z segments;
+// columns: the last summed over the systems of a launch (0: this system alone).
+struct SpreadColsGrid {
+    int x, y, nzt, zseg, blocks;
+    long columns;
+};
+SpreadColsGrid spread_cols_grid(int K, int C, size_t elem, long columns);
+// The z-marching form of the FP32 column gather (spread_march.cu; chosen by
+// launch_spread_cols and its batched form): same records, rows and offsets.
+// launch_spread_march sets A.nzt and A.zseg.  FP32 batches always take it.
+SpreadColsGrid spread_march_grid(int K, int C, long columns);
+cudaError_t launch_spread_march(SpreadColsArgs<float> A, int p, cudaStream_t s);
+cudaError_t launch_spread_march_batch(const SpreadColsSys<float> *sys, const int *prefix, int nsys,
+                                      int total, int C, cudaStream_t s);
 // All systems (same C) in one persistent launch; prefix[k] = the first block
 // of system k (nsys + 1 entries, prefix[nsys] = total), both on the device.
 template <typename T>
 cudaError_t launch_spread_cols_batch(const SpreadColsSys<T> *sys, const int *prefix, int nsys,
                                      int total, int C, cudaStream_t s);
+template <>
+cudaError_t launch_spread_cols_batch<float>(const SpreadColsSys<float> *, const int *, int, int,
+                                            int, cudaStream_t);
+template <>
+cudaError_t launch_spread_cols_batch<double>(const SpreadColsSys<double> *, const int *, int, int,
+                                             int, cudaStream_t);
 template <typename T>
 cudaError_t launch_spread_cols(const int *start_off, const uint32_t *rec_start, const T *rec_w,
                                const T *Fs, int C, const MeshGeom &g, T *mesh, cudaStream_t s);

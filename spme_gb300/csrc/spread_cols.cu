@@ -1,5 +1,7 @@
 // Spread of 3R force components onto the K^3 mesh, column-gather form
-// (restates old-version/spme_kernel.c:231-312: grid[c][ind] += P * f_c).
+// (restates old-version/spme_kernel.c:231-312: grid[c][ind] += P * f_c): FP64
+// engines of many components, FP32 ones of over 16 components on small meshes
+// (the others: spread_box.cu, spread_march.cu).
 //
 // Every mesh point receives ~p^3 rho contributions (rho particles per mesh
 // cell), so the useful work per point is small and any scheme that lets a
@@ -35,72 +37,15 @@
 #include <utility>
 
 #include "kernels.h"
+#include "spread_cols.cuh"
 
 namespace spme {
 
 namespace {
 
-// fn(std::integral_constant<int, i>) for i = 0 .. N-1, unrolled at compile time.
-template <typename Fn, int... Is>
-__device__ __forceinline__ void static_for_impl(Fn &&fn, std::integer_sequence<int, Is...>) {
-    (fn(std::integral_constant<int, Is>{}), ...);
-}
-template <int N, typename Fn>
-__device__ __forceinline__ void static_for(Fn &&fn) {
-    static_for_impl(fn, std::make_integer_sequence<int, N>{});
-}
-
-// Asynchronous global -> shared copies (cp.async, completion tracked per thread).
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
-                 : "memory");
-}
-template <int B>
-__device__ __forceinline__ void cp_async_small(void *dst, const void *src) {
-    static_assert(B == 4 || B == 8, "4 or 8 bytes");
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src),
-                 "n"(B)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
 template <typename T> struct V16;
 template <> struct V16<float> { using type = float4; };
 template <> struct V16<double> { using type = double2; };
-
-// Components per lane for C components (chunks of 16 CPL components per block).
-__host__ __device__ constexpr int cols_cpl(int C) { return C <= 16 ? 1 : (C <= 32 ? 2 : 3); }
-// Padded components per lane in the gathered force rows.
-__host__ __device__ constexpr int cols_pcpl(int cpl) { return cpl == 3 ? 4 : cpl; }
-
-// n values from a 16-byte aligned address, global or shared (vector loads
-// where they fit).
-template <typename T, int NV>
-__device__ __forceinline__ void load_vec(const T *__restrict__ src, T (&w)[NV]) {
-    constexpr int VW = 16 / (int)sizeof(T);
-    constexpr int NQ = NV / VW;
-    using V = typename V16<T>::type;
-#pragma unroll
-    for (int v = 0; v < NQ; v++) {
-        const V q = reinterpret_cast<const V *>(src)[v];
-        if constexpr (VW == 4) {
-            w[4 * v] = q.x;
-            w[4 * v + 1] = q.y;
-            w[4 * v + 2] = q.z;
-            w[4 * v + 3] = q.w;
-        } else {
-            w[2 * v] = q.x;
-            w[2 * v + 1] = q.y;
-        }
-    }
-#pragma unroll
-    for (int j = NQ * VW; j < NV; j++) w[j] = src[j];
-}
 
 // Staged weight row length: FP32 rows hold p + 2 values (the first plane of an
 // odd offset shifted by one, so pairs of planes line up), FP64 rows p; both
@@ -311,7 +256,7 @@ __device__ __forceinline__ void spread_cols_body(const SpreadColsArgs<T> &A, int
                 const T w0 = ox < P ? wy * __ldg(rw + ox) : T(0);
                 const T w1 = (ox1 < P && xa + 1 < K) ? wy * __ldg(rw + ox1) : T(0);
                 T wz[P];
-                load_vec<T, P>(rw + 2 * P, wz);
+                load_vec<P>(rw + 2 * P, wz);
                 // weight rows of both columns (16-byte stores; scalar stores at this
                 // lane stride conflict 16-way)
                 constexpr int VW = 16 / (int)sizeof(T);
@@ -366,7 +311,7 @@ __device__ __forceinline__ void spread_cols_body(const SpreadColsArgs<T> &A, int
             auto visit_force = [&](int j, T (&f)[CPL]) {
                 if constexpr (CPL > 1) {
                     T fv[PC];
-                    load_vec<T, PC>(fst + j * LR + l16 * PC, fv);
+                    load_vec<PC>(fst + j * LR + l16 * PC, fv);
 #pragma unroll
                     for (int c = 0; c < CPL; c++) f[c] = fv[c];
                 } else {
@@ -387,7 +332,7 @@ __device__ __forceinline__ void spread_cols_body(const SpreadColsArgs<T> &A, int
                         T f[CPL];
                         visit_force(j, f);
                         T wt[WR];
-                        load_vec<T, WR>(&ws.wt[j][half][0], wt);
+                        load_vec<WR>(&ws.wt[j][half][0], wt);
                         add_pair_run<P, CPL, TZ, M0, WR>(acc, wt, f);
                     }
                 });
@@ -399,7 +344,7 @@ __device__ __forceinline__ void spread_cols_body(const SpreadColsArgs<T> &A, int
                         T f[CPL];
                         visit_force(j, f);
                         T wt[WR];
-                        load_vec<T, WR>(&ws.wt[j][half][0], wt);
+                        load_vec<WR>(&ws.wt[j][half][0], wt);
                         add_planes<P, CPL, TZ, D, WR>(acc, wt, f);
                     }
                 });
@@ -463,7 +408,7 @@ k_spread_cols(SpreadColsArgs<T> A) {
     spread_cols_body<T, P, CPL, TZ, NW>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// Many systems in one persistent launch: work item w (a block of one system)
+// Many FP64 systems in one persistent launch: work item w (a block of one system)
 // -> system k with prefix[k] <= w < prefix[k + 1]; the order p of each system
 // selects the body.
 template <typename T, int CPL, int TZ, int NW>
@@ -475,7 +420,7 @@ k_spread_cols_batch(const SpreadColsSys<T> *__restrict__ sys, const int *__restr
         const SpreadColsSys<T> S = sys[k];
         const int local = w - prefix[k];
         const int bx = local % S.gx, rest = local / S.gx;
-        const int by = rest % S.args.K, bz = rest / S.args.K;
+        const int by = rest % S.gy, bz = rest / S.gy;
         switch (S.p) {
             case 4: spread_cols_body<T, 4, CPL, TZ, NW>(S.args, bx, by, bz); break;
             case 6: spread_cols_body<T, 6, CPL, TZ, NW>(S.args, bx, by, bz); break;
@@ -552,7 +497,7 @@ cudaError_t launch_cols(const int *soff, const uint32_t *rec_start, const T *rec
     if (e != cudaSuccess) return e;
     dim3 grid((K + XT - 1) / XT, K, nzt * nchunk);
     SpreadColsArgs<T> A{soff, rec_start, rec_w, Fs, mesh, C, spread_cols_row_width(C), K, nzt,
-                        RecordWidth<T, P>::value};
+                        TZ, RecordWidth<T, P>::value};
     kern<<<grid, NW * 32, smem, s>>>(A);
     return cudaGetLastError();
 }
@@ -583,11 +528,23 @@ cudaError_t dispatch_cpl(const int *soff, const uint32_t *rec_start, const T *re
                          int C, const MeshGeom &g, T *mesh, cudaStream_t s) {
     // components per lane: the smallest CPL with 16 CPL >= C, at most 3
     switch (cols_cpl(C)) {
-        case 1: return launch_cols<T, P, 1>(soff, rec_start, rec_w, Fs, C, g, mesh, s);
+        case 1:
+            if constexpr (sizeof(T) == 8)
+                return launch_cols<T, P, 1>(soff, rec_start, rec_w, Fs, C, g, mesh, s);
+            return cudaErrorInvalidValue;  // FP32: spread_march
         case 2: return launch_cols<T, P, 2>(soff, rec_start, rec_w, Fs, C, g, mesh, s);
         default: return launch_cols<T, P, 3>(soff, rec_start, rec_w, Fs, C, g, mesh, s);
     }
 }
+
+// FP32: the z-marching kernel (spread_march.cu) instead of this one.  With up to 16
+// components it is faster at every size (N = 2000, K = 64, R = 4: 0.021 vs 0.023
+// ms; 2e4, 75: 0.039 vs 0.055; 1e5, 128: 0.129 vs 0.215); with more, small meshes
+// have too few columns for its long blocks (R = 16, K = 64: 0.039 vs 0.031 ms;
+// K = 128: 0.285 vs 0.315; R = 8, K = 75: 0.060 vs 0.058; K = 128: 0.211 vs 0.227).
+// A batch's systems fill the GPU together: it always takes that kernel (64 uneven
+// systems, R = 4 / 8 / 16: 1.02 / 1.69 / 2.24 vs 1.90 / 2.14 / 3.24 ms).
+bool march_pays(int K, int C) { return C <= 16 || K >= 100; }
 
 int blocks_for_rows(size_t total) {
     const size_t b = (total + 255) / 256;
@@ -640,6 +597,16 @@ template <typename T>
 cudaError_t launch_spread_cols(const int *start_off, const uint32_t *rec_start, const T *rec_w,
                                const T *Fs, int C, const MeshGeom &g, T *mesh, cudaStream_t s) {
     if (!spread_cols_ok(g.K, C, sizeof(T), g.p)) return cudaErrorInvalidValue;
+    if constexpr (sizeof(T) == 4)
+        if (march_pays(g.K, C)) {
+            const int ws = g.p == 4   ? RecordWidth<float, 4>::value
+                           : g.p == 6 ? RecordWidth<float, 6>::value
+                                      : RecordWidth<float, 8>::value;
+            return launch_spread_march(SpreadColsArgs<float>{start_off, rec_start, rec_w, Fs, mesh,
+                                                             C, spread_cols_row_width(C), g.K, 0,
+                                                             0, ws},
+                                       g.p, s);
+        }
     switch (g.p) {
         case 4: return dispatch_cpl<T, 4>(start_off, rec_start, rec_w, Fs, C, g, mesh, s);
         case 6: return dispatch_cpl<T, 6>(start_off, rec_start, rec_w, Fs, C, g, mesh, s);
@@ -648,26 +615,36 @@ cudaError_t launch_spread_cols(const int *start_off, const uint32_t *rec_start, 
     }
 }
 
-template <typename T>
-cudaError_t launch_spread_cols_batch(const SpreadColsSys<T> *sys, const int *prefix, int nsys,
-                                     int total, int C, cudaStream_t s) {
+template <>
+cudaError_t launch_spread_cols_batch<float>(const SpreadColsSys<float> *sys, const int *prefix,
+                                            int nsys, int total, int C, cudaStream_t s) {
+    return launch_spread_march_batch(sys, prefix, nsys, total, C, s);
+}
+
+template <>
+cudaError_t launch_spread_cols_batch<double>(const SpreadColsSys<double> *sys, const int *prefix,
+                                             int nsys, int total, int C, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     switch (cols_cpl(C)) {
-        case 1: return launch_cols_batch<T, 1>(sys, prefix, nsys, total, s);
-        case 2: return launch_cols_batch<T, 2>(sys, prefix, nsys, total, s);
-        default: return launch_cols_batch<T, 3>(sys, prefix, nsys, total, s);
+        case 1: return launch_cols_batch<double, 1>(sys, prefix, nsys, total, s);
+        case 2: return launch_cols_batch<double, 2>(sys, prefix, nsys, total, s);
+        default: return launch_cols_batch<double, 3>(sys, prefix, nsys, total, s);
     }
 }
 
-int spread_cols_blocks(int K, int C, size_t elem) {
-    const int TZ = elem == 4 ? 16 : 8, XT = 16, CC = 16 * cols_cpl(C);
-    return ((K + XT - 1) / XT) * K * ((K + TZ - 1) / TZ) * ((C + CC - 1) / CC);
+SpreadColsGrid spread_cols_grid(int K, int C, size_t elem, long columns) {
+    if (elem == 4) return spread_march_grid(K, C, columns);
+    const int TZ = 8, CC = 16 * cols_cpl(C);
+    SpreadColsGrid g;
+    g.x = (K + 15) / 16;
+    g.y = K;
+    g.zseg = TZ;
+    g.nzt = (K + TZ - 1) / TZ;
+    g.blocks = g.x * g.y * g.nzt * ((C + CC - 1) / CC);
+    g.columns = g.blocks;
+    return g;
 }
 
-template cudaError_t launch_spread_cols_batch<float>(const SpreadColsSys<float> *, const int *,
-                                                     int, int, int, cudaStream_t);
-template cudaError_t launch_spread_cols_batch<double>(const SpreadColsSys<double> *, const int *,
-                                                      int, int, int, cudaStream_t);
 template void launch_gather_cols_rows<float>(const float *, const int *, int, int, float *,
                                              cudaStream_t);
 template void launch_gather_cols_rows<double>(const double *, const int *, int, int, double *,
