@@ -144,7 +144,7 @@ k_batch_records(const uint32_t *__restrict__ pstart, const T *__restrict__ pfrac
 // packed side where R is a multiple of 4 (FP32), scalars otherwise.
 template <typename T>
 __global__ void k_batch_pack(const T *__restrict__ f, const int *__restrict__ pref, int nsys,
-                             int R, int ntot, T *__restrict__ F) {
+                             int R, int ntot, T *__restrict__ F, T *__restrict__ F2) {
     const int C = 3 * R;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         const int k = batch_find(pref, nsys, i);
@@ -175,6 +175,29 @@ __global__ void k_batch_pack(const T *__restrict__ f, const int *__restrict__ pr
             dst[3 * r] = __ldg(s);
             dst[3 * r + 1] = __ldg(s + 1);
             dst[3 * r + 2] = __ldg(s + 2);
+        }
+        if (F2) {  // the real-space sum's rows (their padding zero)
+            T *d2 = F2 + (size_t)i * real_row(R);
+            if constexpr (sizeof(T) == 4) {
+                if (R > kRealFew && (R & 3) == 0) {
+                    for (int q = 0; q < R; q += 4)
+#pragma unroll
+                        for (int d = 0; d < 3; d++) {
+                            const T *s = src + (size_t)q * 3 * nk + d;
+                            const size_t h = (size_t)3 * nk;
+                            *reinterpret_cast<float4 *>(d2 + d * R + q) = make_float4(
+                                __ldg(s), __ldg(s + h), __ldg(s + 2 * h), __ldg(s + 3 * h));
+                        }
+                    continue;
+                }
+            }
+            const int nq = R <= kRealFew ? R : rows_even(R);
+            for (int q = 0; q < nq; q++) {
+                const T *s = src + (size_t)q * 3 * nk;
+                for (int d = 0; d < 3; d++) d2[real_at(R, q, d)] = q < R ? __ldg(s + d) : T(0);
+            }
+            if (R <= kRealFew)
+                for (int k = 3 * R; k < real_row(R); k++) d2[k] = T(0);
         }
     }
 }
@@ -408,8 +431,9 @@ struct _spme_batch_t {
     uint32_t *d_rst1 = nullptr, *d_rst2 = nullptr;
     void *d_rw1 = nullptr, *d_rw2 = nullptr;
     void *d_F = nullptr, *d_Fs = nullptr, *d_W = nullptr, *d_W2 = nullptr;
+    void *d_F2 = nullptr;  // force rows as the FP32 real-space sum reads them
     void *d_mesh = nullptr, *d_spec = nullptr, *d_tab = nullptr;
-    double *d_pair = nullptr;  // FP64 batches: Chebyshev tables of all systems
+    double *d_pair = nullptr;  // FP64 batches: pair-function tables of all systems
     int *d_err = nullptr;
     // work lists (device): per-system launch arguments and block prefixes
     void *d_spread_sys = nullptr, *d_interp_sys = nullptr, *d_real_sys = nullptr;
@@ -646,6 +670,8 @@ int create_t(_spme_batch_t *b) {
     BTRY(balloc(&b->d_rw1, sizeof(T) * (size_t)b->ws * n));
     BTRY(balloc(&b->d_rw2, sizeof(T) * (size_t)b->ws * n));
     BTRY(balloc(&b->d_F, sizeof(T) * (size_t)C * n));
+    if (sizeof(T) == 4 && !real_row_is_F(b->R))
+        BTRY(balloc(&b->d_F2, sizeof(T) * (size_t)real_row(b->R) * n));
     BTRY(balloc(&b->d_Fs, sizeof(T) * (size_t)spread_cols_row_width(C) * n));
     BTRY(balloc(&b->d_W, sizeof(T) * (size_t)C * n));
     BTRY(balloc(&b->d_W2, sizeof(T) * (size_t)C * n));
@@ -696,29 +722,25 @@ int create_t(_spme_batch_t *b) {
     }
     cudaFree(d_bm);
 
-    // FP64 batches: the pair functions from per-system Chebyshev tables
+    // FP64 batches: the pair functions from per-system tables
     std::vector<PairTable> ptab(ns);
     if (sizeof(T) == 8) {
-        std::vector<std::vector<double>> coefs(ns);
-        size_t total = 0;
+        std::vector<double> all, coef;
         std::vector<size_t> at(ns, 0);
         for (int k = 0; k < ns; k++) {
             const BatchSys &x = b->sys[k];
-            if (build_pair_table(x.s.xi, x.s.radius, x.s.rcut, &coefs[k], &ptab[k])) {
-                at[k] = total;
-                total += coefs[k].size();
-            } else {
+            at[k] = all.size();
+            if (build_pair_table(x.s.xi, x.s.radius, x.s.rcut, &coef, &ptab[k]))
+                all.insert(all.end(), coef.begin(), coef.end());
+            else
                 ptab[k] = PairTable{};
-            }
         }
-        if (total) {
-            BTRY(balloc(&b->d_pair, sizeof(double) * total));
+        if (!all.empty()) {
+            BTRY(balloc(&b->d_pair, sizeof(double) * all.size()));
+            BTRY_CUDA(cudaMemcpy(b->d_pair, all.data(), sizeof(double) * all.size(),
+                                 cudaMemcpyHostToDevice));
             for (int k = 0; k < ns; k++)
-                if (!coefs[k].empty()) {
-                    BTRY_CUDA(cudaMemcpy(b->d_pair + at[k], coefs[k].data(),
-                                         sizeof(double) * coefs[k].size(), cudaMemcpyHostToDevice));
-                    ptab[k].coef = b->d_pair + at[k];
-                }
+                if (ptab[k].hi_bits) ptab[k].coef = b->d_pair + at[k];
         }
     }
 
@@ -742,7 +764,7 @@ int create_t(_spme_batch_t *b) {
         ss[k].gy = sg.y;
         ps[k + 1] = ps[k] + sg.blocks;
         rs[k] = real_args<T>(x.nc, b->d_off3 + x.cell_off, b->d_perm3, b->d_cpos, (const T *)b->d_F,
-                             b->R, x.s.box_size, x.s.rcut, x.s.xi, x.s.radius, 1, ptab[k],
+                             (const T *)(b->d_F2 ? b->d_F2 : b->d_F), b->R, x.s.box_size, x.s.rcut, x.s.xi, x.s.radius, 1, ptab[k],
                              (T *)b->d_W);
         pr[k + 1] = pr[k] + x.nc * x.nc * x.nc;
         const size_t Kc = (size_t)K * K * (K / 2 + 1);
@@ -867,7 +889,7 @@ int apply_body(_spme_batch_t *b, double alpha, const T *f, double beta, T *u) {
     const long total = (long)n * C;
     mark(b, 1);  // (the position build, when it ran, ends here)
     k_batch_pack<T><<<grid_cap(n, 256, 8), 256, 0, s>>>(f, b->d_pref, b->nsys, b->R, n,
-                                                       (T *)b->d_F);
+                                                       (T *)b->d_F, (T *)b->d_F2);
     mark(b, 2);
     // the real-space sum beside the mesh pipeline when asked (serially when
     // profiling, so that every stage is timed alone)
@@ -945,7 +967,7 @@ void destroy_b(_spme_batch_t *b) {
                     b->d_off2,  b->d_cnt3,  b->d_off3,  b->d_scan_tmp, b->d_perm1, b->d_perm2,
                     b->d_perm3, b->d_pstart, b->d_pfrac, b->d_prel, b->d_cpos,  b->d_ridx1,
                     b->d_ridx2, b->d_rst1,  b->d_rst2,  b->d_rw1,   b->d_rw2,   b->d_F,
-                    b->d_Fs,    b->d_W,     b->d_W2,    b->d_mesh,  b->d_spec,  b->d_tab,
+                    b->d_Fs,    b->d_F2,    b->d_W,     b->d_W2,    b->d_mesh,  b->d_spec,  b->d_tab,
                     b->d_pair,  b->d_err,   b->d_spread_sys, b->d_interp_sys,
                     b->d_real_sys, b->d_infl_sys, b->d_pre_spread, b->d_pre_interp,
                     b->d_pre_real, b->d_pre_infl};

@@ -155,13 +155,14 @@ struct _spme_t {
     int *d_ccount = nullptr, *d_coff = nullptr, *d_cperm = nullptr;
     void *d_cpos = nullptr;  // float4 (FP32 engine) or double4_32a (FP64 engine)
     void *d_prel = nullptr;  // the same in particle order (from the keys pass)
-    void *d_pair = nullptr;  // Chebyshev table of the pair functions (FP64 engines)
+    void *d_pair = nullptr;  // table of the pair functions (FP64 engines)
     spme::PairTable pair;
     void *d_mesh = nullptr, *d_cmesh = nullptr, *d_tab = nullptr;
     double *d_bmod2 = nullptr;
     void *d_work = nullptr;
     size_t work_bytes = 0;
     std::vector<PlanPair> plans;
+    void *d_F2 = nullptr;  // force rows as the FP32 real-space sum reads them
     void *d_F = nullptr, *d_W = nullptr, *d_fstage = nullptr, *d_ustage = nullptr;
     void *d_W2 = nullptr;  // mesh part of the result when the real-space part is in d_W
     int *d_err = nullptr;  // device-side error flag (TMA wait timeouts)
@@ -579,7 +580,7 @@ int create_impl(const spme_params &prm, spme_t **out) {
         TRY(dalloc(&e->d_cperm, sizeof(int) * n));
         TRY(dalloc(&e->d_cpos, sizeof(double4_32a) * n));
         TRY(dalloc(&e->d_prel, sizeof(double4_32a) * n));
-        // FP64: the pair functions from a Chebyshev table instead of erfc / exp
+        // FP64: the pair functions from a table in r^2 instead of erfc / exp
         std::vector<double> coef;
         if (!is_fp32(e) && spme::build_pair_table(prm.xi, prm.radius, prm.rcut, &coef, &e->pair)) {
             TRY(dalloc(&e->d_pair, sizeof(double) * coef.size()));
@@ -588,6 +589,12 @@ int create_impl(const spme_params &prm, spme_t **out) {
             e->pair.coef = (const double *)e->d_pair;
         } else {
             e->pair = spme::PairTable{};
+        }
+        if (is_fp32(e)) {
+            // (a pass of fewer right-hand sides may have the wider rows: 4 against 5)
+            size_t row = 0;
+            for (int r = 1; r <= prm.max_nrhs; r++) row = std::max<size_t>(row, spme::real_row(r));
+            TRY(dalloc(&e->d_F2, e->elem * n * row));
         }
     }
     if (prm.terms & SPME_TERM_RECIP) {
@@ -731,7 +738,7 @@ void destroy_impl(spme_t *e) {
                     e->d_zip,    e->d_f2tab,    e->d_scount,  e->d_soff,   e->d_sperm, e->d_srec_idx,
                     e->d_srec_start, e->d_srec_w, e->d_Fs, e->d_W2, e->d_pair, e->d_key2,
                     e->d_key3,   e->d_pstart, e->d_pfrac, e->d_box,
-                    e->d_boxtab};
+                    e->d_boxtab, e->d_F2};
     for (void *b : bufs) dfree(b);
     for (int i = 0; i <= kStages; i++)
         if (e->ev[i]) cudaEventDestroy(e->ev[i]);
@@ -836,6 +843,12 @@ int set_positions_impl(spme_t *e, const double *pos, int mem) {
     return SPME_OK;
 }
 
+// Where the pack writes the real-space sum's rows (null: nowhere, or F's serve).
+template <typename T>
+T *packed_rows(spme_t *e, int R) {
+    return spme::real_row_is_F(R) ? nullptr : (T *)e->d_F2;
+}
+
 template <typename T>
 int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alpha, double beta,
              int rpart) {
@@ -847,7 +860,7 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
     T *F = (T *)e->d_F, *W = (T *)e->d_W;
     if (prof) cudaEventRecord(e->ev[0], s);
     if (f) {  // null: F already packed (host-pointer applies pack on the copy stream)
-        spme::launch_pack_tiled<T>(f, ldf, n, R, F, s);
+        spme::launch_pack_tiled<T>(f, ldf, n, R, 0, R, F, packed_rows<T>(e, R), s);
         e->launches++;
     }
     if (prof) cudaEventRecord(e->ev[1], s);
@@ -864,7 +877,8 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
         if (prof) cudaEventRecord(e->ev_rs[0], rss);
         if (terms & SPME_TERM_REAL) {
             if (!e->d_coff || !e->d_cperm || !e->d_cpos) return SPME_ERR_STATE;
-            TRY_CUDA(spme::launch_realspace<T>(e->nc, e->d_coff, e->d_cperm, e->d_cpos, F, R,
+            TRY_CUDA(spme::launch_realspace<T>(e->nc, e->d_coff, e->d_cperm, e->d_cpos, F,
+                                               spme::real_row_is_F(R) ? F : (T *)e->d_F2, R,
                                                e->prm.box_size, e->prm.rcut, e->prm.xi,
                                                e->prm.radius, (terms & SPME_TERM_SELF) ? 1 : 0,
                                                e->pair, W, rss));
@@ -1089,10 +1103,12 @@ int apply_impl(spme_t *e, int nrhs, double alpha, const void *f, long ldf, doubl
                     TRY_CUDA(cudaStreamWaitEvent(e->stream, e->ev_in[k], 0));
                     if (is_fp32(e))
                         spme::launch_pack_tiled<float>((const float *)e->d_fstage, 3L * n, n, R, q0,
-                                                       q1, (float *)e->d_F, e->stream);
+                                                       q1, (float *)e->d_F,
+                                                       packed_rows<float>(e, R), e->stream);
                     else
                         spme::launch_pack_tiled<double>((const double *)e->d_fstage, 3L * n, n, R,
-                                                        q0, q1, (double *)e->d_F, e->stream);
+                                                        q0, q1, (double *)e->d_F,
+                                                        packed_rows<double>(e, R), e->stream);
                     e->launches++;
                 }
                 TRY_CUDA(cudaGetLastError());

@@ -260,10 +260,24 @@ struct PairTable {
 // false if no fit meets that within 1024 segments per octave.
 bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef, PairTable *t);
 // cpos: float4 for T = float, double4_32a for T = double (cell-relative); FP32 in
-// realspace.cu (tab unused), FP64 in realspace_fp64.cu.
+// realspace.cu (tab unused), FP64 in realspace_fp64.cu.  F2 (FP32; unused in FP64):
+// the force rows as that kernel reads them, real_row(R) values each: for up to
+// kRealFew right-hand sides in F's order padded to 16 bytes, for more by component
+// ([d][rows_even(R)]); the padding is zero.
+constexpr int kRealFew = 4;
+__host__ __device__ constexpr int rows_even(int R) { return (R + 1) & ~1; }
+__host__ __device__ constexpr int real_row(int R) {
+    return R <= kRealFew ? (3 * R + 3) / 4 * 4 : 3 * rows_even(R);
+}
+// Whether F's own rows serve (R = 4: 12 values, whole 16-byte vectors).
+__host__ __device__ constexpr bool real_row_is_F(int R) { return R <= kRealFew && real_row(R) == 3 * R; }
+// The place of right-hand side r, component d in such a row.
+__host__ __device__ constexpr int real_at(int R, int r, int d) {
+    return R <= kRealFew ? 3 * r + d : d * rows_even(R) + r;
+}
 template <typename T>
 cudaError_t launch_realspace(int nc, const int *cell_off, const int *cell_perm, const void *cpos,
-                             const T *F, int R, double L, double rc, double xi, double a,
+                             const T *F, const T *F2, int R, double L, double rc, double xi, double a,
                              int with_self, const PairTable &tab, T *W, cudaStream_t s);
 // FP32 pair-function coefficients of one (xi, a) and the FP32 copies of the
 // geometry (real_args fills them): far field (r >= 2a), with ir = 1/r,
@@ -283,6 +297,7 @@ struct RealArgs {
     const int *cell_perm;
     const void *cpos;
     const T *F;
+    const T *F2;
     T *W;
     int nc, R, with_self;
     double L, h, rc2, xi, a, self_c;
@@ -292,7 +307,7 @@ struct RealArgs {
 double real_self_coeff(double xi, double a);
 template <typename T>
 RealArgs<T> real_args(int nc, const int *cell_off, const int *cell_perm, const void *cpos,
-                      const T *F, int R, double L, double rc, double xi, double a, int with_self,
+                      const T *F, const T *F2, int R, double L, double rc, double xi, double a, int with_self,
                       const PairTable &tab, T *W);
 // All systems (R right-hand sides each) in one persistent launch over their cells
 // (prefix as for the spread).
@@ -302,11 +317,11 @@ cudaError_t launch_realspace_batch(const RealArgs<T> *sys, const int *prefix, in
 
 template <>
 cudaError_t launch_realspace<float>(int, const int *, const int *, const void *, const float *,
-                                    int, double, double, double, double, int, const PairTable &,
+                                    const float *, int, double, double, double, double, int, const PairTable &,
                                     float *, cudaStream_t);
 template <>
 cudaError_t launch_realspace<double>(int, const int *, const int *, const void *, const double *,
-                                     int, double, double, double, double, int, const PairTable &,
+                                     const double *, int, double, double, double, double, int, const PairTable &,
                                      double *, cudaStream_t);
 template <>
 cudaError_t launch_realspace_batch<float>(const RealArgs<float> *, const int *, int, int, int,
@@ -319,7 +334,6 @@ cudaError_t launch_realspace_batch<double>(const RealArgs<double> *, const int *
 // W = self_c * F (the self term alone, when no real-space sum is requested)
 template <typename T>
 void launch_self(const T *F, int n, int R, double self_c, T *W, cudaStream_t s);
-// F[i][3R] = f[r*ld + 3i + d]
 // Fs[s][c] = F[idx[s]][c] for s < n (C components per row).
 template <typename T>
 void launch_gather_rows(const T *F, const int *idx, int n, int C, T *Fs, cudaStream_t s);
@@ -328,11 +342,11 @@ void launch_pack(const T *f, long ld, int n, int R, T *F, cudaStream_t s);
 // u[r*ld + 3i + d] = beta*u + alpha*W[i][3r+d]   (u not read when beta == 0)
 // Tiled (shared-memory) forms of launch_pack / launch_unpack(_sum): coalesced on
 // both sides; W2 may be null (plain unpack).  Up to 48 KB of shared memory.
+// Right-hand sides [r0, r1) of f into their columns of F[n][3R] and, if F2 is not
+// null, their places in F2[n][real_row(R)] (with the last ones, zeros in its padding).
 template <typename T>
-void launch_pack_tiled(const T *f, long ld, int n, int R, T *F, cudaStream_t s);
-// (right-hand sides [r0, r1) of f into their columns of F[n][3R])
-template <typename T>
-void launch_pack_tiled(const T *f, long ld, int n, int R, int r0, int r1, T *F, cudaStream_t s);
+void launch_pack_tiled(const T *f, long ld, int n, int R, int r0, int r1, T *F, T *F2,
+                       cudaStream_t s);
 // (launch_unpack_tiled: right-hand sides [r0, r1) of the R in W / W2.)
 template <typename T>
 void launch_unpack_tiled(const T *W, const T *W2, int n, int R, int r0, int r1, double alpha,

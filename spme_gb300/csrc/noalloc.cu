@@ -119,8 +119,8 @@ extern "C" int spme_realspace_apply_noalloc(int np, const double *pos, double bo
     spme::launch_scatter(key, off, np, perm, slot, s);
     spme::launch_cell_positions(pos, perm, np, box_size, (int)nc, false, cpos, s);
     spme::launch_pack<double>(f, ldf, np, nrhs, F, s);
-    if (spme::launch_realspace<double>((int)nc, off, perm, cpos, F, nrhs, box_size, rcut, xi,
-                                       radius, 1, spme::PairTable{}, W, s) != cudaSuccess)
+    if (spme::launch_realspace<double>((int)nc, off, perm, cpos, F, nullptr, nrhs, box_size, rcut,
+                                       xi, radius, 1, spme::PairTable{}, W, s) != cudaSuccess)
         return SPME_ERR_CUDA;
     spme::launch_unpack<double>(W, np, nrhs, alpha, beta, u, ldu, s);
     return cudaGetLastError() == cudaSuccess ? SPME_OK : SPME_ERR_CUDA;

@@ -70,10 +70,46 @@ constexpr int kPB = 128;
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_pack_tiled(const T *__restrict__ f, long ld, int n, int R, int r0, int r1, int pb, int vec,
-             T *__restrict__ F) {
+             T *__restrict__ F, T *__restrict__ F2) {
     extern __shared__ __align__(16) unsigned char pk_raw[];
     T *tile = reinterpret_cast<T *>(pk_raw);  // [pb][CP + 1]
     const int C = 3 * R, CP = 3 * (r1 - r0), CS = CP + 1;  // row stride, columns written
+    // the tile's right-hand sides in the real-space sum's rows (kernels.h), and with
+    // the last one zeros in their padding
+    const int R2 = rows_even(R), RW = real_row(R), last = r1 == R;
+    auto write_real_rows = [&](int i0, int np) {
+        // a row is 3 runs of NR values (by component) or one of CP + padding
+        const bool by_comp = R > kRealFew;
+        const int nrun = by_comp ? 3 : 1, NR = by_comp ? (last ? R2 : r1) - r0
+                                                       : (last ? RW : 3 * r1) - 3 * r0;
+        const int n_in = by_comp ? r1 - r0 : CP, step = by_comp ? 3 : 1;
+        DivMod dr;
+        if constexpr (sizeof(T) == 4) {
+            if (((R2 | r0 | NR | RW) & 3) == 0 || (!by_comp && r0 == 0)) {  // 16-byte vectors
+                dr.init(NR / 4);
+                for (int t = threadIdx.x; t < np * nrun * (NR / 4); t += blockDim.x) {
+                    int k4;
+                    const int pd = dr.div(t, k4), p = by_comp ? pd / 3 : pd, d = pd - nrun * p;
+                    const T *src = tile + p * CS + (by_comp ? d : 0);
+                    float e[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        e[j] = 4 * k4 + j < n_in ? src[(4 * k4 + j) * step] : 0.f;
+                    *reinterpret_cast<float4 *>(F2 + (size_t)(i0 + p) * RW +
+                                                (by_comp ? d * R2 + r0 : 0) + 4 * k4) =
+                        make_float4(e[0], e[1], e[2], e[3]);
+                }
+                return;
+            }
+        }
+        dr.init(NR);
+        for (int t = threadIdx.x; t < np * nrun * NR; t += blockDim.x) {
+            int k;
+            const int pd = dr.div(t, k), p = by_comp ? pd / 3 : pd, d = pd - nrun * p;
+            F2[(size_t)(i0 + p) * RW + (by_comp ? d * R2 + r0 : 3 * r0) + k] =
+                k < n_in ? tile[p * CS + (by_comp ? d : 0) + k * step] : T(0);
+        }
+    };
     for (int i0 = blockIdx.x * pb; i0 < n; i0 += gridDim.x * pb) {
         const int np = min(pb, n - i0);
         if constexpr (sizeof(T) == 4) {
@@ -102,6 +138,7 @@ k_pack_tiled(const T *__restrict__ f, long ld, int n, int R, int r0, int r1, int
                     *reinterpret_cast<float4 *>(F + (size_t)(i0 + p) * C + 3 * r0 + 4 * c4) =
                         make_float4(src[0], src[1], src[2], src[3]);
                 }
+                if (F2) write_real_rows(i0, np);
                 __syncthreads();
                 continue;
             }
@@ -116,6 +153,7 @@ k_pack_tiled(const T *__restrict__ f, long ld, int n, int R, int r0, int r1, int
             const int p = t / CP, c = t - p * CP;
             F[(size_t)(i0 + p) * C + 3 * r0 + c] = tile[p * CS + c];
         }
+        if (F2) write_real_rows(i0, np);
         __syncthreads();
     }
 }
@@ -249,11 +287,6 @@ int tile_particles(int R, size_t elem) {
     return (int)(pb < 1 ? 1 : pb);
 }
 
-template <typename T>
-void launch_pack_tiled(const T *f, long ld, int n, int R, T *F, cudaStream_t s) {
-    launch_pack_tiled<T>(f, ld, n, R, 0, R, F, s);
-}
-
 // 16-byte vectors on both sides of an FP32 tile: the caller's rows (ld, base) and
 // the packed rows (C, the first column 3 r0, the width 3 (r1 - r0), the base)
 // all 16-byte aligned, and whole tiles of a multiple of 4 particles.
@@ -267,12 +300,14 @@ int vec_tiles(const T *caller, long ld, const T *packed, int R, int r0, int r1, 
 }
 
 template <typename T>
-void launch_pack_tiled(const T *f, long ld, int n, int R, int r0, int r1, T *F, cudaStream_t s) {
+void launch_pack_tiled(const T *f, long ld, int n, int R, int r0, int r1, T *F, T *F2,
+                       cudaStream_t s) {
     if (n <= 0 || R <= 0 || r0 < 0 || r1 > R || r0 >= r1) return;
     const int pb = tile_particles(r1 - r0, sizeof(T));
     const size_t smem = (size_t)pb * (3 * (r1 - r0) + 1) * sizeof(T);
     const int vec = vec_tiles<T>(f, ld, F, R, r0, r1, pb);
-    k_pack_tiled<T><<<tiled_blocks(n, pb), 256, smem, s>>>(f, ld, n, R, r0, r1, pb, vec, F);
+    k_pack_tiled<T><<<tiled_blocks(n, pb), 256, smem, s>>>(f, ld, n, R, r0, r1, pb, vec, F,
+                                                               F2);
 }
 
 template <typename T>
@@ -297,12 +332,10 @@ void launch_self(const T *F, int n, int R, double self_c, T *W, cudaStream_t s) 
     if (total) k_self<T><<<blocks_for(total), 256, 0, s>>>(F, total, (T)self_c, W);
 }
 
-template void launch_pack_tiled<float>(const float *, long, int, int, float *, cudaStream_t);
-template void launch_pack_tiled<double>(const double *, long, int, int, double *, cudaStream_t);
-template void launch_pack_tiled<float>(const float *, long, int, int, int, int, float *,
+template void launch_pack_tiled<float>(const float *, long, int, int, int, int, float *, float *,
                                        cudaStream_t);
 template void launch_pack_tiled<double>(const double *, long, int, int, int, int, double *,
-                                        cudaStream_t);
+                                        double *, cudaStream_t);
 template void launch_unpack_tiled<float>(const float *, const float *, int, int, int, int, double,
                                          double, float *, long, cudaStream_t);
 template void launch_unpack_tiled<double>(const double *, const double *, int, int, int, int,

@@ -1,22 +1,39 @@
 // FP32 real-space Ewald RPY pair sum over a cell list within rc, plus the self
-// term (FP64: realspace_fp64.cu).  The reference has no real-space part (it computes only M_recip,
-// old-version/spme.c:560-726); this restates Beenakker, J. Chem. Phys. 85,
-// 1581 (1986), in the reference's units (mobility x 6 pi eta, matching
-// scalar_recip at old-version/spme.c:43-60), with the RPY overlap form for
-// pairs closer than 2a.
+// term (FP64: realspace_fp64.cu).  The reference has no real-space part (it
+// computes only M_recip, old-version/spme.c:560-726); this restates Beenakker, J.
+// Chem. Phys. 85, 1581 (1986), in the reference's units (mobility x 6 pi eta,
+// matching scalar_recip at old-version/spme.c:43-60), with the RPY overlap form
+// for pairs closer than 2a.
 //
-// One CTA per cell of edge >= rc; a warp per particle of the cell against the
-// candidates of the 27 neighbour cells (details at the kernel below).
+// What bounds it: issued instructions (the sum was 71 % issue-active at 1814 warp
+// instructions per particle for 16 right-hand sides), so pairs are listed first
+// and everything after runs with full warps:
+//   * one CTA per cell of edge >= rc stages the candidates of the 27 neighbour cells
+//     once; each warp lists the pairs within rc of up to 16 of its particles
+//     (ballot-compacted, realspace_pairs.cuh);
+//   * the pair functions are evaluated 32 listed pairs at a time;
+//   * up to kRealFew right-hand sides: the listed pairs are split evenly over the
+//     lanes, which accumulate in registers (realspace_few_body); a partner's row is
+//     padded to 16-byte vectors, as every lane reads another row;
+//   * more: lanes as (pair slot, two right-hand sides) apply the evaluated pairs with
+//     two-lane FMAs (fma.rn.f32x2); the partner's force rows come component by
+//     component (F2[j][d][r]), so a right-hand side pair is one 8-byte load and a
+//     row's load touches one line instead of the whole interleaved row.
+// Sums over up to 16 pairs per slot run in FP32, longer ones with TwoSum.
+// Measured (ms): N = 1e6, R = 16 1.65 -> 1.52; N = 2e5, R = 16 0.445 -> 0.405; N = 1e5,
+// R = 1 0.162 -> 0.102; 64 uneven systems, R = 4 1.53 -> 1.40.  The partners' rows come
+// mostly from L2 (16 % L1 hits), whose latency bounds it now; more warps per SM at
+// fewer registers spill (1.57 ms at 12 blocks), a table of the pair functions in
+// shared-memory-free FP32 cost more in scattered loads than it saved (1.64 ms).
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
-#include "kernels.h"
+#include "realspace_pairs.cuh"
 
 namespace spme {
 
 namespace {
-
-constexpr int kThreads = 64;  // two warps per cell: ~4-5 particles each at typical densities
 
 // M_real(r) = F I + G rhat rhat: Beenakker's real-space form divided by a, and
 // for r < 2a plus (overlap RPY - far-field RPY).  For r < 2a the 1/r and 1/r^3
@@ -75,308 +92,232 @@ __device__ __forceinline__ void real_FG_f32(float r2, const RealCoef &c, float &
     G = ec * fmaf(c.c3, ir3, 0.75f * ir) + e * pG;
 }
 
-// Accumulator across pair batches: FP32 with Knuth's TwoSum error term carried
-// alongside (the FP64 pipe is a small fraction of the FP32 rate on this GPU, and
-// a handful of double adds per particle had become the kernel's limiter).
-struct PairSum {
-    float s = 0.f, c = 0.f;
-    __device__ __forceinline__ void add(float x) {
-        const float t = s + x, bp = t - s;
-        c += (s - (t - bp)) + (x - bp);
-        s = t;
-    }
-    __device__ __forceinline__ void add(const PairSum &o) {
-        add(o.s);
-        c += o.c;
-    }
-    __device__ __forceinline__ float value() const { return s + c; }
+template <int RB>
+__device__ __forceinline__ void real_few(const RealArgs<float> &A, int cell) {
+    realspace_few_body<float, RB>(A, cell, A.cf.L, A.cf.h, A.cf.rc2, A.cf.self_c,
+                                  [&](float s, float &Av, float &Bv) {
+                                      float ir;
+                                      real_FG_f32(s, A.cf, Av, Bv, ir);
+                                      Bv *= ir * ir;
+                                      return true;
+                                  });
+}
+
+constexpr int kWin = 64;      // pairs evaluated together
+constexpr int kListM = 512;   // listed pairs per warp
+constexpr int kFold = 16;     // pairs per slot summed in plain FP32
+
+struct ManyShared {
+    float4 r0[kWin];  // displacement, A
+    float2 r1[kWin];  // B, partner (bits)
+    float4 pf[kGroup];
+    uint32_t list[kListM];
+    int beg[kGroup + 2];
 };
 
-__device__ __forceinline__ PairSum shfl_xor(const PairSum &a, int o) {
-    PairSum b;
-    b.s = __shfl_xor_sync(0xffffffffu, a.s, o);
-    b.c = __shfl_xor_sync(0xffffffffu, a.c, o);
-    return b;
-}
+// One cell, more than kRealFew right-hand sides: RL lanes of two right-hand sides
+// each, 32 / RL pair slots; blocks of 2 RL right-hand sides in sequence.
+template <int RL>
+__device__ __forceinline__ void real_many(const RealArgs<float> &A, int cell) {
+    constexpr int PS = 32 / RL;
+    __shared__ CellShared<float> csh;
+    __shared__ ManyShared wsh[kRsWarps];
+    const int ib0 = __ldg(A.cell_off + cell), ie = __ldg(A.cell_off + cell + 1);
+    if (ib0 == ie) return;  // uniform over the block
+    const Cell<float> cl(csh, cell, A.nc, A.cell_off, A.cell_perm, A.cpos, A.cf.L, A.cf.h,
+                         A.cf.rc2);
+    const int R = A.R, R2 = rows_even(R), C = 3 * R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = lane / RL, rl = lane % RL;
+    ManyShared &ws = wsh[warp];
 
-constexpr int kWarps = kThreads / 32;
-constexpr int kCap = 512;  // candidates staged in shared memory per cell
-
-// Positions are stored relative to the corner of their cell (edge h = L/nc), so
-// the displacement to a candidate in neighbour cell c_i + dc is (o_i - o_j) -
-// dc*h, accurate in FP32 for any box size.
-//
-// One CTA per cell.  The candidates of the 27 neighbour cells are staged once
-// in shared memory (positions in the frame of the CTA's cell), then each warp
-// takes one of the cell's particles at a time:
-//   1. lanes test 32 candidates at a time for r < rc and compact the hits
-//      into a per-warp buffer (ballot + popc);
-//   2. every 32 hits, lanes evaluate the 32 pair functions F, G and unit
-//      vectors (all lanes busy);
-//   3. lanes as (pair, right-hand side) apply the batch to the forces:
-//      u_i[r] += F f_j[r] + G rhat (rhat . f_j[r]).
-// Sums over one batch run in FP32, across batches in compensated FP32 (TwoSum,
-// PairSum).  No block barrier after the staging.  More than kCap candidates (very dense cells)
-// take a second path that reads candidates straight from global memory.
-// 64 registers, 16 blocks (32 warps) per SM (measured faster than the
-// unconstrained 80 registers).
-__device__ __forceinline__ void realspace_body(const RealArgs<float> &A, int cell) {
-    const int nc = A.nc;
-    const int *__restrict__ cell_off = A.cell_off;
-    const int *__restrict__ cell_perm = A.cell_perm;
-    const float4 *__restrict__ cpos = reinterpret_cast<const float4 *>(A.cpos);
-    const float *__restrict__ F = A.F;
-    float *__restrict__ W = A.W;
-    const int R = A.R, with_self = A.with_self;
-    const float L = A.cf.L, h = A.cf.h, rc2 = A.cf.rc2, self_c = A.cf.self_c;
-    __shared__ int nb_beg[27], nb_pre[28], nnb;
-    __shared__ float nb_shift[27][3];
-    // a staged candidate: position in the CTA cell's frame and particle id in
-    // one 16-byte record
-    struct __align__(16) Cand {
-        float x, y, z;
-        int j;
-    };
-    __shared__ Cand cand[kCap];
-    constexpr int kU = 2;  // candidates tested per lane per iteration
-    __shared__ int hits[kWarps][32 + 32 * kU];  // up to 31 carried + 32 kU new
-    // one record per buffered pair: unit vector and F in one 16-byte vector,
-    // then G and the start of the partner's force row (aligned as that vector)
-    struct PairRec {
-        float4 rf;  // (rhat_x, rhat_y, rhat_z, F)
-        const float *frow;
-        float gfac;
-    };
-    __shared__ PairRec prec[kWarps][32];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int C = 3 * R;
-    // neighbour table: lane k of warp 0 takes neighbour cell k (27 of them, or
-    // the cell alone when nc < 3), candidate offsets by a warp scan
-    if (warp == 0) {
-        const int ccx = cell % nc, ccy = (cell / nc) % nc, ccz = cell / (nc * nc);
-        const int nk = nc >= 3 ? 27 : 1;
-        int cnt = 0;
-        if (lane < nk) {
-            const int dx = nk == 1 ? 0 : lane % 3 - 1, dy = nk == 1 ? 0 : (lane / 3) % 3 - 1,
-                      dz = nk == 1 ? 0 : lane / 9 - 1;
-            auto wrap = [nc](int v) { return v < 0 ? v + nc : (v >= nc ? v - nc : v); };
-            const int c2 = (wrap(ccz + dz) * nc + wrap(ccy + dy)) * nc + wrap(ccx + dx);
-            const int b = __ldg(cell_off + c2);
-            cnt = __ldg(cell_off + c2 + 1) - b;
-            nb_beg[lane] = b;
-            nb_shift[lane][0] = dx * h;
-            nb_shift[lane][1] = dy * h;
-            nb_shift[lane][2] = dz * h;
+    // this warp's share of the cell's particles, kGroup at a time
+    const int half = (ie - ib0 + kRsWarps - 1) / kRsWarps;
+    const int wb = ib0 + warp * half, we = min(ie, wb + half);
+    for (int g0 = wb; g0 < we; g0 += kGroup) {
+        const int np = min(kGroup, we - g0);
+        if (lane < np) {
+            const float4 p = cl.cpos[g0 + lane];
+            ws.pf[lane] = make_float4(p.x, p.y, p.z, __int_as_float(A.cell_perm[g0 + lane]));
         }
-        int inc = cnt;
+        __syncwarp();
+        for (int rb = 0; rb < R; rb += 2 * RL) {
+            const int r = rb + 2 * rl;  // this lane's right-hand sides r, r + 1
+            const bool live = r < R;
+            const float *__restrict__ Fr = A.F2 + r;
+            ListState ls;
+            // sums of the current particle: two-lane partial sums, moved to compensated
+            // ones every kFold pairs per slot
+            float2 s0 = make_float2(0.f, 0.f), s1 = s0, s2 = s0;
+            PairSum<float> sum[6];
+            int nfold = 0, cnt = 0;
+            auto fold = [&]() {
+                const float v[6] = {s0.x, s1.x, s2.x, s0.y, s1.y, s2.y};
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane < nk) nb_pre[lane] = inc - cnt;
-        if (lane == nk - 1) {
-            nb_pre[nk] = inc;
-            nnb = nk;
-        }
-    }
-    __syncthreads();
-    const int ncand = nb_pre[nnb];
-    const bool staged = ncand <= kCap;
-    // neighbour k holding candidate q: nb_pre[k] <= q < nb_pre[k + 1]
-    auto find_nb = [&](int q) {
-        int lo = 0, hi = nnb;
-        while (hi - lo > 1) {
-            const int m = (lo + hi) >> 1;
-            if (nb_pre[m] <= q) lo = m; else hi = m;
-        }
-        return lo;
-    };
-    if (staged) {
-        for (int q = tid; q < ncand; q += kThreads) {
-            const int k = find_nb(q);
-            const int js = nb_beg[k] + (q - nb_pre[k]);
-            const auto p = cpos[js];
-            Cand c;
-            c.x = p.x + nb_shift[k][0];
-            c.y = p.y + nb_shift[k][1];
-            c.z = p.z + nb_shift[k][2];
-            c.j = cell_perm[js];
-            cand[q] = c;
-        }
-    }
-    __syncthreads();
-    const bool single = nc < 3;
-    const float invL = 1.f / L;
-    const int ib0 = cell_off[cell], ie = cell_off[cell + 1];
-
-    // candidate q -> position in this cell's frame and particle id
-    auto candidate = [&](int q, float &x, float &y, float &z, int &j) {
-        if (staged) {
-            const Cand c = cand[q];
-            x = c.x;
-            y = c.y;
-            z = c.z;
-            j = c.j;
-        } else {
-            const int k = find_nb(q);
-            const int js = nb_beg[k] + (q - nb_pre[k]);
-            const auto p = cpos[js];
-            x = p.x + nb_shift[k][0];
-            y = p.y + nb_shift[k][1];
-            z = p.z + nb_shift[k][2];
-            j = cell_perm[js];
-        }
-    };
-
-    const int RL = R >= 32 ? 32 : (R > 16 ? 32 : (R > 8 ? 16 : (R > 4 ? 8 : (R > 2 ? 4 : (R > 1 ? 2 : 1)))));
-    const int PR = 32 / RL;             // pairs applied in parallel
-    const int pp = lane / RL, rl = lane % RL;
-
-    for (int i = ib0 + warp; i < ie; i += kWarps) {
-        const auto pi = cpos[i];
-        const int ii = cell_perm[i];
-        for (int rb = 0; rb < R; rb += RL) {
-            const int r = rb + rl;
-            const bool rok = r < R;
-            PairSum a0, a1, a2;
-            int nh = 0;  // buffered hits (warp-uniform)
-            // evaluate and apply `m` buffered hits; returns this lane's partial sums
-            auto flush = [&](int m, float &s0, float &s1, float &s2) {
-                if (lane < m) {
-                    float x, y, z;
-                    int j;
-                    candidate(hits[warp][lane], x, y, z, j);
-                    float d0 = pi.x - x, d1 = pi.y - y, d2 = pi.z - z;
-                    if (single) {
-                        d0 -= L * rintf(d0 * invL);
-                        d1 -= L * rintf(d1 * invL);
-                        d2 -= L * rintf(d2 * invL);
-                    }
-                    float Fv, Gv;
-                    float ir;  // coincident particles (r = 0): no direction, the G term vanishes
-                    real_FG_f32(d0 * d0 + d1 * d1 + d2 * d2, A.cf, Fv, Gv, ir);
-                    PairRec &pq = prec[warp][lane];
-                    pq.rf.x = d0 * ir;
-                    pq.rf.y = d1 * ir;
-                    pq.rf.z = d2 * ir;
-                    pq.rf.w = Fv;
-                    pq.gfac = Gv;
-                    pq.frow = F + (size_t)j * C;
-                }
-                __syncwarp();
-                s0 = s1 = s2 = 0.f;
-                if (rok) {
-#pragma unroll 4
-                    for (int k = pp; k < m; k += PR) {
-                        const PairRec &pq = prec[warp][k];
-                        const auto rf = pq.rf;
-                        const float *fj = pq.frow + 3 * r;
-                        const float f0 = __ldg(fj), f1 = __ldg(fj + 1), f2 = __ldg(fj + 2);
-                        const float rx = rf.x, ry = rf.y, rz = rf.z;
-                        const float Fk = rf.w, Gd = pq.gfac * (rx * f0 + ry * f1 + rz * f2);
-                        s0 += Fk * f0 + Gd * rx;
-                        s1 += Fk * f1 + Gd * ry;
-                        s2 += Fk * f2 + Gd * rz;
-                    }
-                }
-                __syncwarp();
+                for (int q = 0; q < 6; q++) sum[q].add(v[q]);
+                s0 = s1 = s2 = make_float2(0.f, 0.f);
+                nfold++;
+                cnt = 0;
             };
-            // candidate q within rc of particle i (and not i itself)
-            auto test = [&](int q) {
-                bool hit = false;
-                if (q < ncand) {
-                    float x, y, z;
-                    int j;
-                    candidate(q, x, y, z, j);
-                    if (j != ii) {
-                        float d0 = pi.x - x, d1 = pi.y - y, d2 = pi.z - z;
-                        if (single) {
-                            d0 -= L * rintf(d0 * invL);
-                            d1 -= L * rintf(d1 * invL);
-                            d2 -= L * rintf(d2 * invL);
+            while (ls.il < np) {
+                const int ilo = ls.il;
+                const int nh = list_pairs<true, kListM>(cl, ws.pf, np, ws.list, ws.beg, ls, PS);
+                const int last = ls.q0 == 0 ? ls.il - 1 : ls.il;
+                int wend = 0;  // entries [wend - kWin, wend) are evaluated
+                for (int ip = ilo; ip <= last; ip++) {
+                    int k = ws.beg[ip];
+                    const int e = ws.beg[ip + 1];
+                    while (k < e) {
+                        if (k >= wend) {
+                            __syncwarp();
+#pragma unroll
+                            for (int v = 0; v < kWin / 32; v++) {
+                                const int t = wend + 32 * v + lane;
+                                if (t < nh) {
+                                    const uint32_t ent = ws.list[t];
+                                    const float4 me = ws.pf[ent >> 28];
+                                    float d0 = 0.f, d1 = 0.f, d2 = 0.f, Av = 0.f, Bv = 0.f;
+                                    int j = __float_as_int(me.w);
+                                    if ((ent & kNoCand) != kNoCand) {
+                                        float x, y, z;
+                                        cl.candidate((int)(ent & kNoCand), x, y, z, j);
+                                        d0 = me.x - x;
+                                        d1 = me.y - y;
+                                        d2 = me.z - z;
+                                        cl.min_image(d0, d1, d2);
+                                        float ir;
+                                        real_FG_f32(fmaf(d2, d2, fmaf(d1, d1, d0 * d0)), A.cf, Av,
+                                                    Bv, ir);
+                                        Bv *= ir * ir;
+                                    }
+                                    const int q = 32 * v + lane;
+                                    ws.r0[q] = make_float4(d0, d1, d2, Av);
+                                    ws.r1[q] = make_float2(Bv, __int_as_float(j));
+                                }
+                            }
+                            wend += kWin;
+                            __syncwarp();
                         }
-                        hit = d0 * d0 + d1 * d1 + d2 * d2 < rc2;
+                        const int ke = min(e, wend);
+                        const int o = wend - kWin - slot;
+                        if (cnt >= kFold) fold();
+                        cnt += (ke - k) / PS;
+                        if (live) {
+#pragma unroll 2
+                            for (int q = k - o; q < ke - o; q += PS) {
+                                const float4 a = ws.r0[q];
+                                const float2 b = ws.r1[q];
+                                const float *fj =
+                                    Fr + (size_t)__float_as_int(b.y) * (size_t)(3 * R2);
+                                const float2 f0 = __ldg(reinterpret_cast<const float2 *>(fj));
+                                const float2 f1 = __ldg(reinterpret_cast<const float2 *>(fj + R2));
+                                const float2 f2 =
+                                    __ldg(reinterpret_cast<const float2 *>(fj + 2 * R2));
+                                const float2 d0 = make_float2(a.x, a.x), d1 = make_float2(a.y, a.y),
+                                             d2 = make_float2(a.z, a.z), Av = make_float2(a.w, a.w);
+                                const float2 g = __fmul2_rn(
+                                    make_float2(b.x, b.x),
+                                    __ffma2_rn(d2, f2, __ffma2_rn(d1, f1, __fmul2_rn(d0, f0))));
+                                s0 = __ffma2_rn(g, d0, __ffma2_rn(Av, f0, s0));
+                                s1 = __ffma2_rn(g, d1, __ffma2_rn(Av, f1, s1));
+                                s2 = __ffma2_rn(g, d2, __ffma2_rn(Av, f2, s2));
+                            }
+                        }
+                        k = ke;
+                    }
+                    if (ip == ls.il) break;  // cut: goes on in the next list
+                    // the slots' sums, then the self term, to the particle's row
+                    const int ii = __float_as_int(ws.pf[ip].w);
+                    if (nfold) fold();
+                    float v[6] = {s0.x, s1.x, s2.x, s0.y, s1.y, s2.y};
+#pragma unroll
+                    for (int q = 0; q < 6; q++) {
+                        if (nfold) v[q] = sum[q].value();
+                        sum[q] = PairSum<float>();
+#pragma unroll
+                        for (int w = RL; w < 32; w <<= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], w);
+                    }
+                    s0 = s1 = s2 = make_float2(0.f, 0.f);
+                    nfold = cnt = 0;
+                    if (slot == 0 && live) {
+                        const float *fi = Fr + (size_t)ii * (size_t)(3 * R2);
+                        float *o = A.W + (size_t)ii * C + 3 * r;
+#pragma unroll
+                        for (int q = 0; q < 6; q++) {
+                            if (q < 3 || r + 1 < R) {
+                                const float f = A.with_self ? __ldg(fi + q % 3 * R2 + q / 3) : 0.f;
+                                o[q] = fmaf(A.cf.self_c, f, v[q]);
+                            }
+                        }
                     }
                 }
-                return hit;
-            };
-            // kU candidates per lane per iteration: hits are appended in candidate
-            // order and evaluated 32 at a time
-            const unsigned below = (1u << lane) - 1u;
-            for (int q0 = 0; q0 < ncand; q0 += 32 * kU) {
-                bool hu[kU];
-#pragma unroll
-                for (int v = 0; v < kU; v++) hu[v] = test(q0 + 32 * v + lane);
-#pragma unroll
-                for (int v = 0; v < kU; v++) {
-                    const unsigned mv = __ballot_sync(0xffffffffu, hu[v]);
-                    if (hu[v]) hits[warp][nh + __popc(mv & below)] = q0 + 32 * v + lane;
-                    nh += __popc(mv);
-                }
                 __syncwarp();
-                while (nh >= 32) {
-                    float s0, s1, s2;
-                    flush(32, s0, s1, s2);
-                    a0.add(s0);
-                    a1.add(s1);
-                    a2.add(s2);
-                    // the rest (at most 32 kU - 1 entries) moves down by 32
-                    const int rest = nh - 32;
-                    int e[kU];
-#pragma unroll
-                    for (int v = 0; v < kU; v++)
-                        e[v] = lane + 32 * v < rest ? hits[warp][32 + 32 * v + lane] : 0;
-                    __syncwarp();
-#pragma unroll
-                    for (int v = 0; v < kU; v++)
-                        if (lane + 32 * v < rest) hits[warp][32 * v + lane] = e[v];
-                    nh = rest;
-                    __syncwarp();
-                }
-            }
-            if (nh > 0) {
-                float s0, s1, s2;
-                flush(nh, s0, s1, s2);
-                a0.add(s0);
-                a1.add(s1);
-                a2.add(s2);
-            }
-            // sum the PR pair slots of each right-hand side
-            for (int o = RL; o < 32; o <<= 1) {
-                a0.add(shfl_xor(a0, o));
-                a1.add(shfl_xor(a1, o));
-                a2.add(shfl_xor(a2, o));
-            }
-            if (pp == 0 && rok) {
-                const float *fi = F + (size_t)ii * C + 3 * r;
-                if (with_self) {
-                    a0.add(self_c * fi[0]);
-                    a1.add(self_c * fi[1]);
-                    a2.add(self_c * fi[2]);
-                }
-                float *o = W + (size_t)ii * C + 3 * r;
-                o[0] = a0.value();
-                o[1] = a1.value();
-                o[2] = a2.value();
             }
         }
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 16) k_realspace(RealArgs<float> A) {
-    realspace_body(A, blockIdx.x);
+// W: lanes per right-hand side pair group of the many-right-hand-sides form (0: the
+// few-right-hand-sides form with RB right-hand sides per sweep).
+template <int W, int RB>
+__device__ __forceinline__ void real_body(const RealArgs<float> &A, int cell) {
+    if constexpr (W > 0) real_many<W>(A, cell);
+    else real_few<RB>(A, cell);
+}
+
+template <int W, int RB>
+__global__ void __launch_bounds__(kRsThreads, 10) k_realspace(RealArgs<float> A) {
+    real_body<W, RB>(A, blockIdx.x);
 }
 
 // Many systems in one persistent launch over their cells.
-__global__ void __launch_bounds__(kThreads, 16)
+template <int W, int RB>
+__global__ void __launch_bounds__(kRsThreads, 10)
 k_realspace_batch(const RealArgs<float> *__restrict__ sys, const int *__restrict__ prefix,
                   int nsys, int total) {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int k = batch_find(prefix, nsys, w);
-        realspace_body(sys[k], w - prefix[k]);
+        // (a copy: fields read through the list would be loaded again after every store)
+        const RealArgs<float> A = sys[k];
+        real_body<W, RB>(A, w - prefix[k]);
         __syncthreads();
+    }
+}
+
+struct Launch {
+    const RealArgs<float> *sys;  // batched: work list, prefix, systems, cells
+    const int *prefix;
+    int nsys, total;
+    cudaStream_t s;
+};
+
+template <int W, int RB>
+cudaError_t launch_form(const RealArgs<float> *one, const Launch &l) {
+    if (one) {
+        k_realspace<W, RB><<<l.total, kRsThreads, 0, l.s>>>(*one);
+        return cudaGetLastError();
+    }
+    auto kern = k_realspace_batch<W, RB>;
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRsThreads, 0);
+    const int grid = std::max(1, std::min(l.total, sms * std::max(per_sm, 1)));
+    kern<<<grid, kRsThreads, 0, l.s>>>(l.sys, l.prefix, l.nsys, l.total);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_any(const RealArgs<float> *one, int R, const Launch &l) {
+    if (l.total <= 0 || R <= 0) return cudaSuccess;
+    switch (R) {
+        case 1: return launch_form<0, 1>(one, l);
+        case 2: return launch_form<0, 2>(one, l);
+        case 3: return launch_form<0, 3>(one, l);
+        case 4: return launch_form<0, 4>(one, l);
+        default:
+            if (R <= 8) return launch_form<4, 0>(one, l);
+            if (R <= 16) return launch_form<8, 0>(one, l);
+            return launch_form<16, 0>(one, l);
     }
 }
 
@@ -389,7 +330,7 @@ double real_self_coeff(double xi, double a) {
 
 template <typename T>
 RealArgs<T> real_args(int nc, const int *cell_off, const int *cell_perm, const void *cpos,
-                      const T *F, int R, double L, double rc, double xi, double a, int with_self,
+                      const T *F, const T *F2, int R, double L, double rc, double xi, double a, int with_self,
                       const PairTable &tab, T *W) {
     RealArgs<T> A;
     A.nc = nc;
@@ -397,6 +338,7 @@ RealArgs<T> real_args(int nc, const int *cell_off, const int *cell_perm, const v
     A.cell_perm = cell_perm;
     A.cpos = cpos;
     A.F = F;
+    A.F2 = F2;
     A.W = W;
     A.R = R;
     A.with_self = with_self;
@@ -435,35 +377,26 @@ RealArgs<T> real_args(int nc, const int *cell_off, const int *cell_perm, const v
 
 template <>
 cudaError_t launch_realspace<float>(int nc, const int *cell_off, const int *cell_perm,
-                                    const void *cpos, const float *F, int R, double L, double rc,
-                                    double xi, double a, int with_self, const PairTable &tab,
-                                    float *W, cudaStream_t s) {
-    const int ncell = nc * nc * nc;
-    const RealArgs<float> A = real_args<float>(nc, cell_off, cell_perm, cpos, F, R, L, rc, xi, a,
-                                               with_self, tab, W);
-    k_realspace<<<ncell, kThreads, 0, s>>>(A);
-    return cudaGetLastError();
+                                    const void *cpos, const float *F, const float *F2, int R,
+                                    double L, double rc, double xi, double a, int with_self,
+                                    const PairTable &tab, float *W, cudaStream_t s) {
+    if (!F2) return cudaErrorInvalidValue;
+    const RealArgs<float> A = real_args<float>(nc, cell_off, cell_perm, cpos, F, F2, R, L, rc, xi,
+                                               a, with_self, tab, W);
+    return launch_any(&A, R, Launch{nullptr, nullptr, 0, nc * nc * nc, s});
 }
 
 template <>
 cudaError_t launch_realspace_batch<float>(const RealArgs<float> *sys, const int *prefix, int nsys,
-                                          int total, int, cudaStream_t s) {
-    if (total <= 0) return cudaSuccess;
-    auto kern = k_realspace_batch;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
-    const int grid = std::max(1, std::min(total, sms * std::max(per_sm, 1)));
-    kern<<<grid, kThreads, 0, s>>>(sys, prefix, nsys, total);
-    return cudaGetLastError();
+                                          int total, int R, cudaStream_t s) {
+    return launch_any(nullptr, R, Launch{sys, prefix, nsys, total, s});
 }
 
 template RealArgs<float> real_args<float>(int, const int *, const int *, const void *,
-                                          const float *, int, double, double, double, double, int,
-                                          const PairTable &, float *);
+                                          const float *, const float *, int, double, double,
+                                          double, double, int, const PairTable &, float *);
 template RealArgs<double> real_args<double>(int, const int *, const int *, const void *,
-                                            const double *, int, double, double, double, double,
-                                            int, const PairTable &, double *);
+                                            const double *, const double *, int, double, double,
+                                            double, double, int, const PairTable &, double *);
 
 }  // namespace spme

@@ -11,12 +11,10 @@
 //     those of its last round;
 //   * the pair functions come from a table in s = r^2 (PairTable): no square root
 //     and no division, the unit vector is folded in as G/r^2: 29 FP64 instructions
-//     per pair and right-hand side (geometry 6, segment offset 1, two cubic-sextic
-//     Horner chains 12, application 10);
-//   * the listed pairs are split evenly over the lanes (contiguous shares), which
-//     accumulate in registers; a particle's partial sums, one per share it
-//     touches, are added in list order: a fixed order on every run, and a few
-//     additions instead of a 5-step butterfly per particle.
+//     per pair and right-hand side (geometry 6, segment offset 1, two Horner chains
+//     of degree six 12, application 10);
+//   * the listed pairs are split evenly over the lanes (realspace_pairs.cuh), which
+//     accumulate in registers: no 5-step FP64 butterfly per particle.
 // N = 1e6, L = 480, rc = 10 (38 pairs per particle), one right-hand side:
 // 15.19 -> 3.30 ms; N = 1e5, L = 220: 1.645 -> 0.358 ms (FP64 pipe floor 2.0 ms: 36
 // FP64 warp instructions per particle at 16 cycles each).
@@ -25,18 +23,11 @@
 #include <cstring>
 #include <vector>
 
-#include "kernels.h"
+#include "realspace_pairs.cuh"
 
 namespace spme {
 
 namespace {
-
-constexpr int kThreads = 64;  // two warps per cell: ~4-5 particles each at typical densities
-constexpr int kWarps = kThreads / 32;
-constexpr int kCap = 512;    // candidates staged in shared memory per cell
-constexpr int kList = 512;   // listed pairs per warp
-constexpr int kGroup = 16;   // particles listed together (4 bits of a list entry)
-constexpr int kU = 2;        // candidates tested per lane per iteration
 
 // M_real(r) = F I + G rhat rhat: Beenakker's real-space form divided by a, and
 // for r < 2a plus (overlap RPY - far-field RPY), written in the cancellation-free
@@ -105,7 +96,8 @@ __device__ __forceinline__ void pair_AB(const PairTable &tb, double s, double xi
         // offset from the segment's centre: same exponent, so the difference is exact
         const double ctr = __hiloint2double((hw & ~((1 << tb.shift) - 1)) | (1 << (tb.shift - 1)), 0);
         const double v = s - ctr;
-        const double2 *c = reinterpret_cast<const double2 *>(tb.coef) + (size_t)seg * (kPairDeg + 1);
+        const double2 *c =
+            reinterpret_cast<const double2 *>(tb.coef) + (size_t)seg * (kPairDeg + 1);
         double2 q = __ldg(c + kPairDeg);
         Av = q.x;
         Bv = q.y;
@@ -125,283 +117,24 @@ __device__ __forceinline__ void pair_AB(const PairTable &tb, double s, double xi
 }
 
 template <int RB>
-struct WarpSh {
-    static constexpr int S = 3 * RB;
-    double first[32][S], last[32][S];  // a lane's first and last partial sum
-    double mid[kGroup][S];             // a particle wholly inside one lane's share
-    double res[kGroup][S];
-    double px[kGroup], py[kGroup], pz[kGroup];
-    float4 pf[kGroup];                 // FP32 position, particle id (bits)
-    uint32_t list[kList];              // particle (4 bits) | candidate
-    int beg[kGroup + 1];               // first entry of each particle
-};
-
-// One cell: a warp lists the pairs of up to kGroup of its particles and sums
-// them (RB right-hand sides per sweep).
-template <int RB>
 __device__ __forceinline__ void realspace64_body(const RealArgs<double> &A, int cell) {
-    constexpr int S = 3 * RB;
-    __shared__ int nb_beg[27], nb_pre[28], nnb;
-    __shared__ double nb_shift[27][3];
-    __shared__ float4 cf[kCap];  // staged candidates: FP32 position, particle id (bits)
-    __shared__ double cx[kCap], cy[kCap], cz[kCap];
-    __shared__ WarpSh<RB> wsh[kWarps];
-
-    const int nc = A.nc, C = 3 * A.R;
-    const double L = A.L, h = A.h;
-    const double4_32a *__restrict__ cpos = reinterpret_cast<const double4_32a *>(A.cpos);
-    const int *__restrict__ cell_perm = A.cell_perm;
-    const double *__restrict__ F = A.F;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ib0 = __ldg(A.cell_off + cell), ie = __ldg(A.cell_off + cell + 1);
-    if (ib0 == ie) return;  // uniform over the block
-    // neighbour table: lane k of warp 0 takes neighbour cell k (27 of them, or the
-    // cell alone when nc < 3), candidate offsets by a warp scan
-    if (warp == 0) {
-        const int ccx = cell % nc, ccy = (cell / nc) % nc, ccz = cell / (nc * nc);
-        const int nk = nc >= 3 ? 27 : 1;
-        int cnt = 0;
-        if (lane < nk) {
-            const int dx = nk == 1 ? 0 : lane % 3 - 1, dy = nk == 1 ? 0 : (lane / 3) % 3 - 1,
-                      dz = nk == 1 ? 0 : lane / 9 - 1;
-            auto wrap = [nc](int v) { return v < 0 ? v + nc : (v >= nc ? v - nc : v); };
-            const int c2 = (wrap(ccz + dz) * nc + wrap(ccy + dy)) * nc + wrap(ccx + dx);
-            const int b = __ldg(A.cell_off + c2);
-            cnt = __ldg(A.cell_off + c2 + 1) - b;
-            nb_beg[lane] = b;
-            nb_shift[lane][0] = dx * h;
-            nb_shift[lane][1] = dy * h;
-            nb_shift[lane][2] = dz * h;
-        }
-        int inc = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += t;
-        }
-        if (lane < nk) nb_pre[lane] = inc - cnt;
-        if (lane == nk - 1) {
-            nb_pre[nk] = inc;
-            nnb = nk;
-        }
-    }
-    __syncthreads();
-    const int ncand = nb_pre[nnb];
-    const bool staged = ncand <= kCap;
-    // neighbour k holding candidate q: nb_pre[k] <= q < nb_pre[k + 1]
-    auto find_nb = [&](int q) {
-        int lo = 0, hi = nnb;
-        while (hi - lo > 1) {
-            const int m = (lo + hi) >> 1;
-            if (nb_pre[m] <= q) lo = m; else hi = m;
-        }
-        return lo;
-    };
-    if (staged) {
-        for (int q = tid; q < ncand; q += kThreads) {
-            const int k = find_nb(q);
-            const int js = nb_beg[k] + (q - nb_pre[k]);
-            const double4_32a p = cpos[js];
-            const double x = p.x + nb_shift[k][0], y = p.y + nb_shift[k][1],
-                         z = p.z + nb_shift[k][2];
-            cx[q] = x;
-            cy[q] = y;
-            cz[q] = z;
-            cf[q] = make_float4((float)x, (float)y, (float)z, __int_as_float(cell_perm[js]));
-        }
-    }
-    __syncthreads();
-    // candidate q in the frame of this cell
-    auto candidate = [&](int q, double &x, double &y, double &z, int &j) {
-        if (staged) {
-            x = cx[q];
-            y = cy[q];
-            z = cz[q];
-            j = __float_as_int(cf[q].w);
-        } else {
-            const int k = find_nb(q);
-            const int js = nb_beg[k] + (q - nb_pre[k]);
-            const double4_32a p = cpos[js];
-            x = p.x + nb_shift[k][0];
-            y = p.y + nb_shift[k][1];
-            z = p.z + nb_shift[k][2];
-            j = cell_perm[js];
-        }
-    };
-    // The FP32 test accepts a superset of the pairs within rc: coordinates lie
-    // within 3 cells (one cell of edge L: within L, minimum image), so FP32
-    // rounding moves d^2 by far less than the margin.
-    const bool single = nc < 3;
-    const float pre_r2 = (float)(A.rc2 * 1.0001 + 9e-5 * h * h);
-    const float Lf = (float)L, iLf = 1.f / Lf;
-    const double invL = 1.0 / L;
     const long long rc2_bits = __double_as_longlong(A.rc2);
-    const unsigned below = (1u << lane) - 1u;
-    WarpSh<RB> &ws = wsh[warp];
-
-    // this warp's share of the cell's particles, kGroup at a time
-    const int half = (ie - ib0 + kWarps - 1) / kWarps;
-    const int wb = ib0 + warp * half, we = min(ie, wb + half);
-    for (int g0 = wb; g0 < we; g0 += kGroup) {
-        const int np = min(kGroup, we - g0);
-        if (lane < np) {
-            const double4_32a p = cpos[g0 + lane];
-            ws.px[lane] = p.x;
-            ws.py[lane] = p.y;
-            ws.pz[lane] = p.z;
-            ws.pf[lane] = make_float4((float)p.x, (float)p.y, (float)p.z,
-                                      __int_as_float(cell_perm[g0 + lane]));
-        }
-        for (int r0 = 0; r0 < A.R; r0 += RB) {
-            for (int t = lane; t < np * S; t += 32) ws.res[t / S][t % S] = 0.0;
-            if (lane == 0) ws.beg[0] = 0;
-            __syncwarp();
-            float4 me = ws.pf[0];
-            int il = 0, q0 = 0, nh = 0, ilo = 0;
-            while (true) {
-                // list pairs (particle, candidate) while a test's hits are sure to fit
-                while (il < np && nh <= kList - 32 * kU) {
-                    bool hit[kU];
-#pragma unroll
-                    for (int v = 0; v < kU; v++) {
-                        const int q = q0 + 32 * v + lane;
-                        hit[v] = false;
-                        if (q < ncand) {
-                            float4 c;
-                            if (staged) {
-                                c = cf[q];
-                            } else {
-                                double x, y, z;
-                                int j;
-                                candidate(q, x, y, z, j);
-                                c = make_float4((float)x, (float)y, (float)z, __int_as_float(j));
-                            }
-                            float e0 = me.x - c.x, e1 = me.y - c.y, e2 = me.z - c.z;
-                            if (single) {
-                                e0 -= Lf * rintf(e0 * iLf);
-                                e1 -= Lf * rintf(e1 * iLf);
-                                e2 -= Lf * rintf(e2 * iLf);
-                            }
-                            hit[v] = e0 * e0 + e1 * e1 + e2 * e2 < pre_r2 &&
-                                     __float_as_int(c.w) != __float_as_int(me.w);
-                        }
-                    }
-#pragma unroll
-                    for (int v = 0; v < kU; v++) {
-                        const unsigned m = __ballot_sync(0xffffffffu, hit[v]);
-                        if (hit[v])
-                            ws.list[nh + __popc(m & below)] =
-                                (uint32_t)(q0 + 32 * v + lane) | ((uint32_t)il << 28);
-                        nh += __popc(m);
-                    }
-                    q0 += 32 * kU;
-                    if (q0 >= ncand) {
-                        q0 = 0;
-                        il++;
-                        if (il < np) me = ws.pf[il];
-                        if (lane == 0) ws.beg[il] = nh;
-                    }
-                }
-                if (il < np && lane == 0) ws.beg[il + 1] = nh;  // cut: this list's part ends here
-                __syncwarp();
-                // sum the listed pairs: lane's share [lane c, lane c + c)
-                const int c = (nh + 31) >> 5;
-                double acc[S];
-#pragma unroll
-                for (int k = 0; k < S; k++) acc[k] = 0.0;
-                int cur = -1, nseg = 0;
-                const int e1 = min(nh, lane * c + c);
-                for (int t = lane * c; t < e1; t++) {
-                    const uint32_t ent = ws.list[t];
-                    const int ip = (int)(ent >> 28);
-                    if (ip != cur) {
-                        if (cur >= 0) {
-                            double *dst = nseg == 0 ? ws.first[lane] : ws.mid[cur];
-#pragma unroll
-                            for (int k = 0; k < S; k++) dst[k] = acc[k];
-                            nseg++;
-#pragma unroll
-                            for (int k = 0; k < S; k++) acc[k] = 0.0;
-                        }
-                        cur = ip;
-                    }
-                    double x, y, z;
-                    int j;
-                    candidate((int)(ent & 0x0fffffffu), x, y, z, j);
-                    double d0 = ws.px[ip] - x, d1 = ws.py[ip] - y, d2 = ws.pz[ip] - z;
-                    if (single) {
-                        d0 -= L * rint(d0 * invL);
-                        d1 -= L * rint(d1 * invL);
-                        d2 -= L * rint(d2 * invL);
-                    }
-                    const double s = fma(d2, d2, fma(d1, d1, d0 * d0));
-                    if (__double_as_longlong(s) < rc2_bits) {
-                        double Av, Bv;
-                        pair_AB(A.tab, s, A.xi, A.a, Av, Bv);
-                        const double *fj = F + (size_t)j * C + 3 * r0;
-#pragma unroll
-                        for (int r = 0; r < RB; r++) {
-                            if (RB == 1 || r0 + r < A.R) {
-                                const double f0 = __ldg(fj + 3 * r), f1 = __ldg(fj + 3 * r + 1),
-                                             f2 = __ldg(fj + 3 * r + 2);
-                                const double g = Bv * fma(d2, f2, fma(d1, f1, d0 * f0));
-                                acc[3 * r] = fma(g, d0, fma(Av, f0, acc[3 * r]));
-                                acc[3 * r + 1] = fma(g, d1, fma(Av, f1, acc[3 * r + 1]));
-                                acc[3 * r + 2] = fma(g, d2, fma(Av, f2, acc[3 * r + 2]));
-                            }
-                        }
-                    }
-                }
-                if (cur >= 0) {
-                    double *dst = nseg == 0 ? ws.first[lane] : ws.last[lane];
-#pragma unroll
-                    for (int k = 0; k < S; k++) dst[k] = acc[k];
-                }
-                __syncwarp();
-                // a particle's partial sums in share order: a share's first partial sum
-                // when the particle's entries reach its start, its last when they reach
-                // its end, else the one in between
-                const int npl = min(il, np - 1) - ilo + 1;
-                for (int t = lane; t < npl * S; t += 32) {
-                    const int ip = ilo + t / S, k = t % S;
-                    const int b = ws.beg[ip], e = ws.beg[ip + 1];
-                    if (e <= b) continue;
-                    double sum = ws.res[ip][k];
-                    for (int l = b / c; l * c < e; l++) {
-                        const double v = b <= l * c ? ws.first[l][k]
-                                                    : (e >= min(nh, l * c + c) ? ws.last[l][k]
-                                                                               : ws.mid[ip][k]);
-                        sum += v;
-                    }
-                    ws.res[ip][k] = sum;
-                }
-                __syncwarp();
-                if (il >= np) break;
-                nh = 0;
-                ilo = il;
-                if (lane == 0) ws.beg[il] = 0;
-            }
-            for (int t = lane; t < np * S; t += 32) {
-                const int ip = t / S, k = t % S;
-                if (r0 + k / 3 < A.R) {
-                    const size_t at = (size_t)__float_as_int(ws.pf[ip].w) * C + 3 * r0 + k;
-                    const double v = ws.res[ip][k];
-                    A.W[at] = A.with_self ? fma(A.self_c, F[at], v) : v;
-                }
-            }
-            __syncwarp();
-        }
-    }
+    realspace_few_body<double, RB>(A, cell, A.L, A.h, A.rc2, A.self_c,
+                                   [&](double s, double &Av, double &Bv) {
+                                       if (__double_as_longlong(s) >= rc2_bits) return false;
+                                       pair_AB(A.tab, s, A.xi, A.a, Av, Bv);
+                                       return true;
+                                   });
 }
 
 template <int RB>
-__global__ void __launch_bounds__(kThreads, RB == 1 ? 7 : 4) k_realspace64(RealArgs<double> A) {
+__global__ void __launch_bounds__(kRsThreads, RB == 1 ? 7 : 4) k_realspace64(RealArgs<double> A) {
     realspace64_body<RB>(A, blockIdx.x);
 }
 
 // Many systems in one persistent launch over their cells.
 template <int RB>
-__global__ void __launch_bounds__(kThreads, RB == 1 ? 7 : 4)
+__global__ void __launch_bounds__(kRsThreads, RB == 1 ? 7 : 4)
 k_realspace64_batch(const RealArgs<double> *__restrict__ sys, const int *__restrict__ prefix,
                     int nsys, int total) {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
@@ -425,9 +158,9 @@ cudaError_t launch_batch64(const RealArgs<double> *sys, const int *prefix, int n
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRsThreads, 0);
     const int grid = std::max(1, std::min(total, sms * std::max(per_sm, 1)));
-    kern<<<grid, kThreads, 0, s>>>(sys, prefix, nsys, total);
+    kern<<<grid, kRsThreads, 0, s>>>(sys, prefix, nsys, total);
     return cudaGetLastError();
 }
 
@@ -435,18 +168,18 @@ cudaError_t launch_batch64(const RealArgs<double> *sys, const int *prefix, int n
 
 template <>
 cudaError_t launch_realspace<double>(int nc, const int *cell_off, const int *cell_perm,
-                                     const void *cpos, const double *F, int R, double L,
-                                     double rc, double xi, double a, int with_self,
+                                     const void *cpos, const double *F, const double *, int R,
+                                     double L, double rc, double xi, double a, int with_self,
                                      const PairTable &tab, double *W, cudaStream_t s) {
     if (R <= 0) return cudaSuccess;
-    const RealArgs<double> A = real_args<double>(nc, cell_off, cell_perm, cpos, F, R, L, rc, xi,
-                                                 a, with_self, tab, W);
+    const RealArgs<double> A = real_args<double>(nc, cell_off, cell_perm, cpos, F, nullptr, R, L, rc,
+                                                 xi, a, with_self, tab, W);
     const int ncell = nc * nc * nc;
     switch (sweep_width(R)) {
-        case 1: k_realspace64<1><<<ncell, kThreads, 0, s>>>(A); break;
-        case 2: k_realspace64<2><<<ncell, kThreads, 0, s>>>(A); break;
-        case 3: k_realspace64<3><<<ncell, kThreads, 0, s>>>(A); break;
-        default: k_realspace64<4><<<ncell, kThreads, 0, s>>>(A); break;
+        case 1: k_realspace64<1><<<ncell, kRsThreads, 0, s>>>(A); break;
+        case 2: k_realspace64<2><<<ncell, kRsThreads, 0, s>>>(A); break;
+        case 3: k_realspace64<3><<<ncell, kRsThreads, 0, s>>>(A); break;
+        default: k_realspace64<4><<<ncell, kRsThreads, 0, s>>>(A); break;
     }
     return cudaGetLastError();
 }
@@ -471,21 +204,30 @@ long long bits_of(double v) {
     return b;
 }
 
-// Polynomials (degree kPairDeg, in the offset from the segment's centre) of
-// A = F and B = G / s on [s0, s0 + h], interleaved, through the values at the
-// Chebyshev nodes.
+// Polynomials (degree kPairDeg, in the offset from the segment's centre) of A = F
+// and B = G / s on [s0, s0 + h], interleaved, through the values at the Chebyshev
+// nodes.
 void fit_segment(double s0, double h, double xi, double a, bool near, double *out) {
     constexpr int n = kPairDeg + 1;
+    static double node[n], cs[n][n];
+    static const bool once = [] {
+        for (int j = 0; j < n; j++) {
+            node[j] = std::cos(M_PI * (j + 0.5) / n);
+            for (int k = 0; k < n; k++) cs[k][j] = std::cos(M_PI * k * (j + 0.5) / n);
+        }
+        return true;
+    }();
+    (void)once;
     double f[2][n], c[2][n];
     for (int j = 0; j < n; j++) {
-        const double s = s0 + 0.5 * h * (std::cos(M_PI * (j + 0.5) / n) + 1.0);
+        const double s = s0 + 0.5 * h * (node[j] + 1.0);
         real_FG(std::sqrt(s), xi, a, near, f[0][j], f[1][j]);
         f[1][j] /= s;
     }
     for (int w = 0; w < 2; w++) {
         for (int k = 0; k < n; k++) {
             double q = 0.0;
-            for (int j = 0; j < n; j++) q += f[w][j] * std::cos(M_PI * k * (j + 0.5) / n);
+            for (int j = 0; j < n; j++) q += f[w][j] * cs[k][j];
             c[w][k] = (k ? 2.0 : 1.0) * q / n;
         }
         // Chebyshev to powers of t, then of the offset v = t h / 2
@@ -538,8 +280,8 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
             double *c = coef->data() + (size_t)q * (kPairDeg + 1) * 2;
             fit_segment(s0, h, xi, a, near, c);
             // the fit between the nodes, relative to the function scale there
-            for (int p = 0; p <= 16 && ok; p++) {
-                const double s = s0 + h * p / 16.0, v = s - (s0 + 0.5 * h);
+            for (int p = 0; p <= 8 && ok; p++) {
+                const double s = s0 + h * p / 8.0, v = s - (s0 + 0.5 * h);
                 if (s < lo || s > hi || (near != (s < mid))) continue;
                 double F, G;
                 real_FG(std::sqrt(s), xi, a, near, F, G);
