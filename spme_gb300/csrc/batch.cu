@@ -106,23 +106,30 @@ __device__ __forceinline__ void batch_record(const T *__restrict__ pfrac, int i,
     for (int j = 3 * P; j < ws; j++) out[j] = T(0);
 }
 
-// (records assembled in shared memory, written as one contiguous run)
+// (records assembled in shared memory, written as one contiguous run); blockIdx.y:
+// record set 0, 1, then the cell-relative positions in cell order
 constexpr int kRecThreads = 128;
 constexpr int kMaxWs = 24;  // record stride of order 8
 
 template <typename T>
 __global__ void __launch_bounds__(kRecThreads)
 k_batch_records(const uint32_t *__restrict__ pstart, const T *__restrict__ pfrac,
-                const int *__restrict__ perm, int n, const int *__restrict__ sysid,
-                const BatchGeo *__restrict__ geo, int ws, int *__restrict__ rec_idx,
-                uint32_t *__restrict__ rec_start, T *__restrict__ rec_w) {
+                RecordSet<T> set0, RecordSet<T> set1, int n, const int *__restrict__ sysid,
+                const BatchGeo *__restrict__ geo, int ws,
+                const typename V4T<T>::type *__restrict__ prel, const int *__restrict__ cperm,
+                typename V4T<T>::type *__restrict__ cpos) {
     __shared__ __align__(16) T sm[kRecThreads * kMaxWs];
     const int s0 = blockIdx.x * kRecThreads;
     const int s = s0 + threadIdx.x;
+    if (blockIdx.y == 2) {
+        if (s < n) cpos[s] = prel[cperm[s]];
+        return;
+    }
+    const RecordSet<T> set = blockIdx.y == 0 ? set0 : set1;
     if (s < n) {
-        const int i = perm[s];
-        rec_idx[s] = i;
-        rec_start[s] = pstart[i];
+        const int i = set.perm[s];
+        set.idx[s] = i;
+        set.start[s] = pstart[i];
         T *out = sm + (size_t)threadIdx.x * ws;
         switch (geo[sysid[i]].g.p) {
             case 4: batch_record<T, 4>(pfrac, i, ws, out); break;
@@ -133,7 +140,7 @@ k_batch_records(const uint32_t *__restrict__ pstart, const T *__restrict__ pfrac
     __syncthreads();
     const int cnt = min(kRecThreads, n - s0);
     const int vq = ws * (int)sizeof(T) / 16;
-    float4 *dst = reinterpret_cast<float4 *>(rec_w + (size_t)s0 * ws);
+    float4 *dst = reinterpret_cast<float4 *>(set.w + (size_t)s0 * ws);
     const float4 *src = reinterpret_cast<const float4 *>(sm);
     for (int v = threadIdx.x; v < cnt * vq; v += kRecThreads) dst[v] = src[v];
 }
@@ -419,11 +426,11 @@ struct _spme_batch_t {
     // device
     int *d_sysid = nullptr, *d_pref = nullptr;
     BatchGeo *d_geo = nullptr;
-    // d_sort_tmp: scratch of the three counting sorts (the atomic slots are kept
-    // in the sorts' permutation buffers until the scatter)
+    // d_sort_tmp: scratch of the three counting sorts (the atomic slots are kept in the
+    // sorts' permutation buffers until the scatter)
     int *d_key1 = nullptr, *d_key2 = nullptr, *d_key3 = nullptr, *d_sort_tmp = nullptr;
-    int *d_cnt1 = nullptr, *d_off1 = nullptr, *d_cnt2 = nullptr, *d_off2 = nullptr,
-        *d_cnt3 = nullptr, *d_off3 = nullptr, *d_scan_tmp = nullptr;
+    int *d_count = nullptr;  // the sorts' key counts: tiles, real-space cells, start cells
+    int *d_off1 = nullptr, *d_off2 = nullptr, *d_off3 = nullptr, *d_scan_tmp = nullptr;
     int *d_perm1 = nullptr, *d_perm2 = nullptr, *d_perm3 = nullptr;
     uint32_t *d_pstart = nullptr;
     void *d_pfrac = nullptr, *d_prel = nullptr, *d_cpos = nullptr;
@@ -538,12 +545,15 @@ int build_tiles(_spme_batch_t *b) {
         tile_ok = tile_ok && interp_tile_ok(x.g, sizeof(T));
     }
     if (!tile_ok) return SPME_ERR_UNSUPPORTED;
-    cudaFree(b->d_cnt1);
+    cudaFree(b->d_count);
     cudaFree(b->d_off1);
-    b->d_cnt1 = b->d_off1 = nullptr;
+    cudaFree(b->d_scan_tmp);
+    b->d_count = b->d_off1 = b->d_scan_tmp = nullptr;
     b->ntile_keys = off;
-    BTRY(balloc(&b->d_cnt1, sizeof(int) * off));
+    const long nkeys = (long)off + b->ncell_keys + b->nstart_keys;
+    BTRY(balloc(&b->d_count, sizeof(int) * nkeys));
     BTRY(balloc(&b->d_off1, sizeof(int) * (off + 1)));
+    BTRY(balloc(&b->d_scan_tmp, sizeof(int) * scan_tmp_elems(nkeys)));
     // systems ordered by p, one work list (and prefix) per order
     std::vector<int> order(b->nsys);
     for (int k = 0; k < b->nsys; k++) order[k] = k;
@@ -651,10 +661,8 @@ int create_t(_spme_batch_t *b) {
     BTRY(balloc(&b->d_key1, sizeof(int) * n));
     BTRY(balloc(&b->d_key2, sizeof(int) * n));
     BTRY(balloc(&b->d_key3, sizeof(int) * n));
-    BTRY(balloc(&b->d_sort_tmp, sizeof(int) * n));
-    BTRY(balloc(&b->d_cnt2, sizeof(int) * start));
+    BTRY(balloc(&b->d_sort_tmp, sizeof(int) * (size_t)n * kMaxSorts));
     BTRY(balloc(&b->d_off2, sizeof(int) * (start + 1)));
-    BTRY(balloc(&b->d_cnt3, sizeof(int) * cell));
     BTRY(balloc(&b->d_off3, sizeof(int) * (cell + 1)));
     BTRY(balloc(&b->d_perm1, sizeof(int) * n));
     BTRY(balloc(&b->d_perm2, sizeof(int) * n));
@@ -680,8 +688,6 @@ int create_t(_spme_batch_t *b) {
     BTRY(balloc(&b->d_tab, 2 * sizeof(T) * tab));
     BTRY(balloc(&b->d_err, sizeof(int)));
     BTRY_CUDA(cudaMemset(b->d_err, 0, sizeof(int)));
-    // (the tile keys, counted later, are never more than the stencil-start cells)
-    BTRY(balloc(&b->d_scan_tmp, sizeof(int) * scan_tmp_elems(std::max(start, cell))));
     BTRY(balloc(&b->d_spread_sys, sizeof(SpreadColsSys<T>) * ns));
     BTRY(balloc(&b->d_interp_sys, sizeof(InterpSys<T>) * ns));
     BTRY(balloc(&b->d_real_sys, sizeof(RealArgs<T>) * ns));
@@ -822,27 +828,26 @@ int positions_body(_spme_batch_t *b, const double *pos) {
     cudaStream_t s = b->stream;
     const int n = b->ntot;
     mark(b, 0);
-    BTRY_CUDA(cudaMemsetAsync(b->d_cnt1, 0, sizeof(int) * b->ntile_keys, s));
-    BTRY_CUDA(cudaMemsetAsync(b->d_cnt2, 0, sizeof(int) * b->nstart_keys, s));
-    BTRY_CUDA(cudaMemsetAsync(b->d_cnt3, 0, sizeof(int) * b->ncell_keys, s));
+    // first keys of the sorts
+    const long t0 = 0, c0 = b->ntile_keys, s0 = c0 + b->ncell_keys;
+    BTRY_CUDA(cudaMemsetAsync(b->d_count, 0, sizeof(int) * (size_t)(s0 + b->nstart_keys), s));
     k_batch_keys<T><<<nblk(n, 256), 256, 0, s>>>(
-        pos, n, b->d_sysid, b->d_geo, b->d_key1, b->d_cnt1, b->d_perm1, b->d_key2, b->d_cnt2,
-        b->d_perm2, b->d_key3, b->d_cnt3, b->d_perm3, b->d_pstart, (T *)b->d_pfrac,
-        (typename V4T<T>::type *)b->d_prel);
-    launch_scan(b->d_cnt1, b->ntile_keys, b->d_off1, b->d_scan_tmp, s);
-    launch_scatter(b->d_key1, b->d_off1, n, b->d_perm1, b->d_sort_tmp, s);
-    launch_scan(b->d_cnt2, b->nstart_keys, b->d_off2, b->d_scan_tmp, s);
-    launch_scatter(b->d_key2, b->d_off2, n, b->d_perm2, b->d_sort_tmp, s);
-    launch_scan(b->d_cnt3, b->ncell_keys, b->d_off3, b->d_scan_tmp, s);
-    launch_scatter(b->d_key3, b->d_off3, n, b->d_perm3, b->d_sort_tmp, s);
-    k_batch_records<T><<<nblk(n, kRecThreads), kRecThreads, 0, s>>>(b->d_pstart, (const T *)b->d_pfrac,
-                                                    b->d_perm1, n, b->d_sysid, b->d_geo, b->ws,
-                                                    b->d_ridx1, b->d_rst1, (T *)b->d_rw1);
-    k_batch_records<T><<<nblk(n, kRecThreads), kRecThreads, 0, s>>>(b->d_pstart, (const T *)b->d_pfrac,
-                                                    b->d_perm2, n, b->d_sysid, b->d_geo, b->ws,
-                                                    b->d_ridx2, b->d_rst2, (T *)b->d_rw2);
-    launch_cell_gather(b->d_prel, b->d_perm3, n, sizeof(T) == 4, b->d_cpos, s);
-    b->launches += 1 + 3 * 3 + 3 * 2 + 2 + 1;
+        pos, n, b->d_sysid, b->d_geo, b->d_key1, b->d_count + t0, b->d_perm1, b->d_key2,
+        b->d_count + s0, b->d_perm2, b->d_key3, b->d_count + c0, b->d_perm3, b->d_pstart,
+        (T *)b->d_pfrac, (typename V4T<T>::type *)b->d_prel);
+    Sorts sorts{};
+    sorts.s[0] = Sort{b->d_key1, b->d_perm1, b->d_off1, t0, b->ntile_keys};
+    sorts.s[1] = Sort{b->d_key3, b->d_perm3, b->d_off3, c0, b->ncell_keys};
+    sorts.s[2] = Sort{b->d_key2, b->d_perm2, b->d_off2, s0, b->nstart_keys};
+    sorts.count = 3;
+    const int nl = launch_sorts(sorts, b->d_count, n, b->d_scan_tmp, b->d_sort_tmp, s);
+    const RecordSet<T> set1{b->d_perm1, b->d_ridx1, b->d_rst1, (T *)b->d_rw1},
+        set2{b->d_perm2, b->d_ridx2, b->d_rst2, (T *)b->d_rw2};
+    k_batch_records<T><<<dim3(nblk(n, kRecThreads), 3), kRecThreads, 0, s>>>(
+        b->d_pstart, (const T *)b->d_pfrac, set1, set2, n, b->d_sysid, b->d_geo, b->ws,
+        (const typename V4T<T>::type *)b->d_prel, b->d_perm3,
+        (typename V4T<T>::type *)b->d_cpos);
+    b->launches += 2 + nl;
     return from_cuda(cudaGetLastError());
 }
 
@@ -963,8 +968,8 @@ void destroy_b(_spme_batch_t *b) {
         if (g.bwd) cufftDestroy(g.bwd);
     }
     void *bufs[] = {b->d_sysid, b->d_pref,  b->d_geo,   b->d_key1,  b->d_key2,
-                    b->d_key3,  b->d_sort_tmp, b->d_cnt1,  b->d_off1,  b->d_cnt2,
-                    b->d_off2,  b->d_cnt3,  b->d_off3,  b->d_scan_tmp, b->d_perm1, b->d_perm2,
+                    b->d_key3,  b->d_sort_tmp, b->d_count, b->d_off1,
+                    b->d_off2,  b->d_off3,  b->d_scan_tmp, b->d_perm1, b->d_perm2,
                     b->d_perm3, b->d_pstart, b->d_pfrac, b->d_prel, b->d_cpos,  b->d_ridx1,
                     b->d_ridx2, b->d_rst1,  b->d_rst2,  b->d_rw1,   b->d_rw2,   b->d_F,
                     b->d_Fs,    b->d_F2,    b->d_W,     b->d_W2,    b->d_mesh,  b->d_spec,  b->d_tab,

@@ -38,22 +38,30 @@ __host__ __device__ inline int pmod(int x, int m) {
 // Cox-de Boor recursion M_n(x) = [x M_{n-1}(x) + (n - x) M_{n-1}(x-1)]/(n-1),
 // the same polynomials the reference tabulates in monomial form
 // (old-version/spme.c:25-40, evaluated at :258-279).
+// The factors 1/(n - 1) are collected into one 1/(P - 1)! at the end (FP64 work:
+// 44 instead of 85 instructions per axis at P = 6).
 template <typename T, int P>
 __device__ __forceinline__ void bspline_weights(T w, T (&out)[P]) {
-    T a[P];
+    T a[P], up[P], dn[P];  // up[k] = w + k, dn[k] = k - w
+#pragma unroll
+    for (int k = 1; k < P; k++) {
+        up[k] = w + T(k);
+        dn[k] = T(k) - w;
+    }
     a[0] = w;
-    a[1] = T(1) - w;
+    a[1] = dn[1];
+    T f = T(1);
 #pragma unroll
     for (int n = 3; n <= P; n++) {
-        const T inv = T(1) / T(n - 1);
-        a[n - 1] = T(0);
+        f *= T(n - 1);
+        a[n - 1] = dn[1] * a[n - 2];
 #pragma unroll
-        for (int k = n - 1; k >= 1; k--)
-            a[k] = ((w + T(k)) * a[k] + (T(n) - w - T(k)) * a[k - 1]) * inv;
-        a[0] = w * a[0] * inv;
+        for (int k = n - 2; k >= 1; k--) a[k] = up[k] * a[k] + dn[n - k] * a[k - 1];
+        a[0] = w * a[0];
     }
+    const T inv = T(1) / f;
 #pragma unroll
-    for (int k = 0; k < P; k++) out[k] = a[P - 1 - k];
+    for (int k = 0; k < P; k++) out[k] = a[P - 1 - k] * inv;
 }
 
 // Fractional mesh coordinate of position x (wrapped into [0, L)), following

@@ -124,13 +124,15 @@ struct _spme_t {
     int nc = 1;
     bool have_pos = false;
     // device buffers
-    double *d_pos = nullptr;
+    double *d_pos = nullptr;  // host positions staged on the device
     int *d_key2 = nullptr, *d_key3 = nullptr;
     uint32_t *d_pstart = nullptr;  // per-particle stencil start (mesh engines)
     void *d_pfrac = nullptr;       // per-particle fractional mesh coordinates
-    // d_sort_tmp: scratch of the three counting sorts (the atomic slots are kept
-    // in the sorts' permutation buffers until the scatter)
-    int *d_key = nullptr, *d_sort_tmp = nullptr, *d_tcount = nullptr, *d_toff = nullptr,
+    // d_count: the counting sorts' key counts, one after the other; d_sort_tmp: their
+    // scratch (the atomic slots are kept in the sorts' permutation buffers until the
+    // scatter)
+    int *d_count = nullptr;
+    int *d_key = nullptr, *d_sort_tmp = nullptr, *d_toff = nullptr,
         *d_tperm = nullptr, *d_scan_tmp = nullptr;
     int *d_rec_idx = nullptr;
     uint32_t *d_rec_start = nullptr;
@@ -148,11 +150,11 @@ struct _spme_t {
     spme::BoxTable boxtab;
     int boxtab_tile[3] = {0, 0, 0};
     int spread_mode = 1;  // 1: box or column-gather kernel where they apply, 0: tile kernel
-    int *d_scount = nullptr, *d_soff = nullptr, *d_sperm = nullptr, *d_srec_idx = nullptr;
+    int *d_soff = nullptr, *d_sperm = nullptr, *d_srec_idx = nullptr;
     uint32_t *d_srec_start = nullptr;
     void *d_srec_w = nullptr;
     void *d_Fs = nullptr;  // force rows in start-cell order
-    int *d_ccount = nullptr, *d_coff = nullptr, *d_cperm = nullptr;
+    int *d_coff = nullptr, *d_cperm = nullptr;
     void *d_cpos = nullptr;  // float4 (FP32 engine) or double4_32a (FP64 engine)
     void *d_prel = nullptr;  // the same in particle order (from the keys pass)
     void *d_pair = nullptr;  // table of the pair functions (FP64 engines)
@@ -341,17 +343,16 @@ void alloc_box(spme_t *e) {
 int alloc_tiles(spme_t *e) {
     alloc_box(e);
     size_t need = (size_t)e->ntiles;
-    if (need <= e->cap_tiles && e->d_tcount) return SPME_OK;
-    dfree(e->d_tcount);
+    if (need <= e->cap_tiles && e->d_count) return SPME_OK;
+    dfree(e->d_count);
     dfree(e->d_toff);
     dfree(e->d_scan_tmp);
-    e->d_tcount = e->d_toff = e->d_scan_tmp = nullptr;
-    size_t ncell = (size_t)e->nc * e->nc * e->nc;
-    size_t nkeys = std::max(need, ncell);
-    if (e->cols) nkeys = std::max(nkeys, (size_t)e->prm.dim * e->prm.dim * e->prm.dim);
-    TRY(dalloc(&e->d_tcount, sizeof(int) * need));
+    e->d_count = e->d_toff = e->d_scan_tmp = nullptr;
+    const size_t K = e->prm.dim;
+    const size_t nkeys = need + (size_t)e->nc * e->nc * e->nc + (e->cols ? K * K * K : 0);
+    TRY(dalloc(&e->d_count, sizeof(int) * nkeys));
     TRY(dalloc(&e->d_toff, sizeof(int) * (need + 1)));
-    TRY(dalloc(&e->d_scan_tmp, sizeof(int) * spme::scan_tmp_elems((int)nkeys)));
+    TRY(dalloc(&e->d_scan_tmp, sizeof(int) * spme::scan_tmp_elems((long)nkeys)));
     e->cap_tiles = need;
     return SPME_OK;
 }
@@ -545,7 +546,7 @@ int create_impl(const spme_params &prm, spme_t **out) {
     const size_t C = (size_t)e->Cmax;
     TRY(dalloc(&e->d_pos, sizeof(double) * 3 * n));
     TRY(dalloc(&e->d_key, sizeof(int) * n));
-    TRY(dalloc(&e->d_sort_tmp, sizeof(int) * n));
+    TRY(dalloc(&e->d_sort_tmp, sizeof(int) * n * spme::kMaxSorts));
     TRY(dalloc(&e->d_key3, sizeof(int) * n));
     TRY(dalloc(&e->d_tperm, sizeof(int) * n));
     if (prm.terms & SPME_TERM_RECIP) {
@@ -560,7 +561,6 @@ int create_impl(const spme_params &prm, spme_t **out) {
     e->cols = e->cols_fit && !e->box && (e->elem == 8 || C >= 9);
     if (e->cols) {
         const size_t K3 = K * K * K;
-        TRY(dalloc(&e->d_scount, sizeof(int) * K3));
         TRY(dalloc(&e->d_soff, sizeof(int) * (K3 + 1)));
         TRY(dalloc(&e->d_sperm, sizeof(int) * n));
         TRY(dalloc(&e->d_key2, sizeof(int) * n));
@@ -575,7 +575,6 @@ int create_impl(const spme_params &prm, spme_t **out) {
     TRY(dalloc(&e->d_rec_w, e->elem * record_width(e) * n));
     if (prm.terms & SPME_TERM_REAL) {
         size_t ncell = (size_t)e->nc * e->nc * e->nc;
-        TRY(dalloc(&e->d_ccount, sizeof(int) * ncell));
         TRY(dalloc(&e->d_coff, sizeof(int) * (ncell + 1)));
         TRY(dalloc(&e->d_cperm, sizeof(int) * n));
         TRY(dalloc(&e->d_cpos, sizeof(double4_32a) * n));
@@ -730,12 +729,12 @@ void destroy_impl(spme_t *e) {
             cufftDestroy(p.bwd2);
         }
     }
-    void *bufs[] = {e->d_pos,    e->d_key,     e->d_sort_tmp, e->d_tcount,   e->d_toff,
+    void *bufs[] = {e->d_pos,    e->d_key,     e->d_sort_tmp, e->d_count,   e->d_toff,
                     e->d_tperm,  e->d_scan_tmp, e->d_rec_idx, e->d_rec_start, e->d_rec_w,
-                    e->d_ccount, e->d_coff,    e->d_cperm, e->d_cpos,     e->d_prel, e->d_mesh,
+                    e->d_coff,    e->d_cperm, e->d_cpos,     e->d_prel, e->d_mesh,
                     e->d_cmesh,  e->d_tab,     e->d_bmod2, e->d_work,     e->d_F,
                     e->d_W,      e->d_fstage,  e->d_ustage, e->d_err,  e->d_ztw,
-                    e->d_zip,    e->d_f2tab,    e->d_scount,  e->d_soff,   e->d_sperm, e->d_srec_idx,
+                    e->d_zip,    e->d_f2tab,    e->d_soff,   e->d_sperm, e->d_srec_idx,
                     e->d_srec_start, e->d_srec_w, e->d_Fs, e->d_W2, e->d_pair, e->d_key2,
                     e->d_key3,   e->d_pstart, e->d_pfrac, e->d_box,
                     e->d_boxtab, e->d_F2};
@@ -759,65 +758,57 @@ void destroy_impl(spme_t *e) {
     delete e;
 }
 
+template <typename T>
+void build_records(spme_t *e, bool recip, bool cols, bool real) {
+    spme::RecordSet<T> sets[2];
+    int nset = 0;
+    if (recip) sets[nset++] = {e->d_tperm, e->d_rec_idx, e->d_rec_start, (T *)e->d_rec_w};
+    if (cols) sets[nset++] = {e->d_sperm, e->d_srec_idx, e->d_srec_start, (T *)e->d_srec_w};
+    spme::launch_records<T>(e->d_pstart, (const T *)e->d_pfrac, e->prm.np, e->g.p, nset, sets,
+                            e->d_prel, e->d_cperm, real ? e->d_cpos : nullptr, e->stream);
+    e->launches++;
+}
+
+// One pass over the positions for every key this engine sorts by, then all its
+// counting sorts together, then its record sets and cell positions: 6 to 8
+// kernels and a memset (each sort and record set on its own took 22 kernels, which
+// bound small systems: FP64 N = 300, K = 32 0.110 -> 0.030 ms; FP32 N = 1e5, K = 128,
+// R = 1 0.129 -> 0.054 ms).
 int set_positions_body(spme_t *e, const double *pos, int mem) {
     const int n = e->prm.np;
     cudaStream_t s = e->stream;
     if (n > 0) {
         if (!pos) return SPME_ERR_INVALID;
-        TRY_CUDA(cudaMemcpyAsync(e->d_pos, pos, sizeof(double) * 3 * n,
-                                 mem == SPME_MEM_HOST ? cudaMemcpyHostToDevice
-                                                      : cudaMemcpyDeviceToDevice,
-                                 s));
+        if (mem == SPME_MEM_HOST) {
+            TRY_CUDA(cudaMemcpyAsync(e->d_pos, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
+            pos = e->d_pos;
+        }
     }
     const bool recip = (e->prm.terms & SPME_TERM_RECIP) != 0;  // geometry set by the caller
     const bool real = (e->prm.terms & SPME_TERM_REAL) != 0;
     const bool cols = recip && e->cols;
     const int ncell = e->nc * e->nc * e->nc;
     const int K3 = e->g.K * e->g.K * e->g.K;
-    if (recip) TRY_CUDA(cudaMemsetAsync(e->d_tcount, 0, sizeof(int) * e->ntiles, s));
-    if (cols) TRY_CUDA(cudaMemsetAsync(e->d_scount, 0, sizeof(int) * K3, s));
-    if (real) TRY_CUDA(cudaMemsetAsync(e->d_ccount, 0, sizeof(int) * ncell, s));
-    if (recip || real) {
-        // one pass over the positions for every key this engine sorts by
-        spme::launch_all_keys(e->d_pos, n, e->g, e->nc, e->d_key, recip ? e->d_tcount : nullptr,
-                              e->d_tperm, e->d_key2, cols ? e->d_scount : nullptr, e->d_sperm,
-                              e->d_key3, real ? e->d_ccount : nullptr, e->d_cperm,
-                              recip ? e->d_pstart : nullptr, e->d_pfrac,
-                              real ? e->d_prel : nullptr, is_fp32(e), s);
-        e->launches++;
-    }
-    if (recip) {
-        spme::launch_scan(e->d_tcount, e->ntiles, e->d_toff, e->d_scan_tmp, s);
-        spme::launch_scatter(e->d_key, e->d_toff, n, e->d_tperm, e->d_sort_tmp, s);
-        if (is_fp32(e))
-            spme::launch_records<float>(e->d_pstart, (const float *)e->d_pfrac, e->d_tperm, n,
-                                        e->g.p, e->d_rec_idx, e->d_rec_start,
-                                        (float *)e->d_rec_w, s);
-        else
-            spme::launch_records<double>(e->d_pstart, (const double *)e->d_pfrac, e->d_tperm, n,
-                                         e->g.p, e->d_rec_idx, e->d_rec_start,
-                                         (double *)e->d_rec_w, s);
-        e->launches += 6;
-    }
-    if (cols) {
-        spme::launch_scan(e->d_scount, K3, e->d_soff, e->d_scan_tmp, s);
-        spme::launch_scatter(e->d_key2, e->d_soff, n, e->d_sperm, e->d_sort_tmp, s);
-        if (is_fp32(e))
-            spme::launch_records<float>(e->d_pstart, (const float *)e->d_pfrac, e->d_sperm, n,
-                                        e->g.p, e->d_srec_idx, e->d_srec_start,
-                                        (float *)e->d_srec_w, s);
-        else
-            spme::launch_records<double>(e->d_pstart, (const double *)e->d_pfrac, e->d_sperm, n,
-                                         e->g.p, e->d_srec_idx, e->d_srec_start,
-                                         (double *)e->d_srec_w, s);
-        e->launches += 6;
-    }
-    if (real) {
-        spme::launch_scan(e->d_ccount, ncell, e->d_coff, e->d_scan_tmp, s);
-        spme::launch_scatter(e->d_key3, e->d_coff, n, e->d_cperm, e->d_sort_tmp, s);
-        spme::launch_cell_gather(e->d_prel, e->d_cperm, n, is_fp32(e), e->d_cpos, s);
-        e->launches += 6;
-    }
+    spme::Sorts sorts{};
+    long nkeys = 0;
+    auto add = [&](const int *key, int *perm, int *off, int keys) {
+        sorts.s[sorts.count++] = spme::Sort{key, perm, off, nkeys, keys};
+        int *count = e->d_count + nkeys;
+        nkeys += keys;
+        return count;
+    };
+    int *tcount = recip ? add(e->d_key, e->d_tperm, e->d_toff, e->ntiles) : nullptr;
+    int *ccount = real ? add(e->d_key3, e->d_cperm, e->d_coff, ncell) : nullptr;
+    int *scount = cols ? add(e->d_key2, e->d_sperm, e->d_soff, K3) : nullptr;
+    if (sorts.count == 0) return SPME_OK;
+    TRY_CUDA(cudaMemsetAsync(e->d_count, 0, sizeof(int) * (size_t)nkeys, s));
+    spme::launch_all_keys(pos, n, e->g, e->nc, e->d_key, tcount, e->d_tperm, e->d_key2, scount,
+                          e->d_sperm, e->d_key3, ccount, e->d_cperm,
+                          recip ? e->d_pstart : nullptr, e->d_pfrac, real ? e->d_prel : nullptr,
+                          is_fp32(e), s);
+    e->launches += 1 + spme::launch_sorts(sorts, e->d_count, n, e->d_scan_tmp, e->d_sort_tmp, s);
+    if (is_fp32(e)) build_records<float>(e, recip, cols, real);
+    else build_records<double>(e, recip, cols, real);
     TRY_CUDA(cudaGetLastError());
     return SPME_OK;
 }

@@ -24,27 +24,45 @@ void launch_all_keys(const double *pos, int n, const MeshGeom &g, int nc, int *k
                      int *slot1, int *key2, int *count2, int *slot2, int *key3, int *count3,
                      int *slot3, uint32_t *pstart, void *pfrac, void *prel, bool fp32,
                      cudaStream_t s);
-// cpos[s] = prel[perm[s]] (float4 or double4_32a): cell-relative positions in cell order.
-void launch_cell_gather(const void *prel, const int *perm, int n, bool fp32, void *cpos,
-                        cudaStream_t s);
 // Real-space cell key (nc^3 cells of edge L/nc) and slot within its cell.
 void launch_cell_keys(const double *pos, int n, double L, int nc, int *key, int *count,
                       int *slot, cudaStream_t s);
-// Exclusive scan of count[0..nkeys) into off[0..nkeys] (off[nkeys] = total).
-// tmp must hold scan_tmp_elems(nkeys) ints.
-size_t scan_tmp_elems(int nkeys);
-void launch_scan(const int *count, int nkeys, int *off, int *tmp, cudaStream_t s);
-// Counting-sort scatter.  On entry perm[i] is particle i's slot within its key
-// (from the atomic counts, in no fixed order); on return perm[off[k] ..
-// off[k + 1]) lists key k's particles in increasing index.  tmp: n ints.
-void launch_scatter(const int *key, const int *off, int n, int *perm, int *tmp,
-                    cudaStream_t s);
-// B-spline records in sorted order (perm): rec_idx[s] = perm[s], the packed
-// stencil start, and p weights per axis (record width RecordWidth<T,P>), from
-// launch_all_keys' per-particle starts and fractional coordinates.
+// Up to kMaxSorts counting sorts of the same n particles together (one launch for
+// all of them per stage).  Sort j's counts are count[first .. first + nkeys) (first
+// = the keys of the sorts before it); key[i] is particle i's key.  On entry perm[i]
+// is particle i's slot within its key (from the atomic counts, in no fixed order);
+// on return off[0 .. nkeys] holds the keys' offsets and perm[off[k] .. off[k + 1])
+// lists key k's particles in increasing index.  scan_tmp: scan_tmp_elems(all keys)
+// ints; tmp: n ints per sort.  Returns the kernels launched.
+constexpr int kMaxSorts = 3;
+struct Sort {
+    const int *key;
+    int *perm, *off;
+    long first;
+    int nkeys;
+};
+struct Sorts {
+    Sort s[kMaxSorts];
+    int count;
+};
+size_t scan_tmp_elems(long nkeys);
+int launch_sorts(const Sorts &S, const int *count, int n, int *scan_tmp, int *tmp, cudaStream_t s);
+// One set of B-spline records in sorted order (perm): idx[s] = perm[s], the packed
+// stencil start, and p weights per axis (record width RecordWidth<T,P>).
 template <typename T>
-void launch_records(const uint32_t *pstart, const T *pfrac, const int *perm, int n, int p,
-                    int *rec_idx, uint32_t *rec_start, T *rec_w, cudaStream_t s);
+struct RecordSet {
+    const int *perm;
+    int *idx;
+    uint32_t *start;
+    T *w;
+};
+// Up to two record sets from launch_all_keys' per-particle starts and fractional
+// coordinates and, if cpos is not null, the cell-relative positions in cell order,
+// cpos[s] = prel[cperm[s]] (float4 or double4_32a), in one launch.
+template <typename T>
+void launch_records(const uint32_t *pstart, const T *pfrac, int n, int p, int nset,
+                    const RecordSet<T> *sets, const void *prel, const int *cperm, void *cpos,
+                    cudaStream_t s);
 // Cell-sorted positions relative to their cell's lower corner (float4 or double4_32a).
 void launch_cell_positions(const double *pos, const int *perm, int n, double L, int nc,
                            bool fp32, void *cpos, cudaStream_t s);

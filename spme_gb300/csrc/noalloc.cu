@@ -115,8 +115,10 @@ extern "C" int spme_realspace_apply_noalloc(int np, const double *pos, double bo
         return SPME_ERR_CUDA;
     }
     spme::launch_cell_keys(pos, np, box_size, (int)nc, key, count, perm, s);
-    spme::launch_scan(count, ncell, off, tmp, s);
-    spme::launch_scatter(key, off, np, perm, slot, s);
+    spme::Sorts sorts{};
+    sorts.s[0] = spme::Sort{key, perm, off, 0, ncell};
+    sorts.count = 1;
+    spme::launch_sorts(sorts, count, np, tmp, slot, s);
     spme::launch_cell_positions(pos, perm, np, box_size, (int)nc, false, cpos, s);
     spme::launch_pack<double>(f, ldf, np, nrhs, F, s);
     if (spme::launch_realspace<double>((int)nc, off, perm, cpos, F, nullptr, nrhs, box_size, rcut,

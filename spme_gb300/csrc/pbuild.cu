@@ -1,6 +1,8 @@
 // P-build: stencil starts, tile / cell keys, counting sorts and B-spline
 // records (restates old-version/spme.c:158-297 in factored form: p weights per
 // axis instead of the dense p^3 P matrix and index list).
+#include <climits>
+
 #include "kernels.h"
 
 namespace spme {
@@ -162,56 +164,105 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(int *__restrict__ su
     }
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_final(const int *__restrict__ in, int n,
-                                                            const int *__restrict__ sums,
-                                                            int *__restrict__ out) {
+// The sorts' counts lie one after the other and each adds up to n, so one scan
+// serves them all: key q of the concatenation belongs to the last sort j whose
+// keys start at or before q, and its offset is the scan's value - j n.
+__device__ __forceinline__ void put_offset(const Sorts &S, int q, int ex, int n) {
+    int j = 0, first = 0;
+#pragma unroll
+    for (int k = 1; k < kMaxSorts; k++)
+        if (k < S.count && q >= S.s[k].first) {
+            j = k;
+            first = (int)S.s[k].first;
+        }
+    S.s[j].off[q - first] = ex - j * n;
+}
+
+__device__ __forceinline__ void put_ends(const Sorts &S, int n) {
+    if ((int)threadIdx.x < S.count) {
+        const int j = threadIdx.x;
+        S.s[j].off[S.s[j].nkeys] = n;
+    }
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_final(const int *__restrict__ in, int total,
+                                                            const int *__restrict__ sums, Sorts S,
+                                                            int n) {
     long base = (long)blockIdx.x * kScanTile + (long)threadIdx.x * kScanItems;
     int v[kScanItems];
     int s = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        v[k] = base + k < n ? in[base + k] : 0;
+        v[k] = base + k < total ? in[base + k] : 0;
         s += v[k];
     }
-    int total;
-    int ex = block_exclusive_scan(s, total) + sums[blockIdx.x];
+    int all;
+    int ex = block_exclusive_scan(s, all) + sums[blockIdx.x];
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        if (base + k < n) out[base + k] = ex;
+        if (base + k < total) put_offset(S, (int)base + k, ex, n);
         ex += v[k];
     }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = ex;
+    if (blockIdx.x == 0) put_ends(S, n);
 }
 
-__global__ void k_scatter(const int *__restrict__ key, const int *__restrict__ slot,
-                          const int *__restrict__ off, int n, int *__restrict__ perm) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Up to kScanOne keys in one block: the counts staged in shared memory (padded by
+// one word in 32: a thread scans a contiguous chunk).
+constexpr int kScanOneThreads = 1024;
+constexpr int kScanOne = 32 * 1024;
+__device__ __forceinline__ int pad32(int i) { return i + (i >> 5); }
+__global__ void __launch_bounds__(kScanOneThreads) k_scan_one(const int *__restrict__ in, int total,
+                                                              Sorts S, int n) {
+    extern __shared__ int cnt[];
+    for (int i = threadIdx.x; i < total; i += kScanOneThreads) cnt[pad32(i)] = in[i];
+    __syncthreads();
+    const int chunk = (total + kScanOneThreads - 1) / kScanOneThreads;
+    const int b = threadIdx.x * chunk, e = min(total, b + chunk);
+    int sum = 0;
+    for (int i = b; i < e; i++) sum += cnt[pad32(i)];
+    int all;
+    int ex = block_exclusive_scan(sum, all);
+    for (int i = b; i < e; i++) {
+        const int c = cnt[pad32(i)];
+        cnt[pad32(i)] = ex;
+        ex += c;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < total; i += kScanOneThreads) put_offset(S, i, cnt[pad32(i)], n);
+    put_ends(S, n);
+}
+
+// Sort blockIdx.y: particle i to its bucket, in the order of the atomic slots.
+__global__ void k_scatter(Sorts S, int n, int *__restrict__ tmp) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    perm[off[key[i]] + slot[i]] = i;
+    const Sort &s = S.s[blockIdx.y];
+    tmp[(size_t)blockIdx.y * n + __ldg(s.off + s.key[i]) + s.perm[i]] = i;
 }
 
 // Keys holding more particles than this keep the order of the atomic slots:
 // ranking a key's particles costs (its count)^2 / 32 warp steps.
 constexpr int kStableMax = 16384;
 
-// Particle v = in[q] goes to out[b + r], r its rank by particle index among
+// Particle v = in[q] goes to perm[b + r], r its rank by particle index among
 // the particles of its key [b, e): every key's particles in increasing index,
 // so a position build gives the same order (and the sums over particles the
 // same rounding) on every run.  Consecutive q share a key, so the lanes of a
 // warp read the same entries (broadcast loads).
-__global__ void k_stable_place(const int *__restrict__ key, const int *__restrict__ off,
-                               const int *__restrict__ in, int n, int *__restrict__ out) {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_stable_place(Sorts S, int n, const int *__restrict__ tmp) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
+    const Sort &s = S.s[blockIdx.y];
+    const int *__restrict__ in = tmp + (size_t)blockIdx.y * n;
     const int v = in[q];
-    const int k = key[v];
-    const int b = off[k], e = off[k + 1];
+    const int k = s.key[v];
+    const int b = s.off[k], e = s.off[k + 1];
     int r = q - b;
     if (e - b <= kStableMax) {
         r = 0;
         for (int j = b; j < e; j++) r += in[j] < v;
     }
-    out[b + r] = v;
+    s.perm[b + r] = v;
 }
 
 // The block's records are assembled in shared memory and written as one
@@ -219,18 +270,26 @@ __global__ void k_stable_place(const int *__restrict__ key, const int *__restric
 // FP32), and per-thread record stores would touch a separate sector per lane.
 constexpr int kRecThreads = 128;
 
+// blockIdx.y < nset: that record set; nset: the cell-relative positions in cell
+// order (gathered from the keys pass's output).
 template <typename T, int P>
 __global__ void __launch_bounds__(kRecThreads)
-k_records(const uint32_t *__restrict__ pstart, const T *__restrict__ pfrac,
-          const int *__restrict__ perm, int n, int *__restrict__ rec_idx,
-          uint32_t *__restrict__ rec_start, T *__restrict__ rec_w) {
+k_records(const uint32_t *__restrict__ pstart, const T *__restrict__ pfrac, int n, int nset,
+          RecordSet<T> set0, RecordSet<T> set1,
+          const typename Vec4T<T>::type *__restrict__ prel, const int *__restrict__ cperm,
+          typename Vec4T<T>::type *__restrict__ cpos) {
     constexpr int WS = RecordWidth<T, P>::value;
     constexpr int VQ = WS * (int)sizeof(T) / 16;  // 16-byte pieces per record
     __shared__ __align__(16) T sm[kRecThreads * WS];
     const int s0 = blockIdx.x * kRecThreads;
     const int s = s0 + threadIdx.x;
+    if ((int)blockIdx.y == nset) {
+        if (s < n) cpos[s] = prel[cperm[s]];
+        return;
+    }
+    const RecordSet<T> set = blockIdx.y == 0 ? set0 : set1;
     if (s < n) {
-        const int i = perm[s];
+        const int i = set.perm[s];
         T row[WS];
         T w[P];
 #pragma unroll
@@ -241,25 +300,17 @@ k_records(const uint32_t *__restrict__ pstart, const T *__restrict__ pfrac,
         }
 #pragma unroll
         for (int j = 3 * P; j < WS; j++) row[j] = T(0);
-        rec_idx[s] = i;
-        rec_start[s] = pstart[i];
+        set.idx[s] = i;
+        set.start[s] = pstart[i];
         float4 *dst = reinterpret_cast<float4 *>(sm + (size_t)threadIdx.x * WS);
 #pragma unroll
         for (int q = 0; q < VQ; q++) dst[q] = reinterpret_cast<const float4 *>(row)[q];
     }
     __syncthreads();
     const int cnt = min(kRecThreads, n - s0);
-    float4 *out = reinterpret_cast<float4 *>(rec_w + (size_t)s0 * WS);
+    float4 *out = reinterpret_cast<float4 *>(set.w + (size_t)s0 * WS);
     const float4 *src = reinterpret_cast<const float4 *>(sm);
     for (int v = threadIdx.x; v < cnt * VQ; v += kRecThreads) out[v] = src[v];
-}
-
-// Cell-relative positions in cell order, gathered from the keys pass's output.
-template <typename G4>
-__global__ void k_cell_gather(const G4 *__restrict__ prel, const int *__restrict__ perm, int n,
-                              G4 *__restrict__ cpos) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n) cpos[s] = prel[perm[s]];
 }
 
 // Positions relative to the lower corner of their real-space cell.
@@ -304,48 +355,60 @@ void launch_all_keys(const double *pos, int n, const MeshGeom &g, int nc, int *k
                                                         (double *)pfrac, (double4_32a *)prel);
 }
 
-void launch_cell_gather(const void *prel, const int *perm, int n, bool fp32, void *cpos,
-                        cudaStream_t s) {
-    if (n <= 0) return;
-    if (fp32)
-        k_cell_gather<float4><<<nblk(n, 256), 256, 0, s>>>((const float4 *)prel, perm, n,
-                                                           (float4 *)cpos);
-    else
-        k_cell_gather<double4_32a><<<nblk(n, 256), 256, 0, s>>>((const double4_32a *)prel, perm, n,
-                                                            (double4_32a *)cpos);
-}
-
 void launch_cell_keys(const double *pos, int n, double L, int nc, int *key, int *count,
                       int *slot, cudaStream_t s) {
     if (n > 0) k_cell_keys<<<nblk(n, 256), 256, 0, s>>>(pos, n, L, nc, key, count, slot);
 }
 
-size_t scan_tmp_elems(int nkeys) { return (size_t)nblk(nkeys, kScanTile) + 1; }
+size_t scan_tmp_elems(long nkeys) { return (size_t)nblk(nkeys, kScanTile) + 1; }
 
-void launch_scan(const int *count, int nkeys, int *off, int *tmp, cudaStream_t s) {
-    int nb = nblk(nkeys, kScanTile);
-    if (nb < 1) nb = 1;
-    k_scan_reduce<<<nb, kScanThreads, 0, s>>>(count, nkeys, tmp);
-    k_scan_sums<<<1, kScanThreads, 0, s>>>(tmp, nb);
-    k_scan_final<<<nb, kScanThreads, 0, s>>>(count, nkeys, tmp, off);
-}
-
-void launch_scatter(const int *key, const int *off, int n, int *perm, int *tmp,
-                    cudaStream_t s) {
-    if (n <= 0) return;
-    k_scatter<<<nblk(n, 256), 256, 0, s>>>(key, perm, off, n, tmp);
-    k_stable_place<<<nblk(n, 256), 256, 0, s>>>(key, off, tmp, n, perm);
+int launch_sorts(const Sorts &S, const int *count, int n, int *scan_tmp, int *tmp,
+                 cudaStream_t s) {
+    const Sort &last = S.s[S.count - 1];
+    int launches = 0;
+    if (last.first + last.nkeys > INT_MAX) {  // one sort after the other
+        for (int j = 0; j < S.count; j++) {
+            Sorts one{};
+            one.s[0] = S.s[j];
+            one.s[0].first = 0;
+            one.count = 1;
+            launches += launch_sorts(one, count + S.s[j].first, n, scan_tmp, tmp, s);
+        }
+        return launches;
+    }
+    const int total = (int)last.first + last.nkeys;
+    if (total <= kScanOne) {
+        const size_t smem = sizeof(int) * (size_t)(total + total / 32 + 1);
+        cudaFuncSetAttribute(k_scan_one, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(int) * (kScanOne + kScanOne / 32 + 1)));
+        k_scan_one<<<1, kScanOneThreads, smem, s>>>(count, total, S, n);
+        launches = 1;
+    } else {
+        const int nb = nblk(total, kScanTile);
+        k_scan_reduce<<<nb, kScanThreads, 0, s>>>(count, total, scan_tmp);
+        k_scan_sums<<<1, kScanThreads, 0, s>>>(scan_tmp, nb);
+        k_scan_final<<<nb, kScanThreads, 0, s>>>(count, total, scan_tmp, S, n);
+        launches = 3;
+    }
+    if (n <= 0) return launches;
+    const dim3 grid(nblk(n, 256), S.count);
+    k_scatter<<<grid, 256, 0, s>>>(S, n, tmp);
+    k_stable_place<<<grid, 256, 0, s>>>(S, n, tmp);
+    return launches + 2;
 }
 
 template <typename T>
-void launch_records(const uint32_t *pstart, const T *pfrac, const int *perm, int n, int p,
-                    int *rec_idx, uint32_t *rec_start, T *rec_w, cudaStream_t s) {
-    if (n <= 0) return;
-    const int nb = nblk(n, kRecThreads);
+void launch_records(const uint32_t *pstart, const T *pfrac, int n, int p, int nset,
+                    const RecordSet<T> *sets, const void *prel, const int *cperm, void *cpos,
+                    cudaStream_t s) {
+    if (n <= 0 || (nset == 0 && !cpos)) return;
+    using V4 = typename Vec4T<T>::type;
+    const dim3 grid(nblk(n, kRecThreads), nset + (cpos ? 1 : 0));
+    const RecordSet<T> s0 = nset > 0 ? sets[0] : RecordSet<T>{}, s1 = nset > 1 ? sets[1] : s0;
     switch (p) {
-        case 4: k_records<T, 4><<<nb, kRecThreads, 0, s>>>(pstart, pfrac, perm, n, rec_idx, rec_start, rec_w); break;
-        case 6: k_records<T, 6><<<nb, kRecThreads, 0, s>>>(pstart, pfrac, perm, n, rec_idx, rec_start, rec_w); break;
-        case 8: k_records<T, 8><<<nb, kRecThreads, 0, s>>>(pstart, pfrac, perm, n, rec_idx, rec_start, rec_w); break;
+        case 4: k_records<T, 4><<<grid, kRecThreads, 0, s>>>(pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
+        case 6: k_records<T, 6><<<grid, kRecThreads, 0, s>>>(pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
+        case 8: k_records<T, 8><<<grid, kRecThreads, 0, s>>>(pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
         default: break;
     }
 }
@@ -361,9 +424,11 @@ void launch_cell_positions(const double *pos, const int *perm, int n, double L, 
                                                                       (double4_32a *)cpos);
 }
 
-template void launch_records<float>(const uint32_t *, const float *, const int *, int, int, int *,
-                                    uint32_t *, float *, cudaStream_t);
-template void launch_records<double>(const uint32_t *, const double *, const int *, int, int,
-                                     int *, uint32_t *, double *, cudaStream_t);
+template void launch_records<float>(const uint32_t *, const float *, int, int, int,
+                                    const RecordSet<float> *, const void *, const int *, void *,
+                                    cudaStream_t);
+template void launch_records<double>(const uint32_t *, const double *, int, int, int,
+                                     const RecordSet<double> *, const void *, const int *, void *,
+                                     cudaStream_t);
 
 }  // namespace spme
