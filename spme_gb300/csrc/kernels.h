@@ -238,6 +238,11 @@ struct ZPlan {
 bool make_zplan(int K, size_t elem, ZPlan *zp, std::vector<double> *tw, std::vector<int> *perm);
 // Columns per block for K (0 if K does not fit the fused kernel).
 int zfft_width(int K, size_t elem);
+// Two-factor form of the same operation (zfft2.cu; FP32, K <= 256): columns per
+// block (0: not this K), and its launch.
+int zfft2_width(int K);
+cudaError_t launch_zfft2(int K, const CUtensorMap &map, const float *tab2, const float *tw, double L,
+                         int R, int *err, cudaStream_t s);
 // One-pass 2D (y, x) transforms of the mesh's z-planes (FP32; K = 128, 160,
 // 256): real planes [planes][K][K] <-> half spectra [planes][K][K/2+1], cuFFT's
 // layouts and unnormalised conventions.  tables: make_fft2d_tables' bytes on

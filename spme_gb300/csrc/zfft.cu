@@ -1,4 +1,5 @@
-// Fused z-transform + k-space influence + inverse z-transform.
+// Fused z-transform + k-space influence + inverse z-transform: FP64, and the FP32 sizes
+// that zfft2.cu does not take (K < 16, K > 256).
 //
 // The 3D R2C/C2R transforms of the mesh are split: cuFFT does the 2D (y, x)
 // transforms of every z-plane, and this kernel does, for a chunk of W (y, x)
@@ -543,6 +544,7 @@ int zcfg_index(int K, size_t elem) {
 }  // namespace
 
 int zfft_width(int K, size_t elem) {
+    if (elem == 4 && zfft2_width(K) > 0) return zfft2_width(K);
     const int i = zcfg_index(K, elem);
     if (i < 0) return 0;
     return (elem == 4 ? kCfg32 : kCfg64)[i].W;
@@ -577,11 +579,11 @@ bool plan_is(const ZPlan &zp) {
 template <typename T, int W, int CT, int MINB, int MAXP>
 cudaError_t launch_zcfg(const CUtensorMap &map, const T *tab2, const T *tw, const int *perm,
                         const ZPlan &zp, T twopi_L, int R, int zb, int *err, cudaStream_t s) {
-    // a fixed pass sequence when the plan matches one (instantiated for each
-    // precision's first configuration, the one these K get)
-    constexpr ZCfg first = sizeof(T) == 4 ? kCfg32[0] : kCfg64[0];
-    constexpr bool fixed_ok = first.W == W && first.ct == CT && first.minb == MINB &&
-                              first.maxp == MAXP;
+    // a fixed pass sequence when the plan matches one (instantiated for FP64's first
+    // configuration, the one these K get; FP32 runs zfft2.cu for them)
+    constexpr ZCfg first = kCfg64[0];
+    constexpr bool fixed_ok = sizeof(T) == 8 && first.W == W && first.ct == CT &&
+                              first.minb == MINB && first.maxp == MAXP;
     auto kern = k_zfft_influence<T, W, CT, MINB, MAXP, 0>;
     if constexpr (fixed_ok) {
         if (plan_is<256>(zp)) kern = k_zfft_influence<T, W, CT, MINB, MAXP, 256>;
@@ -604,6 +606,10 @@ cudaError_t launch_zfft_influence(const CUtensorMap &map, T *G, const T *tab2, c
                                   cudaStream_t s) {
     (void)G;  // addressed through the tensor map
     const int K = zp.K;
+    // FP32, K = R1 R2 of the supported list: compile-time radices, three passes (influence
+    // stage at K = 256, R = 16 1.80 -> 1.19 ms, K = 160 .780 -> .350, K = 75, R = 8 .154 -> .025)
+    if constexpr (sizeof(T) == 4)
+        if (zfft2_width(K) > 0) return launch_zfft2(K, map, tab2, tw, L, R, err, s);
     const int ci = zcfg_index(K, sizeof(T));
     if (ci < 0) return cudaErrorInvalidValue;
     const T twopi_L = (T)(2.0 * M_PI / L);

@@ -1,0 +1,398 @@
+// Fused z-transform + k-space influence + inverse z-transform for K = R1 R2 (FP32):
+// the operation of zfft.cu with compile-time radices and the influence inside the
+// second pass.
+//
+// Forward, per column and component: R1-point transforms over n1 (z = n2 + R2 n1),
+// twiddles w_K^{n2 k1}, then R2-point transforms over n2 give the frequencies
+// kz = k1 + R1 k2; the inverse runs the same steps backwards.  A thread of the
+// second pass holds the R2 frequencies of its k1 for all three components, so
+// the influence is applied in registers and the inverse R2-point transforms
+// follow at once: three passes over shared memory per right-hand side (forward
+// R1, second pass, inverse R1) with two barriers between them, instead of a pass
+// per radix pair and direction plus one for the influence (five at K = 256), and no
+// digit reversal.  The R1 passes give each component its own threads (3 R2 of them per
+// column), so with R1 near 3 R2 both kinds of pass keep the block's threads busy.
+// Complex sums are two-lane additions.
+// Data movement as in zfft.cu: chunks of W columns of the flattened z-plane
+// (TMA boxes, loads and stores), two buffers per block, a dedicated TMA warp.
+// Right-hand sides are split over blockIdx.y where the chunks alone would leave
+// SMs idle.
+// Bound: HBM (one read and one write of the half spectrum, 0.98 ms at K = 256, R =
+// 16), then shared-memory traffic and latency at one or two blocks per SM.
+// Influence stage, radix passes of zfft.cu -> here: K = 256, R = 16 1.80 -> 1.19 ms;
+// K = 160, R = 16 .780 -> .350; K = 128, R = 1 .037 -> .021; K = 75, R = 8 .154 -> .025.
+// Sixteen- by ten-point factors (K = 160: one thread per column and index for all three
+// components) need 168 registers a thread; 20 x 8 needs 126.
+#pragma once
+
+#include <utility>
+
+#include "kernels.h"
+#include "tma.cuh"
+
+namespace spme {
+namespace {
+
+__device__ __forceinline__ float2 z_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 z_sub(float2 a, float2 b) {
+    return __ffma2_rn(make_float2(-1.f, -1.f), b, a);
+}
+// a (c + i s)
+__device__ __forceinline__ float2 z_mul(float2 a, float c, float s) {
+    return make_float2(a.x * c - a.y * s, a.x * s + a.y * c);
+}
+
+// cos and sin of 2 pi m / n to double rounding (Taylor series after reduction to
+// [-pi/4, pi/4]): twiddles of the composite radices.
+constexpr double kPi = 3.14159265358979323846;
+__host__ __device__ constexpr double ct_sin(double x) {
+    double t = x, s = x;
+    for (int k = 1; k < 12; k++) {
+        t *= -x * x / ((2 * k) * (2 * k + 1));
+        s += t;
+    }
+    return s;
+}
+__host__ __device__ constexpr double ct_cos(double x) {
+    double t = 1, s = 1;
+    for (int k = 1; k < 12; k++) {
+        t *= -x * x / ((2 * k - 1) * (2 * k));
+        s += t;
+    }
+    return s;
+}
+__host__ __device__ constexpr double root_re(int m, int n) {
+    m %= n;
+    const int q = (4 * m + n / 2) / n;  // nearest quarter turn
+    const double x = 2 * kPi * ((double)m / n - q / 4.0);
+    return q % 4 == 0 ? ct_cos(x) : q % 4 == 1 ? -ct_sin(x) : q % 4 == 2 ? -ct_cos(x) : ct_sin(x);
+}
+__host__ __device__ constexpr double root_im(int m, int n) {
+    m %= n;
+    const int q = (4 * m + n / 2) / n;
+    const double x = 2 * kPi * ((double)m / n - q / 4.0);
+    return q % 4 == 0 ? ct_sin(x) : q % 4 == 1 ? ct_cos(x) : q % 4 == 2 ? -ct_sin(x) : -ct_cos(x);
+}
+
+// In-place DFT of v (natural order in and out): out[p] = sum_q v[q] w^{pq}, w =
+// e^{-2 pi i / R}, or its conjugate (INV).
+template <int R, bool INV>
+__device__ __forceinline__ void z_dft(float2 (&v)[R]);
+
+// The first factor of a composite radix.
+__host__ __device__ constexpr int z_split(int R) {
+    return R % 4 == 0 ? 4 : R % 2 == 0 ? 2 : R % 3 == 0 ? 3 : 5;
+}
+
+// y[qb][pa] *= w_R^{qb pa} (conjugated: INV), I = qb A + pa
+template <int R, bool INV, int A, int B, int I>
+__device__ __forceinline__ void z_twiddle(float2 (&y)[B][A]) {
+    constexpr int qb = I / A, pa = I % A;
+    if constexpr (qb * pa != 0) {
+        constexpr float c = (float)root_re(qb * pa, R);
+        constexpr float s = (float)(INV ? root_im(qb * pa, R) : -root_im(qb * pa, R));
+        y[qb][pa] = z_mul(y[qb][pa], c, s);
+    }
+}
+template <int R, bool INV, int A, int B, int... I>
+__device__ __forceinline__ void z_twiddles(float2 (&y)[B][A], std::integer_sequence<int, I...>) {
+    (z_twiddle<R, INV, A, B, I>(y), ...);
+}
+
+template <int R, bool INV>
+__device__ __forceinline__ void z_dft(float2 (&v)[R]) {
+    if constexpr (R == 2) {
+        const float2 a = v[0];
+        v[0] = z_add(a, v[1]);
+        v[1] = z_sub(a, v[1]);
+    } else if constexpr (R == 3) {
+        constexpr float h = 0.86602540378443865f;
+        const float2 t = z_add(v[1], v[2]), u = z_sub(v[1], v[2]);
+        const float2 m = __ffma2_rn(make_float2(-0.5f, -0.5f), t, v[0]);
+        // forward: v1 = m - i h u; inverse: m + i h u
+        const float sx = INV ? -h * u.y : h * u.y, sy = INV ? h * u.x : -h * u.x;
+        v[0] = z_add(v[0], t);
+        v[1] = make_float2(m.x + sx, m.y + sy);
+        v[2] = make_float2(m.x - sx, m.y - sy);
+    } else if constexpr (R == 4) {
+        const float2 s02 = z_add(v[0], v[2]), d02 = z_sub(v[0], v[2]), s13 = z_add(v[1], v[3]);
+        // -i (v1 - v3) forward, +i (v1 - v3) inverse
+        const float2 jd = INV ? make_float2(v[3].y - v[1].y, v[1].x - v[3].x)
+                              : make_float2(v[1].y - v[3].y, v[3].x - v[1].x);
+        v[0] = z_add(s02, s13);
+        v[1] = z_add(d02, jd);
+        v[2] = z_sub(s02, s13);
+        v[3] = z_sub(d02, jd);
+    } else if constexpr (R == 5) {
+        constexpr float c1 = 0.30901699437494742f, c2 = -0.80901699437494742f,
+                        s1 = 0.95105651629515357f, s2 = 0.58778525229247313f;
+        const float2 t1 = z_add(v[1], v[4]), t2 = z_add(v[2], v[3]);
+        const float2 u1 = z_sub(v[1], v[4]), u2 = z_sub(v[2], v[3]);
+        const float2 m1 = __ffma2_rn(make_float2(c2, c2), t2, __ffma2_rn(make_float2(c1, c1), t1, v[0]));
+        const float2 m2 = __ffma2_rn(make_float2(c1, c1), t2, __ffma2_rn(make_float2(c2, c2), t1, v[0]));
+        const float2 n1 = __ffma2_rn(make_float2(s2, s2), u2, __fmul2_rn(make_float2(s1, s1), u1));
+        const float2 n2 = __ffma2_rn(make_float2(-s1, -s1), u2, __fmul2_rn(make_float2(s2, s2), u1));
+        v[0] = z_add(v[0], z_add(t1, t2));
+        // forward: v1 = m1 - i n1, v4 = m1 + i n1; inverse the other way round
+        const float2 a1 = make_float2(m1.x + n1.y, m1.y - n1.x), b1 = make_float2(m1.x - n1.y, m1.y + n1.x);
+        const float2 a2 = make_float2(m2.x + n2.y, m2.y - n2.x), b2 = make_float2(m2.x - n2.y, m2.y + n2.x);
+        v[1] = INV ? b1 : a1;
+        v[4] = INV ? a1 : b1;
+        v[2] = INV ? b2 : a2;
+        v[3] = INV ? a2 : b2;
+    } else {
+        // R = A B: q = qb + B qa, p = pa + A pb
+        constexpr int A = z_split(R), B = R / A;
+        float2 y[B][A];
+#pragma unroll
+        for (int qb = 0; qb < B; qb++) {
+#pragma unroll
+            for (int qa = 0; qa < A; qa++) y[qb][qa] = v[qb + B * qa];
+            z_dft<A, INV>(y[qb]);
+        }
+        z_twiddles<R, INV, A, B>(y, std::make_integer_sequence<int, A * B>{});
+#pragma unroll
+        for (int pa = 0; pa < A; pa++) {
+            float2 t[B];
+#pragma unroll
+            for (int qb = 0; qb < B; qb++) t[qb] = y[qb][pa];
+            z_dft<B, INV>(t);
+#pragma unroll
+            for (int pb = 0; pb < B; pb++) v[pa + A * pb] = t[pb];
+        }
+    }
+}
+
+// Shared-memory layout (bytes from the 128-aligned base): two buffers of three
+// K x W component blocks, the twiddles e^{-2 pi i e / K}, barriers full[b] (TMA
+// load of buffer b landed) and done[b] (the compute warps finished buffer b).
+struct ZSmem2 {
+    size_t comp, buf_bytes, tw_off, bar_off, total;
+    __host__ __device__ constexpr ZSmem2(int K, int W)
+        : comp(((size_t)K * W * sizeof(float2) + 127) & ~(size_t)127),  // TMA: 128-aligned
+          buf_bytes(3 * comp),
+          tw_off(2 * buf_bytes),
+          bar_off(tw_off + (((size_t)K * sizeof(float2) + 15) & ~(size_t)15)),
+          total(bar_off + 4 * sizeof(uint64_t)) {}
+};
+
+__host__ __device__ constexpr int z2_threads(int W, int R1, int R2) {
+    return (W * (R1 > 3 * R2 ? R1 : 3 * R2) + 31) / 32 * 32;
+}
+// Blocks per SM: what shared memory allows, at no less than REGMIN registers a thread.
+__host__ __device__ constexpr int z2_minb(int W, int R1, int R2) {
+    const int regs = 8 * R2 + 32 > 2 * R1 + 32 ? 8 * R2 + 32 : 2 * R1 + 32;
+    const int bs = (int)(224 * 1024 / (ZSmem2(R1 * R2, W).total + 1152));
+    const int br = 65536 / (regs * ((z2_threads(W, R1, R2) + 32 + 127) / 128 * 128));
+    const int m = bs < br ? bs : br;
+    return m < 1 ? 1 : m > 8 ? 8 : m;
+}
+
+template <int N>
+__device__ __forceinline__ void z2_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ bool z2_sync_and(bool p) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred q, o;\n\t"
+        "setp.ne.u32 q, %1, 0;\n\t"
+        "bar.red.and.pred o, 1, %2, q;\n\t"
+        "selp.u32 %0, 1, 0, o;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)p), "n"(N)
+        : "memory");
+    return r != 0;
+}
+
+// One block per chunk of W consecutive columns and range of right-hand sides
+// [blockIdx.y rs, +rs).  Threads 0 .. CT-1 transform (thread = column + W index),
+// the warp after them moves data.
+template <int W, int R1, int R2>
+__global__ void __launch_bounds__(z2_threads(W, R1, R2) + 32, z2_minb(W, R1, R2))
+k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab2,
+        const float2 *__restrict__ tw_g, float twopi_L, int R, int rs, int *__restrict__ err) {
+    constexpr int K = R1 * R2, Kh = K / 2 + 1, CT = z2_threads(W, R1, R2);
+    const int plane = K * Kh;
+    const int f0 = blockIdx.x * W, tid = threadIdx.x;
+    const int rb = blockIdx.y * rs, nr = min(rs, R - rb);
+    extern __shared__ __align__(128) unsigned char zsm_raw[];
+    unsigned char *zsm = zsm_raw + ((128u - (smem_addr(zsm_raw) & 127u)) & 127u);
+    constexpr ZSmem2 lay(K, W);
+    constexpr int GS = (int)(lay.comp / sizeof(float2));  // component stride (complex values)
+    float2 *const buf0 = reinterpret_cast<float2 *>(zsm);
+    float2 *const buf1 = reinterpret_cast<float2 *>(zsm + lay.buf_bytes);
+    float2 *tw = reinterpret_cast<float2 *>(zsm + lay.tw_off);
+    uint64_t *full = reinterpret_cast<uint64_t *>(zsm + lay.bar_off);
+    uint64_t *done = full + 2;
+
+    if (tid == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        mbar_init(&done[0], CT);
+        mbar_init(&done[1], CT);
+        mbar_fence_init();
+    }
+    for (int e = tid; e < K; e += CT + 32) tw[e] = tw_g[e];
+    __syncthreads();
+
+    if (tid >= CT) {
+        // ---- TMA warp (one lane) ----
+        if (tid != CT) return;
+        const uint32_t bytes = (uint32_t)(3 * K * W * sizeof(float2));
+        auto issue_load = [&](int r, int b) {
+            mbar_expect_tx(&full[b], bytes);
+            float2 *dst = b ? buf1 : buf0;
+            for (int d = 0; d < 3; d++)
+                tma_load_3d(dst + d * GS, &gmap, 2 * f0, 0, 3 * (rb + r) + d, &full[b]);
+        };
+        issue_load(0, 0);
+        int issued = 1;
+        if (nr > 1) issue_load(1, 1), issued = 2;
+        int r = 0;
+        for (; r < nr; r++) {
+            const int b = r & 1;
+            if (!mbar_wait(&done[b], (uint32_t)((r >> 1) & 1))) break;
+            const float2 *src = b ? buf1 : buf0;
+            for (int d = 0; d < 3; d++)
+                tma_store_3d(&gmap, 2 * f0, 0, 3 * (rb + r) + d, src + d * GS);
+            bulk_commit_group();
+            if (r + 2 < nr) {
+                bulk_wait_read_all();  // buffer b is free again
+                issue_load(r + 2, b);
+                issued++;
+            }
+        }
+        if (r < nr) {
+            atomicExch(err, 1);
+            // loads of right-hand sides r .. issued-1 may still be in flight
+            for (int q = r; q < issued; q++) mbar_wait(&full[q & 1], (uint32_t)((q >> 1) & 1));
+        }
+        bulk_wait_all();
+        return;
+    }
+
+    // ---- compute warps ----
+    // column; in the R1 passes component d1 and n2, in the second k1 = id
+    const int w = tid % W, id = tid / W, d1 = id / R2, n2 = id - d1 * R2;
+    const int fl = f0 + w;
+    const bool valid = fl < plane;
+    const int ky = valid ? fl / Kh : 0, kx = valid ? fl - ky * Kh : 0;
+    const float kxv = (float)kx * twopi_L;  // kx <= K/2: non-negative wavenumber
+    const float kyv = (float)(ky <= K / 2 ? ky : ky - K) * twopi_L;
+    // kx = 0 and (even K) K/2 planes hold k and -k: there the tensor is averaged with
+    // its mirror (the Hermitian part of the result): with s_i = +1 for a zero or
+    // Nyquist index and -1 otherwise, the ij coupling survives when s_i s_j = +1
+    // (s_x = +1 on these planes)
+    const bool xplane = valid && (kx == 0 || (K % 2 == 0 && kx == K / 2));
+    const bool sy = ky == 0 || (K % 2 == 0 && ky == K / 2);
+    // the influence table of this thread's frequencies, read once for all its
+    // right-hand sides
+    float2 mc[R2];
+#pragma unroll
+    for (int k2 = 0; k2 < R2; k2++)
+        mc[k2] = id < R1 && valid ? __ldg(tab2 + (size_t)(id + R1 * k2) * plane + fl)
+                                  : make_float2(0.f, 0.f);
+
+    for (int r = 0; r < nr; r++) {
+        const int b = r & 1;
+        const bool ok = mbar_wait(&full[b], (uint32_t)((r >> 1) & 1));
+        if (!z2_sync_and<CT>(ok)) {
+            if (tid == 0) atomicExch(err, 1);
+            break;
+        }
+        float2 *B = (b ? buf1 : buf0) + w;
+        float2 *x1 = B + d1 * GS + n2 * W;
+        // forward R1-point transforms over n1, in place (k1 where n1 was)
+        if (id < 3 * R2) {
+            float2 v[R1];
+#pragma unroll
+            for (int n1 = 0; n1 < R1; n1++) v[n1] = x1[n1 * R2 * W];
+            z_dft<R1, false>(v);
+            x1[0] = v[0];
+#pragma unroll
+            for (int k1 = 1; k1 < R1; k1++) {
+                const float2 t = tw[n2 * k1];
+                x1[k1 * R2 * W] = z_mul(v[k1], t.x, t.y);
+            }
+        }
+        z2_sync<CT>();
+        // second pass: R2-point transforms, influence, inverse R2-point transforms
+        if (id < R1) {
+            float2 *x = B + id * R2 * W;
+            float2 v[3][R2];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+#pragma unroll
+                for (int q = 0; q < R2; q++) v[d][q] = x[d * GS + q * W];
+                z_dft<R2, false>(v[d]);
+            }
+#pragma unroll
+            for (int k2 = 0; k2 < R2; k2++) {
+                const int kz = id + R1 * k2;
+                const float kzv = (float)(kz <= K / 2 ? kz : kz - K) * twopi_L;
+                const float m2 = mc[k2].x, c = mc[k2].y;
+                const float cx = c * kxv, cy = c * kyv, cz = c * kzv;
+                float b1 = -cx * kyv, b2 = -cx * kzv, b4 = -cy * kzv;
+                if (xplane) {
+                    const bool sz = kz == 0 || (K % 2 == 0 && kz == K / 2);
+                    if (!sy) b1 = 0.f;
+                    if (!sz) b2 = 0.f;
+                    if (sy != sz) b4 = 0.f;
+                }
+                const float b0 = m2 - cx * kxv, b3 = m2 - cy * kyv, b5 = m2 - cz * kzv;
+                const float2 g0 = v[0][k2], g1 = v[1][k2], g2 = v[2][k2];
+                const float2 B1 = make_float2(b1, b1), B2 = make_float2(b2, b2), B4 = make_float2(b4, b4);
+                v[0][k2] = __ffma2_rn(B2, g2, __ffma2_rn(B1, g1, __fmul2_rn(make_float2(b0, b0), g0)));
+                v[1][k2] = __ffma2_rn(B4, g2, __ffma2_rn(make_float2(b3, b3), g1, __fmul2_rn(B1, g0)));
+                v[2][k2] = __ffma2_rn(make_float2(b5, b5), g2, __ffma2_rn(B4, g1, __fmul2_rn(B2, g0)));
+            }
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                z_dft<R2, true>(v[d]);
+                x[d * GS] = v[d][0];
+#pragma unroll
+                for (int q = 1; q < R2; q++) {
+                    const float2 t = tw[id * q];
+                    x[d * GS + q * W] = z_mul(v[d][q], t.x, -t.y);
+                }
+            }
+        }
+        z2_sync<CT>();
+        // inverse R1-point transforms over k1
+        if (id < 3 * R2) {
+            float2 v[R1];
+#pragma unroll
+            for (int k1 = 0; k1 < R1; k1++) v[k1] = x1[k1 * R2 * W];
+            z_dft<R1, true>(v);
+#pragma unroll
+            for (int n1 = 0; n1 < R1; n1++) x1[n1 * R2 * W] = v[n1];
+        }
+        // hand the buffer to the TMA warp (its store reads what this thread wrote)
+        fence_proxy_async();
+        mbar_arrive(&done[b]);
+    }
+}
+
+template <int W, int R1, int R2>
+cudaError_t launch_z2(const CUtensorMap &map, const float *tab2, const float *tw, double L, int R,
+                      int *err, cudaStream_t s) {
+    constexpr int K = R1 * R2;
+    constexpr size_t smem = ZSmem2(K, W).total + 128;
+    auto kern = k_zfft2<W, R1, R2>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int nchunk = (K * (K / 2 + 1) + W - 1) / W;
+    // right-hand sides per block: all of them, or fewer (at least two, for the second
+    // buffer) until the resident blocks are filled about four times
+    int rs = R;
+    while (rs > 2 && (long)nchunk * ((R + rs - 1) / rs) < 608L * z2_minb(W, R1, R2)) rs = (rs + 1) / 2;
+    kern<<<dim3(nchunk, (R + rs - 1) / rs), z2_threads(W, R1, R2) + 32, smem, s>>>(
+        map, reinterpret_cast<const float2 *>(tab2), reinterpret_cast<const float2 *>(tw),
+        (float)(2.0 * M_PI / L), R, rs, err);
+    return cudaGetLastError();
+}
+
+}  // namespace
+}  // namespace spme
