@@ -80,10 +80,9 @@ constexpr int kGraphSlots = 4;
 
 struct PlanPair {
     int C;
-    cufftHandle fwd;
-    cufftHandle bwd;
+    cufftHandle fwd = 0, bwd = 0;    // 3D transforms
     cufftHandle fwd2 = 0, bwd2 = 0;  // 2D (y, x) transforms of every z-plane
-    bool has2d = false;
+    bool has3d = false, has2d = false;
     spme::InterpMaps maps;  // TMA boxes over the mesh for this C and tile shape
     int maps_tile[3];
 };
@@ -438,6 +437,27 @@ cufftHandle pick_cand(spme_t *e, PlanCand &pc, bool inverse) {
     return h;
 }
 
+// Mode 1 with this library's x and y transforms (fft_xy.cuh) in place of cuFFT's 2D ones:
+// every size they are compiled for.  Transforms and influence in ms against cuFFT 3D
+// (FP64, R = 1) and 2D (FP32, R = 16): FP64 K = 32 .090 -> .053, K = 90 .62 -> .44, K = 128
+// 1.41 -> .94, K = 256 10.9 -> 7.6; FP32 K = 75 .40 -> .20, K = 160 1.98 -> 1.52, K = 256
+// 6.07 -> 5.33.  No cuFFT plan and no work area.
+bool own_xy(const spme_t *e) { return e->fft_mode == 1 && e->d_ztw && spme::fft_xy_ok(e->prm.dim, e->elem); }
+
+void destroy_plans(spme_t *e) {
+    for (PlanPair &p : e->plans) {
+        if (p.has3d) {
+            cufftDestroy(p.fwd);
+            cufftDestroy(p.bwd);
+        }
+        if (p.has2d) {
+            cufftDestroy(p.fwd2);
+            cufftDestroy(p.bwd2);
+        }
+    }
+    e->plans.clear();
+}
+
 int get_plans(spme_t *e, int C, PlanPair **out) {
     for (PlanPair &p : e->plans)
         if (p.C == C) {
@@ -448,6 +468,13 @@ int get_plans(spme_t *e, int C, PlanPair **out) {
     int n[3] = {K, K, K}, re[3] = {K, K, K}, ce[3] = {K, K, K / 2 + 1};
     PlanPair pp;
     pp.C = C;
+    if (own_xy(e)) {  // no cuFFT plan (set_fft_mode drops the entry)
+        pp.maps_tile[0] = pp.maps_tile[1] = pp.maps_tile[2] = 0;
+        e->plans.push_back(pp);
+        *out = &e->plans.back();
+        return SPME_OK;
+    }
+    pp.has3d = true;
     pp.maps_tile[0] = pp.maps_tile[1] = pp.maps_tile[2] = 0;
     cufftType tf = is_fp32(e) ? CUFFT_R2C : CUFFT_D2Z;
     cufftType tb = is_fp32(e) ? CUFFT_C2R : CUFFT_Z2D;
@@ -487,8 +514,9 @@ int get_plans(spme_t *e, int C, PlanPair **out) {
         e->work_bytes = ws;
         bool ok = true;
         for (PlanPair &q : e->plans) {
-            ok = ok && cufftSetWorkArea(q.fwd, e->d_work) == CUFFT_SUCCESS &&
-                 cufftSetWorkArea(q.bwd, e->d_work) == CUFFT_SUCCESS;
+            if (q.has3d)
+                ok = ok && cufftSetWorkArea(q.fwd, e->d_work) == CUFFT_SUCCESS &&
+                     cufftSetWorkArea(q.bwd, e->d_work) == CUFFT_SUCCESS;
             if (q.has2d)
                 ok = ok && cufftSetWorkArea(q.fwd2, e->d_work) == CUFFT_SUCCESS &&
                      cufftSetWorkArea(q.bwd2, e->d_work) == CUFFT_SUCCESS;
@@ -628,9 +656,9 @@ int create_impl(const spme_params &prm, spme_t **out) {
                                     cudaMemcpyHostToDevice));
             }
             TRY_CUDA(cudaMemcpy(e->d_zip, ip.data(), sizeof(int) * K, cudaMemcpyHostToDevice));
-            // measured on GB300 (K = 256): the fused path wins in FP32; in FP64
-            // the 3D transforms + influence are as fast
-            e->fft_mode = is_fp32(e) ? 1 : 0;
+            // FP64 sizes without two-factor transforms: 3D transforms + influence are as
+            // fast as 2D transforms + the fused z transform (K = 320)
+            e->fft_mode = is_fp32(e) || spme::fft_xy_ok((int)K, 8) ? 1 : 0;
             // tables of the one-pass 2D transforms (fft_mode 2, opt-in: measured
             // slower than cuFFT's two-pass 2D transforms on GB300, 3.7 vs 2.55 ms
             // per direction at K = 256, 48 components)
@@ -674,8 +702,10 @@ void drop_graphs(spme_t *e) {
 void use_stream(spme_t *e, cudaStream_t s) {
     e->stream = s;
     for (PlanPair &p : e->plans) {
-        cufftSetStream(p.fwd, s);
-        cufftSetStream(p.bwd, s);
+        if (p.has3d) {
+            cufftSetStream(p.fwd, s);
+            cufftSetStream(p.bwd, s);
+        }
         if (p.has2d) {
             cufftSetStream(p.fwd2, s);
             cufftSetStream(p.bwd2, s);
@@ -721,14 +751,7 @@ void destroy_impl(spme_t *e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     if (e->aux) cudaStreamSynchronize(e->aux);
     drop_graphs(e);
-    for (PlanPair &p : e->plans) {
-        cufftDestroy(p.fwd);
-        cufftDestroy(p.bwd);
-        if (p.has2d) {
-            cufftDestroy(p.fwd2);
-            cufftDestroy(p.bwd2);
-        }
-    }
+    destroy_plans(e);
     void *bufs[] = {e->d_pos,    e->d_key,     e->d_sort_tmp, e->d_count,   e->d_toff,
                     e->d_tperm,  e->d_scan_tmp, e->d_rec_idx, e->d_rec_start, e->d_rec_w,
                     e->d_coff,    e->d_cperm, e->d_cpos,     e->d_prel, e->d_mesh,
@@ -909,15 +932,19 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
                                             (const T *)e->d_rec_w, F, C, e->g, (T *)e->d_mesh, s));
         e->launches++;
         if (prof) cudaEventRecord(e->ev[2], s);
-        // fft_mode 2: this project's one-pass 2D transforms; 1: cuFFT's 2D
-        // transforms; both followed by the fused z transform + influence
-        const bool own2d = e->fft_mode == 2 && e->d_f2tab;
-        const bool fused = own2d || (e->fft_mode == 1 && pp->has2d);
+        // fft_mode 2: one-pass 2D transforms; 1: two-factor x and y transforms, or cuFFT's
+        // 2D transforms; all followed by the fused z transform + influence
+        const bool own2d = e->fft_mode == 2 && e->d_f2tab, ownxy = own_xy(e);
+        const bool fused = own2d || ownxy || (e->fft_mode == 1 && pp->has2d);
         cufftHandle fwd = fused ? pp->fwd2 : pp->fwd, bwd = fused ? pp->bwd2 : pp->bwd;
         if (own2d) {
             TRY_CUDA(spme::launch_fft2d_r2c(K, (const float *)e->d_mesh, (float *)e->d_cmesh,
                                             (long)C * K, e->d_f2tab, s));
             e->launches++;
+        } else if (ownxy) {
+            TRY_CUDA(spme::launch_fft_xy<T>(K, false, (T *)e->d_mesh, (T *)e->d_cmesh, (long)C * K,
+                                            (const T *)e->d_ztw, s));
+            e->launches += 2;
         } else if (sizeof(T) == 4)
             TRY_FFT(cufftExecR2C(fwd, (cufftReal *)e->d_mesh, (cufftComplex *)e->d_cmesh));
         else
@@ -939,6 +966,10 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
             TRY_CUDA(spme::launch_fft2d_c2r(K, (const float *)e->d_cmesh, (float *)e->d_mesh,
                                             (long)C * K, e->d_f2tab, s));
             e->launches++;
+        } else if (ownxy) {
+            TRY_CUDA(spme::launch_fft_xy<T>(K, true, (T *)e->d_mesh, (T *)e->d_cmesh, (long)C * K,
+                                            (const T *)e->d_ztw, s));
+            e->launches += 2;
         } else if (sizeof(T) == 4)
             TRY_FFT(cufftExecC2R(bwd, (cufftComplex *)e->d_cmesh, (cufftReal *)e->d_mesh));
         else
@@ -1271,17 +1302,7 @@ int spme_set_fft_mode(spme_t *e, int mode) {
     if (mode == 2 && !e->d_f2tab) return e->last_error = SPME_ERR_UNSUPPORTED;
     if (e->stream) cudaStreamSynchronize(e->stream);
     drop_graphs(e);
-    if (mode == 1) {
-        for (PlanPair &p : e->plans) {
-            cufftDestroy(p.fwd);
-            cufftDestroy(p.bwd);
-            if (p.has2d) {
-                cufftDestroy(p.fwd2);
-                cufftDestroy(p.bwd2);
-            }
-        }
-        e->plans.clear();  // rebuilt with their 2D companions on the next pass
-    }
+    destroy_plans(e);  // made again for the mode on the next pass
     e->fft_mode = mode;
     return e->last_error = SPME_OK;
 }

@@ -233,7 +233,8 @@ struct ZPlan {
     int pcode[12];        // 10 * R1 + R2 (R2 = 1: single stage)
     int pspan[12];        // span of the pass's first (R1) stage in DIT order
 };
-// Radix plan, twiddles e^{-2 pi i e/K} (re, im pairs) and the digit-reversal
+// Radix plan, twiddles e^{-2 pi i e/K} (re, im pairs; re - 1 for the sizes of the
+// FP64 two-factor kernels) and the digit-reversal
 // permutation (position p holds frequency perm[p]) for length-K transforms.
 bool make_zplan(int K, size_t elem, ZPlan *zp, std::vector<double> *tw, std::vector<int> *perm);
 // Columns per block for K (0 if K does not fit the fused kernel).
@@ -243,6 +244,18 @@ int zfft_width(int K, size_t elem);
 int zfft2_width(int K);
 cudaError_t launch_zfft2(int K, const CUtensorMap &map, const float *tab2, const float *tw, double L,
                          int R, int *err, cudaStream_t s);
+// Its FP64 form (zfft64.cu; K of fft_xy_ok, elem 8), on G in place.
+cudaError_t launch_zfft64(int K, double *G, const double *tab2, const double *tw, double L, int R,
+                          cudaStream_t s);
+// Two-factor x and y transforms of the mesh's z-planes (fft_xy.cuh; K = 2^a 3^b 5^c, 16 to
+// 256, fft_xy_ok): mesh -> G, or G -> mesh (inv; G is overwritten).  tw as for the z transform.
+bool fft_xy_ok(int K, size_t elem);
+template <typename T>
+cudaError_t launch_fft_xy(int K, bool inv, T *mesh, T *G, long planes, const T *tw, cudaStream_t s);
+template <>
+cudaError_t launch_fft_xy<float>(int, bool, float *, float *, long, const float *, cudaStream_t);
+template <>
+cudaError_t launch_fft_xy<double>(int, bool, double *, double *, long, const double *, cudaStream_t);
 // One-pass 2D (y, x) transforms of the mesh's z-planes (FP32; K = 128, 160,
 // 256): real planes [planes][K][K] <-> half spectra [planes][K][K/2+1], cuFFT's
 // layouts and unnormalised conventions.  tables: make_fft2d_tables' bytes on

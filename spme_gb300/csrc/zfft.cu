@@ -500,9 +500,16 @@ bool make_zplan(int K, size_t elem, ZPlan *zp, std::vector<double> *twr, std::ve
     perm->assign(idx.begin(), idx.end());
     twr->resize(2 * (size_t)K);
     for (int e = 0; e < K; e++) {
-        const double a = -2.0 * M_PI * (double)e / (double)K;
-        (*twr)[2 * e] = std::cos(a);
-        (*twr)[2 * e + 1] = std::sin(a);
+        // the angle reduced to a quarter turn's nearest, in integers
+        const int q = (4 * e + K / 2) / K;
+        const long double x = 2.0L * 3.14159265358979323846264338327950288L * (4 * e - q * K) / (4.0L * K);
+        const long double c = std::cos(x), s = std::sin(x);
+        const long double re[4] = {c, -s, -c, s}, im[4] = {s, c, -s, -c};
+        // (the FP64 two-factor kernels read cos - 1)
+        const long double t = std::sin(x / 2);
+        const bool own = elem == 8 && fft_xy_ok(K, 8);
+        (*twr)[2 * e] = (double)(!own ? re[q % 4] : q == 0 ? -2 * t * t : re[q % 4] - 1);
+        (*twr)[2 * e + 1] = (double)-im[q % 4];
     }
     return true;
 }
@@ -604,12 +611,14 @@ template <typename T>
 cudaError_t launch_zfft_influence(const CUtensorMap &map, T *G, const T *tab2, const T *tw,
                                   const int *perm, const ZPlan &zp, double L, int R, int *err,
                                   cudaStream_t s) {
-    (void)G;  // addressed through the tensor map
     const int K = zp.K;
     // FP32, K = R1 R2 of the supported list: compile-time radices, three passes (influence
     // stage at K = 256, R = 16 1.80 -> 1.19 ms, K = 160 .780 -> .350, K = 75, R = 8 .154 -> .025)
-    if constexpr (sizeof(T) == 4)
+    if constexpr (sizeof(T) == 4) {
         if (zfft2_width(K) > 0) return launch_zfft2(K, map, tab2, tw, L, R, err, s);
+    } else {
+        if (fft_xy_ok(K, 8)) return launch_zfft64(K, G, tab2, tw, L, R, s);
+    }
     const int ci = zcfg_index(K, sizeof(T));
     if (ci < 0) return cudaErrorInvalidValue;
     const T twopi_L = (T)(2.0 * M_PI / L);

@@ -25,143 +25,12 @@
 // components) need 168 registers a thread; 20 x 8 needs 126.
 #pragma once
 
-#include <utility>
-
+#include "fft_dft.cuh"
 #include "kernels.h"
 #include "tma.cuh"
 
 namespace spme {
 namespace {
-
-__device__ __forceinline__ float2 z_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 z_sub(float2 a, float2 b) {
-    return __ffma2_rn(make_float2(-1.f, -1.f), b, a);
-}
-// a (c + i s)
-__device__ __forceinline__ float2 z_mul(float2 a, float c, float s) {
-    return make_float2(a.x * c - a.y * s, a.x * s + a.y * c);
-}
-
-// cos and sin of 2 pi m / n to double rounding (Taylor series after reduction to
-// [-pi/4, pi/4]): twiddles of the composite radices.
-constexpr double kPi = 3.14159265358979323846;
-__host__ __device__ constexpr double ct_sin(double x) {
-    double t = x, s = x;
-    for (int k = 1; k < 12; k++) {
-        t *= -x * x / ((2 * k) * (2 * k + 1));
-        s += t;
-    }
-    return s;
-}
-__host__ __device__ constexpr double ct_cos(double x) {
-    double t = 1, s = 1;
-    for (int k = 1; k < 12; k++) {
-        t *= -x * x / ((2 * k - 1) * (2 * k));
-        s += t;
-    }
-    return s;
-}
-__host__ __device__ constexpr double root_re(int m, int n) {
-    m %= n;
-    const int q = (4 * m + n / 2) / n;  // nearest quarter turn
-    const double x = 2 * kPi * ((double)m / n - q / 4.0);
-    return q % 4 == 0 ? ct_cos(x) : q % 4 == 1 ? -ct_sin(x) : q % 4 == 2 ? -ct_cos(x) : ct_sin(x);
-}
-__host__ __device__ constexpr double root_im(int m, int n) {
-    m %= n;
-    const int q = (4 * m + n / 2) / n;
-    const double x = 2 * kPi * ((double)m / n - q / 4.0);
-    return q % 4 == 0 ? ct_sin(x) : q % 4 == 1 ? ct_cos(x) : q % 4 == 2 ? -ct_sin(x) : -ct_cos(x);
-}
-
-// In-place DFT of v (natural order in and out): out[p] = sum_q v[q] w^{pq}, w =
-// e^{-2 pi i / R}, or its conjugate (INV).
-template <int R, bool INV>
-__device__ __forceinline__ void z_dft(float2 (&v)[R]);
-
-// The first factor of a composite radix.
-__host__ __device__ constexpr int z_split(int R) {
-    return R % 4 == 0 ? 4 : R % 2 == 0 ? 2 : R % 3 == 0 ? 3 : 5;
-}
-
-// y[qb][pa] *= w_R^{qb pa} (conjugated: INV), I = qb A + pa
-template <int R, bool INV, int A, int B, int I>
-__device__ __forceinline__ void z_twiddle(float2 (&y)[B][A]) {
-    constexpr int qb = I / A, pa = I % A;
-    if constexpr (qb * pa != 0) {
-        constexpr float c = (float)root_re(qb * pa, R);
-        constexpr float s = (float)(INV ? root_im(qb * pa, R) : -root_im(qb * pa, R));
-        y[qb][pa] = z_mul(y[qb][pa], c, s);
-    }
-}
-template <int R, bool INV, int A, int B, int... I>
-__device__ __forceinline__ void z_twiddles(float2 (&y)[B][A], std::integer_sequence<int, I...>) {
-    (z_twiddle<R, INV, A, B, I>(y), ...);
-}
-
-template <int R, bool INV>
-__device__ __forceinline__ void z_dft(float2 (&v)[R]) {
-    if constexpr (R == 2) {
-        const float2 a = v[0];
-        v[0] = z_add(a, v[1]);
-        v[1] = z_sub(a, v[1]);
-    } else if constexpr (R == 3) {
-        constexpr float h = 0.86602540378443865f;
-        const float2 t = z_add(v[1], v[2]), u = z_sub(v[1], v[2]);
-        const float2 m = __ffma2_rn(make_float2(-0.5f, -0.5f), t, v[0]);
-        // forward: v1 = m - i h u; inverse: m + i h u
-        const float sx = INV ? -h * u.y : h * u.y, sy = INV ? h * u.x : -h * u.x;
-        v[0] = z_add(v[0], t);
-        v[1] = make_float2(m.x + sx, m.y + sy);
-        v[2] = make_float2(m.x - sx, m.y - sy);
-    } else if constexpr (R == 4) {
-        const float2 s02 = z_add(v[0], v[2]), d02 = z_sub(v[0], v[2]), s13 = z_add(v[1], v[3]);
-        // -i (v1 - v3) forward, +i (v1 - v3) inverse
-        const float2 jd = INV ? make_float2(v[3].y - v[1].y, v[1].x - v[3].x)
-                              : make_float2(v[1].y - v[3].y, v[3].x - v[1].x);
-        v[0] = z_add(s02, s13);
-        v[1] = z_add(d02, jd);
-        v[2] = z_sub(s02, s13);
-        v[3] = z_sub(d02, jd);
-    } else if constexpr (R == 5) {
-        constexpr float c1 = 0.30901699437494742f, c2 = -0.80901699437494742f,
-                        s1 = 0.95105651629515357f, s2 = 0.58778525229247313f;
-        const float2 t1 = z_add(v[1], v[4]), t2 = z_add(v[2], v[3]);
-        const float2 u1 = z_sub(v[1], v[4]), u2 = z_sub(v[2], v[3]);
-        const float2 m1 = __ffma2_rn(make_float2(c2, c2), t2, __ffma2_rn(make_float2(c1, c1), t1, v[0]));
-        const float2 m2 = __ffma2_rn(make_float2(c1, c1), t2, __ffma2_rn(make_float2(c2, c2), t1, v[0]));
-        const float2 n1 = __ffma2_rn(make_float2(s2, s2), u2, __fmul2_rn(make_float2(s1, s1), u1));
-        const float2 n2 = __ffma2_rn(make_float2(-s1, -s1), u2, __fmul2_rn(make_float2(s2, s2), u1));
-        v[0] = z_add(v[0], z_add(t1, t2));
-        // forward: v1 = m1 - i n1, v4 = m1 + i n1; inverse the other way round
-        const float2 a1 = make_float2(m1.x + n1.y, m1.y - n1.x), b1 = make_float2(m1.x - n1.y, m1.y + n1.x);
-        const float2 a2 = make_float2(m2.x + n2.y, m2.y - n2.x), b2 = make_float2(m2.x - n2.y, m2.y + n2.x);
-        v[1] = INV ? b1 : a1;
-        v[4] = INV ? a1 : b1;
-        v[2] = INV ? b2 : a2;
-        v[3] = INV ? a2 : b2;
-    } else {
-        // R = A B: q = qb + B qa, p = pa + A pb
-        constexpr int A = z_split(R), B = R / A;
-        float2 y[B][A];
-#pragma unroll
-        for (int qb = 0; qb < B; qb++) {
-#pragma unroll
-            for (int qa = 0; qa < A; qa++) y[qb][qa] = v[qb + B * qa];
-            z_dft<A, INV>(y[qb]);
-        }
-        z_twiddles<R, INV, A, B>(y, std::make_integer_sequence<int, A * B>{});
-#pragma unroll
-        for (int pa = 0; pa < A; pa++) {
-            float2 t[B];
-#pragma unroll
-            for (int qb = 0; qb < B; qb++) t[qb] = y[qb][pa];
-            z_dft<B, INV>(t);
-#pragma unroll
-            for (int pb = 0; pb < B; pb++) v[pa + A * pb] = t[pb];
-        }
-    }
-}
 
 // Shared-memory layout (bytes from the 128-aligned base): two buffers of three
 // K x W component blocks, the twiddles e^{-2 pi i e / K}, barriers full[b] (TMA
@@ -179,7 +48,7 @@ struct ZSmem2 {
 __host__ __device__ constexpr int z2_threads(int W, int R1, int R2) {
     return (W * (R1 > 3 * R2 ? R1 : 3 * R2) + 31) / 32 * 32;
 }
-// Blocks per SM: what shared memory allows, at no less than REGMIN registers a thread.
+// Blocks per SM: what shared memory allows at the registers the passes want.
 __host__ __device__ constexpr int z2_minb(int W, int R1, int R2) {
     const int regs = 8 * R2 + 32 > 2 * R1 + 32 ? 8 * R2 + 32 : 2 * R1 + 32;
     const int bs = (int)(224 * 1024 / (ZSmem2(R1 * R2, W).total + 1152));
@@ -314,7 +183,7 @@ k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab
 #pragma unroll
             for (int k1 = 1; k1 < R1; k1++) {
                 const float2 t = tw[n2 * k1];
-                x1[k1 * R2 * W] = z_mul(v[k1], t.x, t.y);
+                x1[k1 * R2 * W] = z_tw(v[k1], t.x, t.y);
             }
         }
         z2_sync<CT>();
@@ -355,7 +224,7 @@ k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab
 #pragma unroll
                 for (int q = 1; q < R2; q++) {
                     const float2 t = tw[id * q];
-                    x[d * GS + q * W] = z_mul(v[d][q], t.x, -t.y);
+                    x[d * GS + q * W] = z_tw(v[d][q], t.x, -t.y);
                 }
             }
         }
