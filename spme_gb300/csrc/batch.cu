@@ -394,6 +394,13 @@ struct FftGroup {
     int K = 0;
     size_t mesh_off = 0, spec_off = 0;  // of the group's first system
     int nsys = 0;
+    // two-factor transforms with the influence in the z transform (fft_xy.cuh, zfft2.cuh,
+    // zfft64.cuh) where the size has them, else cuFFT's 3D transforms
+    bool own = false;
+    size_t tab_off = 0;
+    int sys_off = 0;      // into d_twopi_L
+    void *d_tw = nullptr;
+    CUtensorMap zmap;     // FP32: over the group's spectra
     cufftHandle fwd = 0, bwd = 0;
 };
 
@@ -440,6 +447,7 @@ struct _spme_batch_t {
     void *d_F = nullptr, *d_Fs = nullptr, *d_W = nullptr, *d_W2 = nullptr;
     void *d_F2 = nullptr;  // force rows as the FP32 real-space sum reads them
     void *d_mesh = nullptr, *d_spec = nullptr, *d_tab = nullptr;
+    double *d_twopi_L = nullptr;  // per system, in group order
     double *d_pair = nullptr;  // FP64 batches: pair-function tables of all systems
     int *d_err = nullptr;
     // work lists (device): per-system launch arguments and block prefixes
@@ -614,6 +622,28 @@ int build_tiles(_spme_batch_t *b) {
     return SPME_OK;
 }
 
+// Twiddles (and FP32 the box over the spectra) of a group whose size has two-factor
+// transforms; its spectra must be in place.
+template <typename T>
+int own_transforms(_spme_batch_t *b, FftGroup &grp) {
+    const int K = grp.K;
+    // (systems and right-hand sides are a grid dimension of the z transform)
+    if (!fft_xy_ok(K, sizeof(T)) || (long)grp.nsys * b->R > 65535) return SPME_OK;
+    if (sizeof(T) == 4 &&
+        (zfft2_width(K) == 0 || zfft_width(K, 4) == 0 ||
+         !make_zfft_map(&grp.zmap, (T *)b->d_spec + 2 * grp.spec_off, K, b->C * grp.nsys, 4)))
+        return SPME_OK;
+    ZPlan zp;
+    std::vector<double> tw;
+    std::vector<int> perm;
+    if (!make_zplan(K, sizeof(T), &zp, &tw, &perm)) return SPME_OK;
+    const std::vector<T> t(tw.begin(), tw.end());
+    BTRY(balloc(&grp.d_tw, sizeof(T) * t.size()));
+    BTRY_CUDA(cudaMemcpy(grp.d_tw, t.data(), sizeof(T) * t.size(), cudaMemcpyHostToDevice));
+    grp.own = true;
+    return SPME_OK;
+}
+
 template <typename T>
 int create_t(_spme_batch_t *b) {
     const int n = b->ntot, C = b->C, ns = b->nsys;
@@ -631,6 +661,7 @@ int create_t(_spme_batch_t *b) {
     std::map<int, std::vector<int>> byK;
     for (int k = 0; k < ns; k++) byK[b->sys[k].s.dim].push_back(k);
     size_t mesh = 0, spec = 0, tab = 0;
+    std::vector<double> twopi_L;  // in group order
     for (auto &kv : byK) {
         FftGroup grp;
         grp.K = kv.first;
@@ -642,12 +673,15 @@ int create_t(_spme_batch_t *b) {
         spec = (spec + 63) / 64 * 64;
         grp.mesh_off = mesh;
         grp.spec_off = spec;
+        grp.tab_off = tab;
+        grp.sys_off = (int)twopi_L.size();
         grp.nsys = (int)kv.second.size();
         const size_t K = (size_t)kv.first, K3 = K * K * K, Kc = K * K * (K / 2 + 1);
         for (int k : kv.second) {
             b->sys[k].mesh_off = mesh;
             b->sys[k].spec_off = spec;
             b->sys[k].tab_off = tab;
+            twopi_L.push_back(2.0 * M_PI / b->sys[k].s.box_size);
             mesh += (size_t)C * K3;
             spec += (size_t)C * Kc;
             tab += Kc;
@@ -750,6 +784,14 @@ int create_t(_spme_batch_t *b) {
         }
     }
 
+    BTRY(balloc(&b->d_twopi_L, sizeof(double) * ns));
+    BTRY_CUDA(cudaMemcpy(b->d_twopi_L, twopi_L.data(), sizeof(double) * ns, cudaMemcpyHostToDevice));
+    for (FftGroup &grp : b->groups) BTRY(own_transforms<T>(b, grp));
+    std::vector<char> own(ns, 0);
+    for (int k = 0; k < ns; k++)
+        for (const FftGroup &grp : b->groups)
+            if (grp.K == b->sys[k].s.dim) own[k] = grp.own;
+
     // work lists that do not depend on the tile
     std::vector<SpreadColsSys<T>> ss(ns);
     std::vector<RealArgs<T>> rs(ns);
@@ -780,7 +822,7 @@ int create_t(_spme_batch_t *b) {
         fs[k].tab_off = x.tab_off;
         fs[k].twopi_L = 2.0 * M_PI / x.s.box_size;
         const int nplane = ((K & 1) ? 1 : 2) * K * K;
-        pf[k + 1] = pf[k] + fs[k].nb_int + (nplane + 255) / 256;
+        pf[k + 1] = pf[k] + (own[k] ? 0 : fs[k].nb_int + (nplane + 255) / 256);
     }
     b->tot_spread = ps[ns];
     b->tot_real = pr[ns];
@@ -792,11 +834,12 @@ int create_t(_spme_batch_t *b) {
     BTRY_CUDA(cudaMemcpy(b->d_pre_real, pr.data(), sizeof(int) * (ns + 1), cudaMemcpyHostToDevice));
     BTRY_CUDA(cudaMemcpy(b->d_pre_infl, pf.data(), sizeof(int) * (ns + 1), cudaMemcpyHostToDevice));
 
-    // one batched 3D plan pair per mesh size
+    // one batched 3D plan pair per mesh size without own transforms
     size_t wsz = 0;
     const cufftType tf = sizeof(T) == 4 ? CUFFT_R2C : CUFFT_D2Z;
     const cufftType tb = sizeof(T) == 4 ? CUFFT_C2R : CUFFT_Z2D;
     for (FftGroup &grp : b->groups) {
+        if (grp.own) continue;
         const int K = grp.K;
         int nn[3] = {K, K, K}, re[3] = {K, K, K}, ce[3] = {K, K, K / 2 + 1};
         const int K3 = K * K * K, Kc = K * K * (K / 2 + 1);
@@ -812,7 +855,8 @@ int create_t(_spme_batch_t *b) {
             return SPME_ERR_CUFFT;
         wsz = std::max({wsz, w1, w2});
     }
-    for (void *&w : b->d_works) BTRY(balloc(&w, wsz));
+    if (wsz > 0)
+        for (void *&w : b->d_works) BTRY(balloc(&w, wsz));
     BTRY(build_tiles<T>(b));
     BTRY_CUDA(cudaStreamSynchronize(b->stream));
     return SPME_OK;
@@ -851,6 +895,28 @@ int positions_body(_spme_batch_t *b, const double *pos) {
     return from_cuda(cudaGetLastError());
 }
 
+// x and y transforms of a group (forward, or inverse), and its z transforms with the
+// influence.
+template <typename T>
+cudaError_t own_xy(_spme_batch_t *b, const FftGroup &grp, bool inverse, cudaStream_t s) {
+    b->launches += 2;
+    return launch_fft_xy<T>(grp.K, inverse, (T *)b->d_mesh + grp.mesh_off,
+                            (T *)b->d_spec + 2 * grp.spec_off, (long)b->C * grp.nsys * grp.K,
+                            (const T *)grp.d_tw, s);
+}
+template <typename T>
+cudaError_t own_z(_spme_batch_t *b, const FftGroup &grp, cudaStream_t s) {
+    b->launches++;
+    const T *tab = (const T *)b->d_tab + 2 * grp.tab_off;
+    const double *tl = b->d_twopi_L + grp.sys_off;
+    if constexpr (sizeof(T) == 4)
+        return launch_zfft2(grp.K, grp.zmap, tab, (const T *)grp.d_tw, 1.0, tl, grp.nsys, b->R,
+                            b->d_err, s);
+    else
+        return launch_zfft64(grp.K, (T *)b->d_spec + 2 * grp.spec_off, tab, (const T *)grp.d_tw, 1.0,
+                             tl, grp.nsys, b->R, s);
+}
+
 // One direction of every group's transform: groups round-robin on the FFT
 // streams (forked from and joined back to the batch's stream), or all on the
 // batch's stream.
@@ -865,6 +931,14 @@ int run_ffts(_spme_batch_t *b, bool inverse, bool conc) {
     for (size_t q = 0; q < b->groups.size(); q++) {
         FftGroup &grp = b->groups[q];
         const int j = (int)(q % ns);
+        if (grp.own) {
+            cudaStream_t gs = conc ? b->fft_stream[j] : s;
+            // concurrent groups run their influence with the forward transform
+            if (!inverse) BTRY_CUDA(own_xy<T>(b, grp, false, gs));
+            if (!inverse && conc) BTRY_CUDA(own_z<T>(b, grp, gs));
+            if (inverse) BTRY_CUDA(own_xy<T>(b, grp, true, gs));
+            continue;
+        }
         cufftHandle h = inverse ? grp.bwd : grp.fwd;
         if (cufftSetStream(h, conc ? b->fft_stream[j] : s) != CUFFT_SUCCESS ||
             cufftSetWorkArea(h, b->d_works[j]) != CUFFT_SUCCESS)
@@ -915,9 +989,15 @@ int apply_body(_spme_batch_t *b, double alpha, const T *f, double beta, T *u) {
     const bool fconc = !b->profiling && (b->overlap & 2);
     BTRY(run_ffts<T>(b, false, fconc));
     mark(b, 5);
-    k_batch_influence<T><<<grid_cap((long)b->tot_infl * 256, 256, 8), 256, 0, s>>>(
-        (Cx2<T> *)b->d_spec, (const T *)b->d_tab, b->d_infl_sys, b->d_pre_infl, b->nsys,
-        b->tot_infl, b->R);
+    if (!fconc)
+        for (FftGroup &grp : b->groups)
+            if (grp.own) BTRY_CUDA(own_z<T>(b, grp, s));
+    if (b->tot_infl > 0) {
+        k_batch_influence<T><<<grid_cap((long)b->tot_infl * 256, 256, 8), 256, 0, s>>>(
+            (Cx2<T> *)b->d_spec, (const T *)b->d_tab, b->d_infl_sys, b->d_pre_infl, b->nsys,
+            b->tot_infl, b->R);
+        b->launches++;
+    }
     mark(b, 6);
     BTRY(run_ffts<T>(b, true, fconc));
     mark(b, 7);
@@ -936,7 +1016,7 @@ int apply_body(_spme_batch_t *b, double alpha, const T *f, double beta, T *u) {
         (T)beta, u);
     mark(b, 9);
     b->stages_valid = b->profiling;
-    b->launches += 6 + (long)b->igroups.size();
+    b->launches += 5 + (long)b->igroups.size();
     return from_cuda(cudaGetLastError());
 }
 
@@ -966,6 +1046,7 @@ void destroy_b(_spme_batch_t *b) {
     for (FftGroup &g : b->groups) {
         if (g.fwd) cufftDestroy(g.fwd);
         if (g.bwd) cufftDestroy(g.bwd);
+        if (g.d_tw) cudaFree(g.d_tw);
     }
     void *bufs[] = {b->d_sysid, b->d_pref,  b->d_geo,   b->d_key1,  b->d_key2,
                     b->d_key3,  b->d_sort_tmp, b->d_count, b->d_off1,
@@ -975,7 +1056,7 @@ void destroy_b(_spme_batch_t *b) {
                     b->d_Fs,    b->d_F2,    b->d_W,     b->d_W2,    b->d_mesh,  b->d_spec,  b->d_tab,
                     b->d_pair,  b->d_err,   b->d_spread_sys, b->d_interp_sys,
                     b->d_real_sys, b->d_infl_sys, b->d_pre_spread, b->d_pre_interp,
-                    b->d_pre_real, b->d_pre_infl};
+                    b->d_pre_real, b->d_pre_infl, b->d_twopi_L};
     for (void *p : bufs)
         if (p) cudaFree(p);
     for (void *w : b->d_works)

@@ -240,13 +240,15 @@ bool make_zplan(int K, size_t elem, ZPlan *zp, std::vector<double> *tw, std::vec
 // Columns per block for K (0 if K does not fit the fused kernel).
 int zfft_width(int K, size_t elem);
 // Two-factor form of the same operation (zfft2.cu; FP32, K <= 256): columns per
-// block (0: not this K), and its launch.
+// block (0: not this K), and its launch.  Batches: nsys systems of R right-hand sides each,
+// spectra and tables consecutive, 2 pi / L of every system at twopi_Ls (L unused);
+// else 1 and null.
 int zfft2_width(int K);
 cudaError_t launch_zfft2(int K, const CUtensorMap &map, const float *tab2, const float *tw, double L,
-                         int R, int *err, cudaStream_t s);
+                         const double *twopi_Ls, int nsys, int R, int *err, cudaStream_t s);
 // Its FP64 form (zfft64.cu; K of fft_xy_ok, elem 8), on G in place.
-cudaError_t launch_zfft64(int K, double *G, const double *tab2, const double *tw, double L, int R,
-                          cudaStream_t s);
+cudaError_t launch_zfft64(int K, double *G, const double *tab2, const double *tw, double L,
+                          const double *twopi_Ls, int nsys, int R, cudaStream_t s);
 // Two-factor x and y transforms of the mesh's z-planes (fft_xy.cuh; K = 2^a 3^b 5^c, 16 to
 // 256, fft_xy_ok): mesh -> G, or G -> mesh (inv; G is overwritten).  tw as for the z transform.
 bool fft_xy_ok(int K, size_t elem);

@@ -615,9 +615,9 @@ cudaError_t launch_zfft_influence(const CUtensorMap &map, T *G, const T *tab2, c
     // FP32, K = R1 R2 of the supported list: compile-time radices, three passes (influence
     // stage at K = 256, R = 16 1.80 -> 1.19 ms, K = 160 .780 -> .350, K = 75, R = 8 .154 -> .025)
     if constexpr (sizeof(T) == 4) {
-        if (zfft2_width(K) > 0) return launch_zfft2(K, map, tab2, tw, L, R, err, s);
+        if (zfft2_width(K) > 0) return launch_zfft2(K, map, tab2, tw, L, nullptr, 1, R, err, s);
     } else {
-        if (fft_xy_ok(K, 8)) return launch_zfft64(K, G, tab2, tw, L, R, s);
+        if (fft_xy_ok(K, 8)) return launch_zfft64(K, G, tab2, tw, L, nullptr, 1, R, s);
     }
     const int ci = zcfg_index(K, sizeof(T));
     if (ci < 0) return cudaErrorInvalidValue;

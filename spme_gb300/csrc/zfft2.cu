@@ -36,9 +36,9 @@ int zfft2_width(int K) {
 }
 
 cudaError_t launch_zfft2(int K, const CUtensorMap &map, const float *tab2, const float *tw, double L,
-                         int R, int *err, cudaStream_t s) {
+                         const double *twopi_Ls, int nsys, int R, int *err, cudaStream_t s) {
 #define SPME_Z2_CASE(A, B) \
-    if (K == A * B) return launch_z2<z2_width(A * B), A, B>(map, tab2, tw, L, R, err, s);
+    if (K == A * B) return launch_z2<z2_width(A * B), A, B>(map, tab2, tw, L, twopi_Ls, nsys, R, err, s);
     SPME_Z2_LIST(SPME_Z2_CASE)
 #undef SPME_Z2_CASE
     return cudaErrorInvalidValue;

@@ -75,17 +75,22 @@ __device__ __forceinline__ bool z2_sync_and(bool p) {
     return r != 0;
 }
 
-// One block per chunk of W consecutive columns and range of right-hand sides
-// [blockIdx.y rs, +rs).  Threads 0 .. CT-1 transform (thread = column + W index),
+// One block per chunk of W consecutive columns, range of right-hand sides
+// [blockIdx.y rs, +rs) and system blockIdx.z (batches: R right-hand sides and one table
+// each, box sizes through twopi_Ls).  Threads 0 .. CT-1 transform (thread = column + W index),
 // the warp after them moves data.
 template <int W, int R1, int R2>
 __global__ void __launch_bounds__(z2_threads(W, R1, R2) + 32, z2_minb(W, R1, R2))
 k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab2,
-        const float2 *__restrict__ tw_g, float twopi_L, int R, int rs, int *__restrict__ err) {
+        const float2 *__restrict__ tw_g, float twopi_L, const double *__restrict__ twopi_Ls, int R,
+        int rs, int *__restrict__ err) {
     constexpr int K = R1 * R2, Kh = K / 2 + 1, CT = z2_threads(W, R1, R2);
     const int plane = K * Kh;
     const int f0 = blockIdx.x * W, tid = threadIdx.x;
     const int rb = blockIdx.y * rs, nr = min(rs, R - rb);
+    const int c0 = 3 * (blockIdx.z * R + rb);  // first component
+    if (twopi_Ls) twopi_L = (float)twopi_Ls[blockIdx.z];
+    tab2 += (size_t)blockIdx.z * K * plane;
     extern __shared__ __align__(128) unsigned char zsm_raw[];
     unsigned char *zsm = zsm_raw + ((128u - (smem_addr(zsm_raw) & 127u)) & 127u);
     constexpr ZSmem2 lay(K, W);
@@ -114,7 +119,7 @@ k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab
             mbar_expect_tx(&full[b], bytes);
             float2 *dst = b ? buf1 : buf0;
             for (int d = 0; d < 3; d++)
-                tma_load_3d(dst + d * GS, &gmap, 2 * f0, 0, 3 * (rb + r) + d, &full[b]);
+                tma_load_3d(dst + d * GS, &gmap, 2 * f0, 0, c0 + 3 * r + d, &full[b]);
         };
         issue_load(0, 0);
         int issued = 1;
@@ -125,7 +130,7 @@ k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab
             if (!mbar_wait(&done[b], (uint32_t)((r >> 1) & 1))) break;
             const float2 *src = b ? buf1 : buf0;
             for (int d = 0; d < 3; d++)
-                tma_store_3d(&gmap, 2 * f0, 0, 3 * (rb + r) + d, src + d * GS);
+                tma_store_3d(&gmap, 2 * f0, 0, c0 + 3 * r + d, src + d * GS);
             bulk_commit_group();
             if (r + 2 < nr) {
                 bulk_wait_read_all();  // buffer b is free again
@@ -245,21 +250,22 @@ k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab
 }
 
 template <int W, int R1, int R2>
-cudaError_t launch_z2(const CUtensorMap &map, const float *tab2, const float *tw, double L, int R,
-                      int *err, cudaStream_t s) {
+cudaError_t launch_z2(const CUtensorMap &map, const float *tab2, const float *tw, double L,
+                      const double *twopi_Ls, int nsys, int R, int *err, cudaStream_t s) {
     constexpr int K = R1 * R2;
     constexpr size_t smem = ZSmem2(K, W).total + 128;
     auto kern = k_zfft2<W, R1, R2>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int nchunk = (K * (K / 2 + 1) + W - 1) / W;
+    const long blocks = (long)nchunk * nsys;
     // right-hand sides per block: all of them, or fewer (at least two, for the second
     // buffer) until the resident blocks are filled about four times
     int rs = R;
-    while (rs > 2 && (long)nchunk * ((R + rs - 1) / rs) < 608L * z2_minb(W, R1, R2)) rs = (rs + 1) / 2;
-    kern<<<dim3(nchunk, (R + rs - 1) / rs), z2_threads(W, R1, R2) + 32, smem, s>>>(
+    while (rs > 2 && blocks * ((R + rs - 1) / rs) < 608L * z2_minb(W, R1, R2)) rs = (rs + 1) / 2;
+    kern<<<dim3(nchunk, (R + rs - 1) / rs, nsys), z2_threads(W, R1, R2) + 32, smem, s>>>(
         map, reinterpret_cast<const float2 *>(tab2), reinterpret_cast<const float2 *>(tw),
-        (float)(2.0 * M_PI / L), R, rs, err);
+        (float)(2.0 * M_PI / L), twopi_Ls, R, rs, err);
     return cudaGetLastError();
 }
 

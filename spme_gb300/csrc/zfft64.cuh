@@ -33,7 +33,7 @@ __host__ __device__ constexpr int z64_minb(int R1, int R2) {
 template <int R1, int R2>
 __global__ void __launch_bounds__(z64_threads(R1, R2), z64_minb(R1, R2))
 k_z64(double2 *__restrict__ G, const double2 *__restrict__ tab2, const double2 *__restrict__ tw,
-      double twopi_L) {
+      double twopi_L, const double *__restrict__ twopi_Ls, int R) {
     constexpr int K = R1 * R2, Kh = K / 2 + 1, W = z64_cols(K), NT = z64_threads(R1, R2);
     constexpr int plane = K * Kh;
     extern __shared__ __align__(16) unsigned char zsm[];
@@ -41,6 +41,11 @@ k_z64(double2 *__restrict__ G, const double2 *__restrict__ tab2, const double2 *
     const int tid = threadIdx.x, w = tid % W, id = tid / W;
     const int fl = blockIdx.x * W + w;
     const bool valid = fl < plane;
+    if (twopi_Ls) {  // batch: blockIdx.y = system and right-hand side
+        const int sys = blockIdx.y / R;
+        twopi_L = twopi_Ls[sys];
+        tab2 += (size_t)sys * K * plane;
+    }
     {
         const int d = id / R2, n2 = id - d * R2;
         if (d < 3 && valid) {
@@ -133,16 +138,17 @@ k_z64(double2 *__restrict__ G, const double2 *__restrict__ tab2, const double2 *
 }
 
 template <int R1, int R2>
-cudaError_t launch_z64_k(double *G, const double *tab2, const double *tw, double L, int R, cudaStream_t s) {
+cudaError_t launch_z64_k(double *G, const double *tab2, const double *tw, double L,
+                         const double *twopi_Ls, int nsys, int R, cudaStream_t s) {
     constexpr int K = R1 * R2, W = z64_cols(K), smem = 3 * K * W * (int)sizeof(double2);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_z64<R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
     const unsigned nb = (K * (K / 2 + 1) + W - 1) / W;
-    k_z64<R1, R2><<<dim3(nb, R), z64_threads(R1, R2), smem, s>>>(
+    k_z64<R1, R2><<<dim3(nb, R * nsys), z64_threads(R1, R2), smem, s>>>(
         reinterpret_cast<double2 *>(G), reinterpret_cast<const double2 *>(tab2),
-        reinterpret_cast<const double2 *>(tw), 2.0 * M_PI / L);
+        reinterpret_cast<const double2 *>(tw), 2.0 * M_PI / L, twopi_Ls, R);
     return cudaGetLastError();
 }
 
