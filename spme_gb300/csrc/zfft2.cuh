@@ -19,7 +19,7 @@
 // SMs idle.
 // Bound: HBM (one read and one write of the half spectrum, 0.98 ms at K = 256, R =
 // 16), then shared-memory traffic and latency at one or two blocks per SM.
-// Influence stage, radix passes of zfft.cu -> here: K = 256, R = 16 1.80 -> 1.19 ms;
+// Influence stage, radix passes of zfft.cu -> here: K = 256, R = 16 1.80 -> 1.20 ms;
 // K = 160, R = 16 .780 -> .350; K = 128, R = 1 .037 -> .021; K = 75, R = 8 .154 -> .025.
 // Sixteen- by ten-point factors (K = 160: one thread per column and index for all three
 // components) need 168 registers a thread; 20 x 8 needs 126.
@@ -55,6 +55,16 @@ __host__ __device__ constexpr int z2_minb(int W, int R1, int R2) {
     const int br = 65536 / (regs * ((z2_threads(W, R1, R2) + 32 + 127) / 128 * 128));
     const int m = bs < br ? bs : br;
     return m < 1 ? 1 : m > 8 ? 8 : m;
+}
+
+// Whether the influence table is read for every right-hand side instead of held: where the
+// radices leave no registers for it.  At K = 256 a block's shared memory leaves too little L1
+// for the spills.  Stage in ms, held / read again, R = 16: K = 256 1.66 / 1.20, K = 250 (25 x 10)
+// 1.87 / 1.37, K = 240 1.14 / 1.06, K = 150 .341 / .313; K = 216 (24 x 9) .793 / .834, K = 160
+// .342 / .366, K = 75 .041 / .043.
+__host__ __device__ constexpr bool z2_reload(int W, int R1, int R2) {
+    const int regs = 65536 / (z2_minb(W, R1, R2) * ((z2_threads(W, R1, R2) + 32 + 127) / 128 * 128));
+    return R1 >= 24 && (R2 >= 10 || regs <= 104);
 }
 
 template <int N>
@@ -161,13 +171,17 @@ k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab
     // (s_x = +1 on these planes)
     const bool xplane = valid && (kx == 0 || (K % 2 == 0 && kx == K / 2));
     const bool sy = ky == 0 || (K % 2 == 0 && ky == K / 2);
-    // the influence table of this thread's frequencies, read once for all its
-    // right-hand sides
+    // the influence table of this thread's frequencies: read once for all its right-hand
+    // sides, or (RELOAD) for each between the passes
+    constexpr bool RELOAD = z2_reload(W, R1, R2);
     float2 mc[R2];
+    auto load_mc = [&]() {
 #pragma unroll
-    for (int k2 = 0; k2 < R2; k2++)
-        mc[k2] = id < R1 && valid ? __ldg(tab2 + (size_t)(id + R1 * k2) * plane + fl)
-                                  : make_float2(0.f, 0.f);
+        for (int k2 = 0; k2 < R2; k2++)
+            mc[k2] = id < R1 && valid ? __ldg(tab2 + (size_t)(id + R1 * k2) * plane + fl)
+                                      : make_float2(0.f, 0.f);
+    };
+    if constexpr (!RELOAD) load_mc();
 
     for (int r = 0; r < nr; r++) {
         const int b = r & 1;
@@ -191,6 +205,7 @@ k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab
                 x1[k1 * R2 * W] = z_tw(v[k1], t.x, t.y);
             }
         }
+        if constexpr (RELOAD) load_mc();
         z2_sync<CT>();
         // second pass: R2-point transforms, influence, inverse R2-point transforms
         if (id < R1) {
