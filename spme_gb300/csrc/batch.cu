@@ -599,7 +599,7 @@ int build_tiles(_spme_batch_t *b) {
         A.ce = b->C;
         A.accumulate = 0;
         // TMA boxes where the mesh rows allow them (K a multiple of 16 bytes / elem);
-        // plain-load staging otherwise
+        // asynchronous copies otherwise
         A.use_tma = make_interp_box(&is[q].tmap, A.mesh, b->C, x.g, sizeof(T)) ? 1 : 0;
         A.ws = b->ws;
         grp.total += x.g.ntx * x.g.nty * x.g.ntz;

@@ -6,6 +6,8 @@
 
 #include <utility>
 
+#include "cp_async.cuh"
+
 namespace spme {
 
 // fn(std::integral_constant<int, i>) for i = 0 .. N-1, unrolled at compile time.
@@ -16,25 +18,6 @@ __device__ __forceinline__ void static_for_impl(Fn &&fn, std::integer_sequence<i
 template <int N, typename Fn>
 __device__ __forceinline__ void static_for(Fn &&fn) {
     static_for_impl(fn, std::make_integer_sequence<int, N>{});
-}
-
-// Asynchronous global -> shared copies (cp.async, completion tracked per thread).
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
-                 : "memory");
-}
-template <int B>
-__device__ __forceinline__ void cp_async_small(void *dst, const void *src) {
-    static_assert(B == 4 || B == 8, "4 or 8 bytes");
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src),
-                 "n"(B)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Components per lane for C components (chunks of 16 CPL components per block).
