@@ -23,6 +23,7 @@
 
 #include "fft_dft.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace spme {
 namespace {
@@ -53,6 +54,7 @@ template <typename T, int R1, int R2>
 __global__ void __launch_bounds__(kXPairs * zmax(R1, R2), xy_minb<T>(kXPairs * zmax(R1, R2), zmax(R1, R2)))
 k_fft_x_fwd(const T *__restrict__ mesh, typename ZVec<T>::type *__restrict__ G,
             const typename ZVec<T>::type *__restrict__ tw, long rows) {
+    pdl_wait();
     using V = typename ZVec<T>::type;
     constexpr int K = R1 * R2, Kh = K / 2 + 1, P = kXPairs, RS = x_stride(R2);
     extern __shared__ __align__(16) unsigned char xsm[];
@@ -123,6 +125,7 @@ template <typename T, int R1, int R2>
 __global__ void __launch_bounds__(kXPairs * zmax(R1, R2), xy_minb<T>(kXPairs * zmax(R1, R2), zmax(R1, R2)))
 k_fft_x_inv(const typename ZVec<T>::type *__restrict__ G, T *__restrict__ mesh,
             const typename ZVec<T>::type *__restrict__ tw, long rows) {
+    pdl_wait();
     using V = typename ZVec<T>::type;
     constexpr int K = R1 * R2, Kh = K / 2 + 1, P = kXPairs, RS = x_stride(R2);
     extern __shared__ __align__(16) unsigned char xsm[];
@@ -208,6 +211,7 @@ template <typename T, int R1, int R2>
 __global__ void __launch_bounds__(xy_cols<T>(R1, R2) * zmax(R1, R2), xy_minb<T>(xy_cols<T>(R1, R2) * zmax(R1, R2), zmax(R1, R2)))
 k_fft_y(typename ZVec<T>::type *__restrict__ G, const typename ZVec<T>::type *__restrict__ tw, long cols,
         int inv) {
+    pdl_wait();
     using V = typename ZVec<T>::type;
     constexpr int K = R1 * R2, Kh = K / 2 + 1, W = xy_cols<T>(R1, R2);
     extern __shared__ __align__(16) unsigned char xsm[];
@@ -267,11 +271,11 @@ cudaError_t launch_xy(bool inv, T *mesh, T *G, long planes, const T *tw, cudaStr
         e = cudaFuncSetAttribute(k_fft_y<T, R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ysmem);
     if (e != cudaSuccess) return e;
     if (inv) {
-        k_fft_y<T, R1, R2><<<yb, W * M, ysmem, s>>>(g, t, cols, 1);
-        k_fft_x_inv<T, R1, R2><<<xb, P * M, xsmem, s>>>(g, mesh, t, rows);
+        pdl_launch(k_fft_y<T, R1, R2>, yb, W * M, ysmem, s, g, t, cols, 1);
+        pdl_launch(k_fft_x_inv<T, R1, R2>, xb, P * M, xsmem, s, g, mesh, t, rows);
     } else {
-        k_fft_x_fwd<T, R1, R2><<<xb, P * M, xsmem, s>>>(mesh, g, t, rows);
-        k_fft_y<T, R1, R2><<<yb, W * M, ysmem, s>>>(g, t, cols, 0);
+        pdl_launch(k_fft_x_fwd<T, R1, R2>, xb, P * M, xsmem, s, mesh, g, t, rows);
+        pdl_launch(k_fft_y<T, R1, R2>, yb, W * M, ysmem, s, g, t, cols, 0);
     }
     return cudaGetLastError();
 }

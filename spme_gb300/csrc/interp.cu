@@ -22,6 +22,7 @@
 #include "cp_async.cuh"
 #include "kernels.h"
 #include "tma.cuh"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -345,6 +346,7 @@ template <typename T, int P, int CG>
 // blocks per SM that the 4-component box's shared memory allows (16x8x4 tiles)
 __global__ void __launch_bounds__(kThreads, 5)
 k_interp(const __grid_constant__ CUtensorMap tmap, InterpArgs<T> A) {
+    pdl_wait();
     // tiles z fastest: blocks launched together are z neighbours, whose boxes
     // share p - 1 of their tz + p - 1 planes (read from L2 by the later ones)
     const int b = blockIdx.x, ntx = A.g.ntx, nty = A.g.nty, ntz = A.g.ntz;
@@ -395,7 +397,7 @@ cudaError_t launch_interp_t(const InterpMaps &maps, const int *tile_off, const i
     const CUtensorMap &m = maps.cg4;
     InterpArgs<T> A{tile_off, rec_idx, rec_start, rec_w, mesh, W, err, g, C, cb, ce,
                     accumulate, use ? 1 : 0, RecordWidth<T, P>::value};
-    kern<<<g.ntx * g.nty * g.ntz, kThreads, smem, s>>>(m, A);
+    pdl_launch(kern, g.ntx * g.nty * g.ntz, kThreads, smem, s, m, A);
     return cudaGetLastError();
 }
 

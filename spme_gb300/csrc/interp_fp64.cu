@@ -20,6 +20,7 @@
 #include "cp_async.cuh"
 #include "kernels.h"
 #include "tma.cuh"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -134,6 +135,7 @@ __device__ __forceinline__ void interp64_body(const CUtensorMap *tmap,
 template <int P>
 __global__ void __launch_bounds__(kThreads)
 k_interp64(const __grid_constant__ CUtensorMap tmap, InterpArgs<double> A) {
+    pdl_wait();
     // tiles z fastest, as in the FP32 kernel: z neighbours share halo planes
     const int b = blockIdx.x, ntx = A.g.ntx, nty = A.g.nty, ntz = A.g.ntz;
     const int tiz = b % ntz, rest = b / ntz;
@@ -168,7 +170,7 @@ cudaError_t launch_p(const CUtensorMap &map, const InterpArgs<double> &A, cudaSt
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(A.g.ntx * A.g.nty * A.g.ntz, A.ce - A.cb), kThreads, smem, s>>>(map, A);
+    pdl_launch(kern, dim3(A.g.ntx * A.g.nty * A.g.ntz, A.ce - A.cb), kThreads, smem, s, map, A);
     return cudaGetLastError();
 }
 

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -71,6 +72,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 k_pack_tiled(const T *__restrict__ f, long ld, int n, int R, int r0, int r1, int pb, int vec,
              T *__restrict__ F, T *__restrict__ F2) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char pk_raw[];
     T *tile = reinterpret_cast<T *>(pk_raw);  // [pb][CP + 1]
     const int C = 3 * R, CP = 3 * (r1 - r0), CS = CP + 1;  // row stride, columns written
@@ -163,6 +165,7 @@ template <typename T, bool SUM>
 __global__ void __launch_bounds__(256)
 k_unpack_tiled(const T *__restrict__ W, const T *__restrict__ W2, int n, int R, int r0, int r1,
                int pb, int vec, T alpha, T beta, T *__restrict__ u, long ld) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char pk_raw[];
     T *tile = reinterpret_cast<T *>(pk_raw);  // [pb][CP + 1]
     const int C = 3 * R, CP = 3 * (r1 - r0), CS = CP + 1;  // row stride, columns taken
@@ -306,7 +309,7 @@ void launch_pack_tiled(const T *f, long ld, int n, int R, int r0, int r1, T *F, 
     const int pb = tile_particles(r1 - r0, sizeof(T));
     const size_t smem = (size_t)pb * (3 * (r1 - r0) + 1) * sizeof(T);
     const int vec = vec_tiles<T>(f, ld, F, R, r0, r1, pb);
-    k_pack_tiled<T><<<tiled_blocks(n, pb), 256, smem, s>>>(f, ld, n, R, r0, r1, pb, vec, F,
+    pdl_launch(k_pack_tiled<T>, tiled_blocks(n, pb), 256, smem, s, f, ld, n, R, r0, r1, pb, vec, F,
                                                                F2);
 }
 
@@ -319,10 +322,10 @@ void launch_unpack_tiled(const T *W, const T *W2, int n, int R, int r0, int r1, 
     const int vec = vec_tiles<T>(u, ld, W, R, r0, r1, pb) &&
                     (!W2 || (uintptr_t)W2 % 16 == 0);
     if (W2)
-        k_unpack_tiled<T, true><<<tiled_blocks(n, pb), 256, smem, s>>>(
+        pdl_launch(k_unpack_tiled<T, true>, tiled_blocks(n, pb), 256, smem, s, 
             W, W2, n, R, r0, r1, pb, vec, (T)alpha, (T)beta, u, ld);
     else
-        k_unpack_tiled<T, false><<<tiled_blocks(n, pb), 256, smem, s>>>(
+        pdl_launch(k_unpack_tiled<T, false>, tiled_blocks(n, pb), 256, smem, s, 
             W, W, n, R, r0, r1, pb, vec, (T)alpha, (T)beta, u, ld);
 }
 

@@ -4,6 +4,7 @@
 #include <climits>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -50,6 +51,7 @@ __global__ void k_all_keys(const double *__restrict__ pos, int n, MeshGeom g, in
                            int *__restrict__ key3, int *__restrict__ count3,
                            int *__restrict__ slot3, uint32_t *__restrict__ pstart,
                            T *__restrict__ pfrac, typename Vec4T<T>::type *__restrict__ prel) {
+    pdl_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int s[3] = {0, 0, 0}, cc[3] = {0, 0, 0};
@@ -126,6 +128,7 @@ __device__ int block_exclusive_scan(int v, int &total) {
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int *__restrict__ in, int n,
                                                              int *__restrict__ sums) {
+    pdl_wait();
     long base = (long)blockIdx.x * kScanTile + (long)threadIdx.x * kScanItems;
     int s = 0;
 #pragma unroll
@@ -138,6 +141,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int *__restr
 
 // Exclusive scan of sums[0..nb) in place, one block, looping with a carry.
 __global__ void __launch_bounds__(kScanThreads) k_scan_sums(int *__restrict__ sums, int nb) {
+    pdl_wait();
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -188,6 +192,7 @@ __device__ __forceinline__ void put_ends(const Sorts &S, int n) {
 __global__ void __launch_bounds__(kScanThreads) k_scan_final(const int *__restrict__ in, int total,
                                                             const int *__restrict__ sums, Sorts S,
                                                             int n) {
+    pdl_wait();
     long base = (long)blockIdx.x * kScanTile + (long)threadIdx.x * kScanItems;
     int v[kScanItems];
     int s = 0;
@@ -213,6 +218,7 @@ constexpr int kScanOne = 32 * 1024;
 __device__ __forceinline__ int pad32(int i) { return i + (i >> 5); }
 __global__ void __launch_bounds__(kScanOneThreads) k_scan_one(const int *__restrict__ in, int total,
                                                               Sorts S, int n) {
+    pdl_wait();
     extern __shared__ int cnt[];
     for (int i = threadIdx.x; i < total; i += kScanOneThreads) cnt[pad32(i)] = in[i];
     __syncthreads();
@@ -234,6 +240,7 @@ __global__ void __launch_bounds__(kScanOneThreads) k_scan_one(const int *__restr
 
 // Sort blockIdx.y: particle i to its bucket, in the order of the atomic slots.
 __global__ void k_scatter(Sorts S, int n, int *__restrict__ tmp) {
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const Sort &s = S.s[blockIdx.y];
@@ -250,6 +257,7 @@ constexpr int kStableMax = 16384;
 // same rounding) on every run.  Consecutive q share a key, so the lanes of a
 // warp read the same entries (broadcast loads).
 __global__ void k_stable_place(Sorts S, int n, const int *__restrict__ tmp) {
+    pdl_wait();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
     const Sort &s = S.s[blockIdx.y];
@@ -278,6 +286,7 @@ k_records(const uint32_t *__restrict__ pstart, const T *__restrict__ pfrac, int 
           RecordSet<T> set0, RecordSet<T> set1,
           const typename Vec4T<T>::type *__restrict__ prel, const int *__restrict__ cperm,
           typename Vec4T<T>::type *__restrict__ cpos) {
+    pdl_wait();
     constexpr int WS = RecordWidth<T, P>::value;
     constexpr int VQ = WS * (int)sizeof(T) / 16;  // 16-byte pieces per record
     __shared__ __align__(16) T sm[kRecThreads * WS];
@@ -346,11 +355,11 @@ void launch_all_keys(const double *pos, int n, const MeshGeom &g, int nc, int *k
                      cudaStream_t s) {
     if (n <= 0) return;
     if (fp32)
-        k_all_keys<float><<<nblk(n, 256), 256, 0, s>>>(pos, n, g, nc, key1, count1, slot1, key2,
+        pdl_launch(k_all_keys<float>, nblk(n, 256), 256, 0, s, pos, n, g, nc, key1, count1, slot1, key2,
                                                        count2, slot2, key3, count3, slot3, pstart,
                                                        (float *)pfrac, (float4 *)prel);
     else
-        k_all_keys<double><<<nblk(n, 256), 256, 0, s>>>(pos, n, g, nc, key1, count1, slot1, key2,
+        pdl_launch(k_all_keys<double>, nblk(n, 256), 256, 0, s, pos, n, g, nc, key1, count1, slot1, key2,
                                                         count2, slot2, key3, count3, slot3, pstart,
                                                         (double *)pfrac, (double4_32a *)prel);
 }
@@ -381,19 +390,19 @@ int launch_sorts(const Sorts &S, const int *count, int n, int *scan_tmp, int *tm
         const size_t smem = sizeof(int) * (size_t)(total + total / 32 + 1);
         cudaFuncSetAttribute(k_scan_one, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(sizeof(int) * (kScanOne + kScanOne / 32 + 1)));
-        k_scan_one<<<1, kScanOneThreads, smem, s>>>(count, total, S, n);
+        pdl_launch(k_scan_one, 1, kScanOneThreads, smem, s, count, total, S, n);
         launches = 1;
     } else {
         const int nb = nblk(total, kScanTile);
-        k_scan_reduce<<<nb, kScanThreads, 0, s>>>(count, total, scan_tmp);
-        k_scan_sums<<<1, kScanThreads, 0, s>>>(scan_tmp, nb);
-        k_scan_final<<<nb, kScanThreads, 0, s>>>(count, total, scan_tmp, S, n);
+        pdl_launch(k_scan_reduce, nb, kScanThreads, 0, s, count, total, scan_tmp);
+        pdl_launch(k_scan_sums, 1, kScanThreads, 0, s, scan_tmp, nb);
+        pdl_launch(k_scan_final, nb, kScanThreads, 0, s, count, total, scan_tmp, S, n);
         launches = 3;
     }
     if (n <= 0) return launches;
     const dim3 grid(nblk(n, 256), S.count);
-    k_scatter<<<grid, 256, 0, s>>>(S, n, tmp);
-    k_stable_place<<<grid, 256, 0, s>>>(S, n, tmp);
+    pdl_launch(k_scatter, grid, 256, 0, s, S, n, tmp);
+    pdl_launch(k_stable_place, grid, 256, 0, s, S, n, tmp);
     return launches + 2;
 }
 
@@ -406,9 +415,9 @@ void launch_records(const uint32_t *pstart, const T *pfrac, int n, int p, int ns
     const dim3 grid(nblk(n, kRecThreads), nset + (cpos ? 1 : 0));
     const RecordSet<T> s0 = nset > 0 ? sets[0] : RecordSet<T>{}, s1 = nset > 1 ? sets[1] : s0;
     switch (p) {
-        case 4: k_records<T, 4><<<grid, kRecThreads, 0, s>>>(pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
-        case 6: k_records<T, 6><<<grid, kRecThreads, 0, s>>>(pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
-        case 8: k_records<T, 8><<<grid, kRecThreads, 0, s>>>(pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
+        case 4: pdl_launch(k_records<T, 4>, grid, kRecThreads, 0, s, pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
+        case 6: pdl_launch(k_records<T, 6>, grid, kRecThreads, 0, s, pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
+        case 8: pdl_launch(k_records<T, 8>, grid, kRecThreads, 0, s, pstart, pfrac, n, nset, s0, s1, (const V4 *)prel, cperm, (V4 *)cpos); break;
         default: break;
     }
 }

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "realspace_pairs.cuh"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -267,6 +268,7 @@ __device__ __forceinline__ void real_body(const RealArgs<float> &A, int cell) {
 
 template <int W, int RB>
 __global__ void __launch_bounds__(kRsThreads, 10) k_realspace(RealArgs<float> A) {
+    pdl_wait();
     real_body<W, RB>(A, blockIdx.x);
 }
 
@@ -294,7 +296,7 @@ struct Launch {
 template <int W, int RB>
 cudaError_t launch_form(const RealArgs<float> *one, const Launch &l) {
     if (one) {
-        k_realspace<W, RB><<<l.total, kRsThreads, 0, l.s>>>(*one);
+        pdl_launch(k_realspace<W, RB>, l.total, kRsThreads, 0, l.s, *one);
         return cudaGetLastError();
     }
     auto kern = k_realspace_batch<W, RB>;

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "realspace_pairs.cuh"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -129,6 +130,7 @@ __device__ __forceinline__ void realspace64_body(const RealArgs<double> &A, int 
 
 template <int RB>
 __global__ void __launch_bounds__(kRsThreads, RB == 1 ? 7 : 4) k_realspace64(RealArgs<double> A) {
+    pdl_wait();
     realspace64_body<RB>(A, blockIdx.x);
 }
 
@@ -176,10 +178,10 @@ cudaError_t launch_realspace<double>(int nc, const int *cell_off, const int *cel
                                                  xi, a, with_self, tab, W);
     const int ncell = nc * nc * nc;
     switch (sweep_width(R)) {
-        case 1: k_realspace64<1><<<ncell, kRsThreads, 0, s>>>(A); break;
-        case 2: k_realspace64<2><<<ncell, kRsThreads, 0, s>>>(A); break;
-        case 3: k_realspace64<3><<<ncell, kRsThreads, 0, s>>>(A); break;
-        default: k_realspace64<4><<<ncell, kRsThreads, 0, s>>>(A); break;
+        case 1: pdl_launch(k_realspace64<1>, ncell, kRsThreads, 0, s, A); break;
+        case 2: pdl_launch(k_realspace64<2>, ncell, kRsThreads, 0, s, A); break;
+        case 3: pdl_launch(k_realspace64<3>, ncell, kRsThreads, 0, s, A); break;
+        default: pdl_launch(k_realspace64<4>, ncell, kRsThreads, 0, s, A); break;
     }
     return cudaGetLastError();
 }

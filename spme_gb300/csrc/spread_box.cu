@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(32)
 k_spread_box(const int *__restrict__ tile_off, const int *__restrict__ rec_idx,
              const uint32_t *__restrict__ rec_start, const T *__restrict__ rec_w,
              const T *__restrict__ F, int C, int c0, MeshGeom g, T *__restrict__ boxes) {
+    pdl_wait();
     constexpr int WS = RecordWidth<T, P>::value;
     constexpr int NP3 = P * P * P, NJ = (NP3 + 31) / 32;
     constexpr int NPR = P * P + P;  // products: w_y w_z (p^2), then w_x f (p)
@@ -143,6 +145,7 @@ template <typename T, int MX, int MY, int MZ>
 __global__ void __launch_bounds__(256)
 k_box_sum(const T *__restrict__ boxes, const int4 *__restrict__ tab, int K, size_t slot, int c0,
           T *__restrict__ mesh) {
+    pdl_wait();
     const int row = blockIdx.x * blockDim.y + threadIdx.y;
     if (row >= K * K) return;
     const int y = row % K, z = row / K;
@@ -190,7 +193,7 @@ void launch_sum(const T *boxes, const BoxTable &bt, const MeshGeom &g, size_t sl
                 : m == 2 ? k_box_sum<T, 2, 4, 2>
                 : m == 4 ? k_box_sum<T, 2, 2, 4>
                          : k_box_sum<T, 4, 4, 4>;
-    kern<<<dim3((g.K * g.K + by - 1) / by, nc), dim3(bx, by), 0, s>>>(boxes, bt.tab, g.K, slot, c0,
+    pdl_launch(kern, dim3((g.K * g.K + by - 1) / by, nc), dim3(bx, by), 0, s, boxes, bt.tab, g.K, slot, c0,
                                                                       mesh);
 }
 
@@ -208,7 +211,7 @@ cudaError_t launch_box_t(const int *tile_off, const int *rec_idx, const uint32_t
     const size_t slot = (size_t)ntiles * b.vol;
     for (int c0 = 0; c0 < C; c0 += nslot) {
         const int nc = C - c0 < nslot ? C - c0 : nslot;
-        kern<<<dim3(ntiles, nc), 32, smem, s>>>(tile_off, rec_idx, rec_start, rec_w, F, C, c0, g,
+        pdl_launch(kern, dim3(ntiles, nc), 32, smem, s, tile_off, rec_idx, rec_start, rec_w, F, C, c0, g,
                                                 boxes);
         launch_sum<T>(boxes, bt, g, slot, c0, nc, mesh, s);
     }

@@ -38,6 +38,7 @@
 
 #include "kernels.h"
 #include "spread_cols.cuh"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -435,6 +436,7 @@ k_spread_cols_batch(const SpreadColsSys<T> *__restrict__ sys, const int *__restr
 template <typename T, int CPL>
 __global__ void k_gather_cols_rows(const T *__restrict__ F, const int *__restrict__ idx, int n,
                                    int C, int RW, int nchunk, T *__restrict__ Fs) {
+    pdl_wait();
     // one thread per (slot, chunk, lane): the lane's CPL components (padded to PC)
     // as one vector store
     constexpr int PC = cols_pcpl(CPL);
@@ -579,15 +581,15 @@ void launch_gather_cols_rows(const T *F, const int *idx, int n, int C, T *Fs, cu
     if (n <= 0) return;
     switch (cpl) {
         case 1:
-            k_gather_cols_rows<T, 1><<<blocks_for_rows(total), 256, 0, s>>>(F, idx, n, C, RW,
+            pdl_launch(k_gather_cols_rows<T, 1>, blocks_for_rows(total), 256, 0, s, F, idx, n, C, RW,
                                                                             nchunk, Fs);
             break;
         case 2:
-            k_gather_cols_rows<T, 2><<<blocks_for_rows(total), 256, 0, s>>>(F, idx, n, C, RW,
+            pdl_launch(k_gather_cols_rows<T, 2>, blocks_for_rows(total), 256, 0, s, F, idx, n, C, RW,
                                                                             nchunk, Fs);
             break;
         default:
-            k_gather_cols_rows<T, 3><<<blocks_for_rows(total), 256, 0, s>>>(F, idx, n, C, RW,
+            pdl_launch(k_gather_cols_rows<T, 3>, blocks_for_rows(total), 256, 0, s, F, idx, n, C, RW,
                                                                             nchunk, Fs);
             break;
     }

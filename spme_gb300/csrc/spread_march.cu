@@ -33,6 +33,7 @@
 
 #include "kernels.h"
 #include "spread_cols.cuh"
+#include "pdl.cuh"
 
 namespace spme {
 
@@ -467,6 +468,7 @@ __host__ __device__ constexpr int march_minb(int cpl) { return cpl == 1 ? 4 : cp
 template <int P, int CPL>
 __global__ void __launch_bounds__(kThreads, march_minb(CPL))
 k_spread_march(SpreadColsArgs<float> A) {
+    pdl_wait();
     spread_march_body<P, CPL>(A, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -514,7 +516,7 @@ cudaError_t launch_t(const SpreadColsArgs<float> &A, const SpreadColsGrid &g, cu
     auto kern = k_spread_march<P, CPL>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(g.x, g.y, g.blocks / (g.x * g.y)), kThreads, smem, s>>>(A);
+    pdl_launch(kern, dim3(g.x, g.y, g.blocks / (g.x * g.y)), kThreads, smem, s, A);
     return cudaGetLastError();
 }
 

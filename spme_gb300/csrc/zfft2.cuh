@@ -28,6 +28,7 @@
 #include "fft_dft.cuh"
 #include "kernels.h"
 #include "tma.cuh"
+#include "pdl.cuh"
 
 namespace spme {
 namespace {
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(z2_threads(W, R1, R2) + 32, z2_minb(W, R1, R2)
 k_zfft2(const __grid_constant__ CUtensorMap gmap, const float2 *__restrict__ tab2,
         const float2 *__restrict__ tw_g, float twopi_L, const double *__restrict__ twopi_Ls, int R,
         int rs, int *__restrict__ err) {
+    pdl_wait();
     constexpr int K = R1 * R2, Kh = K / 2 + 1, CT = z2_threads(W, R1, R2);
     const int plane = K * Kh;
     const int f0 = blockIdx.x * W, tid = threadIdx.x;
@@ -278,7 +280,7 @@ cudaError_t launch_z2(const CUtensorMap &map, const float *tab2, const float *tw
     // buffer) until the resident blocks are filled about four times
     int rs = R;
     while (rs > 2 && blocks * ((R + rs - 1) / rs) < 608L * z2_minb(W, R1, R2)) rs = (rs + 1) / 2;
-    kern<<<dim3(nchunk, (R + rs - 1) / rs, nsys), z2_threads(W, R1, R2) + 32, smem, s>>>(
+    pdl_launch(kern, dim3(nchunk, (R + rs - 1) / rs, nsys), z2_threads(W, R1, R2) + 32, smem, s, 
         map, reinterpret_cast<const float2 *>(tab2), reinterpret_cast<const float2 *>(tw),
         (float)(2.0 * M_PI / L), twopi_Ls, R, rs, err);
     return cudaGetLastError();

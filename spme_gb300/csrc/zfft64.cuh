@@ -16,6 +16,7 @@
 
 #include "fft_dft.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace spme {
 namespace {
@@ -36,6 +37,7 @@ template <int R1, int R2>
 __global__ void __launch_bounds__(z64_threads(R1, R2), z64_minb(R1, R2))
 k_z64(double2 *__restrict__ G, const double2 *__restrict__ tab2, const double2 *__restrict__ tw,
       double twopi_L, const double *__restrict__ twopi_Ls, int R) {
+    pdl_wait();
     constexpr int K = R1 * R2, Kh = K / 2 + 1, W = z64_cols(K), NT = z64_threads(R1, R2);
     constexpr int plane = K * Kh;
     extern __shared__ __align__(16) unsigned char zsm[];
@@ -148,7 +150,7 @@ cudaError_t launch_z64_k(double *G, const double *tab2, const double *tw, double
         if (e != cudaSuccess) return e;
     }
     const unsigned nb = (K * (K / 2 + 1) + W - 1) / W;
-    k_z64<R1, R2><<<dim3(nb, R * nsys), z64_threads(R1, R2), smem, s>>>(
+    pdl_launch(k_z64<R1, R2>, dim3(nb, R * nsys), z64_threads(R1, R2), smem, s, 
         reinterpret_cast<double2 *>(G), reinterpret_cast<const double2 *>(tab2),
         reinterpret_cast<const double2 *>(tw), 2.0 * M_PI / L, twopi_Ls, R);
     return cudaGetLastError();
