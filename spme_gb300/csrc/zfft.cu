@@ -1,5 +1,5 @@
-// Fused z-transform + k-space influence + inverse z-transform: FP64, and the FP32 sizes
-// that zfft2.cu does not take (K < 16, K > 256).
+// Fused z-transform + k-space influence + inverse z-transform, for the sizes that the
+// two-factor kernels (zfft2.cu, zfft64.cu) do not take: K < 16 and K > 256.
 //
 // The 3D R2C/C2R transforms of the mesh are split: cuFFT does the 2D (y, x)
 // transforms of every z-plane, and this kernel does, for a chunk of W (y, x)
@@ -60,26 +60,19 @@ constexpr int kZSmemCap = 224 * 1024;
 // b L3 + j + q1 L + q2 L R1 (L3 = L R1 R2); the R2 stage sees span L R1 and
 // offset j + q1 L.  DIT runs the R1 stage first, DIF the R2 stage first.  A
 // pass with L = 1 has j = 0: its R1-stage twiddles are 1 and are skipped.
-// KC, LC: K and L as compile-time constants (0: taken from the arguments).
-template <typename T, int W, int CT, int R1, int R2, bool DIF, int KC = 0, int LC = 0>
-__device__ __forceinline__ void zpass(Cx<T> *__restrict__ sb, int Kr, int Lr,
+template <typename T, int W, int CT, int R1, int R2, bool DIF>
+__device__ __forceinline__ void zpass(Cx<T> *__restrict__ sb, int K, int L,
                                       const Cx<T> *__restrict__ tw, int bi0) {
     constexpr int BS = CT / (3 * W);
-    const int K = KC ? KC : Kr, L = LC ? LC : Lr;
     const int La = L * R1, L3 = La * R2;
     const int nb = K / (R1 * R2), ts1 = K / La, ts2 = K / L3;
     const bool unit1 = L == 1;
     DivMod dl;
-    if constexpr (LC == 0) dl.init(L);
-#pragma unroll(KC ? 2 : 1)
+    dl.init(L);
+#pragma unroll 1
     for (int bi = bi0; bi < nb; bi += BS) {
-        int j, b;
-        if constexpr (LC != 0) {
-            b = bi / LC;  // compile-time divisor
-            j = bi - b * LC;
-        } else {
-            b = dl.div(bi, j);
-        }
+        int j;
+        const int b = dl.div(bi, j);
         Cx<T> *x = sb + (size_t)(b * L3 + j) * W;
         Cx<T> v[R2][R1];
 #pragma unroll
@@ -221,8 +214,8 @@ struct ZSmem {
 // compute threads, MINB blocks per SM, MAXP influence points per thread
 // (table values kept in registers: points p = p0 + i PS, i < MAXP, so
 // K W <= MAXP CT).  Fewer transform threads with more registers each measured
-// faster than more threads that spill (K = 256 FP32: 192 threads 1.88 ms,
-// 288 threads 1.93 ms, 384 threads 2.51 ms).
+// faster than more threads that spill (at K = 256, FP32, which zfft2.cu runs now: 192
+// threads 1.88 ms, 288 threads 1.93 ms, 384 threads 2.51 ms).
 struct ZCfg {
     int W, ct, minb, maxp;
 };
@@ -231,69 +224,28 @@ constexpr ZCfg kCfg32[] = {{16, 192, 1, 24}, {8, 192, 2, 12},
 constexpr ZCfg kCfg64[] = {{8, 384, 1, 6}, {4, 192, 2, 12}, {8, 192, 1, 12},
                            {2, 192, 1, 24}, {1, 192, 1, 24}};
 
-// One block per chunk of W consecutive (y, x) columns of the flattened z-plane
-// (chunk starts are multiples of W: 16-byte aligned in the global layout), all
-// 3R components.  Threads 0..CT-1 transform; the warp after them moves data: TMA loads into
-// the two buffers, TMA stores of finished buffers.
-// Compile-time pass sequences (codes and spans as in ZPlan, DIT order) for the
-// mesh sizes used most; any other K runs the plan's passes with runtime spans.
-template <int KS>
-struct ZFixed {
-    static constexpr int n = 0;
-};
-template <>
-struct ZFixed<128> {
-    static constexpr int n = 2;
-    static constexpr int code[2] = {44, 42}, span[2] = {1, 16};
-};
-template <>
-struct ZFixed<160> {
-    static constexpr int n = 3;
-    static constexpr int code[3] = {44, 21, 51}, span[3] = {1, 16, 32};
-};
-template <>
-struct ZFixed<256> {
-    static constexpr int n = 2;
-    static constexpr int code[2] = {44, 44}, span[2] = {1, 16};
-};
-
-// Passes I .. (DIF: down to 0, DIT: up to n - 1) of the fixed sequence of KS.
-template <typename T, int W, int CT, int KS, bool DIF, int I>
-__device__ __forceinline__ void zpasses_fixed(Cx<T> *cb, const Cx<T> *tw, int bi0) {
-    using Z = ZFixed<KS>;
-    constexpr int CODE = Z::code[I], SPAN = Z::span[I];
-    zpass<T, W, CT, CODE / 10, CODE % 10, DIF, KS, SPAN>(cb, KS, SPAN, tw, bi0);
-    if constexpr (DIF) {
-        compute_sync<CT>();
-        if constexpr (I > 0) zpasses_fixed<T, W, CT, KS, true, I - 1>(cb, tw, bi0);
-    } else if constexpr (I + 1 < Z::n) {
-        compute_sync<CT>();
-        zpasses_fixed<T, W, CT, KS, false, I + 1>(cb, tw, bi0);
-    }
-}
-
 // The z transform's passes: forward DIF (last pass first, each followed by a
 // barrier) or inverse DIT (first pass first, barriers between passes).
-template <typename T, int W, int CT, int KS, bool DIF>
+template <typename T, int W, int CT, bool DIF>
 __device__ __forceinline__ void zpasses(Cx<T> *cb, const ZPlan &zp, const Cx<T> *tw, int bi0) {
-    if constexpr (ZFixed<KS>::n > 0) {
-        zpasses_fixed<T, W, CT, KS, DIF, DIF ? ZFixed<KS>::n - 1 : 0>(cb, tw, bi0);
+    if constexpr (DIF) {
+        for (int i = zp.npass - 1; i >= 0; i--) {
+            zstage<T, W, CT, true>(cb, zp.K, zp.pcode[i], zp.pspan[i], tw, bi0);
+            compute_sync<CT>();
+        }
     } else {
-        if constexpr (DIF) {
-            for (int i = zp.npass - 1; i >= 0; i--) {
-                zstage<T, W, CT, true>(cb, zp.K, zp.pcode[i], zp.pspan[i], tw, bi0);
-                compute_sync<CT>();
-            }
-        } else {
-            for (int i = 0; i < zp.npass; i++) {
-                zstage<T, W, CT, false>(cb, zp.K, zp.pcode[i], zp.pspan[i], tw, bi0);
-                if (i + 1 < zp.npass) compute_sync<CT>();
-            }
+        for (int i = 0; i < zp.npass; i++) {
+            zstage<T, W, CT, false>(cb, zp.K, zp.pcode[i], zp.pspan[i], tw, bi0);
+            if (i + 1 < zp.npass) compute_sync<CT>();
         }
     }
 }
 
-template <typename T, int W, int CT, int MINB, int MAXP, int KS>
+// One block per chunk of W consecutive (y, x) columns of the flattened z-plane
+// (chunk starts are multiples of W: 16-byte aligned in the global layout), all
+// 3R components.  Threads 0..CT-1 transform; the warp after them moves data: TMA loads into
+// the two buffers, TMA stores of finished buffers.
+template <typename T, int W, int CT, int MINB, int MAXP>
 __global__ void __launch_bounds__(CT + 32, MINB)
 k_zfft_influence(const __grid_constant__ CUtensorMap gmap, const T *__restrict__ tab2,
                  const Cx<T> *__restrict__ tw_g, const int *__restrict__ perm_g,
@@ -415,7 +367,7 @@ k_zfft_influence(const __grid_constant__ CUtensorMap gmap, const T *__restrict__
         Cx<T> *B = b ? buf1 : buf0;
         Cx<T> *cb = B + (size_t)gcol * GS + wcol;
         // forward DIF, passes from the last down
-        zpasses<T, W, CT, KS, true>(cb, zp, tw, bi0);
+        zpasses<T, W, CT, true>(cb, zp, tw, bi0);
         // influence, digit-reversed z order
 #pragma unroll
         for (int i = 0; i < MAXP; i++) {
@@ -443,7 +395,7 @@ k_zfft_influence(const __grid_constant__ CUtensorMap gmap, const T *__restrict__
         }
         compute_sync<CT>();
         // inverse DIT, passes from the first up
-        zpasses<T, W, CT, KS, false>(cb, zp, tw, bi0);
+        zpasses<T, W, CT, false>(cb, zp, tw, bi0);
         // hand the buffer to the TMA warp (its store reads what this thread wrote)
         fence_proxy_async();
         mbar_arrive(&done[b]);
@@ -574,29 +526,10 @@ bool make_zfft_map(CUtensorMap *map, void *G, int K, int C, size_t elem) {
     return r == CUDA_SUCCESS;
 }
 
-template <int KS>
-bool plan_is(const ZPlan &zp) {
-    using Z = ZFixed<KS>;
-    if (zp.K != KS || zp.npass != Z::n) return false;
-    for (int i = 0; i < Z::n; i++)
-        if (zp.pcode[i] != Z::code[i] || zp.pspan[i] != Z::span[i]) return false;
-    return true;
-}
-
 template <typename T, int W, int CT, int MINB, int MAXP>
 cudaError_t launch_zcfg(const CUtensorMap &map, const T *tab2, const T *tw, const int *perm,
                         const ZPlan &zp, T twopi_L, int R, int zb, int *err, cudaStream_t s) {
-    // a fixed pass sequence when the plan matches one (instantiated for FP64's first
-    // configuration, the one these K get; FP32 runs zfft2.cu for them)
-    constexpr ZCfg first = kCfg64[0];
-    constexpr bool fixed_ok = sizeof(T) == 8 && first.W == W && first.ct == CT &&
-                              first.minb == MINB && first.maxp == MAXP;
-    auto kern = k_zfft_influence<T, W, CT, MINB, MAXP, 0>;
-    if constexpr (fixed_ok) {
-        if (plan_is<256>(zp)) kern = k_zfft_influence<T, W, CT, MINB, MAXP, 256>;
-        if (plan_is<160>(zp)) kern = k_zfft_influence<T, W, CT, MINB, MAXP, 160>;
-        if (plan_is<128>(zp)) kern = k_zfft_influence<T, W, CT, MINB, MAXP, 128>;
-    }
+    auto kern = k_zfft_influence<T, W, CT, MINB, MAXP>;
     const int K = zp.K, Kh = K / 2 + 1;
     const size_t smem = zsmem_bytes<T>(K, W);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
