@@ -53,7 +53,7 @@ WORKLOADS = {
 # as the ratio times its algorithmic bytes (the spread and z-FFT traffic grows in
 # proportion; the interpolation's halo re-reads grow with the mesh, so its
 # estimate is a lower bound).
-NCU_TRAFFIC_RATIO = {"spread": 1.080, "influence": 0.984, "interp": 1.678}
+NCU_TRAFFIC_RATIO = {"spread": 1.019, "influence": 0.982, "interp": 1.802}
 
 
 def algorithmic_bytes(w, s=4):
@@ -533,7 +533,7 @@ def run_gb300(args, w):
                                     terms=spme_gb300.TERM_REAL | spme_gb300.TERM_SELF)
             ers.set_stream(stream.cuda_stream)
             ers.set_positions(p64)
-            urs = torch.zeros((2, 3 * N), dtype=torch.float32, device="cuda")
+            urs = torch.zeros_like(f_d[:2])
             ers.apply(f_d[:2].contiguous(), urs)
             torch.cuda.synchronize()
             acc["rel_l2_fp32_real_self_vs_oracle"] = rel_np(urs.double().cpu().numpy(),

@@ -74,7 +74,7 @@ typedef struct spme_params {
  * (the reference's operator); np/dim/porder/box_size/xi/rcut zero. */
 void spme_params_init(spme_params *p);
 
-/* Create an engine (allocates device memory, cuFFT plans, tables). */
+/* Create an engine (allocates device memory, tables, cuFFT plans where it uses them). */
 int spme_create(const spme_params *params, spme_t **out);
 
 /* Destroy an engine; NULL is a no-op. */
@@ -193,7 +193,7 @@ int spme_fma_peak(int precision, double *flops_per_s);
  * precision, and applies the full operator M_k = M_recip + M_real + M_self to
  * each of them; every stage (position build, spread, influence,
  * interpolation, real-space sum, layout conversions) is one launch over a
- * packed work list of all systems, and cuFFT runs one batched plan per
+ * packed work list of all systems, and the transforms run once per
  * distinct K.  Device pointers only; work ordered on the batch's stream.
  *
  * Packed layouts (systems in the order given, P_k = N_0 + ... + N_{k-1}):
@@ -233,7 +233,7 @@ int spme_batch_step(spme_batch_t *batch, const double *pos, double alpha, const 
                     double beta, void *u);
 int spme_batch_set_graphs(spme_batch_t *batch, int on);
 /* Concurrency inside a step (OR of): 1 the real-space sum on a second stream
- * beside the mesh pipeline, 2 the cuFFT groups on four streams.  Default 0. */
+ * beside the mesh pipeline, 2 the transforms' mesh-size groups on four streams.  Default 0. */
 int spme_batch_set_overlap(spme_batch_t *batch, int mode);
 int spme_batch_synchronize(spme_batch_t *batch);
 long spme_batch_launch_count(const spme_batch_t *batch);

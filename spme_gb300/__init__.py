@@ -376,7 +376,7 @@ class Engine:
 
     def set_fft_mode(self, mode: int):
         """2: one-pass 2D transforms + fused z-FFT/influence kernel (FP32, K = 128,
-        160, 256); 1: 2D cuFFT + fused kernel (the FP32 default where it fits);
+        160, 256); 1: 2D transforms + fused z transform (the default where it fits);
         0: 3D cuFFT + influence."""
         _check(load().spme_set_fft_mode(self.h, int(mode)), "spme_set_fft_mode")
 
@@ -390,7 +390,7 @@ class Engine:
 class Batch:
     """Independent systems (uneven N, L, K, p; same right-hand-side count and
     precision) applied together: every stage is one launch over a packed work
-    list of all systems, cuFFT one batched plan per distinct K
+    list of all systems, one set of transform launches per distinct K
     (``spme_batch_*`` in include/spme_gb300.h).  Device (CUDA tensor) data only,
     in the packed layouts: positions ``pack(pos_list)`` (sum N x 3 float64),
     vectors ``pack(f_list)`` with system k's (R, 3 N_k) rows contiguous.  Work
@@ -462,7 +462,7 @@ class Batch:
         _check(load().spme_batch_set_tile(self.h, tx, ty, tz), "spme_batch_set_tile")
 
     def set_overlap(self, mode: int):
-        """1: real-space sum on a second stream; 2: cuFFT groups on four streams."""
+        """1: real-space sum on a second stream; 2: the transforms' mesh-size groups on four streams."""
         _check(load().spme_batch_set_overlap(self.h, int(mode)), "spme_batch_set_overlap")
 
     def set_profiling(self, on: bool = True):

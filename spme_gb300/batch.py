@@ -8,7 +8,7 @@ per-system loop pays ~20 launches per system.
 ``SystemBatch.run`` uses the native batch (:class:`spme_gb300.Batch`,
 ``spme_batch_*`` in include/spme_gb300.h): every stage of the position build
 and of the apply is one persistent launch over a packed work list of all
-systems' blocks, cuFFT runs one batched plan per distinct K, and the whole
+systems' blocks, the transforms run once per distinct K, and the whole
 step is one captured CUDA graph.  Two references run the same systems through
 separate engines: ``run_loop`` one after the other, ``run_engines_graph`` as
 independent branches of one captured graph.

@@ -1,7 +1,7 @@
 // Batches of independent systems (uneven N, L, K, p) applied together: every
 // stage of the position build and of the apply is one launch over a packed
-// work list covering all systems (persistent blocks walk the list), and cuFFT
-// runs one batched plan per distinct mesh size.  No counterpart in the
+// work list covering all systems (persistent blocks walk the list), and the
+// transforms run once per distinct mesh size.  No counterpart in the
 // reference, whose compute_spme (old-version/spme.c:560-726) applies one
 // system; each system's operator is the engine's full M = M_recip + M_real +
 // M_self.
@@ -15,7 +15,7 @@
 //     over the concatenated keys leaves each system's particles in its own
 //     slot range [P_k, P_k + N_k);
 //   * meshes and half spectra are laid out grouped by mesh size K, so each
-//     group is one batched cuFFT plan (component-major, as in the engine).
+//     group is one set of transform launches (component-major, as in the engine).
 #include <cuda_runtime.h>
 #include <cufft.h>
 
@@ -417,7 +417,7 @@ struct _spme_batch_t {
     std::vector<FftGroup> groups;
     cudaStream_t own_stream = nullptr, stream = nullptr;
     // concurrency inside a step: the real-space sum beside the mesh pipeline
-    // (overlap bit 0), the cuFFT groups on kFftStreams streams, each with its
+    // (overlap bit 0), the transform groups on kFftStreams streams, each with its
     // own work area (bit 1)
     static constexpr int kFftStreams = 4;
     int overlap = 0;

@@ -908,8 +908,8 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
         if (!e->d_mesh || !e->d_cmesh || !e->d_tab) return SPME_ERR_STATE;
         PlanPair *pp;
         TRY(get_plans(e, C, &pp));
-        // column gather where it applies; measured on GB300 (K = 256, N = 1e6): in FP64
-        // it wins at every C (8.0 vs 19.6 ms at C = 3), in FP32 from C = 9 on (the
+        // marching or column gather where they apply; against the tile kernel (K = 256, N =
+        // 1e6) the gather wins in FP64 at every C (8.0 vs 19.6 ms at C = 3; the boxes 2.4), in FP32 from C = 9 on (the
         // tile kernel's per-component cost is lower at C = 3, 6)
         // (the kernel stages force-row offsets as 32-bit integers)
         const bool use_cols = e->cols && e->spread_mode == 1 &&

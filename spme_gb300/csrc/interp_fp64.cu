@@ -14,7 +14,7 @@
 // right-hand side per CTA and the right-hand sides in sequence, N = 3e4, K = 90,
 // p = 8, R = 5 took 1.19 ms.
 // N = 1e6, K = 256, p = 6, one right-hand side, 8x8x8 tiles: 3.54 -> 1.50 ms;
-// N = 1e5, K = 128: 0.395 -> 0.170 ms; K = 90, p = 8, R = 5: 0.897 -> 0.576 ms.
+// N = 1e5, K = 128: 0.395 -> 0.168 ms; K = 90, p = 8, R = 5: 0.897 -> 0.561 ms.
 #include <algorithm>
 
 #include "cp_async.cuh"
