@@ -29,7 +29,12 @@ namespace spme {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kHX = kInterpMaxRow;  // staged row width (elements)
+// Staged row width (elements) HX: 24, or 16 for boxes copied without TMA at tiles of at most
+// 8 columns (tx + 7 columns are read): the copies are what those cost.  Interpolation at
+// K = 75, C = 24, p = 4, 8x8x8 tiles 0.111 -> 0.080 ms.  A TMA box stays 24 wide: dense
+// 16-wide components would all start on the same banks.
+constexpr int kHX = kInterpMaxRow;
+__host__ __device__ constexpr bool narrow_row(bool use_tma, int tx) { return !use_tma && tx <= 8; }
 
 template <typename T> struct Vec16;
 template <> struct Vec16<float> { using type = float4; static constexpr int n = 4; };
@@ -62,7 +67,7 @@ __device__ __forceinline__ HalfRec load_pair_rec(const InterpArgs<float> &A, int
 // carry zero weights (the box is 24 columns wide: a pair ends at most at
 // column tx + 6).  The next pair's records are loaded while this pair is
 // interpolated; rec0 is the warp's first pair, loaded once per tile.
-template <int P>
+template <int P, int HX>
 __device__ __forceinline__ void interp_pairs(const float *box, int PS, int HYB,
                                              const InterpArgs<float> &A, int c0, int nc,
                                              int pbeg, int pend, int ox, int oy, int oz,
@@ -99,16 +104,16 @@ __device__ __forceinline__ void interp_pairs(const float *box, int PS, int HYB,
         }
 #pragma unroll
         for (int z = 0; z < P; z++) wz[z] = w(2 * P + z);
-        const float *base = box + (size_t)cl * PS + (lz * HYB + ly) * kHX + (lx - odd) + 2 * xp;
+        const float *base = box + (size_t)cl * PS + (lz * HYB + ly) * HX + (lx - odd) + 2 * xp;
         float2 acc = make_float2(0.f, 0.f);
         // sum over y with w_x w_y first, then one w_z per plane
 #pragma unroll
         for (int z = 0; z < P; z++) {
-            const float *pz = base + z * HYB * kHX;
+            const float *pz = base + z * HYB * HX;
             float2 t = make_float2(0.f, 0.f);
 #pragma unroll
             for (int y = 0; y < P; y++)
-                t = __ffma2_rn(wxy[y], *reinterpret_cast<const float2 *>(pz + y * kHX), t);
+                t = __ffma2_rn(wxy[y], *reinterpret_cast<const float2 *>(pz + y * HX), t);
             acc = __ffma2_rn(make_float2(wz[z], wz[z]), t, acc);
         }
         float a = acc.x + acc.y;
@@ -123,12 +128,12 @@ __device__ __forceinline__ void interp_pairs(const float *box, int PS, int HYB,
 
 // One tile's work (the body of the single-system kernel and of the batched
 // one); tmap is read only when use_tma is set.
-template <typename T, int P, int CG>
+template <typename T, int P, int CG, int HX>
 __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const InterpArgs<T> &A,
                                             int tile) {
     using V = typename Vec16<T>::type;
     constexpr int VW = Vec16<T>::n;
-    constexpr int NV = kHX / VW;  // vectors per staged row
+    constexpr int NV = HX / VW;  // vectors per staged row
     constexpr int NG = CG / 4;    // groups of 4 components per chunk
     const int use_tma = A.use_tma;
     const int *__restrict__ tile_off = A.tile_off;
@@ -149,7 +154,8 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
     if (pbeg == pend) return;
     const int K = g.K;
     const int HYB = g.ty + P - 1, HZB = g.tz + P - 1;
-    const int PS = HZB * HYB * kHX;  // component-plane stride
+    // component-plane stride: 8 or 24 (mod 32) words
+    const int PS = HZB * HYB * HX + (HX == 16 ? 8 : 0);
     const int tix = tile % g.ntx, tiy = (tile / g.ntx) % g.nty, tiz = tile / (g.ntx * g.nty);
     const int ox = tix * g.tx, oy = tiy * g.ty, oz = tiz * g.tz;
     const int hx = min(g.tx, K - ox) + P - 1;
@@ -171,7 +177,7 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
     }
     __syncthreads();
 
-    // rows [c][z][y][0..kHX) of the halo region with asynchronous copies of 16, 8 or 4
+    // rows [c][z][y][0..HX) of the halo region with asynchronous copies of 16, 8 or 4
     // bytes.  Through registers a thread waited for each vector: K = 75, C = 24 0.121 ms, here
     // 0.111; 64 systems of K = 24 to 100, C = 12 1.47, 1.27 ms.
     auto stage_rows = [&](int c0, int nc) {
@@ -191,7 +197,7 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
             gz -= gz >= K ? K : 0;
             const int x0 = ox + v * VW;
             const T *src = mesh + (size_t)(c0 + c) * K3 + (size_t)gz * K2 + (size_t)gy * K;
-            T *dst = box + (size_t)c * PS + (z * HYB + y) * kHX + v * VW;
+            T *dst = box + (size_t)c * PS + (z * HYB + y) * HX + v * VW;
             if (vec) {
                 cp_async16(dst, src + wrap_index(x0, K));
             } else if (two) {
@@ -229,7 +235,7 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
             gy -= gy >= K ? K : 0;
             gz -= gz >= K ? K : 0;
             const T *src = mesh + (size_t)(c0 + c) * K3 + (size_t)gz * K2 + (size_t)gy * K;
-            T *dst = box + (size_t)c * PS + (z * HYB + y) * kHX;
+            T *dst = box + (size_t)c * PS + (z * HYB + y) * HX;
             const int v1 = row_wraps ? NV - 1 : xw1;
             for (int v = row_wraps ? 0 : xw0; v <= v1; v++) {
                 const int x0 = ox + v * VW;
@@ -277,7 +283,7 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
             stage_rows(c0, nc);
         }
         if constexpr (kPairs) {
-            interp_pairs<P>(reinterpret_cast<const float *>(box), PS, HYB,
+            interp_pairs<P, HX>(reinterpret_cast<const float *>(box), PS, HYB,
                             reinterpret_cast<const InterpArgs<float> &>(A), c0, nc, pbeg, pend,
                             ox, oy, oz, hrec_0);
             __syncthreads();  // the box is rewritten by the next chunk
@@ -310,18 +316,18 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
             T acc[NG];
 #pragma unroll
             for (int k = 0; k < NG; k++) acc[k] = T(0);
-            const T *base = box + (size_t)cl * PS + (lz * HYB + ly) * kHX + lx + xs;
+            const T *base = box + (size_t)cl * PS + (lz * HYB + ly) * HX + lx + xs;
             // sum over y with w_x w_y first, then one w_z per plane
 #pragma unroll
             for (int z = 0; z < P; z++) {
-                const T *pz = base + z * HYB * kHX;
+                const T *pz = base + z * HYB * HX;
                 T t[NG];
 #pragma unroll
                 for (int k = 0; k < NG; k++) t[k] = T(0);
 #pragma unroll
                 for (int y = 0; y < P; y++)
 #pragma unroll
-                    for (int k = 0; k < NG; k++) t[k] += wxy[y] * pz[(size_t)k * 4 * PS + y * kHX];
+                    for (int k = 0; k < NG; k++) t[k] += wxy[y] * pz[(size_t)k * 4 * PS + y * HX];
 #pragma unroll
                 for (int k = 0; k < NG; k++) acc[k] += wz[z] * t[k];
             }
@@ -342,7 +348,7 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
     }
 }
 
-template <typename T, int P, int CG>
+template <typename T, int P, int CG, int HX>
 // blocks per SM that the 4-component box's shared memory allows (16x8x4 tiles)
 __global__ void __launch_bounds__(kThreads, 5)
 k_interp(const __grid_constant__ CUtensorMap tmap, InterpArgs<T> A) {
@@ -351,7 +357,7 @@ k_interp(const __grid_constant__ CUtensorMap tmap, InterpArgs<T> A) {
     // share p - 1 of their tz + p - 1 planes (read from L2 by the later ones)
     const int b = blockIdx.x, ntx = A.g.ntx, nty = A.g.nty, ntz = A.g.ntz;
     const int tiz = b % ntz, rest = b / ntz;
-    interp_body<T, P, CG>(&tmap, A, (tiz * nty + rest / ntx) * ntx + rest % ntx);
+    interp_body<T, P, CG, HX>(&tmap, A, (tiz * nty + rest / ntx) * ntx + rest % ntx);
 }
 
 // Many systems in one persistent launch over their tiles: each system's boxes
@@ -369,10 +375,18 @@ k_interp_batch(const InterpSys<T> *__restrict__ sys, const int *__restrict__ pre
         // global memory; never a local copy)
         const CUtensorMap *tmap = A.use_tma ? &sys[k].tmap : nullptr;
         const int tile = w - prefix[k];
-        switch (A.g.p) {
-            case 4: interp_body<T, 4, CG>(tmap, A, tile); break;
-            case 6: interp_body<T, 6, CG>(tmap, A, tile); break;
-            default: interp_body<T, 8, CG>(tmap, A, tile); break;
+        if (narrow_row(A.use_tma, A.g.tx)) {
+            switch (A.g.p) {
+                case 4: interp_body<T, 4, CG, 16>(tmap, A, tile); break;
+                case 6: interp_body<T, 6, CG, 16>(tmap, A, tile); break;
+                default: interp_body<T, 8, CG, 16>(tmap, A, tile); break;
+            }
+        } else {
+            switch (A.g.p) {
+                case 4: interp_body<T, 4, CG, kHX>(tmap, A, tile); break;
+                case 6: interp_body<T, 6, CG, kHX>(tmap, A, tile); break;
+                default: interp_body<T, 8, CG, kHX>(tmap, A, tile); break;
+            }
         }
         __syncthreads();
     }
@@ -388,12 +402,12 @@ cudaError_t launch_interp_t(const InterpMaps &maps, const int *tile_off, const i
                             const uint32_t *rec_start, const T *rec_w, const T *mesh, int C,
                             int cb, int ce, const MeshGeom &g, T *W, int accumulate, int *err,
                             cudaStream_t s) {
+    const bool use = maps.ok4, narrow = narrow_row(use, g.tx);
     const size_t smem = interp_smem<T, P, CG>(g);
-    auto kern = k_interp<T, P, CG>;
+    auto kern = narrow ? k_interp<T, P, CG, 16> : k_interp<T, P, CG, kHX>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    const bool use = maps.ok4;
     const CUtensorMap &m = maps.cg4;
     InterpArgs<T> A{tile_off, rec_idx, rec_start, rec_w, mesh, W, err, g, C, cb, ce,
                     accumulate, use ? 1 : 0, RecordWidth<T, P>::value};
