@@ -901,7 +901,7 @@ template <typename T>
 cudaError_t own_xy(_spme_batch_t *b, const FftGroup &grp, bool inverse, cudaStream_t s) {
     b->launches += 2;
     return launch_fft_xy<T>(grp.K, inverse, (T *)b->d_mesh + grp.mesh_off,
-                            (T *)b->d_spec + 2 * grp.spec_off, (long)b->C * grp.nsys * grp.K,
+                            (T *)b->d_spec + 2 * grp.spec_off, (long)b->C * grp.nsys,
                             (const T *)grp.d_tw, s);
 }
 template <typename T>

@@ -942,7 +942,7 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
                                             (long)C * K, e->d_f2tab, s));
             e->launches++;
         } else if (ownxy) {
-            TRY_CUDA(spme::launch_fft_xy<T>(K, false, (T *)e->d_mesh, (T *)e->d_cmesh, (long)C * K,
+            TRY_CUDA(spme::launch_fft_xy<T>(K, false, (T *)e->d_mesh, (T *)e->d_cmesh, C,
                                             (const T *)e->d_ztw, s));
             e->launches += 2;
         } else if (sizeof(T) == 4)
@@ -967,7 +967,7 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
                                             (long)C * K, e->d_f2tab, s));
             e->launches++;
         } else if (ownxy) {
-            TRY_CUDA(spme::launch_fft_xy<T>(K, true, (T *)e->d_mesh, (T *)e->d_cmesh, (long)C * K,
+            TRY_CUDA(spme::launch_fft_xy<T>(K, true, (T *)e->d_mesh, (T *)e->d_cmesh, C,
                                             (const T *)e->d_ztw, s));
             e->launches += 2;
         } else if (sizeof(T) == 4)

@@ -7,9 +7,11 @@
 // transforms over n2 (frequency k1 + R1 k2); the inverse of x runs the same steps backwards.  Global
 // loads go straight to the first pass's registers and results leave from the last
 // pass's, so a thread has R1 independent loads in flight.
-// x: two consecutive real rows a, b are one complex row a + i b; the spectra are
-// Z[k] + conj Z[K-k] and -i (Z[k] - conj Z[K-k]) up to a factor 1/2, which the first
-// pass's twiddles carry.
+// x: two consecutive real rows a, b of one component are one complex row a + i b; the
+// spectra are Z[k] + conj Z[K-k] and -i (Z[k] - conj Z[K-k]) up to a factor 1/2, which the
+// first pass's twiddles carry.  Rows of two components never share one: they may belong to
+// right-hand sides or systems of other magnitude, whose rounding (or NaN) would pass over.
+// With odd K the last row of a component (it has K^2) is paired with zeros.
 // y: in place, W columns of the flattened (plane, kx) list per block, so no lane is
 // idle at the end of a plane.
 // Bound: FP64 by the FP64 pipe (a warp instruction each 16 cycles; about 14 instructions
@@ -40,6 +42,18 @@ __host__ __device__ constexpr int xy_cols(int R1, int R2) { return sizeof(T) == 
 // reads along k1 fall on different banks.
 __host__ __device__ constexpr int x_stride(int R2) { return R2 | 1; }
 
+// Row pairs of a component; the first row of pair q of all components' pairs (rows and
+// above: past the last), and whether the pair has a second one.
+__host__ __device__ constexpr int x_pairs(int K) { return (K * K + 1) / 2; }
+template <int K>
+__device__ __forceinline__ long x_row(long q) {
+    return K % 2 == 0 ? 2 * q : 2 * q - q / x_pairs(K);
+}
+template <int K>
+__device__ __forceinline__ bool x_two(long ra, long rows) {
+    return K % 2 == 0 ? ra + 1 < rows : (ra + 1) % (K * K) != 0;
+}
+
 template <typename T>
 __host__ __device__ constexpr int xy_minb(int threads, int R) {
     // registers: the transform's values and as many temporaries
@@ -60,13 +74,13 @@ k_fft_x_fwd(const T *__restrict__ mesh, typename ZVec<T>::type *__restrict__ G,
     extern __shared__ __align__(16) unsigned char xsm[];
     V *sm = reinterpret_cast<V *>(xsm);
     const int tid = threadIdx.x;
-    const long row0 = (long)blockIdx.x * (2 * P);
+    const long q0 = (long)blockIdx.x * P;
     {
         const int p = tid / R2, n2 = tid - p * R2;
-        const long ra = row0 + 2 * p;
+        const long ra = x_row<K>(q0 + p);
         if (p < P && ra < rows) {
             const T *a = mesh + ra * K + n2;
-            const bool two = ra + 1 < rows;
+            const bool two = x_two<K>(ra, rows);
             V v[R1];
 #pragma unroll
             for (int n1 = 0; n1 < R1; n1++) v[n1] = z_make(a[n1 * R2], two ? a[K + n1 * R2] : T(0));
@@ -90,7 +104,7 @@ k_fft_x_fwd(const T *__restrict__ mesh, typename ZVec<T>::type *__restrict__ G,
         constexpr int H = (Kh + R1 - 1) / R1 + 1 < R2 ? (Kh + R1 - 1) / R1 + 1 : R2;
         const int p = tid / R1, k1 = tid - p * R1;
         const bool neg = z_signed<T>(k1, R1) < 0;
-        const long ra = row0 + 2 * p;
+        const long ra = x_row<K>(q0 + p);
         V *x = sm + p * (R1 * RS);
         const V *xc = x + (k1 == 0 ? R2 : (R1 - k1) * RS + R2 - 1);  // frequency K - k1
         V v[R2];
@@ -108,7 +122,7 @@ k_fft_x_fwd(const T *__restrict__ mesh, typename ZVec<T>::type *__restrict__ G,
         __syncthreads();
         if (p < P && ra < rows) {
             V *g = G + ra * Kh + k1;
-            const bool two = ra + 1 < rows;
+            const bool two = x_two<K>(ra, rows);
 #pragma unroll
             for (int k2 = 0; k2 < H; k2++) {
                 const int q = z_k2(neg, k2, R2), k = k1 + R1 * q;
@@ -131,7 +145,7 @@ k_fft_x_inv(const typename ZVec<T>::type *__restrict__ G, T *__restrict__ mesh,
     extern __shared__ __align__(16) unsigned char xsm[];
     V *sm = reinterpret_cast<V *>(xsm);
     const int tid = threadIdx.x;
-    const long row0 = (long)blockIdx.x * (2 * P);
+    const long q0 = (long)blockIdx.x * P;
     {
         // Z[k] = A[k] + i B[k], Z[K-k] = conj A[k] + i conj B[k]; the imaginary parts of the
         // zero and Nyquist frequencies are those of a real row, zero.  Thread (p, k1) loads
@@ -142,13 +156,13 @@ k_fft_x_inv(const typename ZVec<T>::type *__restrict__ G, T *__restrict__ mesh,
         constexpr int H = (Kh + R1 - 1) / R1 + 1 < R2 ? (Kh + R1 - 1) / R1 + 1 : R2;
         const int p = tid / R1, k1 = tid - p * R1;
         const bool neg = z_signed<T>(k1, R1) < 0;
-        const long ra = row0 + 2 * p;
+        const long ra = x_row<K>(q0 + p);
         V *x = sm + p * (R1 * RS);
         V *xc = x + (k1 == 0 ? R2 : (R1 - k1) * RS + R2 - 1);  // frequency K - k1
         V v[R2];
         if (p < P && ra < rows) {
             const V *g = G + ra * Kh + k1;
-            const bool two = ra + 1 < rows;
+            const bool two = x_two<K>(ra, rows);
             V a[H], c[H];
 #pragma unroll
             for (int k2 = 0; k2 < H; k2++) {
@@ -187,7 +201,7 @@ k_fft_x_inv(const typename ZVec<T>::type *__restrict__ G, T *__restrict__ mesh,
     __syncthreads();
     {
         const int p = tid / R2, n2 = tid - p * R2;
-        const long ra = row0 + 2 * p;
+        const long ra = x_row<K>(q0 + p);
         if (p < P && ra < rows) {
             const V *x = sm + p * (R1 * RS) + n2;
             V v[R1];
@@ -197,7 +211,7 @@ k_fft_x_inv(const typename ZVec<T>::type *__restrict__ G, T *__restrict__ mesh,
             T *a = mesh + ra * K + n2;
 #pragma unroll
             for (int n1 = 0; n1 < R1; n1++) a[n1 * R2] = v[n1].x;
-            if (ra + 1 < rows) {
+            if (x_two<K>(ra, rows)) {
 #pragma unroll
                 for (int n1 = 0; n1 < R1; n1++) a[K + n1 * R2] = v[n1].y;
             }
@@ -255,12 +269,12 @@ k_fft_y(typename ZVec<T>::type *__restrict__ G, const typename ZVec<T>::type *__
 }
 
 template <typename T, int R1, int R2>
-cudaError_t launch_xy(bool inv, T *mesh, T *G, long planes, const T *tw, cudaStream_t s) {
+cudaError_t launch_xy(bool inv, T *mesh, T *G, long comps, const T *tw, cudaStream_t s) {
     using V = typename ZVec<T>::type;
     constexpr int K = R1 * R2, Kh = K / 2 + 1, P = kXPairs, W = xy_cols<T>(R1, R2), M = zmax(R1, R2);
     constexpr int xsmem = P * R1 * x_stride(R2) * (int)sizeof(V), ysmem = K * W * (int)sizeof(V);
-    const long rows = planes * K, cols = planes * Kh;
-    const unsigned xb = (unsigned)((rows + 2 * P - 1) / (2 * P)), yb = (unsigned)((cols + W - 1) / W);
+    const long rows = comps * K * K, cols = comps * K * Kh;
+    const unsigned xb = (unsigned)((comps * x_pairs(K) + P - 1) / P), yb = (unsigned)((cols + W - 1) / W);
     V *g = reinterpret_cast<V *>(G);
     const V *t = reinterpret_cast<const V *>(tw);
     auto kx = inv ? reinterpret_cast<const void *>(k_fft_x_inv<T, R1, R2>)

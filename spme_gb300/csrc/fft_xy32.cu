@@ -16,10 +16,10 @@ bool fft_xy_ok(int K, size_t elem) {
 }
 
 template <>
-cudaError_t launch_fft_xy<float>(int K, bool inv, float *mesh, float *G, long planes, const float *tw,
+cudaError_t launch_fft_xy<float>(int K, bool inv, float *mesh, float *G, long comps, const float *tw,
                                  cudaStream_t s) {
 #define SPME_CASE(A, B) \
-    if (K == A * B) return launch_xy<float, A, B>(inv, mesh, G, planes, tw, s);
+    if (K == A * B) return launch_xy<float, A, B>(inv, mesh, G, comps, tw, s);
     SPME_FFT_LIST(SPME_CASE)
 #undef SPME_CASE
     return cudaErrorInvalidValue;

@@ -249,11 +249,12 @@ cudaError_t launch_zfft2(int K, const CUtensorMap &map, const float *tab2, const
 // Its FP64 form (zfft64.cu; K of fft_xy_ok, elem 8), on G in place.
 cudaError_t launch_zfft64(int K, double *G, const double *tab2, const double *tw, double L,
                           const double *twopi_Ls, int nsys, int R, cudaStream_t s);
-// Two-factor x and y transforms of the mesh's z-planes (fft_xy.cuh; K = 2^a 3^b 5^c, 16 to
-// 256, fft_xy_ok): mesh -> G, or G -> mesh (inv; G is overwritten).  tw as for the z transform.
+// Two-factor x and y transforms of the z-planes of comps consecutive meshes (fft_xy.cuh; K =
+// 2^a 3^b 5^c, 16 to 256, fft_xy_ok): mesh -> G, or G -> mesh (inv; G is overwritten), every
+// mesh on its own.  tw as for the z transform.
 bool fft_xy_ok(int K, size_t elem);
 template <typename T>
-cudaError_t launch_fft_xy(int K, bool inv, T *mesh, T *G, long planes, const T *tw, cudaStream_t s);
+cudaError_t launch_fft_xy(int K, bool inv, T *mesh, T *G, long comps, const T *tw, cudaStream_t s);
 template <>
 cudaError_t launch_fft_xy<float>(int, bool, float *, float *, long, const float *, cudaStream_t);
 template <>
