@@ -19,8 +19,10 @@
 //     two-lane FMAs (fma.rn.f32x2); the partner's force rows come component by
 //     component (F2[j][d][r]), so a right-hand side pair is one 8-byte load and a
 //     row's load touches one line instead of the whole interleaved row.
-// Sums over up to 16 pairs per slot run in FP32, longer ones with TwoSum.
-// Measured (ms): N = 1e6, R = 16 1.65 -> 1.52; N = 2e5, R = 16 0.445 -> 0.405; N = 1e5,
+// More right-hand sides: sums of a window's pairs (64, split over the slots) are plain FP32;
+// longer runs, the sum over the slots and the self term carry TwoSum.  That and the term's
+// one rounding into the sum cost 5 % of the stage (R = 16 1.525 -> 1.605 ms at N = 1e6).
+// Measured (ms): N = 1e6, R = 16 1.65 -> 1.61; N = 2e5, R = 16 0.442 -> 0.426; N = 1e5,
 // R = 1 0.162 -> 0.102; 64 uneven systems, R = 4 1.53 -> 1.40.  The partners' rows come
 // mostly from L2 (16 % L1 hits), whose latency bounds it now; more warps per SM at
 // fewer registers spill (1.57 ms at 12 blocks), a table of the pair functions in
@@ -106,7 +108,6 @@ __device__ __forceinline__ void real_few(const RealArgs<float> &A, int cell) {
 
 constexpr int kWin = 64;      // pairs evaluated together
 constexpr int kListM = 512;   // listed pairs per warp
-constexpr int kFold = 16;     // pairs per slot summed in plain FP32
 
 struct ManyShared {
     float4 r0[kWin];  // displacement, A
@@ -121,6 +122,7 @@ struct ManyShared {
 template <int RL>
 __device__ __forceinline__ void real_many(const RealArgs<float> &A, int cell) {
     constexpr int PS = 32 / RL;
+    constexpr int kFold = kWin / PS;  // pairs per slot summed in plain FP32, at most
     __shared__ CellShared<float> csh;
     __shared__ ManyShared wsh[kRsWarps];
     const int ib0 = __ldg(A.cell_off + cell), ie = __ldg(A.cell_off + cell + 1);
@@ -148,7 +150,7 @@ __device__ __forceinline__ void real_many(const RealArgs<float> &A, int cell) {
             const float *__restrict__ Fr = A.F2 + r;
             ListState ls;
             // sums of the current particle: two-lane partial sums, moved to compensated
-            // ones every kFold pairs per slot
+            // ones before a slot has more than kFold pairs
             float2 s0 = make_float2(0.f, 0.f), s1 = s0, s2 = s0;
             PairSum<float> sum[6];
             int nfold = 0, cnt = 0;
@@ -201,7 +203,8 @@ __device__ __forceinline__ void real_many(const RealArgs<float> &A, int cell) {
                         }
                         const int ke = min(e, wend);
                         const int o = wend - kWin - slot;
-                        if (cnt >= kFold) fold();
+                        // (whole pairs per slot: the list is padded)
+                        if (cnt + (ke - k) / PS > kFold) fold();
                         cnt += (ke - k) / PS;
                         if (live) {
 #pragma unroll 2
@@ -219,36 +222,51 @@ __device__ __forceinline__ void real_many(const RealArgs<float> &A, int cell) {
                                 const float2 g = __fmul2_rn(
                                     make_float2(b.x, b.x),
                                     __ffma2_rn(d2, f2, __ffma2_rn(d1, f1, __fmul2_rn(d0, f0))));
-                                s0 = __ffma2_rn(g, d0, __ffma2_rn(Av, f0, s0));
-                                s1 = __ffma2_rn(g, d1, __ffma2_rn(Av, f1, s1));
-                                s2 = __ffma2_rn(g, d2, __ffma2_rn(Av, f2, s2));
+                                // (one rounding of a pair's term into the sum)
+                                s0 = __fadd2_rn(s0, __ffma2_rn(g, d0, __fmul2_rn(Av, f0)));
+                                s1 = __fadd2_rn(s1, __ffma2_rn(g, d1, __fmul2_rn(Av, f1)));
+                                s2 = __fadd2_rn(s2, __ffma2_rn(g, d2, __fmul2_rn(Av, f2)));
                             }
                         }
                         k = ke;
                     }
                     if (ip == ls.il) break;  // cut: goes on in the next list
-                    // the slots' sums, then the self term, to the particle's row
+                    // the slots' sums and the self term, compensated, to the particle's row:
+                    // half of the slots take the first right-hand side, half the second
                     const int ii = __float_as_int(ws.pf[ip].w);
-                    if (nfold) fold();
-                    float v[6] = {s0.x, s1.x, s2.x, s0.y, s1.y, s2.y};
+                    const bool second = (lane & RL) != 0;
+                    PairSum<float> t[3];
+                    if (nfold) {
+                        fold();
 #pragma unroll
-                    for (int q = 0; q < 6; q++) {
-                        if (nfold) v[q] = sum[q].value();
-                        sum[q] = PairSum<float>();
+                        for (int d = 0; d < 3; d++) {
+                            t[d] = second ? sum[3 + d] : sum[d];
+                            t[d].join(shfl_xor(second ? sum[d] : sum[3 + d], RL));
+                            sum[d] = sum[3 + d] = PairSum<float>();
+                        }
+                    } else {
+                        const float v[6] = {s0.x, s1.x, s2.x, s0.y, s1.y, s2.y};
 #pragma unroll
-                        for (int w = RL; w < 32; w <<= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], w);
+                        for (int d = 0; d < 3; d++) {
+                            t[d].s = second ? v[3 + d] : v[d];
+                            t[d].add(__shfl_xor_sync(0xffffffffu, second ? v[d] : v[3 + d], RL));
+                        }
                     }
                     s0 = s1 = s2 = make_float2(0.f, 0.f);
                     nfold = cnt = 0;
-                    if (slot == 0 && live) {
-                        const float *fi = Fr + (size_t)ii * (size_t)(3 * R2);
-                        float *o = A.W + (size_t)ii * C + 3 * r;
 #pragma unroll
-                        for (int q = 0; q < 6; q++) {
-                            if (q < 3 || r + 1 < R) {
-                                const float f = A.with_self ? __ldg(fi + q % 3 * R2 + q / 3) : 0.f;
-                                o[q] = fmaf(A.cf.self_c, f, v[q]);
-                            }
+                    for (int w = 2 * RL; w < 32; w <<= 1) {
+#pragma unroll
+                        for (int d = 0; d < 3; d++) t[d].join(shfl_xor(t[d], w));
+                    }
+                    const int rs = r + (int)second;
+                    if (slot < 2 && rs < R) {
+                        const float *fi = A.F2 + (size_t)ii * (size_t)(3 * R2) + rs;
+                        float *o = A.W + (size_t)ii * C + 3 * rs;
+#pragma unroll
+                        for (int d = 0; d < 3; d++) {
+                            if (A.with_self) t[d].add(A.cf.self_c * __ldg(fi + d * R2));
+                            o[d] = t[d].value();
                         }
                     }
                 }

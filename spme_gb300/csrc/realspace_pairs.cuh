@@ -235,18 +235,30 @@ __device__ __forceinline__ int list_pairs(const Cell<G> &cell, const float4 *pf,
 // alongside.
 template <typename T>
 struct PairSum {
-    T s = T(0), c = T(0);
-    __device__ __forceinline__ void add(T x) {
-        if constexpr (sizeof(T) == 8) {
-            s += x;
-        } else {
-            const T t = s + x, bp = t - s;
-            c += (s - (t - bp)) + (x - bp);
-            s = t;
-        }
-    }
-    __device__ __forceinline__ T value() const { return sizeof(T) == 8 ? s : s + c; }
+    T s = T(0);
+    __device__ __forceinline__ void add(T x) { s += x; }
+    __device__ __forceinline__ void join(PairSum o) { s += o.s; }
+    __device__ __forceinline__ T value() const { return s; }
 };
+template <>
+struct PairSum<float> {
+    float s = 0.f, c = 0.f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = s + x, bp = t - s;
+        c += (s - (t - bp)) + (x - bp);
+        s = t;
+    }
+    __device__ __forceinline__ void join(PairSum o) {
+        add(o.s);
+        c += o.c;
+    }
+    __device__ __forceinline__ float value() const { return s + c; }
+};
+__device__ __forceinline__ PairSum<float> shfl_xor(PairSum<float> a, int w) {
+    a.s = __shfl_xor_sync(0xffffffffu, a.s, w);
+    a.c = __shfl_xor_sync(0xffffffffu, a.c, w);
+    return a;
+}
 
 constexpr int kList = 512;  // listed pairs per warp (few right-hand sides)
 
