@@ -712,7 +712,7 @@ int create_t(_spme_batch_t *b) {
     BTRY(balloc(&b->d_rw1, sizeof(T) * (size_t)b->ws * n));
     BTRY(balloc(&b->d_rw2, sizeof(T) * (size_t)b->ws * n));
     BTRY(balloc(&b->d_F, sizeof(T) * (size_t)C * n));
-    if (sizeof(T) == 4 && !real_row_is_F(b->R))
+    if (sizeof(T) == 4)
         BTRY(balloc(&b->d_F2, sizeof(T) * (size_t)real_row(b->R) * n));
     BTRY(balloc(&b->d_Fs, sizeof(T) * (size_t)spread_cols_row_width(C) * n));
     BTRY(balloc(&b->d_W, sizeof(T) * (size_t)C * n));

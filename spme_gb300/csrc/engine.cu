@@ -857,12 +857,6 @@ int set_positions_impl(spme_t *e, const double *pos, int mem) {
     return SPME_OK;
 }
 
-// Where the pack writes the real-space sum's rows (null: nowhere, or F's serve).
-template <typename T>
-T *packed_rows(spme_t *e, int R) {
-    return spme::real_row_is_F(R) ? nullptr : (T *)e->d_F2;
-}
-
 template <typename T>
 int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alpha, double beta,
              int rpart) {
@@ -874,7 +868,7 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
     T *F = (T *)e->d_F, *W = (T *)e->d_W;
     if (prof) cudaEventRecord(e->ev[0], s);
     if (f) {  // null: F already packed (host-pointer applies pack on the copy stream)
-        spme::launch_pack_tiled<T>(f, ldf, n, R, 0, R, F, packed_rows<T>(e, R), s);
+        spme::launch_pack_tiled<T>(f, ldf, n, R, 0, R, F, (T *)e->d_F2, s);
         e->launches++;
     }
     if (prof) cudaEventRecord(e->ev[1], s);
@@ -892,7 +886,7 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
         if (terms & SPME_TERM_REAL) {
             if (!e->d_coff || !e->d_cperm || !e->d_cpos) return SPME_ERR_STATE;
             TRY_CUDA(spme::launch_realspace<T>(e->nc, e->d_coff, e->d_cperm, e->d_cpos, F,
-                                               spme::real_row_is_F(R) ? F : (T *)e->d_F2, R,
+                                               (const T *)e->d_F2, R,
                                                e->prm.box_size, e->prm.rcut, e->prm.xi,
                                                e->prm.radius, (terms & SPME_TERM_SELF) ? 1 : 0,
                                                e->pair, W, rss));
@@ -1126,11 +1120,11 @@ int apply_impl(spme_t *e, int nrhs, double alpha, const void *f, long ldf, doubl
                     if (is_fp32(e))
                         spme::launch_pack_tiled<float>((const float *)e->d_fstage, 3L * n, n, R, q0,
                                                        q1, (float *)e->d_F,
-                                                       packed_rows<float>(e, R), e->stream);
+                                                       (float *)e->d_F2, e->stream);
                     else
                         spme::launch_pack_tiled<double>((const double *)e->d_fstage, 3L * n, n, R,
                                                         q0, q1, (double *)e->d_F,
-                                                        packed_rows<double>(e, R), e->stream);
+                                                        (double *)e->d_F2, e->stream);
                     e->launches++;
                 }
                 TRY_CUDA(cudaGetLastError());

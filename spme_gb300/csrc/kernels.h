@@ -303,13 +303,14 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
 // the force rows as that kernel reads them, real_row(R) values each: for up to
 // kRealFew right-hand sides in F's order padded to 16 bytes, for more by component
 // ([d][rows_even(R)]); the padding is zero.
-constexpr int kRealFew = 4;
+// The line between the forms: with 3 and 4 right-hand sides the compensated sums of the
+// first (per lane) need more registers and shared memory: N = 1e6, R = 3 1.37 against 1.31 ms,
+// R = 4 1.53 against 1.31, at volume fraction 0.12 2.72 against 2.07; at R = 2 1.07 ms.
+constexpr int kRealFew = 2;
 __host__ __device__ constexpr int rows_even(int R) { return (R + 1) & ~1; }
 __host__ __device__ constexpr int real_row(int R) {
     return R <= kRealFew ? (3 * R + 3) / 4 * 4 : 3 * rows_even(R);
 }
-// Whether F's own rows serve (R = 4: 12 values, whole 16-byte vectors).
-__host__ __device__ constexpr bool real_row_is_F(int R) { return R <= kRealFew && real_row(R) == 3 * R; }
 // The place of right-hand side r, component d in such a row.
 __host__ __device__ constexpr int real_at(int R, int r, int d) {
     return R <= kRealFew ? 3 * r + d : d * rows_even(R) + r;

@@ -23,7 +23,8 @@
 // longer runs, the sum over the slots and the self term carry TwoSum.  That and the term's
 // one rounding into the sum cost 5 % of the stage (R = 16 1.525 -> 1.605 ms at N = 1e6).
 // Measured (ms): N = 1e6, R = 16 1.65 -> 1.61; N = 2e5, R = 16 0.442 -> 0.426; N = 1e5,
-// R = 1 0.162 -> 0.102; 64 uneven systems, R = 4 1.53 -> 1.40.  The partners' rows come
+// R = 1 0.161 -> 0.112; N = 1e6, R = 1 1.32 -> 0.92 (with compensated sums per lane; 0.83
+// without), R = 4 1.35 -> 1.31.  The partners' rows come
 // mostly from L2 (16 % L1 hits), whose latency bounds it now; more warps per SM at
 // fewer registers spill (1.57 ms at 12 blocks), a table of the pair functions in
 // shared-memory-free FP32 cost more in scattered loads than it saved (1.64 ms).
@@ -332,9 +333,8 @@ cudaError_t launch_any(const RealArgs<float> *one, int R, const Launch &l) {
     switch (R) {
         case 1: return launch_form<0, 1>(one, l);
         case 2: return launch_form<0, 2>(one, l);
-        case 3: return launch_form<0, 3>(one, l);
-        case 4: return launch_form<0, 4>(one, l);
         default:
+            if (R <= 4) return launch_form<2, 0>(one, l);
             if (R <= 8) return launch_form<4, 0>(one, l);
             if (R <= 16) return launch_form<8, 0>(one, l);
             return launch_form<16, 0>(one, l);

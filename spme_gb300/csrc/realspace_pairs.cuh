@@ -260,13 +260,91 @@ __device__ __forceinline__ PairSum<float> shfl_xor(PairSum<float> a, int w) {
     return a;
 }
 
+// The sum over a lane's pairs of one particle, RB right-hand sides: component k = 3 r + d.
+// FP64: plain.  FP32: component pairs as two-lane operations, moved to compensated
+// sums every kRun pairs (RB = 1: each pair).
+template <typename T, int RB>
+struct ShareSum {
+    T acc[3 * RB] = {};
+    // row: the partner's force row, from right-hand side r0 on, of which nr are left
+    __device__ __forceinline__ void pair(T A, T B, const T (&d)[3], const T *__restrict__ row, int nr) {
+#pragma unroll
+        for (int r = 0; r < RB; r++) {
+            if (RB == 1 || r < nr) {
+                const T f0 = __ldg(row + 3 * r), f1 = __ldg(row + 3 * r + 1), f2 = __ldg(row + 3 * r + 2);
+                const T g = B * fma(d[2], f2, fma(d[1], f1, d[0] * f0));
+                acc[3 * r] = fma(g, d[0], fma(A, f0, acc[3 * r]));
+                acc[3 * r + 1] = fma(g, d[1], fma(A, f1, acc[3 * r + 1]));
+                acc[3 * r + 2] = fma(g, d[2], fma(A, f2, acc[3 * r + 2]));
+            }
+        }
+    }
+    __device__ __forceinline__ void step(int) {}
+    __device__ __forceinline__ void finish() {}
+    __device__ __forceinline__ PairSum<T> get(int k) const { return PairSum<T>{acc[k]}; }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int k = 0; k < 3 * RB; k++) acc[k] = T(0);
+    }
+};
+template <int RB>
+struct ShareSum<float, RB> {
+    static constexpr int H = (3 * RB + 1) / 2, kRun = RB;
+    float2 run[H] = {}, s[H] = {}, c[H] = {};
+    static __device__ __forceinline__ float2 sub(float2 a, float2 b) {
+        return __ffma2_rn(make_float2(-1.f, -1.f), b, a);
+    }
+    __device__ __forceinline__ void pair(float A, float B, const float (&d)[3], const float *row) {
+        float g[RB];
+#pragma unroll
+        for (int r = 0; r < RB; r++)
+            g[r] = B * fmaf(d[2], row[3 * r + 2], fmaf(d[1], row[3 * r + 1], d[0] * row[3 * r]));
+#pragma unroll
+        for (int m = 0; m < H; m++) {
+            constexpr int last = 3 * RB - 1;  // (odd 3 RB: the second lane again, unused)
+            const int k = 2 * m, l = 2 * m + 1 <= last ? 2 * m + 1 : last;
+            const float2 t = __ffma2_rn(make_float2(g[k / 3], g[l / 3]),
+                                        make_float2(d[k % 3], d[l % 3]),
+                                        __fmul2_rn(make_float2(A, A), make_float2(row[k], row[l])));
+            run[m] = kRun == 1 ? t : __fadd2_rn(run[m], t);
+        }
+        if (kRun == 1) fold();
+    }
+    // TwoSum of run into (s, c)
+    __device__ __forceinline__ void fold() {
+#pragma unroll
+        for (int m = 0; m < H; m++) {
+            const float2 t = __fadd2_rn(s[m], run[m]), bp = sub(t, s[m]);
+            c[m] = __fadd2_rn(c[m], __fadd2_rn(sub(s[m], sub(t, bp)), sub(run[m], bp)));
+            s[m] = t;
+            run[m] = make_float2(0.f, 0.f);
+        }
+    }
+    // after the lane's pair i
+    __device__ __forceinline__ void step(int i) {
+        if (kRun > 1 && i % kRun == kRun - 1) fold();
+    }
+    __device__ __forceinline__ void finish() {
+        if (kRun > 1) fold();
+    }
+    __device__ __forceinline__ PairSum<float> get(int k) const {
+        PairSum<float> v;
+        v.s = k & 1 ? s[k / 2].y : s[k / 2].x;
+        v.c = k & 1 ? c[k / 2].y : c[k / 2].x;
+        return v;
+    }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int m = 0; m < H; m++) s[m] = c[m] = make_float2(0.f, 0.f);
+    }
+};
+
 constexpr int kList = 512;  // listed pairs per warp (few right-hand sides)
 
 template <typename T, int RB>
 struct FewShared {
     static constexpr int S = 3 * RB;
-    T first[32][S], last[32][S];  // a lane's first and last partial sum
-    T mid[kGroup][S];             // a particle wholly inside one lane's share
+    PairSum<T> first[32][S], last[32][S];  // a lane's first and last partial sum
     PairSum<T> res[kGroup][S];
     T px[kGroup], py[kGroup], pz[kGroup];
     float4 pf[kGroup];            // FP32 position, particle id (bits)
@@ -279,7 +357,7 @@ struct FewShared {
 // which evaluate (pair_AB: A = F, B = G / r^2 at s = r^2) and accumulate in
 // registers; a particle's partial sums, one per share it touches, are added in
 // list order: the same order on every run, a few additions instead of a butterfly
-// per particle.
+// per particle.  FP32 sums are compensated all the way (ShareSum).
 template <typename T, int RB, typename AB>
 __device__ __forceinline__ void realspace_few_body(const RealArgs<T> &A, int cell, T L, T h, T rc2,
                                                    T self_c, AB pair_AB) {
@@ -316,36 +394,42 @@ __device__ __forceinline__ void realspace_few_body(const RealArgs<T> &A, int cel
                 const int nh = list_pairs<false, kList>(cl, ws.pf, np, ws.list, ws.beg, ls, 0);
                 // sum the listed pairs: lane's share [lane c, lane c + c)
                 const int c = (nh + 31) >> 5;
-                T acc[S];
-#pragma unroll
-                for (int k = 0; k < S; k++) acc[k] = T(0);
+                ShareSum<T, RB> acc;
+                // the sum of particle cur, whose entries in the share end here: the lane's
+                // first or last partial sum, or all of the particle's in this list
                 int cur = -1, nseg = 0;
+                auto put = [&](bool at_end) {
+                    acc.finish();
+                    if (nseg == 0 || at_end) {
+                        PairSum<T> *dst = nseg == 0 ? ws.first[lane] : ws.last[lane];
+#pragma unroll
+                        for (int k = 0; k < S; k++) dst[k] = acc.get(k);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < S; k++) ws.res[cur][k].join(acc.get(k));
+                    }
+                    acc.clear();
+                    nseg++;
+                };
                 const int e1 = min(nh, lane * c + c);
                 for (int t = lane * c; t < e1; t++) {
                     const uint32_t ent = ws.list[t];
                     const int ip = (int)(ent >> 28);
                     if (ip != cur) {
-                        if (cur >= 0) {
-                            T *dst = nseg == 0 ? ws.first[lane] : ws.mid[cur];
-#pragma unroll
-                            for (int k = 0; k < S; k++) dst[k] = acc[k];
-                            nseg++;
-#pragma unroll
-                            for (int k = 0; k < S; k++) acc[k] = T(0);
-                        }
+                        if (cur >= 0) put(false);
                         cur = ip;
                     }
                     T x, y, z;
                     int j;
                     cl.candidate((int)(ent & 0x0fffffffu), x, y, z, j);
-                    T d0 = ws.px[ip] - x, d1 = ws.py[ip] - y, d2 = ws.pz[ip] - z;
-                    cl.min_image(d0, d1, d2);
-                    const T s = fma(d2, d2, fma(d1, d1, d0 * d0));
+                    T d[3] = {ws.px[ip] - x, ws.py[ip] - y, ws.pz[ip] - z};
+                    cl.min_image(d[0], d[1], d[2]);
+                    const T s = fma(d[2], d[2], fma(d[1], d[1], d[0] * d[0]));
                     T Av, Bv;
-                    // FP32 (one sweep of all RB = R): the padded row as 16-byte vectors
-                    constexpr int SV = (S + 3) / 4 * 4;
-                    T row[SV];
                     if constexpr (sizeof(T) == 4) {
+                        // (one sweep of all RB = R) the padded row as 16-byte vectors
+                        constexpr int SV = (S + 3) / 4 * 4;
+                        T row[SV];
                         const float4 *f4 =
                             reinterpret_cast<const float4 *>(A.F2) + (size_t)j * (SV / 4);
 #pragma unroll
@@ -356,35 +440,18 @@ __device__ __forceinline__ void realspace_few_body(const RealArgs<T> &A, int cel
                             row[4 * q + 2] = v.z;
                             row[4 * q + 3] = v.w;
                         }
+                        pair_AB(s, Av, Bv);
+                        acc.pair(Av, Bv, d, row);
+                    } else if (pair_AB(s, Av, Bv)) {
+                        acc.pair(Av, Bv, d, F + (size_t)j * C + 3 * r0, A.R - r0);
                     }
-                    if (pair_AB(s, Av, Bv)) {
-                        const T *fj = F + (size_t)j * C + 3 * r0;
-#pragma unroll
-                        for (int r = 0; r < RB; r++) {
-                            if (RB == 1 || sizeof(T) == 4 || r0 + r < A.R) {
-                                if constexpr (sizeof(T) == 8) {
-                                    row[3 * r] = __ldg(fj + 3 * r);
-                                    row[3 * r + 1] = __ldg(fj + 3 * r + 1);
-                                    row[3 * r + 2] = __ldg(fj + 3 * r + 2);
-                                }
-                                const T f0 = row[3 * r], f1 = row[3 * r + 1], f2 = row[3 * r + 2];
-                                const T g = Bv * fma(d2, f2, fma(d1, f1, d0 * f0));
-                                acc[3 * r] = fma(g, d0, fma(Av, f0, acc[3 * r]));
-                                acc[3 * r + 1] = fma(g, d1, fma(Av, f1, acc[3 * r + 1]));
-                                acc[3 * r + 2] = fma(g, d2, fma(Av, f2, acc[3 * r + 2]));
-                            }
-                        }
-                    }
+                    acc.step(t - lane * c);
                 }
-                if (cur >= 0) {
-                    T *dst = nseg == 0 ? ws.first[lane] : ws.last[lane];
-#pragma unroll
-                    for (int k = 0; k < S; k++) dst[k] = acc[k];
-                }
+                if (cur >= 0) put(true);
                 __syncwarp();
                 // a particle's partial sums in share order: a share's first partial sum
                 // when the particle's entries reach its start, its last when they reach
-                // its end, else the one in between
+                // its end (entries that reach neither are in res)
                 const int npl = min(ls.il, np - 1) - ilo + 1;
                 for (int t = lane; t < npl * S; t += 32) {
                     const int ip = ilo + t / S, k = t % S;
@@ -393,11 +460,10 @@ __device__ __forceinline__ void realspace_few_body(const RealArgs<T> &A, int cel
                     if (ip == ls.il && ls.q0 == 0) continue;
                     const int b = ws.beg[ip], e = ws.beg[ip + 1];
                     if (e <= b) continue;
+                    if (b % c && e < min(nh, b / c * c + c)) continue;
                     PairSum<T> sum = ws.res[ip][k];
                     for (int l = b / c; l * c < e; l++)
-                        sum.add(b <= l * c ? ws.first[l][k]
-                                           : (e >= min(nh, l * c + c) ? ws.last[l][k]
-                                                                      : ws.mid[ip][k]));
+                        sum.join(b <= l * c ? ws.first[l][k] : ws.last[l][k]);
                     ws.res[ip][k] = sum;
                 }
                 __syncwarp();

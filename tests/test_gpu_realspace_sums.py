@@ -18,6 +18,12 @@ BIG = 2.0 ** 20
 
 
 @pytest.mark.parametrize("R,n,who,plus,small,minus", [
+    # up to 4: a lane's share of the 13 x 25 pairs that a warp lists, eleven of them
+    (1, 26, 0, 1, 2, 3),
+    (1, 26, 0, 1, 5, 9),
+    (2, 26, 0, 1, 5, 9),
+    (3, 26, 0, 1, 5, 9),
+    (4, 26, 0, 1, 5, 9),
     # more than 4 right-hand sides: pair slots of 32 / 4, 32 / 8, 32 / 16 lanes
     (5, 26, 0, 1, 2, 3),      # three slots, summed across slots
     (12, 26, 0, 1, 2, 3),
