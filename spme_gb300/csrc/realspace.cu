@@ -55,7 +55,8 @@ namespace {
 __device__ __forceinline__ void real_FG_f32(float r2, const RealCoef &c, float &F, float &G,
                                             float &ir) {
     constexpr float rsp = 0.56418958354775628695f;  // 1/sqrt(pi)
-    ir = r2 > 0.f ? rsqrtf(r2) : 0.f;
+    // (below r = 1e-18 as at r = 0: the caller's 1/r^2 would overflow, and G vanishes there)
+    ir = r2 >= 1e-36f ? rsqrtf(r2) : 0.f;
     const float r = r2 * ir;
     if (r2 < c.a2x4) {
         const float x = c.xi * r, x2 = x * x, e = expf(-x2);
