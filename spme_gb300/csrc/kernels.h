@@ -295,8 +295,9 @@ struct PairTable {
     long long lo_bits = 0, mid_bits = 0, hi_bits = 0;
     int base = 0, shift = 14;
 };
-// Fits the table on the host (checked between nodes to 2e-13 relative);
-// false if no fit meets that within 1024 segments per octave.
+// Fits the table on the host (the segments that meet 2e-13 relative between nodes, halved:
+// the error left is that of the closed form's values); false if no fit meets that within
+// 1024 segments per octave.
 bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef, PairTable *t);
 // cpos: float4 for T = float, double4_32a for T = double (cell-relative); FP32 in
 // realspace.cu (tab unused), FP64 in realspace_fp64.cu.  F2 (FP32; unused in FP64):

@@ -34,7 +34,7 @@ namespace {
 // for r < 2a plus (overlap RPY - far-field RPY), written in the cancellation-free
 // form of realspace.cu: x = xi r, S(x) = erf(x)/x and psi(x) = (erf(x) -
 // 2x e^{-x^2}/sqrt(pi)) / x^3, for x < 0.5 from their Maclaurin series in x^2
-// (ten terms: below 1e-17 relative; the factor 2/sqrt(pi) outside).  `near`
+// (thirteen terms: below 1e-19 relative; the factor 2/sqrt(pi) outside).  `near`
 // selects the form; both are analytic on either side of r = 2a.
 __host__ __device__ inline void real_FG(double r, double xi, double a, bool near, double &F,
                                         double &G) {
@@ -43,16 +43,18 @@ __host__ __device__ inline void real_FG(double r, double xi, double a, bool near
     if (near) {
         double S = 0.0, P = 0.0;
         if (x < 0.5) {
-            const double ks[10] = {1.0, -1.0 / 3, 1.0 / 10, -1.0 / 42, 1.0 / 216,
-                                   -1.0 / 1320, 1.0 / 9360, -1.0 / 75600,
-                                   1.0 / 685440, -1.0 / 6894720};
-            const double kp[10] = {2.0 / 3, -2.0 / 5, 1.0 / 7, -1.0 / 27, 1.0 / 132,
-                                   -1.0 / 780, 1.0 / 5400, -1.0 / 42840,
-                                   1.0 / 383040, -1.0 / 3810240};
+            const double ks[13] = {1.0, -1.0 / 3, 1.0 / 10, -1.0 / 42, 1.0 / 216,
+                                   -1.0 / 1320, 1.0 / 9360, -1.0 / 75600, 1.0 / 685440,
+                                   -1.0 / 6894720, 1.0 / 76204800, -1.0 / 918086400,
+                                   1.0 / 11975040000};
+            const double kp[13] = {2.0 / 3, -2.0 / 5, 1.0 / 7, -1.0 / 27, 1.0 / 132,
+                                   -1.0 / 780, 1.0 / 5400, -1.0 / 42840, 1.0 / 383040,
+                                   -1.0 / 3810240, 1.0 / 41731200, -1.0 / 498960000,
+                                   1.0 / 6466521600};
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
-            for (int k = 9; k >= 0; k--) {
+            for (int k = 12; k >= 0; k--) {
                 S = S * x2 + ks[k];
                 P = P * x2 + kp[k];
             }
@@ -259,7 +261,10 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
     // (a/2)^2 the closed form is evaluated directly (rare pairs).
     const double lo = 0.25 * a * a, mid = 4.0 * a * a, hi = rc * rc;
     if (hi <= lo) return false;
-    for (int m = 6; m <= 10; m++) {  // 2^m segments per octave of s
+    // (2^m segments per octave of s: twice those that pass, so that the fit, 2^-7 of the
+    // bound then, stays below the rounding of the values it goes through)
+    bool passed = false;
+    for (int m = 6; m <= (passed ? 11 : 10); m++) {
         const int shift = 20 - m;
         auto seg_of = [&](double s) { return (int)((bits_of(s) >> 32) >> shift); };
         auto start_of = [&](int g) {
@@ -282,7 +287,7 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
             double *c = coef->data() + (size_t)q * (kPairDeg + 1) * 2;
             fit_segment(s0, h, xi, a, near, c);
             // the fit between the nodes, relative to the function scale there
-            for (int p = 0; p <= 8 && ok; p++) {
+            for (int p = 0; p <= 8 && ok && !passed; p++) {
                 const double s = s0 + h * p / 8.0, v = s - (s0 + 0.5 * h);
                 if (s < lo || s > hi || (near != (s < mid))) continue;
                 double F, G;
@@ -297,6 +302,10 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
             }
         }
         if (!ok) continue;
+        if (!passed) {
+            passed = true;
+            continue;
+        }
         t->coef = nullptr;  // the caller points it at the device copy
         t->lo_bits = bits_of(lo);
         t->mid_bits = bits_of(mid);
