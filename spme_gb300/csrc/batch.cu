@@ -445,7 +445,8 @@ struct _spme_batch_t {
     uint32_t *d_rst1 = nullptr, *d_rst2 = nullptr;
     void *d_rw1 = nullptr, *d_rw2 = nullptr;
     void *d_F = nullptr, *d_Fs = nullptr, *d_W = nullptr, *d_W2 = nullptr;
-    void *d_F2 = nullptr;  // force rows as the FP32 real-space sum reads them
+    void *d_F2 = nullptr;   // force rows as the FP32 real-space sum reads them,
+    void *d_F2z = nullptr;  // after their row of zeros
     void *d_mesh = nullptr, *d_spec = nullptr, *d_tab = nullptr;
     double *d_twopi_L = nullptr;  // per system, in group order
     double *d_pair = nullptr;  // FP64 batches: pair-function tables of all systems
@@ -712,8 +713,12 @@ int create_t(_spme_batch_t *b) {
     BTRY(balloc(&b->d_rw1, sizeof(T) * (size_t)b->ws * n));
     BTRY(balloc(&b->d_rw2, sizeof(T) * (size_t)b->ws * n));
     BTRY(balloc(&b->d_F, sizeof(T) * (size_t)C * n));
-    if (sizeof(T) == 4)
-        BTRY(balloc(&b->d_F2, sizeof(T) * (size_t)real_row(b->R) * n));
+    if (sizeof(T) == 4) {
+        const size_t lead = sizeof(T) * real_lead(b->R);
+        BTRY(balloc(&b->d_F2z, lead + sizeof(T) * (size_t)real_row(b->R) * n));
+        BTRY_CUDA(cudaMemset(b->d_F2z, 0, lead));
+        b->d_F2 = (char *)b->d_F2z + lead;
+    }
     BTRY(balloc(&b->d_Fs, sizeof(T) * (size_t)spread_cols_row_width(C) * n));
     BTRY(balloc(&b->d_W, sizeof(T) * (size_t)C * n));
     BTRY(balloc(&b->d_W2, sizeof(T) * (size_t)C * n));
@@ -1053,7 +1058,7 @@ void destroy_b(_spme_batch_t *b) {
                     b->d_off2,  b->d_off3,  b->d_scan_tmp, b->d_perm1, b->d_perm2,
                     b->d_perm3, b->d_pstart, b->d_pfrac, b->d_prel, b->d_cpos,  b->d_ridx1,
                     b->d_ridx2, b->d_rst1,  b->d_rst2,  b->d_rw1,   b->d_rw2,   b->d_F,
-                    b->d_Fs,    b->d_F2,    b->d_W,     b->d_W2,    b->d_mesh,  b->d_spec,  b->d_tab,
+                    b->d_Fs,    b->d_F2z,   b->d_W,     b->d_W2,    b->d_mesh,  b->d_spec,  b->d_tab,
                     b->d_pair,  b->d_err,   b->d_spread_sys, b->d_interp_sys,
                     b->d_real_sys, b->d_infl_sys, b->d_pre_spread, b->d_pre_interp,
                     b->d_pre_real, b->d_pre_infl, b->d_twopi_L};

@@ -163,7 +163,8 @@ struct _spme_t {
     void *d_work = nullptr;
     size_t work_bytes = 0;
     std::vector<PlanPair> plans;
-    void *d_F2 = nullptr;  // force rows as the FP32 real-space sum reads them
+    void *d_F2 = nullptr;   // force rows as the FP32 real-space sum reads them,
+    void *d_F2z = nullptr;  // after their row of zeros
     void *d_F = nullptr, *d_W = nullptr, *d_fstage = nullptr, *d_ustage = nullptr;
     void *d_W2 = nullptr;  // mesh part of the result when the real-space part is in d_W
     int *d_err = nullptr;  // device-side error flag (TMA wait timeouts)
@@ -621,7 +622,10 @@ int create_impl(const spme_params &prm, spme_t **out) {
             // (a pass of fewer right-hand sides may have the wider rows: 4 against 5)
             size_t row = 0;
             for (int r = 1; r <= prm.max_nrhs; r++) row = std::max<size_t>(row, spme::real_row(r));
-            TRY(dalloc(&e->d_F2, e->elem * n * row));
+            const size_t lead = e->elem * spme::real_lead(prm.max_nrhs);
+            TRY(dalloc(&e->d_F2z, lead + e->elem * n * row));
+            TRY_CUDA(cudaMemset(e->d_F2z, 0, lead));
+            e->d_F2 = (char *)e->d_F2z + lead;
         }
     }
     if (prm.terms & SPME_TERM_RECIP) {
@@ -760,7 +764,7 @@ void destroy_impl(spme_t *e) {
                     e->d_zip,    e->d_f2tab,    e->d_soff,   e->d_sperm, e->d_srec_idx,
                     e->d_srec_start, e->d_srec_w, e->d_Fs, e->d_W2, e->d_pair, e->d_key2,
                     e->d_key3,   e->d_pstart, e->d_pfrac, e->d_box,
-                    e->d_boxtab, e->d_F2};
+                    e->d_boxtab, e->d_F2z};
     for (void *b : bufs) dfree(b);
     for (int i = 0; i <= kStages; i++)
         if (e->ev[i]) cudaEventDestroy(e->ev[i]);

@@ -303,7 +303,9 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
 // realspace.cu (tab unused), FP64 in realspace_fp64.cu.  F2 (FP32; unused in FP64):
 // the force rows as that kernel reads them, real_row(R) values each: for up to
 // kRealFew right-hand sides in F's order padded to 16 bytes, for more by component
-// ([d][rows_even(R)]); the padding is zero.
+// ([d][rows_even(R)]); the padding is zero, and so are the real_lead(R) values before F2
+// (row -1, which padding entries of the pair lists take: a particle's own row there
+// would turn an infinite force into 0 inf).
 // The line between the forms: with 3 and 4 right-hand sides the compensated sums of the
 // first (per lane) need more registers and shared memory: N = 1e6, R = 3 1.37 against 1.31 ms,
 // R = 4 1.53 against 1.31, at volume fraction 0.12 2.72 against 2.07; at R = 2 1.07 ms.
@@ -312,6 +314,8 @@ __host__ __device__ constexpr int rows_even(int R) { return (R + 1) & ~1; }
 __host__ __device__ constexpr int real_row(int R) {
     return R <= kRealFew ? (3 * R + 3) / 4 * 4 : 3 * rows_even(R);
 }
+// Zeros before the rows of up to R right-hand sides (256-byte steps).
+__host__ __device__ constexpr int real_lead(int R) { return (3 * rows_even(R) + 63) / 64 * 64; }
 // The place of right-hand side r, component d in such a row.
 __host__ __device__ constexpr int real_at(int R, int r, int d) {
     return R <= kRealFew ? 3 * r + d : d * rows_even(R) + r;

@@ -182,7 +182,7 @@ __device__ __forceinline__ void real_many(const RealArgs<float> &A, int cell) {
                                     const uint32_t ent = ws.list[t];
                                     const float4 me = ws.pf[ent >> 28];
                                     float d0 = 0.f, d1 = 0.f, d2 = 0.f, Av = 0.f, Bv = 0.f;
-                                    int j = __float_as_int(me.w);
+                                    int j = -1;  // padding: the row of zeros
                                     if ((ent & kNoCand) != kNoCand) {
                                         float x, y, z;
                                         cl.candidate((int)(ent & kNoCand), x, y, z, j);
@@ -214,7 +214,7 @@ __device__ __forceinline__ void real_many(const RealArgs<float> &A, int cell) {
                                 const float4 a = ws.r0[q];
                                 const float2 b = ws.r1[q];
                                 const float *fj =
-                                    Fr + (size_t)__float_as_int(b.y) * (size_t)(3 * R2);
+                                    Fr + (ptrdiff_t)__float_as_int(b.y) * (3 * R2);
                                 const float2 f0 = __ldg(reinterpret_cast<const float2 *>(fj));
                                 const float2 f1 = __ldg(reinterpret_cast<const float2 *>(fj + R2));
                                 const float2 f2 =
