@@ -130,9 +130,9 @@ int spme_set_overlap(spme_t *spme, int on);
  * each mesh column visits only the particles whose stencil covers it; else the
  * tile kernel.  0: tile kernel
  * always, threads own the columns of a mesh tile and visit every particle
- * staged for the tile.  Mode 1 on an engine whose mesh is too small for the
- * column gather (K < p + 15 in FP32, p + 7 in FP64) returns
- * SPME_ERR_UNSUPPORTED (its default kernel stays). */
+ * staged for the tile.  Mode 1 on an engine without boxes whose mesh is too small
+ * for the column gather (K < p + 15 in FP32, p + 7 in FP64) returns
+ * SPME_ERR_UNSUPPORTED (the kernel in use stays). */
 int spme_set_spread_mode(spme_t *spme, int mode);
 
 /* Transform strategy of the mesh pass.  1: 2D (y, x) transforms of every z-plane,

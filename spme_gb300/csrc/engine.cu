@@ -1286,7 +1286,7 @@ int spme_set_overlap(spme_t *e, int on) {
 int spme_set_spread_mode(spme_t *e, int mode) {
     if (!e || (mode != 0 && mode != 1)) return SPME_ERR_INVALID;
     DeviceGuard dg(e->device);
-    if (mode == 1 && !e->cols_fit) return e->last_error = SPME_ERR_UNSUPPORTED;
+    if (mode == 1 && !e->cols_fit && !e->box) return e->last_error = SPME_ERR_UNSUPPORTED;
     if (e->stream) cudaStreamSynchronize(e->stream);
     drop_graphs(e);
     e->spread_mode = mode;
