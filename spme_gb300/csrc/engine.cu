@@ -136,11 +136,12 @@ struct _spme_t {
     int *d_rec_idx = nullptr;
     uint32_t *d_rec_start = nullptr;
     void *d_rec_w = nullptr;
-    // column-gather spread: records sorted by stencil-start cell (K^3 keys)
+    // column-gather spread: records sorted by stencil-start cell (K^3 keys), where it is
+    // the current tile's
     bool cols = false;
     bool cols_fit = false;  // the mesh admits it (spread mode 1 is accepted)
-    // box spread (few components): scratch for box_slots components' boxes of the
-    // current tile (0 slots: not used)
+    // box spread: whether boxes are faster at these sizes; scratch for box_slots
+    // components' boxes of the current tile (0 slots: not used)
     bool box = false;
     void *d_box = nullptr;
     size_t box_cap = 0;
@@ -148,6 +149,7 @@ struct _spme_t {
     int *d_boxtab = nullptr;  // coverage offsets of the current tile (3 K entries of 4)
     spme::BoxTable boxtab;
     int boxtab_tile[3] = {0, 0, 0};
+    int spread_tile[3] = {0, 0, 0};  // the tile that box_slots and cols were chosen for
     int spread_mode = 1;  // 1: box or column-gather kernel where they apply, 0: tile kernel
     int *d_soff = nullptr, *d_sperm = nullptr, *d_srec_idx = nullptr;
     uint32_t *d_srec_start = nullptr;
@@ -175,7 +177,7 @@ struct _spme_t {
     int *d_zip = nullptr;
     void *d_f2tab = nullptr;  // one-pass 2D transform tables (fft_mode 2)
     CUtensorMap zmap;  // over the half spectrum (fft_mode 1)
-    size_t cap_tiles = 0;  // allocated tile-count capacity
+    size_t cap_tiles = 0, cap_keys = 0;  // allocated capacity: tiles, keys of all sorts
     // CUDA graphs: passes and device-pointer position builds are captured once
     // per key and replayed (spme_set_graphs)
     bool use_graphs = false;
@@ -299,15 +301,15 @@ bool box_pays(size_t elem, int p, int C, int K) {
     return K >= 96 && ((p == 4 && C <= 6) || (p == 6 && C <= 3));
 }
 // Scratch bounds: boxes of as many components at a time as fit in kBoxScratch,
-// and no box spread where one component's boxes exceed kBoxMax (then the
-// column-gather or the tile kernel runs).
+// and no box spread where one component's boxes exceed kBoxMax (K = 410, 5x5x5 tiles; then
+// the column-gather or the tile kernel runs).
 constexpr size_t kBoxScratch = (size_t)1 << 30, kBoxMax = (size_t)4 << 30;
 
 // Scratch and coverage table for the current tile; without them (too large, or no
 // memory) the box spread is off.
 void alloc_box(spme_t *e) {
-    if (!e->box || (e->boxtab.tab && e->boxtab_tile[0] == e->g.tx &&
-                    e->boxtab_tile[1] == e->g.ty && e->boxtab_tile[2] == e->g.tz))
+    if ((e->boxtab.tab && e->boxtab_tile[0] == e->g.tx &&
+         e->boxtab_tile[1] == e->g.ty && e->boxtab_tile[2] == e->g.tz))
         return;
     const size_t one = spme::spread_box_bytes(e->g, e->elem);
     e->box_slots = 0;
@@ -340,20 +342,58 @@ void alloc_box(spme_t *e) {
     e->box_slots = slots;
 }
 
+// Records by start cell and force rows in that order (column gather).
+int alloc_cols(spme_t *e) {
+    const size_t n = (size_t)e->prm.np, K = (size_t)e->prm.dim;
+    TRY(dalloc(&e->d_soff, sizeof(int) * (K * K * K + 1)));
+    TRY(dalloc(&e->d_sperm, sizeof(int) * n));
+    TRY(dalloc(&e->d_key2, sizeof(int) * n));
+    TRY(dalloc(&e->d_srec_idx, sizeof(int) * n));
+    TRY(dalloc(&e->d_srec_start, sizeof(uint32_t) * n));
+    TRY(dalloc(&e->d_srec_w, e->elem * record_width(e) * n));
+    return dalloc(&e->d_Fs, e->elem * (size_t)spme::spread_cols_row_width(e->Cmax) * n);
+}
+
+void free_cols(spme_t *e) {
+    void *bufs[] = {e->d_soff, e->d_sperm, e->d_key2, e->d_srec_idx, e->d_srec_start, e->d_srec_w, e->d_Fs};
+    for (void *b : bufs) dfree(b);
+    e->d_soff = e->d_sperm = e->d_key2 = e->d_srec_idx = nullptr;
+    e->d_srec_start = nullptr;
+    e->d_srec_w = e->d_Fs = nullptr;
+}
+
+// The spread of the current tile: boxes where they pay and fit, else the column gather
+// where it applies (its buffers made when it is first needed), else the tile kernel.
+int choose_spread(spme_t *e) {
+    const int tile[3] = {e->g.tx, e->g.ty, e->g.tz};
+    if (!(e->prm.terms & SPME_TERM_RECIP) || !std::memcmp(e->spread_tile, tile, sizeof(tile)))
+        return SPME_OK;
+    std::memcpy(e->spread_tile, tile, sizeof(tile));
+    if (e->box) alloc_box(e);
+    // (FP32 passes of fewer than 9 components never take the column gather)
+    e->cols = e->cols_fit && e->box_slots == 0 && (e->elem == 8 || e->Cmax >= 9);
+    if (!e->cols || e->d_Fs) return SPME_OK;
+    const int st = alloc_cols(e);
+    if (st != SPME_OK) {
+        free_cols(e);
+        e->cols = false;
+    }
+    return st;
+}
+
 int alloc_tiles(spme_t *e) {
-    alloc_box(e);
-    size_t need = (size_t)e->ntiles;
-    if (need <= e->cap_tiles && e->d_count) return SPME_OK;
+    const size_t need = (size_t)e->ntiles, K = e->prm.dim;
+    const size_t nkeys = need + (size_t)e->nc * e->nc * e->nc + (e->cols ? K * K * K : 0);
+    if (need <= e->cap_tiles && nkeys <= e->cap_keys && e->d_count) return SPME_OK;
     dfree(e->d_count);
     dfree(e->d_toff);
     dfree(e->d_scan_tmp);
     e->d_count = e->d_toff = e->d_scan_tmp = nullptr;
-    const size_t K = e->prm.dim;
-    const size_t nkeys = need + (size_t)e->nc * e->nc * e->nc + (e->cols ? K * K * K : 0);
     TRY(dalloc(&e->d_count, sizeof(int) * nkeys));
     TRY(dalloc(&e->d_toff, sizeof(int) * (need + 1)));
     TRY(dalloc(&e->d_scan_tmp, sizeof(int) * spme::scan_tmp_elems((long)nkeys)));
     e->cap_tiles = need;
+    e->cap_keys = nkeys;
     return SPME_OK;
 }
 
@@ -584,20 +624,7 @@ int create_impl(const spme_params &prm, spme_t **out) {
     }
     e->cols_fit = (prm.terms & SPME_TERM_RECIP) && spme::spread_cols_ok((int)K, (int)C, e->elem, prm.porder);
     e->box = (prm.terms & SPME_TERM_RECIP) && box_pays(e->elem, prm.porder, (int)C, (int)K);
-    alloc_box(e);
-    e->box = e->box_slots > 0;
-    // (FP32 passes of fewer than 9 components never take the column gather)
-    e->cols = e->cols_fit && !e->box && (e->elem == 8 || C >= 9);
-    if (e->cols) {
-        const size_t K3 = K * K * K;
-        TRY(dalloc(&e->d_soff, sizeof(int) * (K3 + 1)));
-        TRY(dalloc(&e->d_sperm, sizeof(int) * n));
-        TRY(dalloc(&e->d_key2, sizeof(int) * n));
-        TRY(dalloc(&e->d_srec_idx, sizeof(int) * n));
-        TRY(dalloc(&e->d_srec_start, sizeof(uint32_t) * n));
-        TRY(dalloc(&e->d_srec_w, e->elem * record_width(e) * n));
-        TRY(dalloc(&e->d_Fs, e->elem * (size_t)spme::spread_cols_row_width((int)C) * n));
-    }
+    TRY(choose_spread(e));
     TRY(alloc_tiles(e));
     TRY(dalloc(&e->d_rec_idx, sizeof(int) * n));
     TRY(dalloc(&e->d_rec_start, sizeof(uint32_t) * n));
@@ -844,6 +871,7 @@ int set_positions_impl(spme_t *e, const double *pos, int mem) {
     if (e->prm.np > 0 && !pos) return SPME_ERR_INVALID;
     if (e->prm.terms & SPME_TERM_RECIP) {
         set_geometry(e);
+        choose_spread(e);  // (without memory for the column gather: the tile kernel)
         TRY(alloc_tiles(e));
     }
     // host positions come from pageable memory: never captured

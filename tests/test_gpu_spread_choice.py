@@ -1,5 +1,6 @@
 """The spread that an engine takes: the default (mode 1) can be had back after mode 0,
-on meshes too small for the column gather too."""
+on meshes too small for the column gather too, and a tile whose boxes do not fit takes
+the column gather."""
 import numpy as np
 import pytest
 
@@ -40,3 +41,27 @@ def test_no_other_spread(gpu_lib):
         with pytest.raises(spme_gb300.SpmeError) as err:
             eng.set_spread_mode(1)
         assert err.value.code == spme_gb300.ERR_UNSUPPORTED
+
+
+def test_tile_without_boxes(gpu_lib):
+    # 5x5x5 tiles at K = 410: over 4 GB of boxes for a component.  The column gather's two
+    # kernels against the tile kernel's one (boxes: two per component); results as the
+    # kernels' tests have them (FP64 1e-13 relative L2)
+    n, L, K = 80_000, 700.0, 410
+    rng = np.random.default_rng(K)
+    pos, f = rng.uniform(0, L, (n, 3)), rng.standard_normal((1, 3 * n))
+    out, used = {}, {}
+    with spme_gb300.Engine(n, L, 0.3, K, 6, precision="fp64", max_nrhs=1,
+                           terms=spme_gb300.TERM_RECIP) as eng:
+        for name, tile, mode in (("default", (8, 8, 8), 1), ("small", (5, 5, 5), 1),
+                                 ("tiles", (5, 5, 5), 0), ("again", (8, 8, 8), 1)):
+            eng.set_spread_mode(mode)
+            eng.set_tile(*tile)
+            eng.set_positions(pos)
+            c = eng.launch_count()
+            out[name] = eng.apply(f)
+            used[name] = eng.launch_count() - c
+    assert used["small"] == used["tiles"] + 1
+    assert np.array_equal(out["default"], out["again"])
+    for name in ("small", "tiles"):
+        assert np.linalg.norm(out[name] - out["default"]) < 1e-13 * np.linalg.norm(out["default"])
