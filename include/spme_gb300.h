@@ -124,7 +124,8 @@ long spme_launch_count(const spme_t *spme);
 int spme_set_overlap(spme_t *spme, int on);
 
 /* Spread kernel.  1 (default): for few components (most FP64 engines of up to
- * 3 right-hand sides, FP32 ones of 1 or 2 at K >= 96) per-tile boxes, one
+ * 3 right-hand sides, FP32 ones of 1 or 2 at K >= 96, unless the particles are sparse on
+ * the mesh or the tile leaves narrow boxes) per-tile boxes, one
  * particle's stencil points across the lanes of a warp; else the column gather
  * where it applies (FP32 from 9 components on, mostly in its z-marching form),
  * each mesh column visits only the particles whose stencil covers it; else the

@@ -140,8 +140,8 @@ struct _spme_t {
     // the current tile's
     bool cols = false;
     bool cols_fit = false;  // the mesh admits it (spread mode 1 is accepted)
-    // box spread: whether boxes are faster at these sizes; scratch for box_slots
-    // components' boxes of the current tile (0 slots: not used)
+    // box spread: whether boxes are faster with the current tile; scratch for box_slots
+    // components' boxes of that tile (0 slots: not used)
     bool box = false;
     void *d_box = nullptr;
     size_t box_cap = 0;
@@ -285,20 +285,54 @@ int record_width(const spme_t *e) {
     return (raw + per16 - 1) / per16 * per16;
 }
 
-// Whether an engine of C components spreads through boxes (spread_box.cu; its
-// default 8x8x8 tile).  The box kernel's cost grows with C, the column gather's is
-// per visit up to 16 components and needs its own sort.  Spread + position build
-// measured on GB300, box vs the other kernel (ms):
-// FP64 (vs column gather), p = 6: N = 1e5, K = 128: C = 3 0.42 vs 1.16, C = 9
-// 0.93 vs 1.17, C = 15 1.55 vs 1.17; N = 2000, K = 64: C = 9 0.142 vs 0.163;
-// p = 4: C = 6 0.43 vs 0.50, C = 9 0.59 vs 0.50; p = 8: C = 9 1.56 vs 2.42, but
-// 0.92 vs 0.86 at K = 90, where tiles that do not divide K make the sum slower.
-// FP32 (vs the tile kernel, spread alone): p = 6: C = 3 0.119 vs 0.145, C = 6
-// 0.214 vs 0.197; p = 4: C = 6 0.145 vs 0.170; p = 8: C = 3 0.176 vs 0.166; K = 64:
-// 0.019 vs 0.016 (one more launch).
-bool box_pays(size_t elem, int p, int C, int K) {
-    if (elem == 8) return C <= (p == 4 || K % 8 != 0 ? 6 : 9);
-    return K >= 96 && ((p == 4 && C <= 6) || (p == 6 && C <= 3));
+// How the boxes overlap: axes on which a mesh point can lie in more than two of them (the
+// axis's tiles, or its last one, narrower than the stencil's p - 1; k_box_sum looks at four
+// tiles then), 2 for any two or three of them, 3 where all tiles are so narrow.
+int box_overlap(const MeshGeom &g) {
+    const int t[3] = {g.tx, g.ty, g.tz}, nt[3] = {g.ntx, g.nty, g.ntz};
+    int n = 0, all = 0;
+    for (int a = 0; a < 3; a++) {
+        n += std::min(t[a], g.K - (nt[a] - 1) * t[a]) < g.p - 1;
+        all += t[a] < g.p - 1;
+    }
+    return all == 3 ? 3 : std::min(n, 2);
+}
+
+// The least particles per mesh point at which an engine of C components spreads through
+// boxes (spread_box.cu).  The boxes' traffic and sum grow with K^3 C, their particles with
+// N C; the column gather (FP64) and the tile kernel (FP32, C < 9) clear and write the mesh
+// once, and cost a lane or a pass more per particle.  Lines by the times of whole steps
+// on GB300, other kernel - boxes (us), K = 128, 8x8x8 tiles, at densities .002 .01 .04 .08
+// (the usual one is .06):
+//   FP64 p = 6, C = 3: 66 172 593 1180, C = 6: -56 33 362 826, C = 9: -179 -104 132 471;
+//        p = 4, C = 3: -16 37 144 334, C = 6: -123 -76 6 148, C = 9: -234 -187 -136 -38;
+//        p = 8, C = 3: 145 355 1409 2831, C = 6: 4 166 1019 2162, C = 9: -136 -25 626 1500;
+//   FP32 p = 4, C = 3: -18 -7 39 100, C = 6: -53 -40 15 92; p = 6, C = 3: -30 -22 19 74, C = 6:
+//        -70 -62 -24 34; p = 8, C = 3: -47 -43 -20 18.
+// One narrow axis (8x8x4 tiles at p = 6: FP64 C = 3 10 124, C = 6 -165 -62, .03: 167) moves the
+// line by about two, FP32 (C = 3 .002: -37, .03: 1) by a fifth; more of them (K = 100, p = 6:
+// FP64 C = 3 -167 -110 104 390, C = 6 -416 -377 -205 24; FP32 C = 3 -87 -83 -61 -26) put it above
+// the usual density but for FP64 with C = 3; with 4x4x4 tiles the FP32 tile kernel is slow
+// too (C = 3 -135 -81, .03: 27, .06: 181, at K = 160 -120 175).
+double box_density(size_t elem, int p, int C, int K, int overlap) {
+    constexpr double no = 1e300;
+    static const double fp64[3][3][3] = {  // [p = 4, 6, 8][overlap 0, 1, 2 and 3][C = 3, 6, 9]
+        {{.006, .045, .13}, {.012, .06, .15}, {.08, no, no}},
+        {{.001, .008, .03}, {.002, .018, .04}, {.03, .08, .2}},
+        {{.0003, .002, .013}, {.001, .01, .026}, {.015, .045, .09}}};
+    static const double fp32[2][4][2] = {{{.016, .042}, {.025, .055}, {no, no}, {no, no}},
+                                         {{.027, no}, {.033, no}, {no, no}, {.045, no}}};
+    const int c = C / 3 - 1, q = p / 2 - 2;
+    if (elem == 8) return c <= 2 ? fp64[q][std::min(overlap, 2)][c] : no;
+    // (K < 96: one more launch costs as much as the boxes give)
+    return K >= 96 && c <= 1 && q <= 1 ? fp32[q][overlap][c] : no;
+}
+
+bool box_pays(const spme_t *e) {
+    // (FP64 without column gather: the tile kernel is far slower at any density)
+    if (e->elem == 8 && !e->cols_fit && e->Cmax <= 9) return true;
+    const double K = e->g.K;
+    return e->prm.np >= K * K * K * box_density(e->elem, e->g.p, e->Cmax, e->g.K, box_overlap(e->g));
 }
 // Scratch bounds: boxes of as many components at a time as fit in kBoxScratch,
 // and no box spread where one component's boxes exceed kBoxMax (K = 410, 5x5x5 tiles; then
@@ -308,8 +342,8 @@ constexpr size_t kBoxScratch = (size_t)1 << 30, kBoxMax = (size_t)4 << 30;
 // Scratch and coverage table for the current tile; without them (too large, or no
 // memory) the box spread is off.
 void alloc_box(spme_t *e) {
-    if ((e->boxtab.tab && e->boxtab_tile[0] == e->g.tx &&
-         e->boxtab_tile[1] == e->g.ty && e->boxtab_tile[2] == e->g.tz))
+    if (e->boxtab.tab && e->boxtab_tile[0] == e->g.tx && e->boxtab_tile[1] == e->g.ty &&
+        e->boxtab_tile[2] == e->g.tz)
         return;
     const size_t one = spme::spread_box_bytes(e->g, e->elem);
     e->box_slots = 0;
@@ -342,6 +376,8 @@ void alloc_box(spme_t *e) {
     e->box_slots = slots;
 }
 
+bool use_box(const spme_t *e) { return e->box && e->box_slots > 0; }
+
 // Records by start cell and force rows in that order (column gather).
 int alloc_cols(spme_t *e) {
     const size_t n = (size_t)e->prm.np, K = (size_t)e->prm.dim;
@@ -369,9 +405,10 @@ int choose_spread(spme_t *e) {
     if (!(e->prm.terms & SPME_TERM_RECIP) || !std::memcmp(e->spread_tile, tile, sizeof(tile)))
         return SPME_OK;
     std::memcpy(e->spread_tile, tile, sizeof(tile));
+    e->box = box_pays(e);
     if (e->box) alloc_box(e);
     // (FP32 passes of fewer than 9 components never take the column gather)
-    e->cols = e->cols_fit && e->box_slots == 0 && (e->elem == 8 || e->Cmax >= 9);
+    e->cols = e->cols_fit && !use_box(e) && (e->elem == 8 || e->Cmax >= 9);
     if (!e->cols || e->d_Fs) return SPME_OK;
     const int st = alloc_cols(e);
     if (st != SPME_OK) {
@@ -623,7 +660,6 @@ int create_impl(const spme_params &prm, spme_t **out) {
         TRY(dalloc(&e->d_pfrac, e->elem * 3 * n));
     }
     e->cols_fit = (prm.terms & SPME_TERM_RECIP) && spme::spread_cols_ok((int)K, (int)C, e->elem, prm.porder);
-    e->box = (prm.terms & SPME_TERM_RECIP) && box_pays(e->elem, prm.porder, (int)C, (int)K);
     TRY(choose_spread(e));
     TRY(alloc_tiles(e));
     TRY(dalloc(&e->d_rec_idx, sizeof(int) * n));
@@ -942,7 +978,7 @@ int run_pass(spme_t *e, int R, const T *f, long ldf, T *u, long ldu, double alph
                               spme::spread_cols_ok(K, C, e->elem, e->g.p) &&
                               (e->elem == 8 || C >= 9) &&
                               (long long)n * spme::spread_cols_row_width(C) < (1LL << 31);
-        if (e->box_slots > 0 && e->spread_mode == 1) {
+        if (use_box(e) && e->spread_mode == 1) {
             TRY_CUDA(spme::launch_spread_box<T>(e->d_toff, e->d_rec_idx, e->d_rec_start,
                                                 (const T *)e->d_rec_w, F, C, e->g, (T *)e->d_box,
                                                 e->box_slots, e->boxtab, (T *)e->d_mesh, s));

@@ -260,7 +260,9 @@ cudaError_t launch_spread_box(const int *tile_off, const int *rec_idx, const uin
     switch (g.p) {
         case 4: return launch_box_t<T, 4>(tile_off, rec_idx, rec_start, rec_w, F, C, g, boxes, nslot, bt, mesh, s);
         case 6: return launch_box_t<T, 6>(tile_off, rec_idx, rec_start, rec_w, F, C, g, boxes, nslot, bt, mesh, s);
-        case 8: return launch_box_t<T, 8>(tile_off, rec_idx, rec_start, rec_w, F, C, g, boxes, nslot, bt, mesh, s);
+        case 8:
+            if constexpr (sizeof(T) == 4) return cudaErrorInvalidValue;  // (never chosen)
+            else return launch_box_t<T, 8>(tile_off, rec_idx, rec_start, rec_w, F, C, g, boxes, nslot, bt, mesh, s);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -1,10 +1,13 @@
 """The spread that an engine takes: the default (mode 1) can be had back after mode 0,
 on meshes too small for the column gather too, and a tile whose boxes do not fit takes
-the column gather."""
+the column gather; boxes above the line of particles per mesh point, against the other
+kernels and the oracle (tolerances as the spread kernels' tests have them), and none below."""
 import numpy as np
 import pytest
 
+import oracle
 import spme_gb300
+from conftest import relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +68,69 @@ def test_tile_without_boxes(gpu_lib):
     assert np.array_equal(out["default"], out["again"])
     for name in ("small", "tiles"):
         assert np.linalg.norm(out[name] - out["default"]) < 1e-13 * np.linalg.norm(out["default"])
+
+
+# Sizes at which boxes are taken (particles per mesh point above the line): tile edges of
+# p - 1 and below on no, one (each) and several axes, tiles that do not divide K, a mesh
+# smaller than a tile and its halo, nearly empty tiles.
+@pytest.mark.parametrize("prec,K,p,tile,R,n", [
+    ("fp64", 32, 6, None, 1, 800),
+    ("fp64", 32, 4, None, 2, 2000),
+    ("fp64", 40, 8, None, 3, 1200),
+    ("fp64", 32, 6, (4, 8, 8), 1, 800),
+    ("fp64", 32, 6, (8, 4, 8), 1, 800),
+    ("fp64", 32, 6, (8, 8, 4), 2, 800),
+    ("fp64", 32, 6, (4, 4, 4), 1, 1500),
+    ("fp64", 33, 8, (4, 4, 4), 1, 800),
+    ("fp64", 36, 8, (16, 8, 4), 2, 2500),
+    ("fp64", 30, 6, (7, 5, 4), 1, 1200),
+    ("fp64", 25, 8, (12, 12, 8), 1, 400),
+    ("fp64", 48, 8, None, 1, 40),
+    ("fp32", 96, 6, None, 1, 26_000),
+    ("fp32", 96, 6, (16, 8, 4), 1, 31_000),
+    ("fp32", 96, 6, (4, 4, 4), 1, 41_000),
+    ("fp32", 100, 4, (8, 4, 4), 2, 45_000),
+])
+def test_boxes(gpu_lib, prec, K, p, tile, R, n):
+    L, xi = 40.0, 0.4
+    dt, tol_k, tol_o = (np.float64, 1e-13, 1e-12) if prec == "fp64" else (np.float32, 2e-6, 1e-5)
+    rng = np.random.default_rng(K * p + R)
+    pos = rng.uniform(0, L, (n, 3))
+    pos[: n // 4] = 0.06 * pos[: n // 4] + 7.0  # a cluster within a tile or two
+    f = rng.standard_normal((R, 3 * n)).astype(dt)
+    out = {}
+    # boxes; the tile kernel; an engine of more right-hand sides, which takes another spread
+    for name, mode, most in (("box", 1, R), ("tile", 0, R), ("other", 1, 4)):
+        with spme_gb300.Engine(n, L, xi, K, p, precision=prec, max_nrhs=most, tile=tile,
+                               terms=spme_gb300.TERM_RECIP) as eng:
+            eng.set_spread_mode(mode)
+            eng.set_positions(pos)
+            out[name] = eng.apply(f)
+    assert not np.array_equal(out["box"], out["tile"])
+    assert not np.array_equal(out["box"], out["other"])
+    assert relerr(out["box"], out["tile"]) < tol_k
+    assert relerr(out["box"], out["other"]) < tol_k
+    assert relerr(out["box"], oracle.recip(pos, L, xi, K, p, f.astype(np.float64))) < tol_o
+
+
+# Below the line: the column gather (FP64) or the tile kernel (FP32), as an engine of more
+# right-hand sides takes them.
+@pytest.mark.parametrize("prec,K,p,tile,R,n", [
+    ("fp64", 48, 6, None, 1, 50),
+    ("fp64", 48, 6, None, 2, 700),
+    ("fp64", 32, 6, (4, 4, 4), 1, 800),
+    ("fp64", 50, 6, None, 1, 2500),
+    ("fp32", 96, 6, None, 1, 3000),
+    ("fp32", 100, 6, None, 1, 60_000),
+])
+def test_no_boxes(gpu_lib, prec, K, p, tile, R, n):
+    rng = np.random.default_rng(K * p + R)
+    pos = rng.uniform(0, 40.0, (n, 3))
+    f = rng.standard_normal((R, 3 * n)).astype(np.float64 if prec == "fp64" else np.float32)
+    out = []
+    for most in (R, 4 if prec == "fp64" else 2):
+        with spme_gb300.Engine(n, 40.0, 0.4, K, p, precision=prec, max_nrhs=most, tile=tile,
+                               terms=spme_gb300.TERM_RECIP) as eng:
+            eng.set_positions(pos)
+            out.append(eng.apply(f))
+    assert np.array_equal(*out)
