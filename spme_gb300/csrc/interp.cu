@@ -2,9 +2,9 @@
 // old-version/spme_kernel.c:8-70: v_i = sum_j P_ij grid[c][ind_ij]; FP64 in
 // interp_fp64.cu).
 //
-// One CTA per mesh tile.  For CG components at a time it stages the tile
+// One CTA per mesh tile.  For 4 components at a time it stages the tile
 // plus its (p-1) upper halo in shared memory as a dense box
-// [CG][HZB][HYB][HX] (HX = 24 wide: every lane's x offset fits; at 16x8x4
+// [4][HZB][HYB][HX] (HX = 24 wide: every lane's x offset fits; at 16x8x4
 // tiles the component-plane stride is 24 (mod 32) words, so the gather below
 // is bank-conflict free):
 //   * one TMA (cp.async.bulk.tensor) load per chunk, completing on an mbarrier
@@ -12,7 +12,7 @@
 //     periodic boundary the part past K arrives as zeros and is patched with
 //     16-byte asynchronous copies (all rows with such copies when TMA is unavailable).
 // Each warp then interpolates the tile's own particles from shared memory:
-// FP32 at p = 4, 6 two particles per warp with lanes = (x column pair,
+// at p = 4, 6 two particles per warp with lanes = (x column pair,
 // component) and two-lane FMAs (interp_pairs); otherwise one particle per warp
 // with lanes = (x offset 0..7, component 0..3).  The x offsets are summed with
 // shuffles.  Every particle is handled by exactly one CTA; a tile's halo is
@@ -36,8 +36,7 @@ constexpr int kThreads = 256;
 constexpr int kHX = kInterpMaxRow;
 __host__ __device__ constexpr bool narrow_row(bool use_tma, int tx) { return !use_tma && tx <= 8; }
 
-template <typename T> struct Vec16;
-template <> struct Vec16<float> { using type = float4; static constexpr int n = 4; };
+constexpr int kCG = 4;  // components of a box
 
 // A half-warp's copy of one particle record for interp_pairs: lane j of the
 // half holds weights j and 16 + j (the record's 3p weights: x, y, z), plus
@@ -58,7 +57,7 @@ __device__ __forceinline__ HalfRec load_pair_rec(const InterpArgs<float> &A, int
     return r;
 }
 
-// FP32, 4-component boxes, p = 4 or 6: two particles per warp, one per
+// p = 4 or 6: two particles per warp, one per
 // half-warp, lanes of a half = (x pair 0..3, component 0..3).  A lane's x pair
 // starts at an even box column (the particle's first column, or the one before
 // it when that is odd), is read with one 8-byte load and meets its two x
@@ -128,27 +127,25 @@ __device__ __forceinline__ void interp_pairs(const float *box, int PS, int HYB,
 
 // One tile's work (the body of the single-system kernel and of the batched
 // one); tmap is read only when use_tma is set.
-template <typename T, int P, int CG, int HX>
-__device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const InterpArgs<T> &A,
+template <int P, int HX>
+__device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const InterpArgs<float> &A,
                                             int tile) {
-    using V = typename Vec16<T>::type;
-    constexpr int VW = Vec16<T>::n;
+    constexpr int VW = 4;        // values per 16-byte vector
     constexpr int NV = HX / VW;  // vectors per staged row
-    constexpr int NG = CG / 4;    // groups of 4 components per chunk
     const int use_tma = A.use_tma;
     const int *__restrict__ tile_off = A.tile_off;
     const int *__restrict__ rec_idx = A.rec_idx;
     const uint32_t *__restrict__ rec_start = A.rec_start;
-    const T *__restrict__ rec_w = A.rec_w;
-    const T *__restrict__ mesh = A.mesh;
-    T *__restrict__ W = A.W;
+    const float *__restrict__ rec_w = A.rec_w;
+    const float *__restrict__ mesh = A.mesh;
+    float *__restrict__ W = A.W;
     int *__restrict__ err = A.err;
     const MeshGeom &g = A.g;
     const int C = A.C, cb = A.cb, ce = A.ce, accumulate = A.accumulate, WS = A.ws;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
     // TMA destinations must be 128-byte aligned (128 spare bytes are allocated)
-    T *box = reinterpret_cast<T *>(smem_raw + ((128 - (smem_addr(smem_raw) & 127)) & 127));
+    float *box = reinterpret_cast<float *>(smem_raw + ((128 - (smem_addr(smem_raw) & 127)) & 127));
 
     const int pbeg = tile_off[tile], pend = tile_off[tile + 1];
     if (pbeg == pend) return;
@@ -166,7 +163,7 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
     // TMA too (the part past K arrives as zeros) and the wrapped part patched
     // with asynchronous copies.
     const bool wraps = ox + hx > K || oy + hy > K || oz + hz > K;
-    const bool tma = use_tma && ((size_t)ox * sizeof(T)) % 16 == 0;
+    const bool tma = use_tma && ((size_t)ox * sizeof(float)) % 16 == 0;
     const size_t K2 = (size_t)K * K, K3 = K2 * K;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int xs = lane >> 2, cl = lane & 3;
@@ -196,8 +193,8 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
             gy -= gy >= K ? K : 0;
             gz -= gz >= K ? K : 0;
             const int x0 = ox + v * VW;
-            const T *src = mesh + (size_t)(c0 + c) * K3 + (size_t)gz * K2 + (size_t)gy * K;
-            T *dst = box + (size_t)c * PS + (z * HYB + y) * HX + v * VW;
+            const float *src = mesh + (size_t)(c0 + c) * K3 + (size_t)gz * K2 + (size_t)gy * K;
+            float *dst = box + (size_t)c * PS + (z * HYB + y) * HX + v * VW;
             if (vec) {
                 cp_async16(dst, src + wrap_index(x0, K));
             } else if (two) {
@@ -212,15 +209,14 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
         __syncthreads();
     };
 
-    // FP32 p = 4, 6: two particles per warp, x columns in pairs (interp_pairs)
-    constexpr bool kPairs = sizeof(T) == 4 && CG == 4 && (P == 4 || P == 6);
+    // p = 4, 6: two particles per warp, x columns in pairs (interp_pairs)
+    constexpr bool kPairs = P == 4 || P == 6;
     // after a TMA box of a tile whose halo wraps: the elements past the periodic
     // boundary (zeros in the box) by 16-byte copies, one thread per box row: a
     // row past K in y or z is copied whole, other rows only from column K - ox on
     const int xw0 = ox + hx > K ? (K - ox) / VW : NV;  // first vector holding a wrapped column
     const int xw1 = (hx - 1) / VW;                     // last vector of the halo
     auto patch_wrapped = [&](int c0, int nc) {
-        const bool vec = (K % VW) == 0 && (ox % VW) == 0;
         DivMod dhy, dhz;
         dhy.init(hy);
         dhz.init(hz);
@@ -234,8 +230,8 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
             if (!row_wraps && xw0 == NV) continue;
             gy -= gy >= K ? K : 0;
             gz -= gz >= K ? K : 0;
-            const T *src = mesh + (size_t)(c0 + c) * K3 + (size_t)gz * K2 + (size_t)gy * K;
-            T *dst = box + (size_t)c * PS + (z * HYB + y) * HX;
+            const float *src = mesh + (size_t)(c0 + c) * K3 + (size_t)gz * K2 + (size_t)gy * K;
+            float *dst = box + (size_t)c * PS + (z * HYB + y) * HX;
             const int v1 = row_wraps ? NV - 1 : xw1;
             for (int v = row_wraps ? 0 : xw0; v <= v1; v++) {
                 const int x0 = ox + v * VW;
@@ -249,28 +245,27 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
     // the warp's first particle's record, the same for every component chunk:
     // loaded once, before the first box is waited for
     constexpr int kWarps = kThreads / 32;
-    T wreg_0 = T(0);
+    float wreg_0 = 0.f;
     uint32_t st_0 = 0;
     int idx_0 = 0;
     HalfRec hrec_0{0.f, 0.f, 0u};
     if constexpr (kPairs) {
         if (pbeg + 2 * warp < pend)
-            hrec_0 = load_pair_rec<P>(reinterpret_cast<const InterpArgs<float> &>(A),
-                                      min(pbeg + 2 * warp + (lane >> 4), pend - 1));
+            hrec_0 = load_pair_rec<P>(A, min(pbeg + 2 * warp + (lane >> 4), pend - 1));
     } else if (pbeg + warp < pend) {
         const int s = pbeg + warp;
-        wreg_0 = lane < 3 * P ? __ldg(rec_w + (size_t)s * WS + lane) : T(0);
+        wreg_0 = lane < 3 * P ? __ldg(rec_w + (size_t)s * WS + lane) : 0.f;
         st_0 = __ldg(rec_start + s);
         idx_0 = __ldg(rec_idx + s);
     }
 
     int chunk = 0;
-    for (int c0 = cb; c0 < ce; c0 += CG, chunk++) {
-        const int nc = min(CG, ce - c0);
+    for (int c0 = cb; c0 < ce; c0 += kCG, chunk++) {
+        const int nc = min(kCG, ce - c0);
         if (tma) {
             if (threadIdx.x == 0) {
                 fence_proxy_async();  // order earlier generic reads of the box before the TMA write
-                mbar_expect_tx(&bar, (uint32_t)((size_t)CG * PS * sizeof(T)));
+                mbar_expect_tx(&bar, (uint32_t)((size_t)kCG * PS * sizeof(float)));
                 tma_load_4d(box, tmap, ox, oy, oz, c0, &bar);
             }
             const bool ok = mbar_wait(&bar, (uint32_t)(chunk & 1));
@@ -283,145 +278,110 @@ __device__ __forceinline__ void interp_body(const CUtensorMap *tmap, const Inter
             stage_rows(c0, nc);
         }
         if constexpr (kPairs) {
-            interp_pairs<P, HX>(reinterpret_cast<const float *>(box), PS, HYB,
-                            reinterpret_cast<const InterpArgs<float> &>(A), c0, nc, pbeg, pend,
-                            ox, oy, oz, hrec_0);
+            interp_pairs<P, HX>(box, PS, HYB, A, c0, nc, pbeg, pend, ox, oy, oz, hrec_0);
             __syncthreads();  // the box is rewritten by the next chunk
             continue;
         }
         // the next particle's record is loaded while this one is interpolated
-        T wreg_n = wreg_0;
+        float wreg_n = wreg_0;
         uint32_t st_n = st_0;
         int idx_n = idx_0;
         for (int s = pbeg + warp; s < pend; s += kWarps) {
-            const T wreg = wreg_n;
+            const float wreg = wreg_n;
             const uint32_t st = st_n;
             const int idx = idx_n;
             if (s + kWarps < pend) {
                 const int sn = s + kWarps;
-                wreg_n = lane < 3 * P ? __ldg(rec_w + (size_t)sn * WS + lane) : T(0);
+                wreg_n = lane < 3 * P ? __ldg(rec_w + (size_t)sn * WS + lane) : 0.f;
                 st_n = __ldg(rec_start + sn);
                 idx_n = __ldg(rec_idx + sn);
             }
             int sx, sy, sz;
             unpack_start(st, sx, sy, sz);
             const int lx = sx - ox, ly = sy - oy, lz = sz - oz;  // own tile: no wrap
-            const T wxv = __shfl_sync(0xffffffffu, wreg, xs < P ? xs : P - 1);
-            const T wx = xs < P ? wxv : T(0);
-            T wxy[P], wz[P];
+            const float wxv = __shfl_sync(0xffffffffu, wreg, xs < P ? xs : P - 1);
+            const float wx = xs < P ? wxv : 0.f;
+            float wxy[P], wz[P];
 #pragma unroll
             for (int y = 0; y < P; y++) wxy[y] = wx * __shfl_sync(0xffffffffu, wreg, P + y);
 #pragma unroll
             for (int z = 0; z < P; z++) wz[z] = __shfl_sync(0xffffffffu, wreg, 2 * P + z);
-            T acc[NG];
-#pragma unroll
-            for (int k = 0; k < NG; k++) acc[k] = T(0);
-            const T *base = box + (size_t)cl * PS + (lz * HYB + ly) * HX + lx + xs;
+            float acc = 0.f;
+            const float *base = box + (size_t)cl * PS + (lz * HYB + ly) * HX + lx + xs;
             // sum over y with w_x w_y first, then one w_z per plane
 #pragma unroll
             for (int z = 0; z < P; z++) {
-                const T *pz = base + z * HYB * HX;
-                T t[NG];
+                const float *pz = base + z * HYB * HX;
+                float t = 0.f;
 #pragma unroll
-                for (int k = 0; k < NG; k++) t[k] = T(0);
-#pragma unroll
-                for (int y = 0; y < P; y++)
-#pragma unroll
-                    for (int k = 0; k < NG; k++) t[k] += wxy[y] * pz[(size_t)k * 4 * PS + y * HX];
-#pragma unroll
-                for (int k = 0; k < NG; k++) acc[k] += wz[z] * t[k];
+                for (int y = 0; y < P; y++) t += wxy[y] * pz[y * HX];
+                acc += wz[z] * t;
             }
 #pragma unroll
-            for (int k = 0; k < NG; k++)
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-            if (xs == 0) {
-                T *out = W + (size_t)idx * C + c0;
-#pragma unroll
-                for (int k = 0; k < NG; k++) {
-                    const int c = 4 * k + cl;
-                    if (c < nc) out[c] = accumulate ? out[c] + acc[k] : acc[k];
-                }
+            for (int o = 4; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (xs == 0 && cl < nc) {
+                float *out = W + (size_t)idx * C + c0 + cl;
+                *out = accumulate ? *out + acc : acc;
             }
         }
         __syncthreads();  // the box is rewritten by the next chunk
     }
 }
 
-template <typename T, int P, int CG, int HX>
+template <int P, int HX>
 // blocks per SM that the 4-component box's shared memory allows (16x8x4 tiles)
 __global__ void __launch_bounds__(kThreads, 5)
-k_interp(const __grid_constant__ CUtensorMap tmap, InterpArgs<T> A) {
+k_interp(const __grid_constant__ CUtensorMap tmap, InterpArgs<float> A) {
     pdl_wait();
     // tiles z fastest: blocks launched together are z neighbours, whose boxes
     // share p - 1 of their tz + p - 1 planes (read from L2 by the later ones)
     const int b = blockIdx.x, ntx = A.g.ntx, nty = A.g.nty, ntz = A.g.ntz;
     const int tiz = b % ntz, rest = b / ntz;
-    interp_body<T, P, CG, HX>(&tmap, A, (tiz * nty + rest / ntx) * ntx + rest % ntx);
+    interp_body<P, HX>(&tmap, A, (tiz * nty + rest / ntx) * ntx + rest % ntx);
 }
 
 // Many systems in one persistent launch over their tiles: each system's boxes
 // by TMA through its own descriptor in the work list where its mesh rows allow
 // it, by asynchronous copies otherwise; the order p of each system selects the body
 // (the batch launches one such kernel per order).
-template <typename T, int CG>
 __global__ void __launch_bounds__(kThreads)
-k_interp_batch(const InterpSys<T> *__restrict__ sys, const int *__restrict__ prefix, int nsys,
+k_interp_batch(const InterpSys<float> *__restrict__ sys, const int *__restrict__ prefix, int nsys,
                int total) {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int k = batch_find(prefix, nsys, w);
-        const InterpArgs<T> A = sys[k].args;
+        const InterpArgs<float> A = sys[k].args;
         // the system's TMA box stays in the global work list (a descriptor in
         // global memory; never a local copy)
         const CUtensorMap *tmap = A.use_tma ? &sys[k].tmap : nullptr;
         const int tile = w - prefix[k];
         if (narrow_row(A.use_tma, A.g.tx)) {
             switch (A.g.p) {
-                case 4: interp_body<T, 4, CG, 16>(tmap, A, tile); break;
-                case 6: interp_body<T, 6, CG, 16>(tmap, A, tile); break;
-                default: interp_body<T, 8, CG, 16>(tmap, A, tile); break;
+                case 4: interp_body<4, 16>(tmap, A, tile); break;
+                case 6: interp_body<6, 16>(tmap, A, tile); break;
+                default: interp_body<8, 16>(tmap, A, tile); break;
             }
         } else {
             switch (A.g.p) {
-                case 4: interp_body<T, 4, CG, kHX>(tmap, A, tile); break;
-                case 6: interp_body<T, 6, CG, kHX>(tmap, A, tile); break;
-                default: interp_body<T, 8, CG, kHX>(tmap, A, tile); break;
+                case 4: interp_body<4, kHX>(tmap, A, tile); break;
+                case 6: interp_body<6, kHX>(tmap, A, tile); break;
+                default: interp_body<8, kHX>(tmap, A, tile); break;
             }
         }
         __syncthreads();
     }
 }
 
-template <typename T, int P, int CG>
-size_t interp_smem(const MeshGeom &g) {
-    return (size_t)CG * (g.tz + P - 1) * (g.ty + P - 1) * kHX * sizeof(T) + 128;
-}
-
-template <typename T, int P, int CG>
-cudaError_t launch_interp_t(const InterpMaps &maps, const int *tile_off, const int *rec_idx,
-                            const uint32_t *rec_start, const T *rec_w, const T *mesh, int C,
-                            int cb, int ce, const MeshGeom &g, T *W, int accumulate, int *err,
-                            cudaStream_t s) {
-    const bool use = maps.ok4, narrow = narrow_row(use, g.tx);
-    const size_t smem = interp_smem<T, P, CG>(g);
-    auto kern = narrow ? k_interp<T, P, CG, 16> : k_interp<T, P, CG, kHX>;
+template <int P>
+cudaError_t launch_p(const InterpMaps &maps, InterpArgs<float> A, cudaStream_t s) {
+    const MeshGeom &g = A.g;
+    const size_t smem = interp_smem_bytes(g, sizeof(float));
+    auto kern = narrow_row(maps.ok4, g.tx) ? k_interp<P, 16> : k_interp<P, kHX>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    const CUtensorMap &m = maps.cg4;
-    InterpArgs<T> A{tile_off, rec_idx, rec_start, rec_w, mesh, W, err, g, C, cb, ce,
-                    accumulate, use ? 1 : 0, RecordWidth<T, P>::value};
-    pdl_launch(kern, g.ntx * g.nty * g.ntz, kThreads, smem, s, m, A);
+    A.ws = RecordWidth<float, P>::value;
+    pdl_launch(kern, g.ntx * g.nty * g.ntz, kThreads, smem, s, maps.cg4, A);
     return cudaGetLastError();
-}
-
-template <typename T, int P>
-cudaError_t dispatch_cg(const InterpMaps &maps, const int *tile_off, const int *rec_idx,
-                        const uint32_t *rec_start, const T *rec_w, const T *mesh, int C,
-                        int cb, int ce, const MeshGeom &g, T *W, int accumulate, int *err,
-                        cudaStream_t s) {
-    return launch_interp_t<T, P, 4>(maps, tile_off, rec_idx, rec_start, rec_w, mesh, C, cb, ce, g,
-                                    W, accumulate, err, s);
 }
 
 bool encode_box(CUtensorMap *m, const void *mesh, int K, int C, const MeshGeom &g, size_t elem,
@@ -466,27 +426,29 @@ bool make_interp_maps(InterpMaps *maps, const void *mesh, int C, const MeshGeom 
     return maps->ok4;
 }
 
-template <typename T>
-cudaError_t launch_interp(const InterpMaps &maps, const int *tile_off, int n, const int *rec_idx,
-                          const uint32_t *rec_start, const T *rec_w, const T *mesh, int C,
-                          int cb, int ce, const MeshGeom &g, T *W, int accumulate, int *err,
-                          cudaStream_t s) {
+template <>
+cudaError_t launch_interp<float>(const InterpMaps &maps, const int *tile_off, int n, const int *rec_idx,
+                                 const uint32_t *rec_start, const float *rec_w, const float *mesh,
+                                 int C, int cb, int ce, const MeshGeom &g, float *W, int accumulate,
+                                 int *err, cudaStream_t s) {
     if (n <= 0 || cb >= ce) return cudaSuccess;
     if (cb < 0 || ce > C) return cudaErrorInvalidValue;
     if (g.tx + 7 > kHX || g.tx + g.p - 1 > kHX) return cudaErrorInvalidValue;
+    const InterpArgs<float> A{tile_off, rec_idx, rec_start, rec_w, mesh, W, err, g, C, cb, ce,
+                              accumulate, maps.ok4 ? 1 : 0, 0};
     switch (g.p) {
-        case 4: return dispatch_cg<T, 4>(maps, tile_off, rec_idx, rec_start, rec_w, mesh, C, cb, ce, g, W, accumulate, err, s);
-        case 6: return dispatch_cg<T, 6>(maps, tile_off, rec_idx, rec_start, rec_w, mesh, C, cb, ce, g, W, accumulate, err, s);
-        case 8: return dispatch_cg<T, 8>(maps, tile_off, rec_idx, rec_start, rec_w, mesh, C, cb, ce, g, W, accumulate, err, s);
+        case 4: return launch_p<4>(maps, A, s);
+        case 6: return launch_p<6>(maps, A, s);
+        case 8: return launch_p<8>(maps, A, s);
         default: return cudaErrorInvalidValue;
     }
 }
 
-template <typename T>
-cudaError_t launch_interp_batch(const InterpSys<T> *sys, const int *prefix, int nsys, int total,
-                                size_t smem, cudaStream_t s, size_t smem_limit) {
+template <>
+cudaError_t launch_interp_batch<float>(const InterpSys<float> *sys, const int *prefix, int nsys,
+                                       int total, size_t smem, cudaStream_t s, size_t smem_limit) {
     if (total <= 0) return cudaSuccess;
-    auto kern = k_interp_batch<T, 4>;
+    auto kern = k_interp_batch;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)std::max(smem, smem_limit));
     if (e != cudaSuccess) return e;
@@ -498,12 +460,5 @@ cudaError_t launch_interp_batch(const InterpSys<T> *sys, const int *prefix, int 
     kern<<<grid, kThreads, smem, s>>>(sys, prefix, nsys, total);
     return cudaGetLastError();
 }
-
-template cudaError_t launch_interp_batch<float>(const InterpSys<float> *, const int *, int, int,
-                                                size_t, cudaStream_t, size_t);
-template cudaError_t launch_interp<float>(const InterpMaps &, const int *, int, const int *,
-                                          const uint32_t *, const float *, const float *, int,
-                                          int, int, const MeshGeom &, float *, int, int *,
-                                          cudaStream_t);
 
 }  // namespace spme

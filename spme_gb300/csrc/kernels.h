@@ -203,6 +203,13 @@ cudaError_t launch_interp(const InterpMaps &maps, const int *tile_off, int n, co
                           int cb, int ce, const MeshGeom &g, T *W, int accumulate, int *err,
                           cudaStream_t s);
 template <>
+cudaError_t launch_interp<float>(const InterpMaps &, const int *, int, const int *,
+                                 const uint32_t *, const float *, const float *, int, int, int,
+                                 const MeshGeom &, float *, int, int *, cudaStream_t);
+template <>
+cudaError_t launch_interp_batch<float>(const InterpSys<float> *, const int *, int, int, size_t,
+                                       cudaStream_t, size_t);
+template <>
 cudaError_t launch_interp<double>(const InterpMaps &, const int *, int, const int *,
                                   const uint32_t *, const double *, const double *, int, int, int,
                                   const MeshGeom &, double *, int, int *, cudaStream_t);
@@ -379,9 +386,6 @@ cudaError_t launch_realspace_batch<double>(const RealArgs<double> *, const int *
 // W = self_c * F (the self term alone, when no real-space sum is requested)
 template <typename T>
 void launch_self(const T *F, int n, int R, double self_c, T *W, cudaStream_t s);
-// Fs[s][c] = F[idx[s]][c] for s < n (C components per row).
-template <typename T>
-void launch_gather_rows(const T *F, const int *idx, int n, int C, T *Fs, cudaStream_t s);
 template <typename T>
 void launch_pack(const T *f, long ld, int n, int R, T *F, cudaStream_t s);
 // u[r*ld + 3i + d] = beta*u + alpha*W[i][3r+d]   (u not read when beta == 0)

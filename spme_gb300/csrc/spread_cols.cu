@@ -412,20 +412,20 @@ k_spread_cols(SpreadColsArgs<T> A) {
 // Many FP64 systems in one persistent launch: work item w (a block of one system)
 // -> system k with prefix[k] <= w < prefix[k + 1]; the order p of each system
 // selects the body.
-template <typename T, int CPL, int TZ, int NW>
-__global__ void __launch_bounds__(NW * 32, (sizeof(T) == 4 ? 3 : 1))
-k_spread_cols_batch(const SpreadColsSys<T> *__restrict__ sys, const int *__restrict__ prefix,
+template <int CPL, int TZ, int NW>
+__global__ void __launch_bounds__(NW * 32)
+k_spread_cols_batch(const SpreadColsSys<double> *__restrict__ sys, const int *__restrict__ prefix,
                     int nsys, int total) {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int k = batch_find(prefix, nsys, w);
-        const SpreadColsSys<T> S = sys[k];
+        const SpreadColsSys<double> S = sys[k];
         const int local = w - prefix[k];
         const int bx = local % S.gx, rest = local / S.gx;
         const int by = rest % S.gy, bz = rest / S.gy;
         switch (S.p) {
-            case 4: spread_cols_body<T, 4, CPL, TZ, NW>(S.args, bx, by, bz); break;
-            case 6: spread_cols_body<T, 6, CPL, TZ, NW>(S.args, bx, by, bz); break;
-            default: spread_cols_body<T, 8, CPL, TZ, NW>(S.args, bx, by, bz); break;
+            case 4: spread_cols_body<double, 4, CPL, TZ, NW>(S.args, bx, by, bz); break;
+            case 6: spread_cols_body<double, 6, CPL, TZ, NW>(S.args, bx, by, bz); break;
+            default: spread_cols_body<double, 8, CPL, TZ, NW>(S.args, bx, by, bz); break;
         }
         __syncthreads();  // shared memory is reused by the next work item
     }
@@ -504,16 +504,13 @@ cudaError_t launch_cols(const int *soff, const uint32_t *rec_start, const T *rec
     return cudaGetLastError();
 }
 
-template <typename T, int CPL>
-cudaError_t launch_cols_batch(const SpreadColsSys<T> *sys, const int *prefix, int nsys,
+template <int CPL>
+cudaError_t launch_cols_batch(const SpreadColsSys<double> *sys, const int *prefix, int nsys,
                               int total, cudaStream_t s) {
-    constexpr int NW = 8;
-    constexpr int TZ = sizeof(T) == 4 ? 16 : 8;
-    constexpr int XT = 2 * NW, CC = 16 * CPL;
-    const size_t smem = (((size_t)CC * (TZ * XT + (sizeof(T) == 4 ? 2 : 1)) * sizeof(T) + 15) &
-                         ~(size_t)15) +
-                        NW * sizeof(WarpScratch<T, 8>);  // the largest order's scratch
-    auto kern = k_spread_cols_batch<T, CPL, TZ, NW>;
+    constexpr int NW = 8, TZ = 8, XT = 2 * NW, CC = 16 * CPL;
+    const size_t smem = (((size_t)CC * (TZ * XT + 1) * sizeof(double) + 15) & ~(size_t)15) +
+                        NW * sizeof(WarpScratch<double, 8>);  // the largest order's scratch
+    auto kern = k_spread_cols_batch<CPL, TZ, NW>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0, per_sm = 0;
@@ -628,9 +625,9 @@ cudaError_t launch_spread_cols_batch<double>(const SpreadColsSys<double> *sys, c
                                              int nsys, int total, int C, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     switch (cols_cpl(C)) {
-        case 1: return launch_cols_batch<double, 1>(sys, prefix, nsys, total, s);
-        case 2: return launch_cols_batch<double, 2>(sys, prefix, nsys, total, s);
-        default: return launch_cols_batch<double, 3>(sys, prefix, nsys, total, s);
+        case 1: return launch_cols_batch<1>(sys, prefix, nsys, total, s);
+        case 2: return launch_cols_batch<2>(sys, prefix, nsys, total, s);
+        default: return launch_cols_batch<3>(sys, prefix, nsys, total, s);
     }
 }
 
