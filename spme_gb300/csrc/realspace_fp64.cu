@@ -213,38 +213,32 @@ long long bits_of(double v) {
 // nodes.
 void fit_segment(double s0, double h, double xi, double a, bool near, double *out) {
     constexpr int n = kPairDeg + 1;
-    static double node[n], cs[n][n];
+    static double node[n], cs[n][n], cheb[n][n];  // cheb[k][i]: the power i in T_k
     static const bool once = [] {
         for (int j = 0; j < n; j++) {
             node[j] = std::cos(M_PI * (j + 0.5) / n);
             for (int k = 0; k < n; k++) cs[k][j] = std::cos(M_PI * k * (j + 0.5) / n);
         }
+        cheb[0][0] = cheb[1][1] = 1.0;
+        for (int k = 2; k < n; k++)
+            for (int i = 0; i < n; i++) cheb[k][i] = (i ? 2.0 * cheb[k - 1][i - 1] : 0.0) - cheb[k - 2][i];
         return true;
     }();
     (void)once;
-    double f[2][n], c[2][n];
+    double f[2][n];
     for (int j = 0; j < n; j++) {
         const double s = s0 + 0.5 * h * (node[j] + 1.0);
         real_FG(std::sqrt(s), xi, a, near, f[0][j], f[1][j]);
         f[1][j] /= s;
     }
     for (int w = 0; w < 2; w++) {
+        // Chebyshev coefficients, then powers of t, then of the offset v = t h / 2
+        double o[n] = {};
         for (int k = 0; k < n; k++) {
             double q = 0.0;
             for (int j = 0; j < n; j++) q += f[w][j] * cs[k][j];
-            c[w][k] = (k ? 2.0 : 1.0) * q / n;
-        }
-        // Chebyshev to powers of t, then of the offset v = t h / 2
-        double t0[n] = {1.0}, t1[n] = {0.0, 1.0}, o[n];
-        for (int i = 0; i < n; i++) o[i] = c[w][0] * t0[i] + c[w][1] * t1[i];
-        for (int k = 2; k < n; k++) {
-            double t2[n];
-            for (int i = 0; i < n; i++) t2[i] = (i ? 2.0 * t1[i - 1] : 0.0) - t0[i];
-            for (int i = 0; i < n; i++) {
-                o[i] += c[w][k] * t2[i];
-                t0[i] = t1[i];
-                t1[i] = t2[i];
-            }
+            const double c = (k ? 2.0 : 1.0) * q / n;
+            for (int i = k & 1; i <= k; i += 2) o[i] += c * cheb[k][i];
         }
         double sc = 1.0;
         for (int i = 0; i < n; i++) {
@@ -262,7 +256,9 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
     const double lo = 0.25 * a * a, mid = 4.0 * a * a, hi = rc * rc;
     if (hi <= lo) return false;
     // (2^m segments per octave of s: twice those that pass, so that the fit, 2^-7 of the
-    // bound then, stays below the rounding of the values it goes through)
+    // bound then, stays below the rounding of the values it goes through.  Every fourth
+    // segment, and the ends of either form, is tried: the error varies slowly along s, and
+    // all of them took an engine's creation from 1.26 to 1.70 ms at N = 300)
     bool passed = false;
     for (int m = 6; m <= (passed ? 11 : 10); m++) {
         const int shift = 20 - m;
@@ -282,6 +278,7 @@ bool build_pair_table(double xi, double a, double rc, std::vector<double> *coef,
         bool ok = true;
         for (int q = 0; q < n && ok; q++) {
             const bool near = q <= gm - base;
+            if (!passed && q % 4 && q != n - 1 && q != gm - base && q != gm - base + 1) continue;
             const int g = base + q - (near ? 0 : 1);
             const double s0 = start_of(g), h = start_of(g + 1) - s0;
             double *c = coef->data() + (size_t)q * (kPairDeg + 1) * 2;
