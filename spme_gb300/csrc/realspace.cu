@@ -20,13 +20,12 @@
 //     component (F2[j][d][r]), so a right-hand side pair is one 8-byte load and a
 //     row's load touches one line instead of the whole interleaved row.
 // More right-hand sides: sums of a window's pairs (64, split over the slots) are plain FP32;
-// longer runs, the sum over the slots and the self term carry TwoSum.  That and the term's
-// one rounding into the sum cost 5 % of the stage (R = 16 1.525 -> 1.605 ms at N = 1e6).
-// Measured (ms): N = 1e6, R = 16 1.65 -> 1.61; N = 2e5, R = 16 0.442 -> 0.426; N = 1e5,
-// R = 1 0.161 -> 0.112; N = 1e6, R = 1 1.32 -> 0.92 (with compensated sums per lane; 0.83
-// without), R = 4 1.35 -> 1.31.  The partners' rows come
-// mostly from L2 (16 % L1 hits), whose latency bounds it now; more warps per SM at
-// fewer registers spill (1.57 ms at 12 blocks), a table of the pair functions in
+// longer runs, the sum over the slots and the self term carry TwoSum; fewer: ShareSum
+// (realspace_pairs.cuh).  Plain sums were 5 % (R = 16) to 11 % (R = 1) faster and 1 to 2 % less exact.
+// Measured (ms): N = 1e6, R = 16 1.65 -> 1.62, R = 4 1.35 -> 1.32, R = 1 1.32 -> 0.92; N = 2e5, R = 16
+// 0.442 -> 0.428; N = 1e5, R = 1 0.161 -> 0.112; 64 uneven systems, R = 4 1.53 -> 1.50.  The
+// partners' rows come mostly from L2 (12 % L1 hits), whose latency bounds it now; more warps
+// per SM at fewer registers spill (1.57 ms at 12 blocks where 10 took 1.52), a table of the pair functions in
 // shared-memory-free FP32 cost more in scattered loads than it saved (1.64 ms).
 #include <algorithm>
 #include <cmath>

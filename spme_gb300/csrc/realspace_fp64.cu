@@ -16,7 +16,7 @@
 //   * the listed pairs are split evenly over the lanes (realspace_pairs.cuh), which
 //     accumulate in registers: no 5-step FP64 butterfly per particle.
 // N = 1e6, L = 480, rc = 10 (38 pairs per particle), one right-hand side:
-// 15.19 -> 3.37 ms; N = 1e5, L = 220: 1.645 -> 0.364 ms (FP64 pipe floor 2.0 ms: 36
+// 15.19 -> 3.28 ms; N = 1e5, L = 220: 1.645 -> 0.357 ms (FP64 pipe floor 2.0 ms: 36
 // FP64 warp instructions per particle at 16 cycles each).
 #include <algorithm>
 #include <cmath>
