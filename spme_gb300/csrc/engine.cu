@@ -1330,11 +1330,19 @@ int spme_set_tile(spme_t *e, int tx, int ty, int tz) {
     g.ty = ty;
     g.tz = tz;
     if (!spme::interp_tile_ok(g, e->elem)) return e->last_error = SPME_ERR_UNSUPPORTED;
+    DeviceGuard dg(e->device);
     e->tile[0] = tx;
     e->tile[1] = ty;
     e->tile[2] = tz;
     e->have_pos = false;
     drop_graphs(e);
+    if (e->prm.terms & SPME_TERM_RECIP) {
+        // buffers of this tile now (the next position build may be captured by the caller);
+        // without memory that build tries again and reports it
+        set_geometry(e);
+        choose_spread(e);
+        (void)alloc_tiles(e);
+    }
     return e->last_error = SPME_OK;
 }
 
@@ -1364,8 +1372,13 @@ int spme_set_fft_mode(spme_t *e, int mode) {
     if (mode == 2 && !e->d_f2tab) return e->last_error = SPME_ERR_UNSUPPORTED;
     if (e->stream) cudaStreamSynchronize(e->stream);
     drop_graphs(e);
-    destroy_plans(e);  // made again for the mode on the next pass
+    if (mode == e->fft_mode) return e->last_error = SPME_OK;
+    destroy_plans(e);
     e->fft_mode = mode;
+    // the whole mesh's plans now, as at creation (a pass may be captured by the caller);
+    // without memory the next pass tries again and reports it
+    PlanPair *pp;
+    (void)get_plans(e, e->Cmax, &pp);
     return e->last_error = SPME_OK;
 }
 
