@@ -1006,14 +1006,10 @@ int apply_body(_spme_batch_t *b, double alpha, const T *f, double beta, T *u) {
     mark(b, 6);
     BTRY(run_ffts<T>(b, true, fconc));
     mark(b, 7);
-    // the kernel's shared-memory limit covers every group (a captured graph replays
-    // all the launches against the limit last set)
-    size_t smem_max = 0;
-    for (const auto &grp : b->igroups) smem_max = std::max(smem_max, grp.smem);
     for (const auto &grp : b->igroups)
         BTRY_CUDA(launch_interp_batch<T>((const InterpSys<T> *)b->d_interp_sys + grp.first,
                                          b->d_pre_interp + grp.pre_off, grp.count, grp.total,
-                                         grp.smem, s, smem_max));
+                                         grp.smem, s));
     mark(b, 8);
     if (conc) BTRY_CUDA(cudaStreamWaitEvent(s, b->ev_rs_join, 0));
     k_batch_unpack<T><<<grid_cap(n, 256, 8), 256, 0, s>>>(

@@ -376,8 +376,7 @@ cudaError_t launch_p(const InterpMaps &maps, InterpArgs<float> A, cudaStream_t s
     const MeshGeom &g = A.g;
     const size_t smem = interp_smem_bytes(g, sizeof(float));
     auto kern = narrow_row(maps.ok4, g.tx) ? k_interp<P, 16> : k_interp<P, kHX>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     A.ws = RecordWidth<float, P>::value;
     pdl_launch(kern, g.ntx * g.nty * g.ntz, kThreads, smem, s, maps.cg4, A);
@@ -446,11 +445,10 @@ cudaError_t launch_interp<float>(const InterpMaps &maps, const int *tile_off, in
 
 template <>
 cudaError_t launch_interp_batch<float>(const InterpSys<float> *sys, const int *prefix, int nsys,
-                                       int total, size_t smem, cudaStream_t s, size_t smem_limit) {
+                                       int total, size_t smem, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     auto kern = k_interp_batch;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)std::max(smem, smem_limit));
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);

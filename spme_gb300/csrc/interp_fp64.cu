@@ -167,8 +167,7 @@ template <int P>
 cudaError_t launch_p(const CUtensorMap &map, const InterpArgs<double> &A, cudaStream_t s) {
     const size_t smem = interp_smem_bytes(A.g, sizeof(double));
     auto kern = k_interp64<P>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     pdl_launch(kern, dim3(A.g.ntx * A.g.nty * A.g.ntz, A.ce - A.cb), kThreads, smem, s, map, A);
     return cudaGetLastError();
@@ -197,12 +196,10 @@ cudaError_t launch_interp<double>(const InterpMaps &maps, const int *tile_off, i
 
 template <>
 cudaError_t launch_interp_batch<double>(const InterpSys<double> *sys, const int *prefix, int nsys,
-                                        int total, size_t smem, cudaStream_t s,
-                                        size_t smem_limit) {
+                                        int total, size_t smem, cudaStream_t s) {
     if (total <= 0) return cudaSuccess;
     auto kern = k_interp64_batch;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)std::max(smem, smem_limit));
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);

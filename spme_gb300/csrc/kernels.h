@@ -12,6 +12,17 @@
 
 namespace spme {
 
+// Lets a kernel take smem bytes of dynamic shared memory.  The limit belongs to the kernel,
+// not to a launch: a smaller one set for another engine's tile would hold for launches of
+// other threads and for graphs captured before, so kernels whose need varies always get
+// the same one (above every tile the engines accept).
+constexpr size_t kSmemLimit = 220 * 1024;
+template <typename F>
+cudaError_t allow_smem(F kern, size_t smem) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(smem > kSmemLimit ? smem : kSmemLimit));
+}
+
 // ---- P-build and counting sorts (pbuild.cu) -------------------------------
 // Sort keys with a slot within each key (atomic counts): the mesh tile of the
 // stencil start (key1), the stencil-start cell ((sy K + sx) K + sz, K^3 keys;
@@ -190,11 +201,10 @@ struct InterpSys {
 // not a multiple of 16 bytes, an unaligned mesh, or no driver entry point).
 bool make_interp_box(CUtensorMap *map, const void *mesh, int C, const MeshGeom &g, size_t elem);
 // All systems in one persistent launch over their tiles (prefix as for the
-// spread; smem = the largest interp_smem_bytes of the systems; the kernel's
-// dynamic shared-memory limit is set to max(smem, smem_limit)).
+// spread; smem = the largest interp_smem_bytes of the systems).
 template <typename T>
 cudaError_t launch_interp_batch(const InterpSys<T> *sys, const int *prefix, int nsys, int total,
-                                size_t smem, cudaStream_t s, size_t smem_limit = 0);
+                                size_t smem, cudaStream_t s);
 // Components [cb, ce) of the C-component mesh (cb a multiple of 12, or 0) into
 // W[n][C]; err: device flag set to 1 if a TMA wait timed out.
 template <typename T>
@@ -208,14 +218,14 @@ cudaError_t launch_interp<float>(const InterpMaps &, const int *, int, const int
                                  const MeshGeom &, float *, int, int *, cudaStream_t);
 template <>
 cudaError_t launch_interp_batch<float>(const InterpSys<float> *, const int *, int, int, size_t,
-                                       cudaStream_t, size_t);
+                                       cudaStream_t);
 template <>
 cudaError_t launch_interp<double>(const InterpMaps &, const int *, int, const int *,
                                   const uint32_t *, const double *, const double *, int, int, int,
                                   const MeshGeom &, double *, int, int *, cudaStream_t);
 template <>
 cudaError_t launch_interp_batch<double>(const InterpSys<double> *, const int *, int, int, size_t,
-                                        cudaStream_t, size_t);
+                                        cudaStream_t);
 
 // ---- host tables (engine.cu) ----------------------------------------------
 // |b(m)|^2 = 1 / |sum_{j<p-1} M_p(j+1) e^{i j 2 pi m'/K}|^2 (old-version/spme.c:109-126).

@@ -219,8 +219,7 @@ cudaError_t launch_spread_t(const int *tile_off, const int *rec_idx, const uint3
     size_t smem = ((size_t)kChunk * CPT * ng + (size_t)WL * (kChunk + 1)) * sizeof(T) +
                   (size_t)kChunk * sizeof(int);
     auto kern = k_spread<T, P, CPT, TZ>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(g.ntx * g.nty * g.ntz, (C + CPT * ng - 1) / (CPT * ng));
     kern<<<grid, threads, smem, s>>>(tile_off, rec_idx, rec_start, rec_w, F, C, g, mesh);

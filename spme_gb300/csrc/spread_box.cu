@@ -205,8 +205,7 @@ cudaError_t launch_box_t(const int *tile_off, const int *rec_idx, const uint32_t
     const size_t smem = (size_t)b.vol * sizeof(T);
     const int ntiles = g.ntx * g.nty * g.ntz;
     auto kern = k_spread_box<T, P>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     const size_t slot = (size_t)ntiles * b.vol;
     for (int c0 = 0; c0 < C; c0 += nslot) {

@@ -532,7 +532,8 @@ cudaError_t launch_zcfg(const CUtensorMap &map, const T *tab2, const T *tw, cons
     auto kern = k_zfft_influence<T, W, CT, MINB, MAXP>;
     const int K = zp.K, Kh = K / 2 + 1;
     const size_t smem = zsmem_bytes<T>(K, W);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the same for every K: allow_smem)
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kZSmemCap);
     if (e != cudaSuccess) return e;
     const int nchunk = (K * Kh + W - 1) / W;
     kern<<<nchunk, CT + 32, smem, s>>>(map, tab2, reinterpret_cast<const Cx<T> *>(tw), perm, zp,
