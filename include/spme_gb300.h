@@ -202,7 +202,9 @@ int spme_fma_peak(int precision, double *flops_per_s);
  *   vectors:   system k's R right-hand sides at element 3 R P_k, right-hand
  *              side r of particle i, Cartesian d at 3 R P_k + r 3 N_k + 3 i + d
  *              (compute_spme's layout with ld = 3 N_k, per system).
- * Each system needs K >= p + 15 (FP32) or K >= p + 7 (FP64), rc < L/2. */
+ * Each system needs K >= p + 15 (FP32) or K >= p + 7 (FP64), rc < L/2.  All systems
+ * together have less than 2^31 mesh points and 3 R sum(N_k) < 2^31 (FP64: with 3 R from 17
+ * on rounded up to rows of 32, from 33 on of 64 per 48), else SPME_ERR_UNSUPPORTED. */
 typedef struct spme_batch_system {
     int np;
     int dim;

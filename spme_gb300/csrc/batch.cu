@@ -1111,12 +1111,19 @@ int spme_batch_create(const spme_batch_system *systems, int count, int nrhs, int
     *out = nullptr;
     if (!systems || count < 1 || nrhs < 1 || nrhs > 1024) return SPME_ERR_INVALID;
     if (precision != SPME_FP32 && precision != SPME_FP64) return SPME_ERR_INVALID;
-    long long ntot = 0;
+    // packed sort keys (a key per mesh point, tile and real-space cell) and vectors are
+    // indexed with 32 bits, and so are the force rows of the FP64 column gather
+    long long ntot = 0, points = 0, cells = 0;
     for (int k = 0; k < count; k++) {
         BTRY(validate_sys(systems[k], precision));
+        const long long K = systems[k].dim, nc = real_cells(systems[k]);
         ntot += systems[k].np;
+        points += K * K * K;
+        cells += nc * nc * nc;
     }
-    if (ntot * 3LL * nrhs >= (1LL << 31)) return SPME_ERR_UNSUPPORTED;
+    const long long row = precision == SPME_FP64 ? spread_cols_row_width(3 * nrhs) : 3 * nrhs;
+    if (ntot * row >= (1LL << 31) || points >= (1LL << 31) || cells >= (1LL << 31))
+        return SPME_ERR_UNSUPPORTED;
     _spme_batch_t *b = new (std::nothrow) _spme_batch_t();
     if (!b) return SPME_ERR_NOMEM;
     cudaGetDevice(&b->device);
